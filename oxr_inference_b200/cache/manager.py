@@ -91,12 +91,16 @@ class CacheManager:
             for s in plan.states:
                 self.states.append(torch.zeros((max_requests + 1, *s.shape), dtype=s.dtype, device=device))
         self.kv_maps: list = [None] * len(self.k_pools)
+        self.long_maps: list = [None] * len(self.k_pools)
         if device is not None and torch.device(device).type == "cuda":
             from oxr_inference_b200 import ops
 
             # TMA maps serve the kernels of plain grouped-query attention: keys and values of one size, causal or windowed
             self.kv_maps = [ops.make_kv_maps(k, v, page_size) if (g.need.value_dim is None and g.need.chunk == 0) else None
                             for g, k, v in zip(plan.groups, self.k_pools, self.v_pools)]
+            # masked groups, and groups whose key rows are the values, use them for their long tiles
+            self.long_maps = [own or (ops.make_kv_maps(k, k if v is None else v, page_size) if g.need.v_dim in (0, g.need.head_dim) else None)
+                              for own, g, k, v in zip(self.kv_maps, plan.groups, self.k_pools, self.v_pools)]
 
     # ---- sizes
     @staticmethod
@@ -262,4 +266,4 @@ class CacheManager:
     def group_view(self, group: int, block_table: torch.Tensor, slots: torch.Tensor) -> GroupView:
         return GroupView(self.page_size, self.k_pools[group] if self.k_pools else None,
                          self.v_pools[group] if self.v_pools else None, block_table, slots,
-                         self.kv_maps[group] if self.k_pools else None)
+                         self.kv_maps[group] if self.k_pools else None, self.long_maps[group] if self.k_pools else None)

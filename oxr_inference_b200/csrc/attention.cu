@@ -1773,6 +1773,45 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
+// The bias by distance in shared memory: per head of the tile one column of the table in log2 units, entry i for the distance i - (TC_BN - 1), with
+// the first row's value before distance 0 (those keys are hidden) and the last row's for TC_BN - 1 distances behind the table. A row reads the
+// 128 entries of a block downwards from one place without a comparison per key. The pitch is 8 modulo 32 words: the 8 tokens x 4 heads of a
+// warp then read from 32 different banks.
+__host__ __device__ constexpr int bias_pitch(int rows) { return ((rows + 2 * (TC_BN - 1)) + 23) / 32 * 32 + 8; }
+constexpr size_t TC_SMEM_MAX = 227 * 1024;
+inline bool bias_fits(int rows, int heads) { return TC_SMEM + (size_t)heads * bias_pitch(rows) * sizeof(float) <= TC_SMEM_MAX; }
+
+// What a row of a block sees: all of it (`whole`), or the keys with index lo .. lo + span and those below `keep`.
+struct RowMask {
+    bool whole;
+    int lo, span, keep;
+};
+// first_kept: the block is one of kept first keys behind every row's window (only the keys below `keep_end` count).
+__device__ __forceinline__ RowMask row_mask(bool row_ok, int row_pos, int row_lo, int key0, bool first_kept, int keep_end) {
+    RowMask m;
+    m.whole = row_ok && key0 + TC_BN - 1 <= row_pos && ((!first_kept && key0 >= row_lo) || key0 + TC_BN <= keep_end);
+    m.lo = row_lo - key0;
+    m.span = row_pos - key0 - m.lo;
+    if (!row_ok || first_kept || m.span < 0) { m.lo = 1 << 30; m.span = 0; }
+    m.keep = row_ok ? min(keep_end, row_pos + 1) - key0 : 0;
+    return m;
+}
+
+// Rows of a stage that TMA brought in with their page piece but that no row of the tile may see (before `lo`, from `end` on) become zero: their
+// probability is zero, but a cache row may hold anything, and 0 * NaN is not 0. `dst`: the piece's rows of 128 bytes, the first is key `kp`.
+__device__ __forceinline__ void zero_hidden_rows(unsigned char* dst, int kp, int box_rows, int lo, int end) {
+    for (int r = 0; r < box_rows; ++r)
+        if (kp + r < lo || kp + r >= end) {
+            uint4* z = reinterpret_cast<uint4*>(dst + (size_t)r * 128);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) z[j] = make_uint4(0, 0, 0, 0);
+        }
+}
+
+// MASKED: the extras of AttnArgs (chunk, kept first keys, bias by distance, sink). The mma.sync kernel for 64-row
+// tiles took 230 us for 2,048 tokens of 32 / 8 heads of 128 with a window of 1,024 and 64 kept keys, this 64; with chunks of 1,024 and a bias of 513
+// distances it takes 50.
+template <bool MASKED>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_q, int q_by_tma,
@@ -1793,6 +1832,8 @@ attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
     uint64_t* o_done = p_full + 2;               // [half] O += P(b) V(b) has completed
     uint64_t* q_ready = o_done + 2;              // Q is in shared memory
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_ready + 1);
+    [[maybe_unused]] uint64_t* fix_bar = q_ready + 28;   // MASKED: a V block with rows to zero has arrived
+    [[maybe_unused]] float* bias_tab = reinterpret_cast<float*>(smem_dyn + TC_SMEM);
 #ifdef OXR_TIMELINE
     unsigned long long* tl = reinterpret_cast<unsigned long long*>(q_ready + 2);   // eight stamps in the spare bytes behind the barriers
     unsigned long long* tl2 = tl + 8;
@@ -1815,9 +1856,13 @@ attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int k_end = g.pos0 + g.tok_end;
-    const int k_lo = a.window > 0 ? max(0, g.pos0 + g.tok0 - a.window + 1) : 0;
-    const int k_first = (k_lo / TC_BN) * TC_BN;
-    const int count = (k_end - k_first + TC_BN - 1) / TC_BN;
+    const KeyWalk kw = key_walk(a, g.pos0 + g.tok0, TC_BN);
+    const int n_kept = MASKED ? kw.n_kept : 0;
+    const int k_lo = kw.k_lo, k_first = kw.k_first;
+    const int count = n_kept + (k_end - k_first + TC_BN - 1) / TC_BN;
+    auto block_key0 = [&](int b) { return MASKED ? kw.key0(b, TC_BN) : k_first + b * TC_BN; };
+    auto block_lo = [&](int b) { return MASKED ? kw.lo(b) : k_lo; };
+    auto block_end = [&](int b) { return MASKED ? kw.end(b, k_end) : k_end; };
     // A lane of the producer warp fetches one page piece of a block's K and of its V (a block has at most 16 pieces of 8 keys
     // and 2 panels): the pool row of this lane's piece of block b, or -1 if it is not fetched. The first block's pages are
     // looked up here, before the set-up, and every later block's while the block before it waits for its place in the rings.
@@ -1825,8 +1870,8 @@ attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
     const int pieces = (TC_BN / box_rows) * PANELS;
     const int my_box = lane / PANELS, my_pnl = lane % PANELS;
     auto lookup = [&](int b) -> int {
-        const int kp = k_first + b * TC_BN + my_box * box_rows;
-        if (lane < pieces && kp < k_end && kp + box_rows > k_lo) {
+        const int kp = block_key0(b) + my_box * box_rows;
+        if (lane < pieces && kp < block_end(b) && kp + box_rows > block_lo(b)) {
             const int page = table_row[a.page_shift >= 0 ? (kp >> a.page_shift) : (kp / a.page_size)];
             if (page >= 0 && page < a.num_pages)
                 return pool_row0 + page * a.page_size + (a.page_shift >= 0 ? (kp & (a.page_size - 1)) : (kp % a.page_size));
@@ -1840,11 +1885,23 @@ attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
         for (int i = 0; i < TC_STAGES; ++i) { mbar_init(k_full + i, 1); mbar_init(k_empty + i, 1); mbar_init(v_full + i, 1); mbar_init(v_empty + i, 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(s_full + i, 1); mbar_init(p_full + i, 4); mbar_init(o_done + i, 1); }
         mbar_init(q_ready, q_by_tma ? 1 : TC_THREADS / 32 - 2);
+        if constexpr (MASKED) mbar_init(fix_bar, 1);
         mbar_fence_init();
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(TC_TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if constexpr (MASKED) {
+        if (a.dist_bias != nullptr) {
+            const int pitch = bias_pitch(a.bias_rows), entries = a.bias_rows + 2 * (TC_BN - 1);
+            for (int i = threadIdx.x; i < entries * g.heads_per_tile; i += TC_THREADS) {
+                const int h = i % g.heads_per_tile, e = i / g.heads_per_tile;
+                const int gh = g.hg * g.heads_per_tile + h;
+                const int dist = min(max(e - (TC_BN - 1), 0), a.bias_rows - 1);
+                bias_tab[h * pitch + e] = gh < g.G ? __ldg(a.dist_bias + (size_t)dist * a.H + (size_t)g.kvh * g.G + gh) * LOG2E : 0.f;
+            }
+        }
     }
     // Nothing else stands before the first loads: the producer warp goes ahead while Q comes in (the MMA warp waits for
     // `q_ready` before its first product).
@@ -1891,12 +1948,36 @@ attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
         }
         // K(0), V(0), K(1), V(1), ...: each into its own ring
         int row = row_first;
+        // MASKED: V of block `fix_b` is on its way and waits for its hidden rows to be zeroed (the next block's K is asked for first)
+        [[maybe_unused]] int fix_b = -1, fix_row = -1;
+        [[maybe_unused]] uint32_t fix_phase = 0;
+        auto finish_fix = [&]() -> bool {
+            if (fix_b < 0) return true;
+            if (!mbar_wait(fix_bar, fix_phase)) { if (lane == 0) oxr_report(a.status, OXR_WAIT_EXPIRED, 38); return false; }
+            fix_phase ^= 1;
+            const int st = fix_b % TC_STAGES;
+            if (fix_row >= 0)
+                zero_hidden_rows(v_ring + (size_t)st * TC_HALF_STAGE + (size_t)my_pnl * TC_PANEL_BYTES + (size_t)my_box * box_rows * 128,
+                                 block_key0(fix_b) + my_box * box_rows, box_rows, block_lo(fix_b), block_end(fix_b));
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(v_full + st);
+            fix_b = -1;
+            return true;
+        };
         for (int b = 0; b < count; ++b) {
             const int row_next = b + 1 < count ? lookup(b + 1) : -1;
             const int st = b % TC_STAGES;
             const int total = __reduce_add_sync(0xffffffffu, row >= 0 ? box_rows * 128 : 0);
-            bool ok = true;
+            bool ok = true, partial = false;
+            if constexpr (MASKED) {
+                const int kp = block_key0(b) + my_box * box_rows;
+                partial = __any_sync(0xffffffffu, row >= 0 && (kp < block_lo(b) || kp + box_rows > block_end(b)));
+            }
             for (int is_v = 0; is_v < 2; ++is_v) {
+                if constexpr (MASKED) {
+                    if (is_v && !finish_fix()) { ok = false; break; }
+                }
                 uint64_t* full = (is_v ? v_full : k_full) + st;
                 if (!mbar_wait((is_v ? v_empty : k_empty) + st, ((b / TC_STAGES) & 1) ^ 1)) { if (lane == 0) oxr_report(a.status, OXR_WAIT_EXPIRED, 30); ok = false; break; }
                 unsigned char* dst = (is_v ? v_ring : k_ring) + (size_t)st * TC_HALF_STAGE;
@@ -1913,6 +1994,9 @@ attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
                     fence_proxy_async();
                     __syncwarp();
                 }
+                if constexpr (MASKED) {
+                    if (is_v && partial) { full = fix_bar; fix_b = b; fix_row = row; }
+                }
                 if (lane == 0) {
                     if (total > 0) mbar_expect_tx(full, (uint32_t)total);
                     else mbar_arrive(full);
@@ -1928,6 +2012,7 @@ attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
             if (!ok) break;
             row = row_next;
         }
+        if constexpr (MASKED) finish_fix();   // (after an expired wait: another bounded one at most)
     } else if (warp == 1) {
         // ---------------------------------------------------------------------- MMA issuer
         if (elect_one_lane()) {
@@ -2003,11 +2088,13 @@ attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
         int tok, gh;
         const bool row_ok = g.row(half * HALF_ROWS + rr, tok, gh);
         const int row_pos = g.pos0 + tok;
-        const float scale_log2 = a.scale * LOG2E;
+        const bool biased = MASKED && a.dist_bias != nullptr;
+        const float scale_log2 = biased ? 1.f : a.scale * LOG2E;   // a biased score is scaled before its bias is added
+        const int row_lo = key_lo(a, row_pos);
         float m_used = -INFINITY, l = 0.f;                   // the maximum P is taken against, the running sum
         bool alive = true;
         for (int b = 0; b < count; ++b) {
-            const int key0 = k_first + b * TC_BN;
+            const int key0 = block_key0(b);
             if (!mbar_wait(s_full + half, b & 1)) { if (lane == 0) oxr_report(a.status, OXR_WAIT_EXPIRED, 34); alive = false; break; }
 #ifdef OXR_TIMELINE
             if (b == 0 && warp == 2 && lane == 0) tl[3] = OXR_TL_NOW();
@@ -2024,18 +2111,29 @@ attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
             if (tl_me) tl2[9 + 4 * half] = OXR_TL_NOW();
 #endif
             // Blocks that this row sees in full need no per-key test; on the others the hidden keys become -inf.
-            const bool whole = row_ok && key0 + TC_BN - 1 <= row_pos && key0 >= k_lo && (a.window <= 0 || key0 > row_pos - a.window);
-            if (!whole) {
-                // the keys of this block that the row sees are those with index lo .. lo + span: one subtraction and one
-                // unsigned comparison per key
-                int lo = max(k_lo, a.window > 0 ? row_pos - a.window + 1 : 0) - key0;
-                int span = row_pos - key0 - lo;
-                if (!row_ok || span < 0) { lo = 1 << 30; span = 0; }
+            if constexpr (MASKED) {
+                if (biased) {
+                    const float* tab = bias_tab + (gh - g.hg * g.heads_per_tile) * bias_pitch(a.bias_rows) +
+                                       min(max(row_pos - key0, 0), a.bias_rows - 1 + TC_BN - 1) + TC_BN - 1;
+                    const float scale = a.scale * LOG2E;
+#pragma unroll
+                    for (int c = 0; c < TC_BN / 32; ++c)
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) sv[c][j] = __float_as_uint(fmaf(__uint_as_float(sv[c][j]), scale, tab[-(c * 32 + j)]));
+                }
+            }
+            // the keys of this block that the row sees are those with index lo .. lo + span: one subtraction and one
+            // unsigned comparison per key (and, MASKED, those below `keep`)
+            const RowMask rm = row_mask(row_ok, row_pos, row_lo, key0, MASKED && b < n_kept, MASKED ? (b < n_kept ? kw.kept_end : kw.keep) : 0);
+            if (!rm.whole) {
 #pragma unroll
                 for (int c = 0; c < TC_BN / 32; ++c)
 #pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if ((unsigned)(c * 32 + j - lo) > (unsigned)span) sv[c][j] = __float_as_uint(-INFINITY);
+                    for (int j = 0; j < 32; ++j) {
+                        bool hidden = (unsigned)(c * 32 + j - rm.lo) > (unsigned)rm.span;
+                        if constexpr (MASKED) hidden = hidden && c * 32 + j >= rm.keep;
+                        if (hidden) sv[c][j] = __float_as_uint(-INFINITY);
+                    }
             }
             // the row's maximum of the raw scores (four independent chains); the (positive) scale is applied once
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -2109,7 +2207,11 @@ attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
 #endif
         if (alive) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const float inv = l > 0.f ? 1.f / l : 0.f;
+            float keep = 1.f;
+            if constexpr (MASKED) {
+                if (a.sink != nullptr && row_ok) keep = add_sink(__ldg(a.sink + g.kvh * g.G + gh), m_used, l);
+            }
+            const float inv = l > 0.f ? keep / l : 0.f;
             // The row goes, as bf16, into the place of this half's Q (every product that read Q has completed), 16-byte pieces
             // swizzled by the row; then the warp writes its 32 rows out two at a time, 256 contiguous bytes each.
             unsigned char* oh = Qs + (size_t)half * PANELS * Q_PANEL_BYTES;
@@ -2164,6 +2266,313 @@ attn_tc5_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TC_TMEM_COLS) : "memory");
     }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Prefill attention for head sizes of 192 and 256 whose values ARE the keys (a compressed cache: one row per token is key and value of every
+// head), on tcgen05. Beside the kernel above two things differ:
+//  * O of 128 rows takes up to 256 of the 512 TMEM columns, so a tile is ONE half of 128 rows, and the tensor pipe is kept busy during the
+//    softmax by a second S instead of a second half: S(b + 1) is issued before O += P(b) V(b), into the other 128 columns;
+//  * a block of 128 keys is fetched ONCE and read by both products: K-major for S, MN-major for P V. Shared memory holds Q (64 KB at 256) and
+//    a ring of five slots of 32 KB, each two 64-wide panels of a block's 128 keys (a block is two slots): P V frees the slots one after the
+//    other, so that two and a half blocks are in flight where whole blocks would leave two.
+// The mma.sync kernel that took these before fetched every row twice, reloaded K and V for each 64-row tile and was bound by the legacy tensor
+// path: 2,048 tokens of 32 heads over rows of 256 took 375 us, and take 112 here; prompts of 402, 670 and 939 tokens 281 and 80.
+// Warps: 0 = TMA producer, 1 = MMA issuer and owner of the TMEM allocation, 2..5 = softmax and epilogue, one thread per row.
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr bool SHARED_OK = TMA_OK && D > 128;
+[[maybe_unused]] constexpr int SH_PAIRS = (PANELS + 1) / 2;                    // slots of a block
+constexpr int SH_SLOT = 2 * TC_PANEL_BYTES;
+constexpr int SH_SLOTS = 5;
+constexpr int SH_THREADS = 192;
+constexpr size_t SH_SMEM = (size_t)PANELS * Q_PANEL_BYTES + (size_t)SH_SLOTS * SH_SLOT + 512;
+
+__global__ void __launch_bounds__(SH_THREADS, 1)
+attn_tc5_shared_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, const __grid_constant__ CUtensorMap map_k,
+                       const __grid_constant__ CUtensorMap map_q, int q_by_tma, int pool_row0, int box_rows, int n_tiles, int n_y, const AttnArgs a) {
+#if HEAD_DIM > 128 && HEAD_DIM % 64 == 0
+    extern __shared__ __align__(1024) unsigned char smem_dyn[];
+    unsigned char* Qs = smem_dyn;                                           // PANELS panels of [128 rows][128 B], swizzled
+    unsigned char* ring = Qs + (size_t)PANELS * Q_PANEL_BYTES;               // SH_SLOTS x 2 panels of [128 keys][128 B]
+    uint64_t* full = reinterpret_cast<uint64_t*>(ring + (size_t)SH_SLOTS * SH_SLOT);
+    uint64_t* empty = full + SH_SLOTS;
+    uint64_t* fix_bar = empty + SH_SLOTS;        // [2] a slot with rows to zero has arrived (items take turns)
+    uint64_t* s_full = fix_bar + 2;              // [2] S(b) is in TMEM (b & 1)
+    uint64_t* p_full = s_full + 2;               // [2] P(b) is in TMEM and O is rescaled (4 arrivals)
+    uint64_t* o_done = p_full + 2;               // O += P(b) V(b) has completed
+    uint64_t* q_ready = o_done + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_ready + 1);
+    if (threadIdx.x == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
+        if (q_by_tma) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
+    }
+    const TileGeometry g = tile_geometry(a, HALF_ROWS, n_tiles - 1 - (int)(blockIdx.x / (unsigned)n_y), (int)(blockIdx.x % (unsigned)n_y));
+    if (g.tok0 >= g.tok_end) return;
+    if (smem_addr(smem_dyn) & 1023u) {   // cannot happen without static shared memory; refuse rather than compute rubbish
+        if (threadIdx.x == 0) oxr_report(a.status, OXR_BAD_ARGUMENT, 1024);
+        return;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k_end = g.pos0 + g.tok_end;
+    const KeyWalk kw = key_walk(a, g.pos0 + g.tok0, TC_BN);
+    const int count = kw.n_kept + (k_end - kw.k_first + TC_BN - 1) / TC_BN;
+    // a lane of the producer warp fetches one page piece of one panel: two lanes per piece (a block has at most 16 of 8 keys)
+    const int* table_row = a.block_table + (size_t)g.req * a.table_width;
+    const int boxes = TC_BN / box_rows, my_box = lane >> 1, my_pnl = lane & 1;
+    auto lookup = [&](int b) -> int {
+        const int kp = kw.key0(b, TC_BN) + my_box * box_rows;
+        if (my_box < boxes && kp < kw.end(b, k_end) && kp + box_rows > kw.lo(b)) {
+            const int page = table_row[kp >> a.page_shift];
+            if (page >= 0 && page < a.num_pages) return pool_row0 + page * a.page_size + (kp & (a.page_size - 1));
+            oxr_report(a.status, OXR_BAD_PAGE, g.req);
+        }
+        return -1;
+    };
+    const int row_first = warp == 0 ? lookup(0) : -1;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < SH_SLOTS; ++i) { mbar_init(full + i, 1); mbar_init(empty + i, 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(fix_bar + i, 1); mbar_init(s_full + i, 1); mbar_init(p_full + i, 4); }
+        mbar_init(o_done, 1);
+        mbar_init(q_ready, q_by_tma ? 1 : 4);
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(TC_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;   // S(b) | P(b) at 128 (b & 1), O at 256
+
+    if (warp == 0) {
+        // ---------------------------------------------------------------------- TMA producer (all 32 lanes issue)
+        if (q_by_tma && lane == 0) {
+            mbar_expect_tx(q_ready, (uint32_t)(PANELS * Q_PANEL_BYTES));
+            for (int pnl = 0; pnl < PANELS; ++pnl)
+                tma_load_3d(Qs + (size_t)pnl * Q_PANEL_BYTES, &map_q, pnl * 64, g.kvh * g.G, g.q_begin + g.tok0, q_ready);
+        }
+        int row = row_first, item = 0;
+        // an item whose hidden rows are zeroed once it has landed, after the next item has been asked for
+        int fix_item = -1, fix_row = -1, fix_b = 0, fixes_asked = 0, fixes_done = 0;
+        bool fix_lane = false;
+        auto finish_fix = [&](int it, int b, int r, bool mine) -> bool {
+            if (!mbar_wait(fix_bar + (fixes_done & 1), (fixes_done >> 1) & 1)) { if (lane == 0) oxr_report(a.status, OXR_WAIT_EXPIRED, 48); return false; }
+            ++fixes_done;
+            if (mine && r >= 0)
+                zero_hidden_rows(ring + (size_t)(it % SH_SLOTS) * SH_SLOT + (size_t)my_pnl * TC_PANEL_BYTES + (size_t)my_box * box_rows * 128,
+                                 kw.key0(b, TC_BN) + my_box * box_rows, box_rows, kw.lo(b), kw.end(b, k_end));
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full + it % SH_SLOTS);
+            return true;
+        };
+        bool ok = true;
+        for (int b = 0; b < count && ok; ++b) {
+            const int row_next = b + 1 < count ? lookup(b + 1) : -1;
+            const int kp = kw.key0(b, TC_BN) + my_box * box_rows;
+            const bool partial = __any_sync(0xffffffffu, row >= 0 && (kp < kw.lo(b) || kp + box_rows > kw.end(b, k_end)));
+            for (int pr = 0; pr < SH_PAIRS; ++pr, ++item) {
+                const int slot = item % SH_SLOTS;
+                const bool mine = my_box < boxes && 2 * pr + my_pnl < PANELS;   // the last slot of three panels holds one
+                unsigned char* dst = ring + (size_t)slot * SH_SLOT + (size_t)my_pnl * TC_PANEL_BYTES + (size_t)my_box * box_rows * 128;
+                if (!mbar_wait(empty + slot, ((item / SH_SLOTS) & 1) ^ 1)) { if (lane == 0) oxr_report(a.status, OXR_WAIT_EXPIRED, 40); ok = false; break; }
+                const int total = __reduce_add_sync(0xffffffffu, mine && row >= 0 ? box_rows * 128 : 0);
+                if (__any_sync(0xffffffffu, mine && row < 0)) {   // pieces that are not fetched must hold finite numbers
+                    if (mine && row < 0)
+                        for (int j = 0; j < box_rows * 8; ++j) reinterpret_cast<uint4*>(dst)[j] = make_uint4(0, 0, 0, 0);
+                    fence_proxy_async();
+                    __syncwarp();
+                }
+                const bool fix = partial && total > 0;
+                uint64_t* bar = fix ? fix_bar + (fixes_asked & 1) : full + slot;
+                if (lane == 0) {
+                    if (total > 0) mbar_expect_tx(bar, (uint32_t)total);
+                    else mbar_arrive(bar);
+                }
+                __syncwarp();
+                if (mine && row >= 0) tma_load_2d(dst, &map_k, g.kvh * D + (2 * pr + my_pnl) * 64, row, bar);
+                if (fix_item >= 0 && !finish_fix(fix_item, fix_b, fix_row, fix_lane)) { ok = false; break; }
+                fix_item = -1;
+                if (fix) { fix_item = item; fix_b = b; fix_row = row; fix_lane = mine; ++fixes_asked; }
+            }
+            row = row_next;
+        }
+        if (ok && fix_item >= 0) finish_fix(fix_item, fix_b, fix_row, fix_lane);
+    } else if (warp == 1) {
+        // ---------------------------------------------------------------------- MMA issuer
+        if (elect_one_lane()) {
+            constexpr uint32_t idesc_s = attn_idesc(HALF_ROWS, TC_BN, false);
+            const uint32_t q_addr = smem_addr(Qs), ring_addr = smem_addr(ring);
+            auto issue_s = [&](int b) -> bool {
+#pragma unroll
+                for (int pr = 0; pr < SH_PAIRS; ++pr) {
+                    const int item = b * SH_PAIRS + pr, slot = item % SH_SLOTS;
+                    if (!mbar_wait(full + slot, (item / SH_SLOTS) & 1)) { oxr_report(a.status, OXR_WAIT_EXPIRED, 41); return false; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                    for (int kk = 0; kk < (2 * pr + 2 <= PANELS ? 8 : 4); ++kk)
+                        tc_mma(tmem_base + (uint32_t)((b & 1) * TC_BN), desc_kmajor(q_addr + (2 * pr + (kk >> 2)) * Q_PANEL_BYTES + (kk & 3) * 32),
+                               desc_kmajor(ring_addr + slot * SH_SLOT + (kk >> 2) * TC_PANEL_BYTES + (kk & 3) * 32), idesc_s, (pr > 0 || kk > 0) ? 1u : 0u);
+                }
+                tc_commit(s_full + (b & 1));
+                return true;
+            };
+            bool ok = true;
+            if (!mbar_wait(q_ready, 0)) { oxr_report(a.status, OXR_WAIT_EXPIRED, 46); ok = false; }
+            ok = ok && issue_s(0);
+            for (int b = 0; b < count && ok; ++b) {
+                // S(b + 1) goes where P(b - 1) stood: the products that read it were issued before
+                if (b + 1 < count && !issue_s(b + 1)) { ok = false; break; }
+                if (!mbar_wait(p_full + (b & 1), (b >> 1) & 1)) { oxr_report(a.status, OXR_WAIT_EXPIRED, 43); ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int pr = 0; pr < SH_PAIRS; ++pr) {
+                    const int slot = (b * SH_PAIRS + pr) % SH_SLOTS;
+                    const uint32_t idesc_o = attn_idesc(HALF_ROWS, 2 * pr + 2 <= PANELS ? 128 : 64, true);
+#pragma unroll
+                    for (int kk = 0; kk < TC_BN / 16; ++kk)
+                        tc_mma_a_tmem(tmem_base + 256 + (uint32_t)(pr * 128), tmem_base + (uint32_t)((b & 1) * TC_BN + kk * 8),
+                                      desc_mnmajor(ring_addr + slot * SH_SLOT + kk * 16 * 128), idesc_o, (b > 0 || kk > 0) ? 1u : 0u);
+                    tc_commit(empty + slot);
+                }
+                tc_commit(o_done);
+            }
+        }
+    } else {
+        // ---------------------------------------------------------------------- softmax and epilogue: one thread per row
+        const int quarter = warp & 3;
+        const int rr = quarter * 32 + lane;
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        const uint32_t tmem_o = tmem_base + lane_base + 256;
+        int tok, gh;
+        const bool row_ok = g.row(rr, tok, gh);
+        if (!q_by_tma) {   // every thread copies its own row of Q; rows without a (token, head) are zero
+            const uint4* src = reinterpret_cast<const uint4*>(q + ((size_t)(g.q_begin + (row_ok ? tok : 0)) * a.H + (size_t)g.kvh * g.G + (row_ok ? gh : 0)) * D);
+#pragma unroll 8
+            for (int c = 0; c < D / 8; ++c)
+                *reinterpret_cast<uint4*>(Qs + (size_t)(c >> 3) * Q_PANEL_BYTES + (size_t)rr * 128 + (((c & 7) ^ (rr & 7)) << 4)) =
+                    row_ok ? __ldg(src + c) : make_uint4(0, 0, 0, 0);
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(q_ready);
+        }
+        const int row_pos = g.pos0 + tok;
+        const int row_lo = key_lo(a, row_pos);
+        const float scale_log2 = a.scale * LOG2E;
+        float m_used = -INFINITY, l = 0.f;
+        bool alive = true;
+        for (int b = 0; b < count; ++b) {
+            const int key0 = kw.key0(b, TC_BN);
+            const uint32_t tmem_s = tmem_base + lane_base + (uint32_t)((b & 1) * TC_BN);
+            if (!mbar_wait(s_full + (b & 1), (b >> 1) & 1)) { if (lane == 0) oxr_report(a.status, OXR_WAIT_EXPIRED, 44); alive = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint32_t sv[TC_BN / 32][32];
+#pragma unroll
+            for (int c = 0; c < TC_BN / 32; ++c) tc_ld32_nowait(tmem_s + (uint32_t)(c * 32), sv[c]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            const RowMask rm = row_mask(row_ok, row_pos, row_lo, key0, b < kw.n_kept, b < kw.n_kept ? kw.kept_end : kw.keep);
+            if (!rm.whole) {
+#pragma unroll
+                for (int c = 0; c < TC_BN / 32; ++c)
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        if ((unsigned)(c * 32 + j - rm.lo) > (unsigned)rm.span && c * 32 + j >= rm.keep) sv[c][j] = __float_as_uint(-INFINITY);
+            }
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int c = 0; c < TC_BN / 32; ++c)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) mx4[j & 3] = max3(mx4[j & 3], __uint_as_float(sv[c][2 * j]), __uint_as_float(sv[c][2 * j + 1]));
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
+            float alpha = 1.f;
+            const bool raise = mx > m_used + RESCALE_THRESHOLD || (m_used == -INFINITY && mx != -INFINITY);
+            if (raise) {
+                alpha = (m_used == -INFINITY) ? 0.f : fast_exp2(m_used - mx);
+                m_used = mx;
+            }
+            if (__any_sync(0xffffffffu, raise && b > 0)) {
+                // S(b) was issued before O += P(b - 1) V(b - 1): that product must be complete before O changes
+                if (!mbar_wait(o_done, (b - 1) & 1)) { if (lane == 0) oxr_report(a.status, OXR_WAIT_EXPIRED, 45); alive = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+                for (int c = 0; c < D / 32; ++c) {
+                    uint32_t ov[32];
+                    tc_ld32(tmem_o + (uint32_t)(c * 32), ov);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * alpha);
+                    tc_st32(tmem_o + (uint32_t)(c * 32), ov);
+                }
+            }
+            const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
+            const uint64_t scale2 = pair_of(scale_log2, scale_log2), neg_m2 = pair_of(neg_m, neg_m);
+            uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+            for (int c = 0; c < TC_BN / 32; ++c) {
+                uint32_t pv[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    float x0, x1;
+                    unpair(fma2(pair_of(__uint_as_float(sv[c][2 * e]), __uint_as_float(sv[c][2 * e + 1])), scale2, neg_m2), x0, x1);
+                    const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+                    sum2[e & 3] = add2(sum2[e & 3], pair_of(p0, p1));
+                    const __nv_bfloat162 pk = __floats2bfloat162_rn(p0, p1);
+                    pv[e] = *reinterpret_cast<const uint32_t*>(&pk);
+                }
+                tc_st16(tmem_s + (uint32_t)(c * 16), pv);
+            }
+            float sum4[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { float lo, hi; unpair(sum2[i], lo, hi); sum4[i] = lo + hi; }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            l = l * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_full + (b & 1));
+        }
+        // S(count - 1) was complete when O += P(count - 2) V(count - 2) may not have been: both phases are waited for, in order (of the last one alone a
+        // parity could not be told from that of the phase two before it)
+        if (alive && ((count > 1 && !mbar_wait(o_done, (count - 2) & 1)) || !mbar_wait(o_done, (count - 1) & 1))) { if (lane == 0) oxr_report(a.status, OXR_WAIT_EXPIRED, 47); alive = false; }
+        alive = __all_sync(0xffffffffu, alive);
+        if (alive) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            float keep = 1.f;
+            if (a.sink != nullptr && row_ok) keep = add_sink(__ldg(a.sink + g.kvh * g.G + gh), m_used, l);
+            const float inv = l > 0.f ? keep / l : 0.f;
+            // as above: the row goes, as bf16, into Q's place, then the warp writes its 32 rows out one after the other
+#pragma unroll 1
+            for (int c = 0; c < D / 32; ++c) {
+                uint32_t ov[32];
+                tc_ld32(tmem_o + (uint32_t)(c * 32), ov);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint4 o4;
+                    __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o4);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        op[e] = __floats2bfloat162_rn(__uint_as_float(ov[8 * j + 2 * e]) * inv, __uint_as_float(ov[8 * j + 2 * e + 1]) * inv);
+                    *reinterpret_cast<uint4*>(Qs + (size_t)rr * (D * 2) + (((c * 4 + j) ^ (rr & 7)) << 4)) = o4;
+                }
+            }
+            __syncwarp();
+            const unsigned long long my_dst = row_ok ? (unsigned long long)(out + ((size_t)(g.q_begin + tok) * a.H + (size_t)g.kvh * g.G + gh) * D) : 0ull;
+#pragma unroll 4
+            for (int it = 0; it < 32; ++it) {
+                const unsigned long long dst2 = __shfl_sync(0xffffffffu, my_dst, it);
+                if (dst2 != 0ull && lane < D / 8)
+                    reinterpret_cast<uint4*>(dst2)[lane] =
+                        *reinterpret_cast<const uint4*>(Qs + (size_t)(quarter * 32 + it) * (D * 2) + ((lane ^ (it & 7)) << 4));
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TC_TMEM_COLS) : "memory");
+    }
+#endif
 }
 }  // namespace
 
@@ -2241,13 +2650,14 @@ static int launch_tma_decode(void* out, const void* q, int n_short, int groups_y
     return oxr_launch_status();
 }
 // Rows of a tile for each kind of tile list that the host builds: 0 generic, 1 decode, 2 prefill (mma.sync), 3 prefill
-// (tcgen05). The host keeps the same numbers and compares them when it loads the library.
+// (tcgen05), 4 prefill over rows that are key and value at once (tcgen05, head sizes 192 and 256). The host keeps the same numbers and compares them when it loads the library.
 OXR_API int oxr_attn_tile_rows(int kind) {
     switch (kind) {
         case 0: return BM;
         case 1: return DECODE_ROWS;
         case 2: return PREFILL_ROWS;
         case 3: return BIG_ROWS;
+        case 4: return HALF_ROWS;
         default: return -1;
     }
 }
@@ -2278,7 +2688,7 @@ static int paged_attention_bf16(void* out, const void* q, const void* k_cache, c
                                 const int* block_table, int table_width, int page_size, int num_pages, int H, int KV,
                                 float scale, int window, int splits, float* part_o, float* part_ml, int* counters,
                                 const void* kv_maps, int pool_row0, int long_rows, int q_tokens, int cut, int* status, cudaStream_t stream,
-                                const MaskExtras& extras);
+                                const MaskExtras& extras, const void* long_maps = nullptr);
 
 OXR_API int oxr_paged_attention_bf16(void* out, const void* q, const void* k_cache, const void* v_cache,
                                      const int* short_req, const int* short_tok0, int n_short, const int* long_req,
@@ -2291,22 +2701,28 @@ OXR_API int oxr_paged_attention_bf16(void* out, const void* q, const void* k_cac
                                 long_rows, q_tokens, cut, status, stream, MaskExtras{});
 }
 
-// The same attention with the extras of AttnArgs: a chunk mask, first keys kept in sight behind a window, a bias by distance and a sink (see there). These run on the
-// cp.async tensor-core kernels only: no kv_maps, long tiles of 64 rows, cut 0.
+// Whether the tcgen05 kernel for long tiles of 256 rows has room for a bias table of `rows` distances for `heads` heads of a tile.
+OXR_API int oxr_attn_bias_fits(int rows, int heads) { return D <= 128 && rows > 0 && heads > 0 && bias_fits(rows, heads) ? 1 : 0; }
+
+// The same attention with the extras of AttnArgs: a chunk mask, first keys kept in sight behind a window, a bias by distance and a sink (see there). Short
+// tiles run on the cp.async tensor-core kernel. Long tiles: of 64 rows on the cp.async kernel; with `long_maps` (the two tensor maps of
+// oxr_attn_make_kv_maps, the same map twice where the values are the keys; pool_row0 as above) of 256 rows on the tcgen05 kernel (head sizes 64 and
+// 128, a bias that oxr_attn_bias_fits) or of 128 rows on the tcgen05 kernel for rows that are key and value at once (head sizes 192 and 256,
+// v_cache == k_cache, no bias).
 OXR_API int oxr_paged_attention_masked_bf16(void* out, const void* q, const void* k_cache, const void* v_cache,
                                             const int* short_req, const int* short_tok0, int n_short, const int* long_req,
                                             const int* long_tok0, int n_long, const int* cu_q, const int* ctx_lens,
                                             const int* block_table, int table_width, int page_size, int num_pages, int H, int KV,
                                             float scale, int window, int chunk, int keep_first, const float* dist_bias, int bias_rows,
-                                            const float* sink, int splits, float* part_o, float* part_ml, int* counters, int* status,
-                                            cudaStream_t stream) {
+                                            const float* sink, int splits, float* part_o, float* part_ml, int* counters, const void* long_maps,
+                                            int pool_row0, int long_rows, int q_tokens, int* status, cudaStream_t stream) {
     if (chunk < 0 || keep_first < 0 || (dist_bias != nullptr && bias_rows <= 0)) return OXR_BAD_ARGUMENT;
     MaskExtras extras;
     extras.chunk = chunk; extras.dist_bias = dist_bias; extras.bias_rows = bias_rows; extras.sink = sink;
     extras.keep_first = window > 0 ? keep_first : 0;
     return paged_attention_bf16(out, q, k_cache, v_cache, short_req, short_tok0, n_short, long_req, long_tok0, n_long, cu_q, ctx_lens, block_table,
-                                table_width, page_size, num_pages, H, KV, scale, window, splits, part_o, part_ml, counters, nullptr, 0,
-                                PREFILL_ROWS, 0, 0, status, stream, extras);
+                                table_width, page_size, num_pages, H, KV, scale, window, splits, part_o, part_ml, counters, nullptr, pool_row0,
+                                long_rows, q_tokens, 0, status, stream, extras, long_maps);
 }
 
 static int paged_attention_bf16(void* out, const void* q, const void* k_cache, const void* v_cache,
@@ -2315,10 +2731,13 @@ static int paged_attention_bf16(void* out, const void* q, const void* k_cache, c
                                 const int* block_table, int table_width, int page_size, int num_pages, int H, int KV,
                                 float scale, int window, int splits, float* part_o, float* part_ml, int* counters,
                                 const void* kv_maps, int pool_row0, int long_rows, int q_tokens, int cut, int* status, cudaStream_t stream,
-                                const MaskExtras& extras) {
+                                const MaskExtras& extras, const void* long_maps) {
     if (n_short <= 0 && n_long <= 0) return 0;
     const bool masked = extras.chunk > 0 || extras.dist_bias != nullptr || extras.sink != nullptr || extras.keep_first > 0;
-    if (masked && (kv_maps != nullptr || cut != 0 || (n_long > 0 && long_rows != PREFILL_ROWS))) return OXR_BAD_ARGUMENT;
+    if (masked && (kv_maps != nullptr || cut != 0 || (n_long > 0 && long_rows != PREFILL_ROWS && long_maps == nullptr))) return OXR_BAD_ARGUMENT;
+    // calls that the cp.async kernel took before keep its care for cache rows that no query sees (they may hold NaN)
+    const bool careful = long_maps != nullptr;
+    if (long_maps == nullptr) long_maps = kv_maps;
     if (H <= 0 || KV <= 0 || H % KV != 0 || page_size <= 0 || table_width <= 0 || window < 0 || splits < 1) return OXR_BAD_ARGUMENT;
     if ((splits > 1 || cut != 0) && n_short > 0 && (part_o == nullptr || part_ml == nullptr || counters == nullptr)) return OXR_BAD_ARGUMENT;
     static bool configured = false;
@@ -2340,10 +2759,13 @@ static int paged_attention_bf16(void* out, const void* q, const void* k_cache, c
     a.chunk = extras.chunk; a.dist_bias = extras.dist_bias; a.bias_rows = extras.bias_rows; a.sink = extras.sink; a.keep_first = extras.keep_first;
     if (n_long > 0 && long_rows == BIG_ROWS) {
         // long tiles of 256 rows: the tcgen05 kernel (the host made the tile list for 256 rows)
-        if (!TMA_OK || D > 128 || kv_maps == nullptr || a.page_shift < 3 || !(scale > 0.f)) return OXR_BAD_ARGUMENT;
+        if (!TMA_OK || D > 128 || long_maps == nullptr || a.page_shift < 3 || !(scale > 0.f)) return OXR_BAD_ARGUMENT;
+        if (a.dist_bias != nullptr && !bias_fits(a.bias_rows, G < BIG_ROWS ? G : BIG_ROWS)) return OXR_BAD_ARGUMENT;
         static bool big_configured = false;
         if (!big_configured) {
-            cudaError_t e = cudaFuncSetAttribute(attn_tc5_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
+            cudaError_t e = cudaFuncSetAttribute(attn_tc5_prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(attn_tc5_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_MAX);
             if (e != cudaSuccess) return 1000 + (int)e;
             big_configured = true;
         }
@@ -2351,14 +2773,41 @@ static int paged_attention_bf16(void* out, const void* q, const void* k_cache, c
         const int groups = (G + hpt - 1) / hpt;
         if ((size_t)KV * groups * (size_t)n_long > 0x7fffffffull) return OXR_BAD_ARGUMENT;
         a.tile_req = long_req; a.tile_tok0 = long_tok0;
-        const CUtensorMap* maps = reinterpret_cast<const CUtensorMap*>(kv_maps);
+        const CUtensorMap* maps = reinterpret_cast<const CUtensorMap*>(long_maps);
         const int box_rows = page_size < MMA_BN ? page_size : MMA_BN;
         // Q by TMA when a half's 128 rows are whole tokens (a [tokens, H, D] map made for this call: q moves from call to call)
         CUtensorMap map_q = maps[0];
         const int q_by_tma = (q_tokens > 0 && HALF_ROWS % G == 0 &&
                               oxr_make_map_bf16_3d(&map_q, q, (unsigned long long)q_tokens, (unsigned long long)H, D, HALF_ROWS / G, G)) ? 1 : 0;
-        attn_tc5_prefill_kernel<<<dim3((unsigned)(n_long * KV * groups)), TC_THREADS, TC_SMEM, stream>>>(
-            (bf16*)out, (const bf16*)q, maps[0], maps[1], map_q, q_by_tma, pool_row0, box_rows, n_long, KV * groups, a);
+        const size_t smem = TC_SMEM + (a.dist_bias != nullptr ? (size_t)hpt * bias_pitch(a.bias_rows) * sizeof(float) : 0);
+        if (careful)
+            attn_tc5_prefill_kernel<true><<<dim3((unsigned)(n_long * KV * groups)), TC_THREADS, smem, stream>>>(
+                (bf16*)out, (const bf16*)q, maps[0], maps[1], map_q, q_by_tma, pool_row0, box_rows, n_long, KV * groups, a);
+        else
+            attn_tc5_prefill_kernel<false><<<dim3((unsigned)(n_long * KV * groups)), TC_THREADS, smem, stream>>>(
+                (bf16*)out, (const bf16*)q, maps[0], maps[1], map_q, q_by_tma, pool_row0, box_rows, n_long, KV * groups, a);
+        int rc = oxr_launch_status();
+        if (rc) return rc;
+    } else if (n_long > 0 && long_rows == HALF_ROWS) {
+        // long tiles of 128 rows: the tcgen05 kernel for rows that are key and value at once
+        if (!SHARED_OK || long_maps == nullptr || k_cache != v_cache || a.dist_bias != nullptr || a.page_shift < 3 || !(scale > 0.f)) return OXR_BAD_ARGUMENT;
+        static bool shared_configured = false;
+        if (!shared_configured) {
+            cudaError_t e = cudaFuncSetAttribute(attn_tc5_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH_SMEM);
+            if (e != cudaSuccess) return 1000 + (int)e;
+            shared_configured = true;
+        }
+        const int hpt = G < HALF_ROWS ? G : HALF_ROWS;
+        const int groups = (G + hpt - 1) / hpt;
+        if ((size_t)KV * groups * (size_t)n_long > 0x7fffffffull) return OXR_BAD_ARGUMENT;
+        a.tile_req = long_req; a.tile_tok0 = long_tok0;
+        const CUtensorMap* maps = reinterpret_cast<const CUtensorMap*>(long_maps);
+        const int box_rows = page_size < MMA_BN ? page_size : MMA_BN;
+        CUtensorMap map_q = maps[0];
+        const int q_by_tma = (q_tokens > 0 && HALF_ROWS % G == 0 &&
+                              oxr_make_map_bf16_3d(&map_q, q, (unsigned long long)q_tokens, (unsigned long long)H, D, HALF_ROWS / G, G)) ? 1 : 0;
+        attn_tc5_shared_kernel<<<dim3((unsigned)(n_long * KV * groups)), SH_THREADS, SH_SMEM, stream>>>(
+            (bf16*)out, (const bf16*)q, maps[0], map_q, q_by_tma, pool_row0, box_rows, n_long, KV * groups, a);
         int rc = oxr_launch_status();
         if (rc) return rc;
     } else if (n_long > 0) {

@@ -224,8 +224,10 @@ def _attn_lib(head_dim: int):
         lib.oxr_paged_attention.argtypes = [p, p, p, p, p, p, i, p, p, p, i, i, i, i, i, f, i, i, p, p]
         lib.oxr_paged_attention.restype = c_int
         lib.oxr_paged_attention_bf16.argtypes = [p, p, p, p, p, p, i, p, p, i, p, p, p, i, i, i, i, i, f, i, i, p, p, p, p, i, i, i, i, p, p]
-        lib.oxr_paged_attention_masked_bf16.argtypes = [p, p, p, p, p, p, i, p, p, i, p, p, p, i, i, i, i, i, f, i, i, i, p, i, p, i, p, p, p, p, p]
+        lib.oxr_paged_attention_masked_bf16.argtypes = [p, p, p, p, p, p, i, p, p, i, p, p, p, i, i, i, i, i, f, i, i, i, p, i, p, i, p, p, p, p, i, i, i, p, p]
         lib.oxr_paged_attention_masked_bf16.restype = c_int
+        lib.oxr_attn_bias_fits.argtypes = [i, i]
+        lib.oxr_attn_bias_fits.restype = c_int
         lib.oxr_attn_make_kv_maps.argtypes = [p, p, p, ctypes.c_ulonglong, i, i]
         lib.oxr_attn_make_kv_maps.restype = c_int
         lib.oxr_paged_attention_fused_decode_bf16.argtypes = [p, p, p, p, p, p, i, p, p, p, i, i, i, i, i, f, i, i, p, p, p, p, i, i, p, p, p, p, f, i, i,
@@ -242,10 +244,10 @@ def _attn_lib(head_dim: int):
         lib.oxr_attn_last_short_kernel.restype = c_int
         if lib.oxr_attn_head_dim() != head_dim:
             raise BuildError(f"attention library for head size {head_dim} reports {lib.oxr_attn_head_dim()}")
-        rows = tuple(lib.oxr_attn_tile_rows(kind) for kind in range(4))
-        if rows != (GENERIC_ROWS, DECODE_ROWS, PREFILL_ROWS, PREFILL_ROWS_TMA):
+        rows = tuple(lib.oxr_attn_tile_rows(kind) for kind in range(5))
+        if rows != (GENERIC_ROWS, DECODE_ROWS, PREFILL_ROWS, PREFILL_ROWS_TMA, PREFILL_ROWS_SHARED):
             raise BuildError(f"attention library tiles have {rows} rows; the host builds its tile lists for "
-                             f"{(GENERIC_ROWS, DECODE_ROWS, PREFILL_ROWS, PREFILL_ROWS_TMA)}")
+                             f"{(GENERIC_ROWS, DECODE_ROWS, PREFILL_ROWS, PREFILL_ROWS_TMA, PREFILL_ROWS_SHARED)}")
         lib.oxr_set_chain.argtypes = [c_int]
         lib.oxr_set_chain.restype = None
         lib.oxr_set_chain(int(CHAIN_KERNELS))
@@ -458,7 +460,7 @@ def qk_norm_rope_store(qkv: torch.Tensor, q_weight: torch.Tensor | None, k_weigh
     return q
 
 
-GENERIC_ROWS, DECODE_ROWS, PREFILL_ROWS, PREFILL_ROWS_TMA = 16, 16, 64, 256
+GENERIC_ROWS, DECODE_ROWS, PREFILL_ROWS, PREFILL_ROWS_TMA, PREFILL_ROWS_SHARED = 16, 16, 64, 256, 128
 SHORT_MAX_TOKENS = 8
 """Requests that bring at most this many tokens go to the split-KV kernel, longer portions to the prefill kernel."""
 MAX_SPLITS = 32
@@ -484,6 +486,34 @@ def tma_gathers_possible(head_dim: int, page_size: int, dtype: torch.dtype) -> b
 
 def _long_rows(head_dim: int, tma: bool) -> int:
     return PREFILL_ROWS_TMA if tma and head_dim <= 128 else PREFILL_ROWS
+
+
+LONG_MASK_BYTES = 35328
+"""Shared memory that the tcgen05 kernel for tiles of 256 rows leaves for a bias-by-distance table (head size 128)."""
+
+
+def masked_long_rows(num_heads: int, num_kv_heads: int, head_dim: int, dtype: torch.dtype, page_size: int, *, shared: bool = False,
+                     bias_rows: int = 0, scale: float = 1.0) -> int:
+    """Rows of a long tile for attention under the masks and extras of :func:`paged_attention`, or with keys that are the values (``shared``):
+    256 for the tcgen05 kernel at head sizes 64 and 128 (a bias table has to fit beside its operands: two bytes short of 35 KB for the heads of one
+    KV head), 128 for the tcgen05 kernel over shared rows at 192 and 256, else 64 for the mma.sync kernel, which takes everything (a scale
+    that is not positive too: the tcgen05 kernels scale a row's maximum, not its scores)."""
+    if not tma_gathers_possible(head_dim, page_size, dtype) or not scale > 0:
+        return PREFILL_ROWS
+    if head_dim <= 128:
+        pitch = (bias_rows + 2 * 127 + 23) // 32 * 32 + 8 if bias_rows else 0
+        return PREFILL_ROWS_TMA if 4 * min(num_heads // num_kv_heads, PREFILL_ROWS_TMA) * pitch <= LONG_MASK_BYTES else PREFILL_ROWS
+    return PREFILL_ROWS_SHARED if shared and not bias_rows else PREFILL_ROWS
+
+
+def masked_tile_specs(num_heads: int, num_kv_heads: int, head_dim: int, dtype: torch.dtype, page_size: int, *, shared: bool = False,
+                      bias_rows: int = 0, scale: float = 1.0) -> list[tuple[int, int, int]]:
+    """:func:`attention_tile_specs` for a mixer that hands ``paged_attention`` its group's ``long_maps``."""
+    short, *rest = attention_tile_specs(num_heads, num_kv_heads, head_dim, dtype)
+    if not rest:
+        return [short]
+    rows = masked_long_rows(num_heads, num_kv_heads, head_dim, dtype, page_size, shared=shared, bias_rows=bias_rows, scale=scale)
+    return [short, (_tokens_per_tile(num_heads, num_kv_heads, rows), *rest[0][1:])]
 
 
 def attention_tile_specs(num_heads: int, num_kv_heads: int, head_dim: int, dtype: torch.dtype,
@@ -544,7 +574,7 @@ class KVMaps:
 
 def make_kv_maps(k_pool: torch.Tensor, v_pool: torch.Tensor, page_size: int) -> KVMaps | None:
     """Tensor maps over a group's whole pool ``[layers, pages, page_size, KV, D]`` so that the split-KV kernel can
-    fetch K and V by TMA; None when the sizes do not allow it (the kernel then gathers with cp.async)."""
+    fetch K and V by TMA; None when the sizes do not allow it (the kernel then gathers with cp.async). ``v_pool`` may be ``k_pool`` itself."""
     if k_pool.dtype != torch.bfloat16 or not k_pool.is_cuda:
         return None
     layers, pages, page, kv, d = k_pool.shape
@@ -568,7 +598,7 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
                     ctx_lens: torch.Tensor, block_table: torch.Tensor, page_size: int, scale: float, window: int,
                     kv_len_bound: int, status: torch.Tensor, generic: bool = False, kv_maps: KVMaps | None = None,
                     layer_in_pool: int = 0, uneven: bool = False, chunk: int = 0, dist_bias: torch.Tensor | None = None,
-                    sink: torch.Tensor | None = None, keep_first: int = 0) -> torch.Tensor:
+                    sink: torch.Tensor | None = None, keep_first: int = 0, long_maps: KVMaps | None = None) -> torch.Tensor:
     """Causal grouped-query attention of the step's new tokens over the paged cache
     (oxr_runtime/attention.py:47-109). ``q`` is ``[tokens, H, D]``; ``k_cache`` / ``v_cache`` are one layer's pool
     ``[pages, page_size, KV, D]``; ``window`` > 0 limits a query to its last ``window`` keys; ``tiles`` maps each
@@ -582,7 +612,9 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     ``j // chunk == p // chunk``; ``dist_bias [rows, H]`` (fp32) is added to the scaled score by distance p - j (the last row for all
     larger ones); ``sink [H]`` (fp32) adds ``exp(sink)`` to the softmax denominator; with a window, ``keep_first`` > 0 keeps the request's
     first ``keep_first`` keys visible to every later query. ``v_cache`` may be ``k_cache`` itself (a latent
-    cache whose rows are key and value at once)."""
+    cache whose rows are key and value at once). ``long_maps`` (the pool's tensor maps; not beside ``kv_maps``): the tiles are those of
+    :func:`masked_tile_specs`, and long ones run on the tcgen05 kernels where that function says so (2,048 tokens on a B200: 64 against 230 us at
+    head size 128, 112 against 375 us over shared rows of 256)."""
     _need(q, "q")
     _need(k_cache, "k_cache", q.dtype)
     _need(v_cache, "v_cache", q.dtype)
@@ -607,8 +639,16 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
                                        tile_tok0.data_ptr(), n, *common, _dtype_code(q), status.data_ptr(), _stream())
         _done(code, "paged_attention")
         return out
-    long_rows = _long_rows(head_dim, kv_maps is not None)
-    short, long_ = attention_tile_specs(num_heads, num_kv_heads, head_dim, torch.bfloat16, page_size if kv_maps is not None else None)
+    if long_maps is not None:
+        if kv_maps is not None:
+            raise KernelError("paged_attention: long_maps are for calls without kv_maps")
+        how = dict(shared=v_cache is k_cache or v_cache.data_ptr() == k_cache.data_ptr(), bias_rows=dist_bias.shape[0] if dist_bias is not None else 0,
+                   scale=scale)
+        long_rows = masked_long_rows(num_heads, num_kv_heads, head_dim, torch.bfloat16, page_size, **how)
+        short, long_ = masked_tile_specs(num_heads, num_kv_heads, head_dim, torch.bfloat16, page_size, **how)
+    else:
+        long_rows = _long_rows(head_dim, kv_maps is not None)
+        short, long_ = attention_tile_specs(num_heads, num_kv_heads, head_dim, torch.bfloat16, page_size if kv_maps is not None else None)
     if long_ not in tiles:
         raise KernelError(f"no tile list for long tiles of {long_rows} rows: the batch was cut for {sorted(tiles)}")
     s_req, s_tok, n_short = tiles[short]
@@ -617,7 +657,7 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     seen = min(kv_len_bound, window + keep_first + SHORT_MAX_TOKENS) if masked and window > 0 else kv_len_bound
     splits, cut, part_o, part_ml, counters = _split_kv_plan(lib, n_short, num_heads, num_kv_heads, head_dim, seen, kv_maps is not None,
                                                             uneven, q.device)
-    if masked:
+    if masked or long_maps is not None:
         for t, nm in ((dist_bias, "dist_bias"), (sink, "sink")):
             if t is not None:
                 _need(t, nm, torch.float32)
@@ -628,7 +668,9 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
         code = lib.oxr_paged_attention_masked_bf16(out.data_ptr(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), s_req.data_ptr(),
                                                    s_tok.data_ptr(), n_short, l_req.data_ptr(), l_tok.data_ptr(), n_long, *common, int(chunk), keep_first,
                                                    _ptr(dist_bias), dist_bias.shape[0] if dist_bias is not None else 0, _ptr(sink), splits,
-                                                   _ptr(part_o), _ptr(part_ml), _ptr(counters), status.data_ptr(), _stream())
+                                                   _ptr(part_o), _ptr(part_ml), _ptr(counters), long_maps.address if long_maps is not None else None,
+                                                   layer_in_pool * long_maps.rows_per_layer if long_maps is not None else 0, long_rows, q.shape[0],
+                                                   status.data_ptr(), _stream())
         global launch_count
         _done(code, "paged_attention_masked_bf16")
         launch_count += 1 if n_long and n_short else 0

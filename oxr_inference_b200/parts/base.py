@@ -116,6 +116,8 @@ class GroupView:
     """int32 [tokens]: where each new token's K and V go (page * page_size + offset)."""
     kv_maps: object | None = None
     """TMA tensor maps over the pools (``ops.make_kv_maps``), when the sizes allow them."""
+    long_maps: object | None = None
+    """The same for mixers whose masks, or whose keys that are the values, keep them off ``kv_maps`` (``ops.masked_tile_specs``)."""
 
 
 @dataclass

@@ -148,7 +148,9 @@ class GatedAttention(Mixer):
     def tile_specs(self) -> list[tuple[int, int, int]]:
         if not self.tiled:
             return []
-        return ops.attention_tile_specs(self.H, self.KV, self.DK, self.runtime.dtype, self.runtime.page_size if self.plain else None)
+        if self.plain:
+            return ops.attention_tile_specs(self.H, self.KV, self.DK, self.runtime.dtype, self.runtime.page_size)
+        return ops.masked_tile_specs(self.H, self.KV, self.DK, self.runtime.dtype, self.runtime.page_size, scale=self.scale)
 
     # ---- the step
     def forward(self, h: torch.Tensor, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
@@ -178,7 +180,8 @@ class GatedAttention(Mixer):
             else:
                 o = ops.paged_attention(q3, k_pool, v_pool, tiles=ctx.tiles, cu_q=ctx.cu_q, ctx_lens=ctx.ctx_lens, block_table=group.block_table,
                                         page_size=group.page_size, scale=self.scale, window=self.window, keep_first=self.keep_first,
-                                        kv_len_bound=ctx.kv_len_bound, status=ctx.status, sink=sink)
+                                        kv_len_bound=ctx.kv_len_bound, status=ctx.status, sink=sink, long_maps=group.long_maps,
+                                        layer_in_pool=cache.layer_in_group)
             o = o.view(n, self.H * self.DV)
         else:
             o = ops.attention_rows(q, self.H, k_pool, v_pool, value_dim=self.DV, positions=ctx.positions, req_of_token=ctx.req_of_token,

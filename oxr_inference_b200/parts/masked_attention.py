@@ -22,6 +22,11 @@ def distance_bucket(n: int, rows: int, far: float) -> int:
     return min(rows - 1, half + int(math.floor(math.log(n / half) / math.log(far / half) * (rows - half))))
 
 
+def bias_distances(rows: int, far: float) -> int:
+    """How many distances :func:`bias_by_distance` gives a row of their own."""
+    return max(rows // 2, int(math.ceil(far))) + 1
+
+
 def bias_by_distance(table: torch.Tensor, far: float) -> torch.Tensor:
     """Expand a bucketed bias table ``[rows, heads]`` into one row per distance ``0 .. ceil(far)``; the last row stands for every
     larger distance (all of them fall into the last bucket). The buckets are worked out on the host in double precision, once."""
@@ -29,8 +34,7 @@ def bias_by_distance(table: torch.Tensor, far: float) -> torch.Tensor:
     half = rows // 2
     if rows < 2 or far <= half:
         raise ValueError(f"a distance-bias table of {rows} rows needs its far distance ({far}) beyond {half}")
-    last = max(half, int(math.ceil(far)))
-    index = [distance_bucket(n, rows, far) for n in range(last + 1)]
+    index = [distance_bucket(n, rows, far) for n in range(bias_distances(rows, far))]
     if index[-1] != rows - 1:
         raise ValueError("the far distance does not reach the table's last row")
     return table[torch.tensor(index, device=table.device)].contiguous()
@@ -162,7 +166,10 @@ class MaskedAttention(Mixer):
     def tile_specs(self) -> list[tuple[int, int, int]]:
         if not self.tiled:
             return []
-        return ops.attention_tile_specs(self.H, self.KV, self.padded or self.DK, self.runtime.dtype, self.runtime.page_size if self.plain else None)
+        if self.plain:
+            return ops.attention_tile_specs(self.H, self.KV, self.padded or self.DK, self.runtime.dtype, self.runtime.page_size)
+        return ops.masked_tile_specs(self.H, self.KV, self.DK, self.runtime.dtype, self.runtime.page_size,
+                                     bias_rows=bias_distances(self.bias_rows, self.bias_far) if self.bias_rows else 0, scale=self.scale)
 
     def forward(self, h: torch.Tensor, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
         y = self.out(self._attend(h, ctx, cache))
@@ -211,7 +218,8 @@ class MaskedAttention(Mixer):
             else:
                 o = ops.paged_attention(q, k_pool, v_pool, tiles=ctx.tiles, cu_q=ctx.cu_q, ctx_lens=ctx.ctx_lens, block_table=group.block_table,
                                         page_size=group.page_size, scale=self.scale, window=self.window, kv_len_bound=ctx.kv_len_bound,
-                                        status=ctx.status, chunk=self.chunk, dist_bias=self.dist_bias)
+                                        status=ctx.status, chunk=self.chunk, dist_bias=self.dist_bias, long_maps=group.long_maps,
+                                        layer_in_pool=cache.layer_in_group)
             return o.view(ctx.n_tokens, self.H * self.DV)
         return ops.attention_rows(q, self.H, k_pool, v_pool, value_dim=self.DV, positions=ctx.positions, req_of_token=ctx.req_of_token,
                                   block_table=group.block_table, scale=self.scale, chunk=self.chunk, window=self.window,
@@ -298,7 +306,8 @@ class LatentAttention(Mixer):
         return (self.L + self.R,) if self.tiled else ()
 
     def tile_specs(self) -> list[tuple[int, int, int]]:
-        return ops.attention_tile_specs(self.H, 1, self.L + self.R, self.runtime.dtype) if self.tiled else []
+        return ops.masked_tile_specs(self.H, 1, self.L + self.R, self.runtime.dtype, self.runtime.page_size, shared=True,
+                                     scale=self.scale) if self.tiled else []
 
     def forward(self, h: torch.Tensor, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
         group = cache.group
@@ -325,7 +334,8 @@ class LatentAttention(Mixer):
         if self.tiled and pool.dtype == torch.bfloat16:
             o_lat = ops.paged_attention(q_abs, pool, pool, tiles=ctx.tiles, cu_q=ctx.cu_q, ctx_lens=ctx.ctx_lens, block_table=group.block_table,
                                         page_size=group.page_size, scale=self.scale, window=self.window, kv_len_bound=ctx.kv_len_bound,
-                                        status=ctx.status, sink=self.sink)                       # [n, H, L + R]: the first L entries are the latent output
+                                        status=ctx.status, sink=self.sink, long_maps=group.long_maps,
+                                        layer_in_pool=cache.layer_in_group)                      # [n, H, L + R]: the first L entries are the latent output
         else:
             o_lat = ops.attention_rows(q_abs.view(n, H * (L + R)), H, pool, None, value_dim=L, positions=ctx.positions,
                                        req_of_token=ctx.req_of_token, block_table=group.block_table, scale=self.scale, window=self.window,
