@@ -23,7 +23,7 @@
 // kernel of its own (below).
 //
 // Token by token in the order of the sequence whatever the cut, so a position's result does not depend on how a prompt was cut into steps.
-#include "common.cuh"
+#include "scan_columns.cuh"
 
 struct DeltaArgs {
     int stride, r_col0, k_col0, v_col0;       // projections
@@ -45,12 +45,6 @@ constexpr int DELTA_TT = 8, DELTA_COLS = 32, DELTA_WARPS = 4, DELTA_PREP_WARPS =
 
 __device__ __forceinline__ float delta_sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
 
-typedef unsigned long long f32x2;      // two floats, the lower half first
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) { f32x2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi)); return d; }
-__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-
 template <int J, int KW> struct DeltaShape {
     static constexpr int DKP = 4 * J * KW, CPT = J / 4, NV = 2 * CPT;
     static constexpr int VEC = DELTA_TT * DKP;                                            // one vector of every token of a tile
@@ -60,22 +54,6 @@ template <int J, int KW> struct DeltaShape {
         (size_t)(2 * TILE + 2 * DELTA_TT * DELTA_COLS) * sizeof(float) + (size_t)DELTA_STAGES * DELTA_TT * TOKEN<T>;
     static_assert(DELTA_WARPS * (32 / J) * CPT == DELTA_COLS, "the warps hold the block's columns");
 };
-
-// The sums of v[0 .. N - 1] over a group of 2 N neighbouring lanes, number j / 2 of them for lane j of the group: every step sends half of the
-// numbers that are left to the lane N, N / 2, ... away and keeps the other half; the last step adds the two lanes of a pair.
-template <int N> __device__ __forceinline__ float delta_reduce(float (&v)[N], int lane) {
-    if constexpr (N == 1) return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-    else {
-        float half[N / 2];
-        const bool up = (lane & N) != 0;       // this lane keeps the upper half of the numbers
-#pragma unroll
-        for (int i = 0; i < N / 2; ++i) {
-            const float send = up ? v[i] : v[N / 2 + i], keep = up ? v[N / 2 + i] : v[i];
-            half[i] = keep + __shfl_xor_sync(0xffffffffu, send, N);
-        }
-        return delta_reduce<N / 2>(half, lane);
-    }
-}
 
 // N neighbouring floats from an address that is a multiple of N
 template <int N> __device__ __forceinline__ void delta_columns(const float* p, float (&v)[N]) {
@@ -97,7 +75,7 @@ __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delt
     constexpr int DKP = Sh::DKP, CPT = Sh::CPT, KL = (DKP + 31) / 32;      // KL: key entries per lane when a warp prepares a token
     extern __shared__ __align__(16) float dsm[];      // [2][TILE], then the results [2][TT][COLS]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int p0 = blockIdx.x * DELTA_COLS, h = blockIdx.y, r = blockIdx.z;
+    const int p0 = blockIdx.x * DELTA_COLS, h = blockIdx.y, r = longest_first(a.cu_q, gridDim.z, blockIdx.z);
     const int t0 = a.cu_q[r], t1 = a.cu_q[r + 1];
     if (t1 <= t0) return;
     const int DK = a.DK, DV = a.DV, n_tiles = (t1 - t0 + DELTA_TT - 1) / DELTA_TT;
@@ -304,7 +282,7 @@ __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delt
                 uu[i] = vec[DKP / 4 + J * i];
                 wr[i] = vec[Sh::VEC / 4 + DKP / 4 + J * i];
             }
-            const float sum = delta_reduce<2 * CPT>(d, lane);
+            const float sum = group_reduce<2 * CPT>(d, lane);
             // the part of the update that does not wait for the sums
 #pragma unroll
             for (int c = 0; c < CPT; ++c) {
@@ -420,7 +398,7 @@ __global__ void __launch_bounds__(32 * DELTA_WARPS) delta_step_kernel(float* __r
             d[CPT + c] = fmaf(s[c][i], rd[i], d[CPT + c]);
         }
     }
-    const float sum = delta_reduce<2 * CPT>(d, lane), held = __shfl_xor_sync(0xffffffffu, sum, J / 2);
+    const float sum = group_reduce<2 * CPT>(d, lane), held = __shfl_xor_sync(0xffffffffu, sum, J / 2);
     const int mine = (j >> 1) - CPT;
 #pragma unroll
     for (int c = 0; c < CPT; ++c) {

@@ -15,7 +15,7 @@
 // state, which is what hides the loop's latencies when a step brings many tokens of a request; keys of up to 128). A tile of TT tokens goes through shared memory at
 // a time (thread d brings entry d of k, q and the decay of each token; the next tile's loads are in flight while this one is computed); the
 // warps' partial sums of S^T q meet in shared memory and are added in the order of the warps after the tile.
-#include "common.cuh"
+#include "scan_columns.cuh"
 
 __device__ __forceinline__ float gla_log_sigmoid(float v) { return fminf(v, 0.f) - log1pf(expf(-fabsf(v))); }
 
@@ -123,11 +123,38 @@ __global__ void __launch_bounds__(32 * NW) gla_scan_kernel(
         if (n0 + k < DK && p < DV) S[(size_t)(n0 + k) * DV + p] = s[k];
 }
 
+// decay[t, i] = sigmoid(z[t, i] + bias[i])^(1 / tau), four entries a thread: once per token and key channel, where the recurrence's blocks (one per 32 value
+// columns) would each work it out again
+__global__ void gla_decay_kernel(float4* __restrict__ decay, const float4* __restrict__ z, const float4* __restrict__ z_bias, float inv_tau, int width4, size_t total) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= total) return;
+    const float4 v = z[i], b = z_bias[i % width4];
+    decay[i] = make_float4(expf(gla_log_sigmoid(v.x + b.x) * inv_tau), expf(gla_log_sigmoid(v.y + b.y) * inv_tau), expf(gla_log_sigmoid(v.z + b.z) * inv_tau),
+                           expf(gla_log_sigmoid(v.w + b.w) * inv_tau));
+}
+
+// decay: fp32 scratch [n_tokens, heads * DK] for steps of many tokens per request, which the kernel of scan_columns.cuh takes where the sizes are its own; null:
+// the kernel above.
 OXR_API int oxr_gla_scan(float* y, const void* proj, int n_requests, int proj_stride, int q_col0, int k_col0, int v_col0, const float* z,
                          const float* z_bias, float tau, int heads, int DK, int DV, float q_scale, float* state, long long slot_stride, const int* cu_q,
-                         const int* state_slots, int dtype, int key_entries_per_thread, cudaStream_t stream) {
+                         const int* state_slots, int dtype, int key_entries_per_thread, float* decay, int n_tokens, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (heads <= 0 || DK <= 0 || DK > 256 || DV <= 0 || heads > 65535 || n_requests > 65535 || !(tau > 0.f)) return OXR_BAD_ARGUMENT;
+    if (decay != nullptr && n_tokens > 0) {
+        const size_t size = dtype == 0 ? 4 : 2;
+        ScanArgs a = {};
+        a.k = (const char*)proj + k_col0 * size; a.q = (const char*)proj + q_col0 * size; a.x = (const char*)proj + v_col0 * size;
+        a.stride = proj_stride; a.k_group = 1; a.decay = decay; a.q_scale = q_scale; a.y = y; a.state = state; a.slot_stride = slot_stride; a.cu_q = cu_q;
+        a.state_slots = state_slots; a.heads = heads; a.DV = DV; a.n_requests = n_requests;
+        if ((dtype == 0 ? scan_fits<float>(a, DK) : scan_fits<__nv_bfloat16>(a, DK)) && (uintptr_t)z % 16 == 0 && (uintptr_t)z_bias % 16 == 0) {
+            const size_t total = (size_t)n_tokens * heads * DK / 4;
+            gla_decay_kernel<<<(unsigned)((total + 127) / 128), 128, 0, stream>>>((float4*)decay, (const float4*)z, (const float4*)z_bias, 1.f / tau,
+                                                                                 heads * DK / 4, total);
+            int rc = oxr_launch_status();
+            if (rc) return rc;
+            return dtype == 0 ? scan_launch<float, true>(a, DK, stream) : scan_launch<__nv_bfloat16, true>(a, DK, stream);
+        }
+    }
     dim3 grid((DV + 31) / 32, heads, n_requests);
     // 16 key entries a thread (twice the warps per head) where that still fits a block of 8 warps; key_entries_per_thread 16 or 32 forces one
     const bool narrow = key_entries_per_thread == 16 ? DK <= 128 : (key_entries_per_thread == 32 ? false : DK <= 128);

@@ -11,7 +11,7 @@
 // The recurrence runs token by token in the order of the sequence whatever the cut, so a position's result does not
 // depend on how the prompt was cut into steps. Columns of S (one value dimension p each) are independent: a block takes
 // 32 columns of one head of one request.
-#include "common.cuh"
+#include "scan_columns.cuh"
 
 // ---------------------------------------------------------------------------------------------- convolution
 // out[t, c] = silu(bias[c] + sum_j w[c, j] * in[t - (taps-1-j), c]); inputs before the step's first token come from the
@@ -237,9 +237,21 @@ static void mamba_scan(float* y, const void* xbc, const void* proj, int n_reques
 
 OXR_API int oxr_mamba_scan(float* y, const void* xbc, const void* proj, int n_requests, int proj_stride, int dt_col0, int heads, int vdim, int N, int groups,
                            const float* dt_bias, const float* a_log, const float* d_skip, float* state, long long slot_stride, const int* cu_q,
-                           const int* state_slots, int dtype, cudaStream_t stream) {
+                           const int* state_slots, int dtype, int n_tokens, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (heads <= 0 || vdim <= 0 || N <= 0 || N > 256 || groups <= 0 || heads % groups || n_requests > 65535 || heads > 65535) return OXR_BAD_ARGUMENT;
+    // Many tokens of a request (not decode steps, whose cost is the state's way through the registers): the kernel of scan_columns.cuh
+    if (n_tokens > 2 * n_requests) {
+        const size_t size = dtype == 0 ? 4 : 2;
+        const int inner = heads * vdim;
+        ScanArgs a = {};
+        a.x = xbc; a.k = (const char*)xbc + inner * size; a.q = (const char*)xbc + (inner + groups * N) * size;
+        a.stride = inner + 2 * groups * N; a.k_group = heads / groups; a.dt = (const char*)proj + dt_col0 * size; a.dt_stride = proj_stride;
+        a.dt_bias = dt_bias; a.a_log = a_log; a.skip = d_skip; a.y = y; a.state = state; a.slot_stride = slot_stride; a.cu_q = cu_q; a.state_slots = state_slots;
+        a.heads = heads; a.DV = vdim; a.n_requests = n_requests;
+        if (dtype == 0 ? scan_fits<float>(a, N) : scan_fits<__nv_bfloat16>(a, N))
+            return dtype == 0 ? scan_launch<float, false>(a, N, stream) : scan_launch<__nv_bfloat16, false>(a, N, stream);
+    }
     const int nw = (N + 31) / 32;
 #define OXR_SCAN(NW) \
     (dtype == 0 ? mamba_scan<float, NW>(y, xbc, proj, n_requests, proj_stride, dt_col0, heads, vdim, N, groups, dt_bias, a_log, d_skip, state, \

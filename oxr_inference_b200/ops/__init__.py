@@ -140,7 +140,7 @@ def _lib():
         lib.oxr_clamped_glu.argtypes = [p, p, i, i, i, f, f, i, p]
         lib.oxr_rotary_angles.argtypes = [p, p, p, p, c_double, i, i, p]
         lib.oxr_mamba_conv.argtypes = [p, p, i, i, i, i, i, i, p, p, p, ll, p, p, p, i, p]
-        lib.oxr_mamba_scan.argtypes = [p, p, p, i, i, i, i, i, i, i, p, p, p, p, ll, p, p, i, p]
+        lib.oxr_mamba_scan.argtypes = [p, p, p, i, i, i, i, i, i, i, p, p, p, p, ll, p, p, i, i, p]
         lib.oxr_gated_group_norm.argtypes = [p, p, p, i, i, i, p, i, i, f, i, p]
         lib.oxr_attention_rows.argtypes = [p, p, i, p, ll, i, p, ll, i, i, i, i, i, i, p, p, p, i, i, i, f, i, i, i, p, i, p, i, p, p]
         lib.oxr_scatter_rows.argtypes = [p, ll, ll, p, i, i, i, p, i, i, p, p, ll, i, p]
@@ -173,7 +173,7 @@ def _lib():
         lib.oxr_expert_clamped_glu.argtypes = [p, p, p, i, i, i, f, f, i, p]
         lib.oxr_head_prep.argtypes = [p, p, p, p, i, i, i, i, i, i, i, i, i, i, i, i, p, p, p, i, p, ll, i, i, p, p, p, f, p, p, i, p, ll, p, p, p, i, p, p]
         lib.oxr_sigmoid_gate.argtypes = [p, p, i, i, i, i, i, i, i, p]
-        lib.oxr_gla_scan.argtypes = [p, p, i, i, i, i, i, p, p, f, i, i, i, f, p, ll, p, p, i, i, p]
+        lib.oxr_gla_scan.argtypes = [p, p, i, i, i, i, i, p, p, f, i, i, i, f, p, ll, p, p, i, i, p, i, p]
         lib.oxr_pair_norm_mean.argtypes = [p, p, p, p, p, i, i, f, i, p]
         lib.oxr_tanh_cap.argtypes = [p, f, ll, p]
         lib.oxr_expert_silu_glu.argtypes = [p, p, p, i, i, i, i, i, p]
@@ -1504,7 +1504,7 @@ def mamba_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col0: int, *, heads: in
     y = torch.empty((n, heads * vdim), dtype=torch.float32, device=xbc.device)
     _done(_lib().oxr_mamba_scan(y.data_ptr(), xbc.data_ptr(), proj.data_ptr(), n_requests, proj.shape[1], dt_col0, heads, vdim, state, groups,
                                 dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), ssm.data_ptr(), ssm.stride(0), cu_q.data_ptr(),
-                                state_slots.data_ptr(), _dtype_code(xbc), _stream()), "mamba_scan")
+                                state_slots.data_ptr(), _dtype_code(xbc), n, _stream()), "mamba_scan")
     return y
 
 
@@ -2007,7 +2007,7 @@ def gla_scan(proj: torch.Tensor, q_col0: int, k_col0: int, v_col0: int, z: torch
     ``alpha_t = sigmoid(z_t + z_bias)^(1 / tau)`` per key channel. ``proj`` holds q, k and v head by head from the given columns; ``z [tokens, heads *
     key_dim]`` is fp32; ``state`` (fp32, first axis the slot: S ``[heads, key_dim, value_dim]``) is read and left at the state after each request's
     last token. Returns fp32 ``o [tokens, heads * value_dim]``. ``key_entries_per_thread`` (16 or 32) forces the kernel's split of a head's
-    key channels over threads; 0 chooses by the step's shape."""
+    key channels over threads; 0 chooses the kernel and the split by the step's shape."""
     _need(proj, "proj")
     _need(z, "z", torch.float32)
     _need(z_bias, "z_bias", torch.float32)
@@ -2017,13 +2017,17 @@ def gla_scan(proj: torch.Tensor, q_col0: int, k_col0: int, v_col0: int, z: torch
     if z.shape != (n, heads * key_dim) or z_bias.numel() != heads * key_dim:
         raise KernelError("gla_scan: the decay logits must be [tokens, heads * key_dim] with one bias each")
     y = torch.empty((n, heads * value_dim), dtype=torch.float32, device=proj.device)
+    decay = None
     if not key_entries_per_thread:
-        # portions of prompts: twice the warps per head hide the loop's latencies (1,069 -> 770 us for 2,048 tokens of 16 heads of 128 x 256);
-        # single tokens: the state's trip through the registers is all there is, and fewer partial sums are cheaper (20.5 against 24.6 us)
-        key_entries_per_thread = 16 if n > 2 * n_requests else 32
+        # portions of prompts: the kernel whose threads hold several columns, where it takes the sizes, else twice the warps per head (2,048 tokens of
+        # 16 heads of 128 x 256: 409 against 739 us); single tokens: the state's trip through the registers is all there is, and fewer
+        # partial sums are cheaper (20.5 against 24.6 us)
+        many = n > 2 * n_requests
+        key_entries_per_thread = 16 if many else 32
+        decay = torch.empty_like(z) if many else None
     _done(_lib().oxr_gla_scan(y.data_ptr(), proj.data_ptr(), int(n_requests), proj.shape[1], int(q_col0), int(k_col0), int(v_col0), z.data_ptr(),
                               z_bias.data_ptr(), float(tau), int(heads), int(key_dim), int(value_dim), float(q_scale), state.data_ptr(), state.stride(0),
-                              cu_q.data_ptr(), state_slots.data_ptr(), _dtype_code(proj), int(key_entries_per_thread), _stream()), "gla_scan")
+                              cu_q.data_ptr(), state_slots.data_ptr(), _dtype_code(proj), int(key_entries_per_thread), _ptr(decay), n, _stream()), "gla_scan")
     return y
 
 
