@@ -39,6 +39,24 @@ __global__ void embedding_vec_kernel(T* __restrict__ out, const T* __restrict__ 
     for (int i = threadIdx.x; i < words_per_row; i += blockDim.x) dst[i] = __ldg(src + i);
 }
 
+// bf16 rows of whole 16-byte words to fp32 (the stream of blocks that keep it whole): eight entries a thread. An entry at a time 8 rows of 4,096 took 9 us and
+// 2,048 rows 19; here 2.6 and 12.
+__global__ void embedding_widen_kernel(float* __restrict__ out, const uint4* __restrict__ table, const int* __restrict__ ids, int words_per_row, int vocab,
+                                       float scale, int* status) {
+    const int t = blockIdx.x;
+    const int id = ids[t];
+    float4* dst = reinterpret_cast<float4*>(out) + (size_t)t * words_per_row * 2;
+    const bool ok = id >= 0 && id < vocab;
+    if (!ok && threadIdx.x == 0) oxr_report(status, OXR_BAD_TOKEN_ID, t);
+    for (int i = threadIdx.x; i < words_per_row; i += blockDim.x) {
+        const uint4 w = ok ? __ldg(table + (size_t)id * words_per_row + i) : make_uint4(0, 0, 0, 0);
+        dst[2 * i] = make_float4(__uint_as_float(w.x << 16) * scale, __uint_as_float(w.x & 0xffff0000u) * scale, __uint_as_float(w.y << 16) * scale,
+                                 __uint_as_float(w.y & 0xffff0000u) * scale);
+        dst[2 * i + 1] = make_float4(__uint_as_float(w.z << 16) * scale, __uint_as_float(w.z & 0xffff0000u) * scale, __uint_as_float(w.w << 16) * scale,
+                                     __uint_as_float(w.w & 0xffff0000u) * scale);
+    }
+}
+
 // table_dtype / out_dtype: 0 = float32, 1 = bfloat16. out = table[id] * scale, the product in fp32, rounded once.
 OXR_API int oxr_embedding(void* out, const void* table, const int* ids, int n_tokens, int hidden, int vocab,
                           int table_dtype, int out_dtype, float scale, int* status, cudaStream_t stream) {
@@ -55,6 +73,10 @@ OXR_API int oxr_embedding(void* out, const void* table, const int* ids, int n_to
                 embedding_vec_kernel<__nv_bfloat16><<<n_tokens, threads, 0, stream>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)table, ids, words, vocab, status);
             return oxr_launch_status();
         }
+    }
+    if (table_dtype == 1 && out_dtype == 0 && hidden % 8 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)table % 16 == 0) {
+        embedding_widen_kernel<<<n_tokens, threads, 0, stream>>>((float*)out, (const uint4*)table, ids, hidden / 8, vocab, scale, status);
+        return oxr_launch_status();
     }
     if (table_dtype == 0 && out_dtype == 0)
         embedding_kernel<float, float><<<n_tokens, threads, 0, stream>>>((float*)out, (const float*)table, ids, hidden, vocab, scale, status);

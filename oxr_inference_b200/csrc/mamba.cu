@@ -36,6 +36,67 @@ __global__ void causal_conv_silu_kernel(T* __restrict__ out, const T* __restrict
     out[(size_t)t * channels + c] = Num<T>::from_f32(acc / (1.f + expf(-acc)));
 }
 
+// Four taps on bf16 rows of whole 16-byte words: a thread takes eight channels of CONV_RUN tokens, one word a token, and keeps the last three inputs and the
+// weights in registers. Element by element the kernel above fetched every input four times and its weight row 16 bytes apart: 2,048 tokens of
+// 10,240 channels took 131 to 142 us, 56 to 62 here (reading and writing each value once takes 13 us). The arithmetic is that of the kernel above, entry by entry.
+constexpr int CONV_RUN = 16, CONV_THREADS = 128;
+__device__ __forceinline__ void conv_widen(const uint4& w, float (&v)[8]) {
+    const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(u[i] << 16); v[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u); }
+}
+__global__ void __launch_bounds__(CONV_THREADS) causal_conv4_silu_words_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ proj, int proj_stride,
+                                                                               int col0, int channels, int n_tokens, const float* __restrict__ w,
+                                                                               const float* __restrict__ bias, const float* __restrict__ state,
+                                                                               long long slot_stride, const int* __restrict__ req_of_token,
+                                                                               const int* __restrict__ cu_q, const int* __restrict__ state_slots) {
+    const int c = (blockIdx.x * CONV_THREADS + threadIdx.x) * 8;
+    if (c >= channels) return;
+    float wt[8][4], b[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const float4 x = *reinterpret_cast<const float4*>(w + (size_t)(c + e) * 4);
+        wt[e][0] = x.x; wt[e][1] = x.y; wt[e][2] = x.z; wt[e][3] = x.w;
+        b[e] = bias[c + e];
+    }
+    const int first = blockIdx.y * CONV_RUN, last = min(first + CONV_RUN, n_tokens);
+    float past[3][8];      // the inputs of the tokens three, two and one back
+    int r = -1;
+#pragma unroll 4
+    for (int t = first; t < last; ++t) {
+        const int rt = req_of_token[t];
+        if (rt != r) {     // the run's first token or a request's: what lies before it comes from the rows before, or from the request's tail
+            r = rt;
+            const int i = t - cu_q[r];
+            const float* tail = state + (long long)state_slots[r] * slot_stride + (long long)c * 3;
+#pragma unroll
+            for (int back = 3; back >= 1; --back) {
+                if (i - back >= 0) conv_widen(*reinterpret_cast<const uint4*>(proj + (size_t)(t - back) * proj_stride + col0 + c), past[3 - back]);
+                else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) past[3 - back][e] = tail[e * 3 + 3 + (i - back)];
+                }
+            }
+        }
+        float now[8], o[8];
+        conv_widen(*reinterpret_cast<const uint4*>(proj + (size_t)t * proj_stride + col0 + c), now);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            float acc = fmaf(wt[e][0], past[0][e], b[e]);
+            acc = fmaf(wt[e][1], past[1][e], acc);
+            acc = fmaf(wt[e][2], past[2][e], acc);
+            acc = fmaf(wt[e][3], now[e], acc);
+            o[e] = acc / (1.f + expf(-acc));
+            past[0][e] = past[1][e]; past[1][e] = past[2][e]; past[2][e] = now[e];
+        }
+        uint4 word;
+        __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&word);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) p[e] = __floats2bfloat162_rn(o[2 * e], o[2 * e + 1]);
+        *reinterpret_cast<uint4*>(out + (size_t)t * channels + c) = word;
+    }
+}
+
 // After the convolution read it: the tail becomes the last taps-1 inputs of (old tail ++ the step's inputs).
 template <typename T>
 __global__ void conv_tail_roll_kernel(float* __restrict__ state, long long slot_stride, const T* __restrict__ proj, int proj_stride, int col0,
@@ -195,15 +256,53 @@ __global__ void gated_group_norm_kernel(T* __restrict__ out, const float* __rest
     }
 }
 
+// The same on whole 16-byte words, eight entries a thread, each read once and kept in registers between the sum and the output: the kernel above reads y and z
+// twice, an entry at a time, and works the silu out twice. 2,048 tokens x 8,192 in 8 parts: 75 -> 32 us (20 us of bytes).
+__global__ void gated_group_norm_words_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ y, const __nv_bfloat16* __restrict__ proj, int proj_stride,
+                                              int z_col0, const float* __restrict__ weight, int inner, int part, float eps) {
+    __shared__ float red[32];
+    const int t = blockIdx.y, at = blockIdx.x * part + 8 * threadIdx.x;
+    const bool ok = 8 * (int)threadIdx.x < part;
+    float v[8] = {};
+    float ss = 0.f;
+    if (ok) {
+        float z[8];
+        conv_widen(*reinterpret_cast<const uint4*>(proj + (size_t)t * proj_stride + z_col0 + at), z);
+        const float4 a = *reinterpret_cast<const float4*>(y + (size_t)t * inner + at), b = *reinterpret_cast<const float4*>(y + (size_t)t * inner + at + 4);
+        const float ye[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            v[e] = ye[e] * (z[e] / (1.f + expf(-z[e])));
+            ss = fmaf(v[e], v[e], ss);
+        }
+    }
+    ss = block_sum(ss, red);
+    const float inv = 1.f / sqrtf(ss / (float)part + eps);
+    if (ok) {
+        uint4 word;
+        __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&word);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) p[e] = __floats2bfloat162_rn(v[2 * e] * inv * weight[at + 2 * e], v[2 * e + 1] * inv * weight[at + 2 * e + 1]);
+        *reinterpret_cast<uint4*>(out + (size_t)t * inner + at) = word;
+    }
+}
+
 // ---------------------------------------------------------------------------------------------- launchers
 // proj: the in-projection's output [tokens, proj_stride], columns [z: inner | x, B, C: channels | dt: heads].
 template <typename T>
 static int mamba_conv(void* out, const void* proj, int n_tokens, int n_requests, int proj_stride, int col0, int channels, int taps,
                       const float* w, const float* bias, float* state, long long slot_stride, const int* req_of_token, const int* cu_q,
                       const int* state_slots, cudaStream_t stream) {
-    dim3 grid((channels + 127) / 128, n_tokens);
-    causal_conv_silu_kernel<T><<<grid, 128, 0, stream>>>((T*)out, (const T*)proj, proj_stride, col0, channels, taps, w, bias, state, slot_stride,
-                                                        req_of_token, cu_q, state_slots);
+    // the 16-byte form wants whole words and, to fill the chip with a thread per eight channels of 16 tokens, more than a decode step's rows
+    const auto words = [](const void* p) { return (uintptr_t)p % 16 == 0; };
+    if (sizeof(T) == 2 && taps == 4 && n_tokens > CONV_RUN && channels % 8 == 0 && proj_stride % 8 == 0 && col0 % 8 == 0 && words(out) && words(proj) && words(w))
+        causal_conv4_silu_words_kernel<<<dim3((channels / 8 + CONV_THREADS - 1) / CONV_THREADS, (n_tokens + CONV_RUN - 1) / CONV_RUN), CONV_THREADS, 0, stream>>>(
+            (__nv_bfloat16*)out, (const __nv_bfloat16*)proj, proj_stride, col0, channels, n_tokens, w, bias, state, slot_stride, req_of_token, cu_q, state_slots);
+    else {
+        dim3 grid((channels + 127) / 128, n_tokens);
+        causal_conv_silu_kernel<T><<<grid, 128, 0, stream>>>((T*)out, (const T*)proj, proj_stride, col0, channels, taps, w, bias, state, slot_stride,
+                                                            req_of_token, cu_q, state_slots);
+    }
     if (taps > 1) {
         dim3 grid2((channels + 127) / 128, n_requests);
         conv_tail_roll_kernel<T><<<grid2, 128, 0, stream>>>(state, slot_stride, (const T*)proj, proj_stride, col0, channels, taps, cu_q, state_slots);
@@ -279,6 +378,12 @@ OXR_API int oxr_gated_group_norm(void* out, const float* y, const void* proj, in
     const int part = inner / parts;
     const int threads = part >= 1024 ? 256 : 128;
     dim3 grid(parts, n_tokens);
+    const auto words = [](const void* p) { return (uintptr_t)p % 16 == 0; };
+    if (dtype == 1 && part % 8 == 0 && part <= 8192 && proj_stride % 8 == 0 && z_col0 % 8 == 0 && words(out) && words(y) && words(proj)) {
+        gated_group_norm_words_kernel<<<grid, (part / 8 + 31) / 32 * 32, 0, stream>>>((__nv_bfloat16*)out, y, (const __nv_bfloat16*)proj, proj_stride, z_col0, weight,
+                                                                                     inner, part, eps);
+        return oxr_launch_status();
+    }
     if (dtype == 0) gated_group_norm_kernel<float><<<grid, threads, 0, stream>>>((float*)out, y, (const float*)proj, proj_stride, z_col0, weight, inner, part, eps);
     else gated_group_norm_kernel<__nv_bfloat16><<<grid, threads, 0, stream>>>((__nv_bfloat16*)out, y, (const __nv_bfloat16*)proj, proj_stride, z_col0, weight,
                                                                               inner, part, eps);
