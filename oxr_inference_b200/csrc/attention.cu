@@ -324,8 +324,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// Gather keys [k0, k0 + MMA_BN) of one request into Ks / Vs (rows of LDS elements); keys outside [k_lo, k_end)
-// become zeros. All MMA_THREADS threads take part: a thread keeps its 16-byte column and walks down the rows, so
+// Gather keys [k0, k0 + MMA_BN) of one request into Ks / Vs (rows of LDS elements; Vs null: the keys are the values, one copy serves); keys outside
+// [k_lo, k_end) become zeros. All MMA_THREADS threads take part: a thread keeps its 16-byte column and walks down the rows, so
 // that per row it needs one block-table lookup, one multiply and two cp.async. page_shift >= 0 when the page size
 // is a power of two.
 __device__ __forceinline__ void load_kv_block(bf16* Ks, bf16* Vs, const bf16* __restrict__ k_cache,
@@ -360,7 +360,7 @@ __device__ __forceinline__ void load_kv_block(bf16* Ks, bf16* Vs, const bf16* __
             }
         }
         cp_async_16(Ks + j * LDS + smem_col, k_cache + base, ok);
-        cp_async_16(Vs + j * LDS + smem_col, v_cache + base, ok);
+        if (Vs != nullptr) cp_async_16(Vs + j * LDS + smem_col, v_cache + base, ok);
     }
 }
 
@@ -657,10 +657,12 @@ attn_mma_prefill_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, cons
 
 constexpr int DECODE_ROWS = 16;
 constexpr int DECODE_STAGES = 3;
-constexpr size_t DECODE_STAGE_SMEM = (size_t)(DECODE_ROWS + DECODE_STAGES * 2 * MMA_BN) * LDS * sizeof(bf16);
 constexpr int MERGE_STRIDE = D + 4;             // floats per row of the warps' merge area: O, m, l, and 16-byte alignment
 constexpr size_t DECODE_MERGE_SMEM = (size_t)4 * DECODE_ROWS * MERGE_STRIDE * sizeof(float);
-constexpr size_t DECODE_SMEM = DECODE_STAGE_SMEM > DECODE_MERGE_SMEM ? DECODE_STAGE_SMEM : DECODE_MERGE_SMEM;
+constexpr size_t decode_smem(bool shared) {   // shared: a stage holds the keys alone, which are the values as well
+    const size_t stages = (size_t)(DECODE_ROWS + DECODE_STAGES * (shared ? 1 : 2) * MMA_BN) * LDS * sizeof(bf16);
+    return stages > DECODE_MERGE_SMEM ? stages : DECODE_MERGE_SMEM;
+}
 
 // The four warps of a block have each seen a quarter of the block's keys: their (O, m, l) per row stand in shared
 // memory `mo` [warp][row][MERGE_STRIDE]. Merge them in the order of the warps; with one piece per unit that is the
@@ -709,51 +711,74 @@ __device__ __forceinline__ void merge_warps(const float* mo, int nrows, int spli
 // eight pieces are issued together and none depends on a value loaded before it, because what the merge costs is the
 // latency of its loads from L2, not their number. An empty piece wrote (-inf, 0) and no O: its O is read (it is
 // memory of the workspace) and dropped by a select, never multiplied.
+// One block does this for a whole unit, so its time is that of the trips to L2 it makes: NI (row, four d) items a thread and pass keep 8 NI
+// loads in flight (at head size 256, 16 rows and 16 pieces: 4 trips where one item at a time made 16).
+constexpr int MERGE_ITEMS = D > 128 ? 4 : 1;     // two at head size 128 cost a short context's decode step 1 us a layer
+template <int NI>
 __device__ __forceinline__ void merge_pieces(bf16* __restrict__ out, const float* __restrict__ all_ml, const float* __restrict__ all_o,
                                              int splits, int rows_live, const TileGeometry& g, const AttnArgs& a) {
     constexpr int CHUNK = 8, DV = D / 4;
-    for (int idx = threadIdx.x; idx < rows_live * DV; idx += MMA_THREADS) {
-        const int r = idx / DV, d = (idx % DV) * 4;
-        int tok, gh;
-        if (!g.row(r, tok, gh)) continue;
-        float M = -INFINITY, L = 0.f;
-        float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int total = rows_live * DV;
+    for (int idx0 = threadIdx.x; idx0 < total; idx0 += MMA_THREADS * NI) {
+        float M[NI], L[NI];
+        float4 O[NI];
+        int row[NI], d[NI];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int idx = min(idx0 + i * MMA_THREADS, total - 1);      // beyond the last item: the last one again, not written
+            row[i] = idx / DV;
+            d[i] = (idx % DV) * 4;
+            M[i] = -INFINITY;
+            L[i] = 0.f;
+            O[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
         for (int s0 = 0; s0 < splits; s0 += CHUNK) {
-            float2 pml[CHUNK];
-            float4 po[CHUNK];
+            float2 pml[NI][CHUNK];
+            float4 po[NI][CHUNK];
 #pragma unroll
             for (int j = 0; j < CHUNK; ++j) {
                 const int s2 = min(s0 + j, splits - 1);
-                pml[j] = __ldcg(reinterpret_cast<const float2*>(all_ml + ((size_t)s2 * DECODE_ROWS + r) * 2));
-                po[j] = __ldcg(reinterpret_cast<const float4*>(all_o + ((size_t)s2 * DECODE_ROWS + r) * D + d));
-            }
-            float m_new = M;
 #pragma unroll
-            for (int j = 0; j < CHUNK; ++j) {
-                if (s0 + j >= splits) pml[j].x = -INFINITY;   // a clamped repeat of the last piece
-                m_new = fmaxf(m_new, pml[j].x);
+                for (int i = 0; i < NI; ++i) {
+                    pml[i][j] = __ldcg(reinterpret_cast<const float2*>(all_ml + ((size_t)s2 * DECODE_ROWS + row[i]) * 2));
+                    po[i][j] = __ldcg(reinterpret_cast<const float4*>(all_o + ((size_t)s2 * DECODE_ROWS + row[i]) * D + d[i]));
+                }
             }
-            const float keep = (M == -INFINITY) ? 0.f : exp2f(M - m_new);
-            L *= keep;
-            O.x *= keep; O.y *= keep; O.z *= keep; O.w *= keep;
 #pragma unroll
-            for (int j = 0; j < CHUNK; ++j) {
-                if (pml[j].x == -INFINITY) continue;          // compile-time unrolled: a select, no load depends on it
-                const float f = exp2f(pml[j].x - m_new);
-                L += pml[j].y * f;
-                O.x += po[j].x * f; O.y += po[j].y * f; O.z += po[j].z * f; O.w += po[j].w * f;
+            for (int i = 0; i < NI; ++i) {
+                float m_new = M[i];
+#pragma unroll
+                for (int j = 0; j < CHUNK; ++j) {
+                    if (s0 + j >= splits) pml[i][j].x = -INFINITY;   // a clamped repeat of the last piece
+                    m_new = fmaxf(m_new, pml[i][j].x);
+                }
+                const float keep = (M[i] == -INFINITY) ? 0.f : exp2f(M[i] - m_new);
+                L[i] *= keep;
+                O[i].x *= keep; O[i].y *= keep; O[i].z *= keep; O[i].w *= keep;
+#pragma unroll
+                for (int j = 0; j < CHUNK; ++j) {
+                    if (pml[i][j].x == -INFINITY) continue;          // compile-time unrolled: a select, no load depends on it
+                    const float f = exp2f(pml[i][j].x - m_new);
+                    L[i] += pml[i][j].y * f;
+                    O[i].x += po[i][j].x * f; O[i].y += po[i][j].y * f; O[i].z += po[i][j].z * f; O[i].w += po[i][j].w * f;
+                }
+                M[i] = m_new;
             }
-            M = m_new;
         }
-        if (a.sink != nullptr) {
-            const float keep = add_sink(a.sink[g.kvh * g.G + gh], M, L);
-            O.x *= keep; O.y *= keep; O.z *= keep; O.w *= keep;
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            int tok, gh;
+            if (idx0 + i * MMA_THREADS >= total || !g.row(row[i], tok, gh)) continue;
+            if (a.sink != nullptr) {
+                const float keep = add_sink(a.sink[g.kvh * g.G + gh], M[i], L[i]);
+                O[i].x *= keep; O[i].y *= keep; O[i].z *= keep; O[i].w *= keep;
+            }
+            const float inv = L[i] > 0.f ? 1.f / L[i] : 0.f;
+            uint2 packed;
+            packed.x = pack_bf16(O[i].x * inv, O[i].y * inv);
+            packed.y = pack_bf16(O[i].z * inv, O[i].w * inv);
+            *reinterpret_cast<uint2*>(out + ((size_t)(g.q_begin + tok) * a.H + (size_t)g.kvh * g.G + gh) * D + d[i]) = packed;
         }
-        const float inv = L > 0.f ? 1.f / L : 0.f;
-        uint2 packed;
-        packed.x = pack_bf16(O.x * inv, O.y * inv);
-        packed.y = pack_bf16(O.z * inv, O.w * inv);
-        *reinterpret_cast<uint2*>(out + ((size_t)(g.q_begin + tok) * a.H + (size_t)g.kvh * g.G + gh) * D + d) = packed;
     }
 }
 
@@ -764,6 +789,10 @@ __device__ __forceinline__ void merge_pieces(bf16* __restrict__ out, const float
 //   part_ml [unit, split, 16, 2] = (maximum in log2 units, sum)
 // and takes a ticket from counters[unit]; the block that draws the last ticket merges all pieces and resets the
 // counter to zero for the next launch. Nobody waits for anybody.
+// SHARED: the keys are the values (a compressed cache). Fetched once, a stage takes half the bytes, and at head size 256 two blocks fit an SM where
+// two copies left room for one (half a round of the pieces that `attention_splits` deals out): a decode step of
+// 13 requests of 225 to 1,800 keys, 32 heads, 48 -> 39 us a layer, and 37 with four items of the merge in flight
+template <bool SHARED>
 __global__ void __launch_bounds__(MMA_THREADS)
 attn_mma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
                        int* __restrict__ counters, const bf16* __restrict__ q, const bf16* __restrict__ k_cache,
@@ -772,7 +801,7 @@ attn_mma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float
     __shared__ int s_ticket;
     bf16* Qs = reinterpret_cast<bf16*>(smem_raw);
     bf16* Ks = Qs + DECODE_ROWS * LDS;                      // DECODE_STAGES stages
-    bf16* Vs = Ks + DECODE_STAGES * MMA_BN * LDS;           // DECODE_STAGES stages
+    bf16* Vs = SHARED ? Ks : Ks + DECODE_STAGES * MMA_BN * LDS;   // DECODE_STAGES stages
     const TileGeometry g = tile_geometry(a, DECODE_ROWS);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int splits = gridDim.z, split = blockIdx.z;
@@ -799,7 +828,7 @@ attn_mma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float
 #pragma unroll
         for (int st = 0; st < DECODE_STAGES - 1; ++st) {
             if (st < count)
-                load_kv_block(Ks + st * MMA_BN * LDS, Vs + st * MMA_BN * LDS, k_cache, v_cache, table_row, a, g.kvh,
+                load_kv_block(Ks + st * MMA_BN * LDS, SHARED ? nullptr : Vs + st * MMA_BN * LDS, k_cache, v_cache, table_row, a, g.kvh,
                               kw.key0(first + st, MMA_BN), kw.lo(first + st), kw.end(first + st, k_end), g.req);
             cp_async_commit();
         }
@@ -828,7 +857,7 @@ attn_mma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float
             // iteration made it free
             const int nb = b + DECODE_STAGES - 1;
             if (nb < count)
-                load_kv_block(Ks + (nb % DECODE_STAGES) * MMA_BN * LDS, Vs + (nb % DECODE_STAGES) * MMA_BN * LDS, k_cache, v_cache,
+                load_kv_block(Ks + (nb % DECODE_STAGES) * MMA_BN * LDS, SHARED ? nullptr : Vs + (nb % DECODE_STAGES) * MMA_BN * LDS, k_cache, v_cache,
                               table_row, a, g.kvh, kw.key0(first + nb, MMA_BN), kw.lo(first + nb), kw.end(first + nb, k_end), g.req);
             cp_async_commit();
             cp_async_wait<DECODE_STAGES - 1>();
@@ -890,7 +919,7 @@ attn_mma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float
     if (threadIdx.x == 0) counters[unit] = 0;   // ready for the next launch (nobody else touches it any more)
     const float* all_ml = part_ml + unit * splits * DECODE_ROWS * 2;
     const float* all_o = part_o + unit * splits * DECODE_ROWS * D;
-    merge_pieces(out, all_ml, all_o, splits, rows_live, g, a);
+    merge_pieces<MERGE_ITEMS>(out, all_ml, all_o, splits, rows_live, g, a);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -1289,7 +1318,7 @@ attn_tma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float
     if (threadIdx.x == 0) counters[unit] = 0;
     const float* all_ml = part_ml + unit * splits * DECODE_ROWS * 2;
     const float* all_o = part_o + unit * splits * DECODE_ROWS * D;
-    merge_pieces(out, all_ml, all_o, splits, rows_live, g, a);
+    merge_pieces<MERGE_ITEMS>(out, all_ml, all_o, splits, rows_live, g, a);
 #ifdef OXR_TIMELINE
     consumer_sync();
     if (threadIdx.x == 0) OXR_TL_PUT(5, tl_released, OXR_TL_NOW(), tl_first, tl_streamed, blockIdx.x);   // id 5: the block that merged its unit
@@ -1630,7 +1659,7 @@ attn_tma_decode_walk_kernel(bf16* __restrict__ out, float* __restrict__ part_o, 
             __threadfence();
             if (threadIdx.x == 0) counters[p.unit] = 0;
             const size_t slot0 = p.slot - (size_t)p.split;
-            merge_pieces(out, part_ml + slot0 * DECODE_ROWS * 2, part_o + slot0 * DECODE_ROWS * D, p.parts, p.rows_live, g, a);
+            merge_pieces<1>(out, part_ml + slot0 * DECODE_ROWS * 2, part_o + slot0 * DECODE_ROWS * D, p.parts, p.rows_live, g, a);
         }
     }
 }
@@ -2744,7 +2773,9 @@ static int paged_attention_bf16(void* out, const void* q, const void* k_cache, c
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attn_mma_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(attn_mma_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DECODE_SMEM);
+            e = cudaFuncSetAttribute(attn_mma_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_smem(false));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(attn_mma_decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_smem(true));
         if (e != cudaSuccess) return 1000 + (int)e;
         configured = true;
     }
@@ -2829,8 +2860,12 @@ static int paged_attention_bf16(void* out, const void* q, const void* k_cache, c
         if (TMA_OK && kv_maps != nullptr && a.page_shift >= 3)
             return launch_tma_decode<false>(out, q, n_short, KV * groups, splits, part_o, part_ml, counters, kv_maps, pool_row0, cut, a, FuseQkv{}, stream);
         oxr_last_short_kernel = 1;
-        attn_mma_decode_kernel<<<dim3(n_short, KV * groups, splits), MMA_THREADS, DECODE_SMEM, stream>>>(
-            (bf16*)out, part_o, part_ml, counters, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, a);
+        if (k_cache == v_cache)
+            attn_mma_decode_kernel<true><<<dim3(n_short, KV * groups, splits), MMA_THREADS, decode_smem(true), stream>>>(
+                (bf16*)out, part_o, part_ml, counters, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, a);
+        else
+            attn_mma_decode_kernel<false><<<dim3(n_short, KV * groups, splits), MMA_THREADS, decode_smem(false), stream>>>(
+                (bf16*)out, part_o, part_ml, counters, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, a);
         int rc = oxr_launch_status();
         if (rc) return rc;
     }
