@@ -60,16 +60,14 @@ __global__ void __launch_bounds__(256) gemm_f32_few_kernel(float* __restrict__ C
 
 // More rows: tiles of 8 TM x 16 TN on 128 threads, TM x TN sums per thread. What bounds it is the FMA rate (128 lanes of an SM,
 // 74 TFLOP/s at the full clock), so everything else has to stay out of the way of the multiply-adds:
-//  * sums in pairs of columns with fma.rn.f32x2 (each half rounds as fmaf does): half the issue slots, which leaves room for the loads;
-//    for that a[m] is kept twice in shared memory, so that one 16-byte load brings two rows' pairs ready (a broadcast: 16 lanes read
-//    the same address, so the doubled bytes cost nothing);
+//  * sums in pairs of columns with fma.rn.f32x2 (each half rounds as fmaf does): half the issue slots, which leaves room for the loads and for doubling
+//    a[m] in registers (kept twice in shared memory, as it was first, its loads took longer than the multiply-adds);
 //  * a thread's columns lie V apart in groups (group j of a thread starts at V (16 j + tx)), so that a warp reads consecutive words;
 //  * the next 16 k of A and W are fetched into registers while the current ones are multiplied, and put into the other half of a
 //    double buffer: one barrier per 16 k.
 // Four warps fill an SM's four schedulers by themselves. The tile is chosen by the launcher, see there.
-// 333 rows on a B200, against 64 x 64 tiles of 4 x 4 a thread filled element by element: 3,072 x 2,048 168 us (324), 2,048 x 2,048 122 (315),
-// 16,384 x 2,048 652 (1,403), 2,048 x 8,192 475 (1,477): 23 to 34 TFLOP/s. What is left is shared memory: at 8 x 8 a k takes 6 loads of 16 bytes a
-// thread, whose return to the registers (64 bytes a cycle, measured) takes longer than the 32 pairs of multiply-adds.
+// 333 rows on a B200, against 64 x 64 tiles of 4 x 4 a thread filled element by element: 3,072 x 2,048 127 us (324), 2,048 x 2,048 109 (315),
+// 16,384 x 2,048 530 (1,403), 2,048 x 8,192 433 (1,477): 26 to 42 TFLOP/s. Stages of 32 k instead of 16 cost registers and with them blocks: slower.
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
     unsigned long long r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -86,8 +84,8 @@ template <int TM, int TN, bool VEC>
 __global__ void __launch_bounds__(F32_THREADS) gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
                                                                     int M, int N, int K) {
     constexpr int BK = F32_BK, BM = 8 * TM, BN = 16 * TN;
-    constexpr int V = TN % 4 == 0 ? 4 : 2, G = TN / V;                     // columns per group, groups per thread
-    constexpr int LA = 2 * BM + 4, LW = BN + 4;                            // floats per k of the two tiles
+    constexpr int V = TN % 4 == 0 ? 4 : 2, G = TN / V, RV = TM % 4 == 0 ? 4 : 2;                     // columns per group, groups per thread
+    constexpr int LA = BM + 4, LW = BN + 4;                            // floats per k of the two tiles
     constexpr int QA = (BM * 4 + F32_THREADS - 1) / F32_THREADS, QW = (BN * 4 + F32_THREADS - 1) / F32_THREADS;   // 16-byte words per thread
     static_assert(TM % 2 == 0 && TN % 2 == 0, "rows and columns come in pairs");
     __shared__ __align__(16) float As[2][BK * LA];
@@ -126,7 +124,7 @@ __global__ void __launch_bounds__(F32_THREADS) gemm_f32_tile_kernel(float* __res
             if (q >= BM * 4) break;
             const float e[4] = {ra[i].x, ra[i].y, ra[i].z, ra[i].w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) *reinterpret_cast<float2*>(&As[b][((q & 3) * 4 + j) * LA + 2 * (q >> 2)]) = make_float2(e[j], e[j]);
+            for (int j = 0; j < 4; ++j) As[b][((q & 3) * 4 + j) * LA + (q >> 2)] = e[j];
         }
 #pragma unroll
         for (int i = 0; i < QW; ++i) {
@@ -151,16 +149,20 @@ __global__ void __launch_bounds__(F32_THREADS) gemm_f32_tile_kernel(float* __res
     for (int k0 = 0; k0 < K; k0 += BK) {
         const bool more = k0 + BK < K;
         if (more) fetch_tiles(k0 + BK);
-        const float* as = As[buf] + 2 * TM * ty;
+        const float* as = As[buf] + TM * ty;
         const float* ws = Ws[buf] + V * tx;
 #pragma unroll
         for (int k = 0; k < BK; ++k) {
             unsigned long long a[TM], b[TN / 2];
 #pragma unroll
-            for (int i = 0; i < TM; i += 2) {
-                const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(as + k * LA + 2 * i);
-                a[i] = p.x;
-                a[i + 1] = p.y;
+            for (int i = 0; i < TM; i += RV) {      // one word feeds RV rows; each is doubled in registers
+                if constexpr (RV == 4) {
+                    const float4 p = *reinterpret_cast<const float4*>(as + k * LA + i);
+                    a[i] = pack2(p.x, p.x); a[i + 1] = pack2(p.y, p.y); a[i + 2] = pack2(p.z, p.z); a[i + 3] = pack2(p.w, p.w);
+                } else {
+                    const float2 p = *reinterpret_cast<const float2*>(as + k * LA + i);
+                    a[i] = pack2(p.x, p.x); a[i + 1] = pack2(p.y, p.y);
+                }
             }
 #pragma unroll
             for (int g = 0; g < G; ++g) {
@@ -205,11 +207,11 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, cu
     return oxr_launch_status();
 }
 
-// Tile shapes (TM, TN) and what a k of a tile costs a scheduler in issue slots: the multiply-adds at the FMA pipe's rate, a slot for
-// each load of a fragment and one for the loop's share of moving the tiles.
-struct F32Tile { int tm, tn, cost; };
-constexpr F32Tile F32_TILES[] = {{8, 8, 64 + 6 + 4}, {8, 6, 48 + 7 + 4}, {6, 8, 48 + 5 + 4}, {6, 6, 36 + 6 + 4}, {8, 4, 32 + 5 + 3}, {6, 4, 24 + 4 + 3},
-                                 {4, 4, 16 + 3 + 3}, {2, 4, 8 + 2 + 3}};
+// Tile shapes (TM, TN) and what a k costs, in tenths of a nanosecond, measured on a B200: `loaded`, a tile's share of an SM that is full of them (1,000 rows
+// x 16,384 columns); `lone`, a tile alone on its SM, which waits for its own loads and barriers (40 rows x 2,048 columns). Between the two
+// n tiles on an SM take n * loaded + (lone - loaded) / n: within 8 % of what 40 to 1,000 rows by 2,048 to 32,768 columns measured, for every shape.
+struct F32Tile { int tm, tn; float loaded, lone; };
+constexpr F32Tile F32_TILES[] = {{8, 8, 465, 595}, {8, 6, 365, 520}, {6, 8, 390, 545}, {6, 6, 307, 440}, {8, 4, 271, 460}, {6, 4, 231, 450}, {4, 4, 190, 480}, {2, 4, 159, 340}};
 
 OXR_API int oxr_gemm_f32_nt(float* C, const float* A, const float* W, int M, int N, int K, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
@@ -218,20 +220,20 @@ OXR_API int oxr_gemm_f32_nt(float* C, const float* A, const float* W, int M, int
         gemm_f32_few_kernel<<<dim3((N + 63) / 64), 256, 0, stream>>>(C, A, W, M, N, K);
         return oxr_launch_status();
     }
-    // The SM that gets the most tiles decides: take the shape with the least (tiles of the fullest SM) x (cost of a tile). A few
-    // hundred rows make few large tiles (2,048 columns: 96 of 64 x 128 on 148 SMs), smaller ones fill the chip better.
+    // The SM that gets the most tiles decides. A few hundred rows make few large tiles (2,048 columns: 96 of 64 x 128 on 148 SMs), smaller ones fill
+    // the chip better: 100 rows x 2,048 columns, k 8,192: 297 us in tiles of 16 x 64, 425 in tiles of 32 x 64, 489 in tiles of 64 x 128.
     static int sms = 0;
     if (sms == 0) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     }
     int best = 0;
-    long long best_cost = -1;
+    float best_cost = -1.f;
     for (int i = 0; i < (int)(sizeof(F32_TILES) / sizeof(F32_TILES[0])); ++i) {
         const F32Tile& t = F32_TILES[i];
         const long long tiles = (long long)((M + 8 * t.tm - 1) / (8 * t.tm)) * ((N + 16 * t.tn - 1) / (16 * t.tn));
-        const long long cost = (tiles + sms - 1) / sms * t.cost;
-        if (best_cost < 0 || cost < best_cost) { best = i; best_cost = cost; }
+        const float n = (float)((tiles + sms - 1) / sms), cost = n * t.loaded + (t.lone - t.loaded) / n;
+        if (best_cost < 0.f || cost < best_cost) { best = i; best_cost = cost; }
     }
     switch (best) {
         case 0: return launch_f32<8, 8>(C, A, W, M, N, K, stream);
