@@ -29,6 +29,8 @@ __global__ void conv_qkv_store_kernel(
     const int* __restrict__ req_of_token, const int* __restrict__ cu_q, const int* __restrict__ state_slots,
     const int* __restrict__ positions, float temp_coef, int temp_every, const float* __restrict__ blend, const T* __restrict__ first,
     T* __restrict__ k_pool, T* __restrict__ v_pool, const int* __restrict__ slots, long long n_slots, int* status, const HeadWidths hw) {
+    pdl_wait();
+    pdl_trigger();
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
     const int t = blockIdx.x;
     const int channels = cq + ck + cv;
@@ -131,6 +133,8 @@ __global__ void conv_qkv_store_bf16x8_kernel(
     const int* __restrict__ req_of_token, const int* __restrict__ cu_q, const int* __restrict__ state_slots, const int* __restrict__ positions,
     float temp_coef, int temp_every, const float* __restrict__ blend, const __nv_bfloat16* __restrict__ first, __nv_bfloat16* __restrict__ k_pool,
     __nv_bfloat16* __restrict__ v_pool, const int* __restrict__ slots, long long n_slots, int* status, const HeadWidths hw) {
+    pdl_wait();
+    pdl_trigger();
     // a block: 8 neighbouring tokens (one per warp) x 256 channels (8 per lane), so that the rows a token shares with its neighbours
     // come out of this SM's L1
     const int c = (blockIdx.y * 32 + (threadIdx.x & 31)) * 8;
@@ -202,6 +206,8 @@ __global__ void __launch_bounds__(256) conv_qkv_store_bf16x8_window_kernel(
     const int* __restrict__ req_of_token, const int* __restrict__ cu_q, const int* __restrict__ state_slots, const int* __restrict__ positions,
     float temp_coef, int temp_every, const float* __restrict__ blend, const __nv_bfloat16* __restrict__ first, __nv_bfloat16* __restrict__ k_pool,
     __nv_bfloat16* __restrict__ v_pool, const int* __restrict__ slots, long long n_slots, int* status, const HeadWidths hw) {
+    pdl_wait();
+    pdl_trigger();
     const int c = (blockIdx.y * 32 + (threadIdx.x & 31)) * 8;
     const int t0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * TOK;
     const int channels = cq + ck + cv;
@@ -279,6 +285,8 @@ __global__ void __launch_bounds__(256) conv_qkv_store_bf16x8_window_kernel(
 template <typename T>
 __global__ void conv_qkv_roll_kernel(float* __restrict__ tails, long long slot_stride, const T* __restrict__ proj, int proj_stride, int channels,
                                      int taps, const float* __restrict__ bias, const int* __restrict__ cu_q, const int* __restrict__ state_slots) {
+    pdl_wait();
+    pdl_trigger();
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
     const int r = blockIdx.x;
     if (c >= channels) return;
@@ -309,11 +317,11 @@ OXR_API int oxr_conv_qkv_store(void* q_out, void* v_out, const void* proj, int n
     if (grid.y > 65535) return OXR_BAD_ARGUMENT;
 #define OXR_CONV_QKV(T) \
     do { \
-        conv_qkv_store_kernel<T><<<grid, threads, 0, stream>>>((T*)q_out, (T*)v_out, (const T*)proj, proj_stride, cq, ck, cv, taps, w, bias, tails, \
+        oxr_launch_small(conv_qkv_store_kernel<T>, dim3(grid), dim3(threads), 0, stream, (T*)q_out, (T*)v_out, (const T*)proj, proj_stride, cq, ck, cv, taps, w, bias, tails, \
                                                               slot_stride, req_of_token, cu_q, state_slots, positions, temp_coef, temp_every, blend, \
                                                               (const T*)first, (T*)k_pool, (T*)v_pool, slots, n_slots, status, hw); \
         if (taps > 1) \
-            conv_qkv_roll_kernel<T><<<roll, threads, 0, stream>>>(tails, slot_stride, (const T*)proj, proj_stride, channels, taps, bias, cu_q, \
+            oxr_launch_small(conv_qkv_roll_kernel<T>, dim3(roll), dim3(threads), 0, stream, tails, slot_stride, (const T*)proj, proj_stride, channels, taps, bias, cu_q, \
                                                                  state_slots); \
     } while (0)
     const auto aligned = [](const void* p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
@@ -323,11 +331,11 @@ OXR_API int oxr_conv_qkv_store(void* q_out, void* v_out, const void* proj, int n
         dim3 vgrid((n_tokens + 7) / 8, (channels / 8 + 31) / 32);
         const bool single = n_tokens == n_requests && single_tokens;
 #define OXR_CONV_QKV8(ROLL) \
-        conv_qkv_store_bf16x8_kernel<ROLL><<<vgrid, 256, 0, stream>>>((B*)q_out, (B*)v_out, (const B*)proj, n_tokens, proj_stride, cq, ck, cv, taps, wt, bias, \
+        oxr_launch_small(conv_qkv_store_bf16x8_kernel<ROLL>, dim3(vgrid), dim3(256), 0, stream, (B*)q_out, (B*)v_out, (const B*)proj, n_tokens, proj_stride, cq, ck, cv, taps, wt, bias, \
                                                                          tails, slot_stride, req_of_token, cu_q, state_slots, positions, temp_coef, \
                                                                          temp_every, blend, (const B*)first, (B*)k_pool, (B*)v_pool, slots, n_slots, status, hw)
 #define OXR_CONV_QKV8W(TAPS) \
-        conv_qkv_store_bf16x8_window_kernel<TAPS, 8><<<dim3((n_tokens + 63) / 64, (channels / 8 + 31) / 32), 256, 0, stream>>>( \
+        oxr_launch_small(conv_qkv_store_bf16x8_window_kernel<TAPS, 8>, dim3((n_tokens + 63) / 64, (channels / 8 + 31) / 32), dim3(256), 0, stream,  \
             (B*)q_out, (B*)v_out, (const B*)proj, n_tokens, proj_stride, cq, ck, cv, wt, bias, tails, slot_stride, req_of_token, cu_q, state_slots, \
             positions, temp_coef, temp_every, blend, (const B*)first, (B*)k_pool, (B*)v_pool, slots, n_slots, status, hw)
         if (single) {
@@ -338,7 +346,7 @@ OXR_API int oxr_conv_qkv_store(void* q_out, void* v_out, const void* proj, int n
             else if (taps == 4 && n_tokens >= 64) OXR_CONV_QKV8W(4);
             else OXR_CONV_QKV8(false);
             if (taps > 1)
-                conv_qkv_roll_kernel<B><<<roll, threads, 0, stream>>>(tails, slot_stride, (const B*)proj, proj_stride, channels, taps, bias, cu_q, state_slots);
+                oxr_launch_small(conv_qkv_roll_kernel<B>, dim3(roll), dim3(threads), 0, stream, tails, slot_stride, (const B*)proj, proj_stride, channels, taps, bias, cu_q, state_slots);
         }
 #undef OXR_CONV_QKV8W
 #undef OXR_CONV_QKV8
@@ -353,6 +361,8 @@ OXR_API int oxr_conv_qkv_store(void* q_out, void* v_out, const void* proj, int n
 // x[t, c] += row[c] in place, the sum in fp32
 template <typename T>
 __global__ void add_bias_kernel(T* __restrict__ x, const float* __restrict__ row, size_t total, int width) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < total) x[i] = Num<T>::from_f32(Num<T>::to_f32(x[i]) + row[i % width]);
 }
@@ -362,18 +372,20 @@ OXR_API int oxr_add_bias(void* x, const float* row, int n, int width, int dtype,
     if (width <= 0) return OXR_BAD_ARGUMENT;
     const size_t total = (size_t)n * width;
     const unsigned blocks = (unsigned)((total + 255) / 256);
-    if (dtype == 0) add_bias_kernel<float><<<blocks, 256, 0, stream>>>((float*)x, row, total, width);
-    else add_bias_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((__nv_bfloat16*)x, row, total, width);
+    if (dtype == 0) oxr_launch_small(add_bias_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)x, row, total, width);
+    else oxr_launch_small(add_bias_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (__nv_bfloat16*)x, row, total, width);
     return oxr_launch_status();
 }
 
 __global__ void scale_f32_kernel(float* __restrict__ x, float scale, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < total) x[i] *= scale;
 }
 
 OXR_API int oxr_scale_f32(float* x, float scale, long long total, cudaStream_t stream) {
     if (total <= 0) return 0;
-    scale_f32_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(x, scale, (size_t)total);
+    oxr_launch_small(scale_f32_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, x, scale, (size_t)total);
     return oxr_launch_status();
 }

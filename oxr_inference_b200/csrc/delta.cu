@@ -71,6 +71,7 @@ template <int N> __device__ __forceinline__ void delta_columns(const float* p, f
 
 template <typename T, int J, int KW>
 __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delta_scan_kernel(float* __restrict__ y, const T* __restrict__ proj, const DeltaArgs a) {
+    pdl_wait();
     using Sh = DeltaShape<J, KW>;
     constexpr int DKP = Sh::DKP, CPT = Sh::CPT, KL = (DKP + 31) / 32;      // KL: key entries per lane when a warp prepares a token
     extern __shared__ __align__(16) float dsm[];      // [2][TILE], then the results [2][TT][COLS]
@@ -335,6 +336,8 @@ __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delt
 // shared memory; every group of lanes prepares the token's vectors for its own key entries. grid (columns / 32, heads, requests).
 template <typename T, int J, int KW>
 __global__ void __launch_bounds__(32 * DELTA_WARPS) delta_step_kernel(float* __restrict__ y, const T* __restrict__ proj, const DeltaArgs a) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int CPT = DeltaShape<J, KW>::CPT;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane % J, c0 = (warp * (32 / J) + lane / J) * CPT;
     const int p0 = blockIdx.x * DELTA_COLS + c0, h = blockIdx.y, r = blockIdx.z, DK = a.DK, DV = a.DV;
@@ -428,7 +431,7 @@ static int delta_launch(float* y, const T* proj, const DeltaArgs& a, int n_reque
     using Sh = DeltaShape<J, KW>;
     const dim3 grid((a.DV + DELTA_COLS - 1) / DELTA_COLS, a.heads, n_requests);
     if (single) {
-        delta_step_kernel<T, J, KW><<<grid, 32 * DELTA_WARPS, 0, stream>>>(y, proj, a);
+        oxr_launch(delta_step_kernel<T, J, KW>, dim3(grid), dim3(32 * DELTA_WARPS), 0, stream, false, y, proj, a);
         return oxr_launch_status();
     }
     constexpr size_t SMEM = Sh::template SMEM<T>;
@@ -437,7 +440,7 @@ static int delta_launch(float* y, const T* proj, const DeltaArgs& a, int n_reque
         cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<T, J, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
         if (e != cudaSuccess) return 1000 + (int)e;
     }
-    delta_scan_kernel<T, J, KW><<<grid, 32 * (DELTA_WARPS + DELTA_PREP_WARPS), SMEM, stream>>>(y, proj, a);
+    oxr_launch(delta_scan_kernel<T, J, KW>, dim3(grid), dim3(32 * (DELTA_WARPS + DELTA_PREP_WARPS)), SMEM, stream, false, y, proj, a);
     return oxr_launch_status();
 }
 
@@ -470,6 +473,8 @@ OXR_API int oxr_delta_scan(float* y, const void* proj, int n_requests, int strid
 // out[t, c] = tanh(z[t, col0 + c]), evaluated in fp32 and rounded once: the activation inside a low-rank map whose first half left fp32.
 template <typename T>
 __global__ void tanh_cols_kernel(T* __restrict__ out, const float* __restrict__ z, int stride, int col0, int width, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t t = i / width;
@@ -481,7 +486,7 @@ OXR_API int oxr_tanh_cols(void* out, const float* z, int n, int stride, int col0
     if (width <= 0 || col0 < 0 || col0 + width > stride) return OXR_BAD_ARGUMENT;
     const size_t total = (size_t)n * width;
     const unsigned blocks = (unsigned)((total + 127) / 128);
-    if (dtype == 0) tanh_cols_kernel<float><<<blocks, 128, 0, stream>>>((float*)out, z, stride, col0, width, total);
-    else tanh_cols_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>((__nv_bfloat16*)out, z, stride, col0, width, total);
+    if (dtype == 0) oxr_launch_small(tanh_cols_kernel<float>, dim3(blocks), dim3(128), 0, stream, (float*)out, z, stride, col0, width, total);
+    else oxr_launch_small(tanh_cols_kernel<__nv_bfloat16>, dim3(blocks), dim3(128), 0, stream, (__nv_bfloat16*)out, z, stride, col0, width, total);
     return oxr_launch_status();
 }

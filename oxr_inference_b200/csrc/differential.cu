@@ -49,6 +49,8 @@ template <> struct DiffWord<__nv_bfloat16, 8> {
 template <typename T, int VEC>
 __global__ void __launch_bounds__(128) diff_prep_kernel(T* __restrict__ q_out, T* __restrict__ k_pool, T* __restrict__ v_pool, const T* __restrict__ proj,
                                                         const DiffArgs a) {
+    pdl_wait();
+    pdl_trigger();
     const int t = blockIdx.y;
     int i = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
     const int q_cols = 2 * a.H * a.W, k_cols = 2 * a.G * a.D, v_cols = a.G * a.DV;
@@ -106,12 +108,12 @@ OXR_API int oxr_diff_prep(void* q_out, void* k_pool, void* v_pool, const void* p
     const bool words = dtype == 1 && D % 8 == 0 && DV % 8 == 0 && W % 8 == 0 && WV % 8 == 0 && stride % 8 == 0 && q_col0 % 8 == 0 && k_col0 % 8 == 0 &&
                        v_col0 % 8 == 0 && (uintptr_t)proj % 16 == 0 && (uintptr_t)q_out % 16 == 0 && (uintptr_t)k_pool % 16 == 0 && (uintptr_t)v_pool % 16 == 0;
     if (words)
-        diff_prep_kernel<__nv_bfloat16, 8><<<dim3((cols / 8 + 127) / 128, n_tokens), 128, 0, stream>>>((__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool,
+        oxr_launch_small(diff_prep_kernel<__nv_bfloat16, 8>, dim3((cols / 8 + 127) / 128, n_tokens), dim3(128), 0, stream, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool,
                                                                                                       (__nv_bfloat16*)v_pool, (const __nv_bfloat16*)proj, a);
     else if (dtype == 0)
-        diff_prep_kernel<float, 1><<<dim3((cols + 127) / 128, n_tokens), 128, 0, stream>>>((float*)q_out, (float*)k_pool, (float*)v_pool, (const float*)proj, a);
+        oxr_launch_small(diff_prep_kernel<float, 1>, dim3((cols + 127) / 128, n_tokens), dim3(128), 0, stream, (float*)q_out, (float*)k_pool, (float*)v_pool, (const float*)proj, a);
     else
-        diff_prep_kernel<__nv_bfloat16, 1><<<dim3((cols + 127) / 128, n_tokens), 128, 0, stream>>>((__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool,
+        oxr_launch_small(diff_prep_kernel<__nv_bfloat16, 1>, dim3((cols + 127) / 128, n_tokens), dim3(128), 0, stream, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool,
                                                                                                   (__nv_bfloat16*)v_pool, (const __nv_bfloat16*)proj, a);
     return oxr_launch_status();
 }
@@ -120,6 +122,8 @@ OXR_API int oxr_diff_prep(void* q_out, void* k_pool, void* v_pool, const void* p
 template <typename T, int VEC, int G>
 __global__ void __launch_bounds__(128) diff_combine_kernel(T* __restrict__ out, const T* __restrict__ o, int o_head, int H, int DV, const float* __restrict__ lambda,
                                                            float eps, float factor, int n_tokens) {
+    pdl_wait();
+    pdl_trigger();
     const int l = threadIdx.x % G;
     const long long at = (long long)blockIdx.x * (128 / G) + threadIdx.x / G;
     const bool live = at < (long long)n_tokens * H;      // the others walk along: the sums are for whole warps
@@ -184,7 +188,7 @@ OXR_API int oxr_diff_combine(void* out, const void* o, int n_tokens, int o_head,
     if (H <= 0 || DV <= 0 || o_head < DV) return OXR_BAD_ARGUMENT;
     const long long total = (long long)n_tokens * H;
 #define OXR_COMBINE(T, VEC, G) \
-    diff_combine_kernel<T, VEC, G><<<(unsigned)((total + 128 / G - 1) / (128 / G)), 128, 0, stream>>>((T*)out, (const T*)o, o_head, H, DV, lambda, eps, factor, n_tokens)
+    oxr_launch_small(diff_combine_kernel<T, VEC, G>, dim3((unsigned)((total + 128 / G - 1) / (128 / G))), dim3(128), 0, stream, (T*)out, (const T*)o, o_head, H, DV, lambda, eps, factor, n_tokens)
     if (dtype == 1 && DV % 8 == 0 && o_head % 8 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)o % 16 == 0) {
         // two words a lane where a head has that many
         if (DV <= 128) OXR_COMBINE(__nv_bfloat16, 8, 8);

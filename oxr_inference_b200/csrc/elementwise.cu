@@ -11,6 +11,8 @@ OXR_TL_DEFINE(oxr_tl_read_elem)
 template <typename TT, typename TO>
 __global__ void embedding_kernel(TO* __restrict__ out, const TT* __restrict__ table, const int* __restrict__ ids,
                                  int hidden, int vocab, float scale, int* status) {
+    pdl_wait();
+    pdl_trigger();
     const int t = blockIdx.x;
     const int id = ids[t];
     TO* dst = out + (size_t)t * hidden;
@@ -27,6 +29,8 @@ __global__ void embedding_kernel(TO* __restrict__ out, const TT* __restrict__ ta
 template <typename T>
 __global__ void embedding_vec_kernel(T* __restrict__ out, const T* __restrict__ table, const int* __restrict__ ids,
                                      int words_per_row, int vocab, int* status) {
+    pdl_wait();
+    pdl_trigger();
     const int t = blockIdx.x;
     const int id = ids[t];
     uint4* dst = reinterpret_cast<uint4*>(out) + (size_t)t * words_per_row;
@@ -43,6 +47,8 @@ __global__ void embedding_vec_kernel(T* __restrict__ out, const T* __restrict__ 
 // 2,048 rows 19; here 2.6 and 12.
 __global__ void embedding_widen_kernel(float* __restrict__ out, const uint4* __restrict__ table, const int* __restrict__ ids, int words_per_row, int vocab,
                                        float scale, int* status) {
+    pdl_wait();
+    pdl_trigger();
     const int t = blockIdx.x;
     const int id = ids[t];
     float4* dst = reinterpret_cast<float4*>(out) + (size_t)t * words_per_row * 2;
@@ -101,6 +107,8 @@ template <typename T>
 __global__ void add_rms_norm_kernel(T* __restrict__ out, float* __restrict__ residual_out, const T* __restrict__ x,
                                     const float* __restrict__ residual_in, const float* __restrict__ weight,
                                     const int* __restrict__ rows, int hidden, float eps, int row_floats_in_smem) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ float smem[];
     float* red = smem;            // 32 floats
     float* rowbuf = smem + 32;    // row_floats_in_smem floats
@@ -233,9 +241,9 @@ OXR_API int oxr_add_rms_norm(void* out, float* residual_out, const void* x, cons
     const int cache_floats = hidden <= 10240 ? hidden : 0;   // 40 KB of row cache at most
     const size_t smem = (32 + cache_floats) * sizeof(float);
     if (dtype == 0)
-        add_rms_norm_kernel<float><<<n_rows, threads, smem, stream>>>((float*)out, residual_out, (const float*)x, residual_in, weight, rows, hidden, eps, cache_floats);
+        oxr_launch_small(add_rms_norm_kernel<float>, dim3(n_rows), dim3(threads), smem, stream, (float*)out, residual_out, (const float*)x, residual_in, weight, rows, hidden, eps, cache_floats);
     else if (dtype == 1)
-        add_rms_norm_kernel<__nv_bfloat16><<<n_rows, threads, smem, stream>>>((__nv_bfloat16*)out, residual_out, (const __nv_bfloat16*)x, residual_in, weight, rows, hidden, eps, cache_floats);
+        oxr_launch_small(add_rms_norm_kernel<__nv_bfloat16>, dim3(n_rows), dim3(threads), smem, stream, (__nv_bfloat16*)out, residual_out, (const __nv_bfloat16*)x, residual_in, weight, rows, hidden, eps, cache_floats);
     else
         return OXR_BAD_ARGUMENT;
     return oxr_launch_status();
@@ -257,6 +265,8 @@ __device__ __forceinline__ void gate_up_at(size_t row, size_t col, int inter, in
 }
 template <typename T>
 __global__ void silu_mul_kernel(T* __restrict__ out, const T* __restrict__ gate_up, int inter, int interleave, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         size_t gi, ui;
         gate_up_at(i / inter, i % inter, inter, interleave, gi, ui);
@@ -267,6 +277,8 @@ __global__ void silu_mul_kernel(T* __restrict__ out, const T* __restrict__ gate_
 }
 template <>
 __global__ void silu_mul_kernel<float>(float* __restrict__ out, const float* __restrict__ gate_up, int inter, int interleave, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         size_t gi, ui;
         gate_up_at(i / inter, i % inter, inter, interleave, gi, ui);
@@ -280,6 +292,8 @@ __global__ void silu_mul_kernel<float>(float* __restrict__ out, const float* __r
 // With INTERLEAVED the gate word of output word `col` is word 2 col of the row and its up word the next one.
 template <bool INTERLEAVED>
 __global__ void silu_mul_bf16x8_kernel(uint4* __restrict__ out, const uint4* __restrict__ gate_up, int inter8) {
+    pdl_wait();
+    pdl_trigger();
     const size_t row = blockIdx.y;
     const uint4* g_row = gate_up + row * 2 * inter8;
     uint4* o_row = out + row * inter8;
@@ -316,17 +330,17 @@ OXR_API int oxr_silu_mul(void* out, const void* gate_up, int n_rows, int inter, 
             dim3 grid((inter8 + threads - 1) / threads, rows);
             uint4* o = (uint4*)out + (size_t)rows_done * inter8;
             const uint4* gu = (const uint4*)gate_up + (size_t)rows_done * 2 * inter8;
-            if (interleave) silu_mul_bf16x8_kernel<true><<<grid, threads, 0, stream>>>(o, gu, inter8);
-            else silu_mul_bf16x8_kernel<false><<<grid, threads, 0, stream>>>(o, gu, inter8);
+            if (interleave) oxr_launch_small(silu_mul_bf16x8_kernel<true>, dim3(grid), dim3(threads), 0, stream, o, gu, inter8);
+            else oxr_launch_small(silu_mul_bf16x8_kernel<false>, dim3(grid), dim3(threads), 0, stream, o, gu, inter8);
             rows_done += rows;
         }
         return oxr_launch_status();
     }
     const int blocks = (int)((total + threads - 1) / threads < 148 * 16 ? (total + threads - 1) / threads : 148 * 16);
     if (dtype == 0)
-        silu_mul_kernel<float><<<blocks, threads, 0, stream>>>((float*)out, (const float*)gate_up, inter, interleave, total);
+        oxr_launch_small(silu_mul_kernel<float>, dim3(blocks), dim3(threads), 0, stream, (float*)out, (const float*)gate_up, inter, interleave, total);
     else if (dtype == 1)
-        silu_mul_kernel<__nv_bfloat16><<<blocks, threads, 0, stream>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)gate_up, inter, interleave, total);
+        oxr_launch_small(silu_mul_kernel<__nv_bfloat16>, dim3(blocks), dim3(threads), 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)gate_up, inter, interleave, total);
     else
         return OXR_BAD_ARGUMENT;
     return oxr_launch_status();
@@ -335,6 +349,8 @@ OXR_API int oxr_silu_mul(void* out, const void* gate_up, int n_rows, int inter, 
 // ---------------------------------------------------------------------------------------------- casts
 template <typename TS, typename TD>
 __global__ void cast_kernel(TD* __restrict__ dst, const TS* __restrict__ src, size_t n) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         dst[i] = Num<TD>::from_f32(Num<TS>::to_f32(src[i]));
 }
@@ -344,9 +360,9 @@ OXR_API int oxr_cast(void* dst, const void* src, size_t n, int src_dtype, int ds
     const int threads = 256;
     const int blocks = (int)((n + threads - 1) / threads < 148 * 16 ? (n + threads - 1) / threads : 148 * 16);
     if (src_dtype == 0 && dst_dtype == 1)
-        cast_kernel<float, __nv_bfloat16><<<blocks, threads, 0, stream>>>((__nv_bfloat16*)dst, (const float*)src, n);
+        oxr_launch_small(cast_kernel<float, __nv_bfloat16>, dim3(blocks), dim3(threads), 0, stream, (__nv_bfloat16*)dst, (const float*)src, n);
     else if (src_dtype == 1 && dst_dtype == 0)
-        cast_kernel<__nv_bfloat16, float><<<blocks, threads, 0, stream>>>((float*)dst, (const __nv_bfloat16*)src, n);
+        oxr_launch_small(cast_kernel<__nv_bfloat16, float>, dim3(blocks), dim3(threads), 0, stream, (float*)dst, (const __nv_bfloat16*)src, n);
     else
         return OXR_BAD_ARGUMENT;
     return oxr_launch_status();

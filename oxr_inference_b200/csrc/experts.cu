@@ -26,6 +26,8 @@ constexpr int ROUTE_MAX_GROUPS = 64;
 __global__ void route_kernel(float* __restrict__ gate, int* __restrict__ ids, float* __restrict__ wts, const float* __restrict__ z, int n_tokens,
                              int E, int top, int groups, int keep, float scale, int score_kind, int group_kind, int renorm, const float* __restrict__ correction,
                              int real, float* __restrict__ kept, const float* __restrict__ bias) {
+    pdl_wait();
+    pdl_trigger();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n_tokens) return;
     auto logit = [&](int e) { return bias != nullptr ? z[(size_t)t * E + e] + bias[e] : z[(size_t)t * E + e]; };
@@ -112,6 +114,8 @@ __global__ void __launch_bounds__(128) route_warp_kernel(float* __restrict__ gat
                                                         int n_tokens, int E, int top, int groups, int keep, float scale, int score_kind,
                                                         int group_kind, int renorm, const float* __restrict__ correction, int real,
                                                         float* __restrict__ kept, const float* __restrict__ bias) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float sc[4][ROUTE_WARP_MAX_E], ch[4][ROUTE_WARP_MAX_E];     // scores, choice scores
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.x * 4 + warp;
@@ -197,15 +201,17 @@ OXR_API int oxr_route(float* gate, int* ids, float* wts, const float* z, int n_t
         top > keep * (E / groups) || score_kind < 0 || score_kind > 2 || (score_kind == 2 && (!renorm || correction != nullptr)) || group_kind < 0 || group_kind > 1)
         return OXR_BAD_ARGUMENT;
     if (E <= ROUTE_WARP_MAX_E && groups <= 32)
-        route_warp_kernel<<<(n_tokens + 3) / 4, 128, 0, stream>>>(gate, ids, wts, z, n_tokens, E, top, groups, keep, scale, score_kind, group_kind, renorm, correction, real, kept, bias);
+        oxr_launch_small(route_warp_kernel, dim3((n_tokens + 3) / 4), dim3(128), 0, stream, gate, ids, wts, z, n_tokens, E, top, groups, keep, scale, score_kind, group_kind, renorm, correction, real, kept, bias);
     else
-        route_kernel<<<(n_tokens + 63) / 64, 64, 0, stream>>>(gate, ids, wts, z, n_tokens, E, top, groups, keep, scale, score_kind, group_kind, renorm, correction, real, kept, bias);
+        oxr_launch_small(route_kernel, dim3((n_tokens + 63) / 64), dim3(64), 0, stream, gate, ids, wts, z, n_tokens, E, top, groups, keep, scale, score_kind, group_kind, renorm, correction, real, kept, bias);
     return oxr_launch_status();
 }
 
 // a[t, c] = gate[t, c / ff] * relu(u[t, c])^2 over the stacked columns of all experts; the product in fp32, rounded once.
 template <typename T>
 __global__ void gated_relu2_kernel(T* __restrict__ a, const T* __restrict__ u, const float* __restrict__ gate, size_t total, int cols, int ff, int E) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t t = i / cols;
@@ -218,6 +224,8 @@ __global__ void gated_relu2_kernel(T* __restrict__ a, const T* __restrict__ u, c
 // the same for bfloat16 with 16-byte accesses: 8 neighbouring columns of one expert (ff a multiple of 8)
 __global__ void gated_relu2_bf16x8_kernel(__nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ u, const float* __restrict__ gate,
                                           size_t total8, int cols, int ff, int E) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i8 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i8 >= total8) return;
     const size_t i = i8 * 8, t = i / cols;
@@ -240,13 +248,13 @@ OXR_API int oxr_gated_relu2(void* a, const void* u, const float* gate, int n_tok
     if (E <= 0 || ff <= 0) return OXR_BAD_ARGUMENT;
     const size_t total = (size_t)n_tokens * E * ff;
     if (dtype == 1 && ff % 8 == 0 && (uintptr_t)a % 16 == 0 && (uintptr_t)u % 16 == 0) {
-        gated_relu2_bf16x8_kernel<<<(unsigned)((total / 8 + 255) / 256), 256, 0, stream>>>((__nv_bfloat16*)a, (const __nv_bfloat16*)u, gate, total / 8,
+        oxr_launch_small(gated_relu2_bf16x8_kernel, dim3((unsigned)((total / 8 + 255) / 256)), dim3(256), 0, stream, (__nv_bfloat16*)a, (const __nv_bfloat16*)u, gate, total / 8,
                                                                                             E * ff, ff, E);
         return oxr_launch_status();
     }
     const unsigned blocks = (unsigned)((total + 255) / 256);
-    if (dtype == 0) gated_relu2_kernel<float><<<blocks, 256, 0, stream>>>((float*)a, (const float*)u, gate, total, E * ff, ff, E);
-    else gated_relu2_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((__nv_bfloat16*)a, (const __nv_bfloat16*)u, gate, total, E * ff, ff, E);
+    if (dtype == 0) oxr_launch_small(gated_relu2_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)a, (const float*)u, gate, total, E * ff, ff, E);
+    else oxr_launch_small(gated_relu2_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (__nv_bfloat16*)a, (const __nv_bfloat16*)u, gate, total, E * ff, ff, E);
     return oxr_launch_status();
 }
 
@@ -255,6 +263,8 @@ OXR_API int oxr_gated_relu2(void* a, const void* u, const float* gate, int n_tok
 template <typename T>
 __global__ void expert_clamped_glu_kernel(T* __restrict__ a, const T* __restrict__ gu, const float* __restrict__ gate_w, size_t total, int ff, int E,
                                           float alpha, float limit) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const int cols = E * ff;
@@ -273,8 +283,8 @@ OXR_API int oxr_expert_clamped_glu(void* a, const void* gu, const float* gate_w,
     if (E <= 0 || ff <= 0) return OXR_BAD_ARGUMENT;
     const size_t total = (size_t)n_tokens * E * ff;
     const unsigned blocks = (unsigned)((total + 255) / 256);
-    if (dtype == 0) expert_clamped_glu_kernel<float><<<blocks, 256, 0, stream>>>((float*)a, (const float*)gu, gate_w, total, ff, E, alpha, limit);
-    else expert_clamped_glu_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((__nv_bfloat16*)a, (const __nv_bfloat16*)gu, gate_w, total, ff, E, alpha, limit);
+    if (dtype == 0) oxr_launch_small(expert_clamped_glu_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)a, (const float*)gu, gate_w, total, ff, E, alpha, limit);
+    else oxr_launch_small(expert_clamped_glu_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (__nv_bfloat16*)a, (const __nv_bfloat16*)gu, gate_w, total, ff, E, alpha, limit);
     return oxr_launch_status();
 }
 
@@ -287,6 +297,8 @@ constexpr int SORT_MAX_EXPERTS = 1024;
 __global__ void __launch_bounds__(1024) expert_sort_kernel(int* __restrict__ counts, int* __restrict__ order, int* __restrict__ place,
                                                           int* __restrict__ tile_group, const int* __restrict__ ids, int total, int E, int pad,
                                                           int capacity) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int hist[SORT_MAX_EXPERTS], cursor[SORT_MAX_EXPERTS];
     for (int e = threadIdx.x; e < E; e += blockDim.x) hist[e] = 0;
     for (int i = threadIdx.x; i < capacity; i += blockDim.x) order[i] = -1;
@@ -328,13 +340,15 @@ OXR_API int oxr_expert_sort(int* counts, int* order, int* place, int* tile_group
                             cudaStream_t stream) {
     if (total <= 0) return 0;
     if (E <= 0 || E > SORT_MAX_EXPERTS || pad <= 0 || capacity % pad != 0 || capacity < total + (pad > 1 ? E * (pad - 1) : 0)) return OXR_BAD_ARGUMENT;
-    expert_sort_kernel<<<1, 1024, 0, stream>>>(counts, order, place, tile_group, ids, total, E, pad, capacity);
+    oxr_launch_small(expert_sort_kernel, dim3(1), dim3(1024), 0, stream, counts, order, place, tile_group, ids, total, E, pad, capacity);
     return oxr_launch_status();
 }
 
 // out[i] = x[order[i] / per_row] (zeros where order[i] is -1): 16-byte copies where the rows allow them
 template <typename T>
 __global__ void gather_rows_kernel(T* __restrict__ out, const T* __restrict__ x, const int* __restrict__ order, int width, int per_row) {
+    pdl_wait();
+    pdl_trigger();
     const int from = order[blockIdx.x];          // -1: a padding place, filled with zeros
     const size_t dst = (size_t)blockIdx.x * width, src = (size_t)(from < 0 ? 0 : from / per_row) * width;
     if (from < 0) {
@@ -354,8 +368,8 @@ __global__ void gather_rows_kernel(T* __restrict__ out, const T* __restrict__ x,
 OXR_API int oxr_gather_rows(void* out, const void* x, const int* order, int rows, int width, int per_row, int dtype, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (width <= 0 || per_row <= 0) return OXR_BAD_ARGUMENT;
-    if (dtype == 0) gather_rows_kernel<float><<<rows, 128, 0, stream>>>((float*)out, (const float*)x, order, width, per_row);
-    else gather_rows_kernel<__nv_bfloat16><<<rows, 128, 0, stream>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)x, order, width, per_row);
+    if (dtype == 0) oxr_launch_small(gather_rows_kernel<float>, dim3(rows), dim3(128), 0, stream, (float*)out, (const float*)x, order, width, per_row);
+    else oxr_launch_small(gather_rows_kernel<__nv_bfloat16>, dim3(rows), dim3(128), 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)x, order, width, per_row);
     return oxr_launch_status();
 }
 
@@ -364,6 +378,8 @@ OXR_API int oxr_gather_rows(void* out, const void* x, const int* order, int rows
 template <typename T>
 __global__ void combine_rows_kernel(T* __restrict__ out, const T* __restrict__ y, const int* __restrict__ place, const float* __restrict__ weights,
                                     int top, int width, const T* __restrict__ x, const float* __restrict__ kept) {
+    pdl_wait();
+    pdl_trigger();
     const int t = blockIdx.x;
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
         float acc = 0.f;
@@ -380,8 +396,8 @@ OXR_API int oxr_combine_rows(void* out, const void* y, const int* place, const f
                              int dtype, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (top <= 0 || width <= 0) return OXR_BAD_ARGUMENT;
-    if (dtype == 0) combine_rows_kernel<float><<<n_tokens, 256, 0, stream>>>((float*)out, (const float*)y, place, weights, top, width, (const float*)x, kept);
-    else combine_rows_kernel<__nv_bfloat16><<<n_tokens, 256, 0, stream>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)y, place, weights, top, width, (const __nv_bfloat16*)x, kept);
+    if (dtype == 0) oxr_launch_small(combine_rows_kernel<float>, dim3(n_tokens), dim3(256), 0, stream, (float*)out, (const float*)y, place, weights, top, width, (const float*)x, kept);
+    else oxr_launch_small(combine_rows_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(256), 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)y, place, weights, top, width, (const __nv_bfloat16*)x, kept);
     return oxr_launch_status();
 }
 
@@ -393,6 +409,8 @@ OXR_API int oxr_combine_rows(void* out, const void* y, const int* place, const f
 template <typename T>
 __global__ void expert_silu_glu_kernel(T* __restrict__ a, const T* __restrict__ gu, const float* __restrict__ gate_w, size_t total, int ff, int E,
                                        int on_input) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const int cols = E * ff;
@@ -414,6 +432,8 @@ __global__ void expert_silu_glu_kernel(T* __restrict__ a, const T* __restrict__ 
 // The same for bf16 and expert widths that are whole 16-byte words: eight columns of one expert per thread.
 __global__ void expert_silu_glu_bf16x8_kernel(__nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ gu, const float* __restrict__ gate_w,
                                               size_t words, int ff, int E, int on_input) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= words) return;
     const int cols = E * ff, per_row = cols / 8;
@@ -445,11 +465,11 @@ OXR_API int oxr_expert_silu_glu(void* a, const void* gu, const float* gate_w, in
     const unsigned blocks = (unsigned)((total + 255) / 256);
     if (dtype == 1 && ff % 8 == 0 && (uintptr_t)a % 16 == 0 && (uintptr_t)gu % 16 == 0) {
         const size_t words = total / 8;
-        expert_silu_glu_bf16x8_kernel<<<(unsigned)((words + 255) / 256), 256, 0, stream>>>((__nv_bfloat16*)a, (const __nv_bfloat16*)gu, gate_w, words, ff, E, on_input);
+        oxr_launch_small(expert_silu_glu_bf16x8_kernel, dim3((unsigned)((words + 255) / 256)), dim3(256), 0, stream, (__nv_bfloat16*)a, (const __nv_bfloat16*)gu, gate_w, words, ff, E, on_input);
         return oxr_launch_status();
     }
-    if (dtype == 0) expert_silu_glu_kernel<float><<<blocks, 256, 0, stream>>>((float*)a, (const float*)gu, gate_w, total, ff, E, on_input);
-    else expert_silu_glu_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((__nv_bfloat16*)a, (const __nv_bfloat16*)gu, gate_w, total, ff, E, on_input);
+    if (dtype == 0) oxr_launch_small(expert_silu_glu_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)a, (const float*)gu, gate_w, total, ff, E, on_input);
+    else oxr_launch_small(expert_silu_glu_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (__nv_bfloat16*)a, (const __nv_bfloat16*)gu, gate_w, total, ff, E, on_input);
     return oxr_launch_status();
 }
 
@@ -457,6 +477,8 @@ OXR_API int oxr_expert_silu_glu(void* a, const void* gu, const float* gate_w, in
 // rounded once). One block per pair.
 template <typename T>
 __global__ void scale_placed_rows_kernel(T* __restrict__ x, const int* __restrict__ place, const float* __restrict__ weights, int hidden) {
+    pdl_wait();
+    pdl_trigger();
     const int row = place[blockIdx.x];
     if (row < 0) return;
     const float w = weights[blockIdx.x];
@@ -467,8 +489,8 @@ __global__ void scale_placed_rows_kernel(T* __restrict__ x, const int* __restric
 OXR_API int oxr_scale_placed_rows(void* x, const int* place, const float* weights, int pairs, int hidden, int dtype, cudaStream_t stream) {
     if (pairs <= 0) return 0;
     if (hidden <= 0) return OXR_BAD_ARGUMENT;
-    if (dtype == 0) scale_placed_rows_kernel<float><<<pairs, 128, 0, stream>>>((float*)x, place, weights, hidden);
-    else scale_placed_rows_kernel<__nv_bfloat16><<<pairs, 128, 0, stream>>>((__nv_bfloat16*)x, place, weights, hidden);
+    if (dtype == 0) oxr_launch_small(scale_placed_rows_kernel<float>, dim3(pairs), dim3(128), 0, stream, (float*)x, place, weights, hidden);
+    else oxr_launch_small(scale_placed_rows_kernel<__nv_bfloat16>, dim3(pairs), dim3(128), 0, stream, (__nv_bfloat16*)x, place, weights, hidden);
     return oxr_launch_status();
 }
 
@@ -476,6 +498,8 @@ OXR_API int oxr_scale_placed_rows(void* x, const int* place, const float* weight
 // fp32 logit) or z itself (`raw`).
 template <typename T>
 __global__ void add_row_gated_kernel(T* __restrict__ y, const T* __restrict__ s, const float* __restrict__ z, int hidden, int raw, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const float zt = z[i / hidden], g = raw ? zt : 1.f / (1.f + expf(-zt));
@@ -487,7 +511,7 @@ OXR_API int oxr_add_row_gated(void* y, const void* s, const float* z, int n, int
     if (hidden <= 0) return OXR_BAD_ARGUMENT;
     const size_t total = (size_t)n * hidden;
     const unsigned blocks = (unsigned)((total + 255) / 256);
-    if (dtype == 0) add_row_gated_kernel<float><<<blocks, 256, 0, stream>>>((float*)y, (const float*)s, z, hidden, raw, total);
-    else add_row_gated_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((__nv_bfloat16*)y, (const __nv_bfloat16*)s, z, hidden, raw, total);
+    if (dtype == 0) oxr_launch_small(add_row_gated_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)y, (const float*)s, z, hidden, raw, total);
+    else oxr_launch_small(add_row_gated_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (__nv_bfloat16*)y, (const __nv_bfloat16*)s, z, hidden, raw, total);
     return oxr_launch_status();
 }

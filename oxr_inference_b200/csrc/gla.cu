@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(32 * NW) gla_scan_kernel(
     float* __restrict__ y, const T* __restrict__ proj, int proj_stride, int q_col0, int k_col0, int v_col0, const float* __restrict__ z,
     const float* __restrict__ z_bias, float inv_tau, int heads, int DK, int DV, float q_scale, float* __restrict__ state, long long slot_stride,
     const int* __restrict__ cu_q, const int* __restrict__ state_slots) {
+    pdl_wait();
     constexpr int DKP = KPT * NW, NT = 32 * NW;      // NT >= DKP: thread d brings key entry d of every token
     __shared__ __align__(16) float ks[TT][DKP];
     __shared__ __align__(16) float qs[TT][DKP];
@@ -126,6 +127,8 @@ __global__ void __launch_bounds__(32 * NW) gla_scan_kernel(
 // decay[t, i] = sigmoid(z[t, i] + bias[i])^(1 / tau), four entries a thread: once per token and key channel, where the recurrence's blocks (one per 32 value
 // columns) would each work it out again
 __global__ void gla_decay_kernel(float4* __restrict__ decay, const float4* __restrict__ z, const float4* __restrict__ z_bias, float inv_tau, int width4, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const float4 v = z[i], b = z_bias[i % width4];
@@ -148,7 +151,7 @@ OXR_API int oxr_gla_scan(float* y, const void* proj, int n_requests, int proj_st
         a.state_slots = state_slots; a.heads = heads; a.DV = DV; a.n_requests = n_requests;
         if ((dtype == 0 ? scan_fits<float>(a, DK) : scan_fits<__nv_bfloat16>(a, DK)) && (uintptr_t)z % 16 == 0 && (uintptr_t)z_bias % 16 == 0) {
             const size_t total = (size_t)n_tokens * heads * DK / 4;
-            gla_decay_kernel<<<(unsigned)((total + 127) / 128), 128, 0, stream>>>((float4*)decay, (const float4*)z, (const float4*)z_bias, 1.f / tau,
+            oxr_launch_small(gla_decay_kernel, dim3((unsigned)((total + 127) / 128)), dim3(128), 0, stream, (float4*)decay, (const float4*)z, (const float4*)z_bias, 1.f / tau,
                                                                                  heads * DK / 4, total);
             int rc = oxr_launch_status();
             if (rc) return rc;
@@ -161,9 +164,9 @@ OXR_API int oxr_gla_scan(float* y, const void* proj, int n_requests, int proj_st
     const int nw = narrow ? (DK + 15) / 16 : (DK + 31) / 32;
 #define OXR_GLA(T, NW) \
     do { \
-        if (narrow) gla_scan_kernel<T, NW, 8, 16><<<grid, 32 * NW, 0, stream>>>(y, (const T*)proj, proj_stride, q_col0, k_col0, v_col0, z, z_bias, 1.f / tau, \
+        if (narrow) oxr_launch(gla_scan_kernel<T, NW, 8, 16>, dim3(grid), dim3(32 * NW), 0, stream, false, y, (const T*)proj, proj_stride, q_col0, k_col0, v_col0, z, z_bias, 1.f / tau, \
                                                                                 heads, DK, DV, q_scale, state, slot_stride, cu_q, state_slots); \
-        else gla_scan_kernel<T, NW, 8, 32><<<grid, 32 * NW, 0, stream>>>(y, (const T*)proj, proj_stride, q_col0, k_col0, v_col0, z, z_bias, 1.f / tau, heads, \
+        else oxr_launch(gla_scan_kernel<T, NW, 8, 32>, dim3(grid), dim3(32 * NW), 0, stream, false, y, (const T*)proj, proj_stride, q_col0, k_col0, v_col0, z, z_bias, 1.f / tau, heads, \
                                                                          DK, DV, q_scale, state, slot_stride, cu_q, state_slots); \
     } while (0)
 #define OXR_GLA_T(T) \

@@ -49,6 +49,8 @@ struct PrepArgs {
 template <typename T>
 __global__ void __launch_bounds__(128) head_prep_kernel(T* __restrict__ q_out, T* __restrict__ k_pool, T* __restrict__ v_pool,
                                                         const T* __restrict__ proj, const PrepArgs a) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ float prep_smem[];   // [warps, max(DK, DV)]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int t = blockIdx.x, head = blockIdx.y * warps + warp;
@@ -163,6 +165,8 @@ __device__ __forceinline__ float prep_head_sum(float v, int g0, int lph) {
 __global__ void __launch_bounds__(128) head_prep_bf16x8_kernel(__nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_pool,
                                                                __nv_bfloat16* __restrict__ v_pool, const __nv_bfloat16* __restrict__ proj,
                                                                const PrepArgs a, int lph, int hpw) {
+    pdl_wait();
+    pdl_trigger();
     using bf16 = __nv_bfloat16;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int t = blockIdx.x;
@@ -277,6 +281,8 @@ __global__ void __launch_bounds__(128) head_prep_bf16x8_kernel(__nv_bfloat16* __
 template <int LPH, int HPG>
 __global__ void __launch_bounds__(128, HPG == 2 ? 8 : 5) head_prep_heads_kernel(__nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_pool,
                                                               __nv_bfloat16* __restrict__ v_pool, const __nv_bfloat16* __restrict__ proj, const PrepArgs a) {
+    pdl_wait();
+    pdl_trigger();
     using bf16 = __nv_bfloat16;
     constexpr int HPW = 32 / LPH, GROUPS = 4 * HPW, DK = 8 * LPH;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -374,6 +380,8 @@ __global__ void __launch_bounds__(128, HPG == 2 ? 8 : 5) head_prep_heads_kernel(
 // (request, channel); it reads the whole old tail before it writes.
 template <typename T>
 __global__ void prep_tail_kernel(const T* __restrict__ proj, const PrepArgs a, int channels, int n_requests) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_requests * channels) return;
     const int r = i / channels, c = i % channels;
@@ -425,21 +433,21 @@ OXR_API int oxr_head_prep(void* q_out, void* k_pool, void* v_pool, const void* p
         if (taps == nullptr && n_tokens >= 64 && heads >= 2 * per_block && (lph == 8 || lph == 16)) {      // heads of 64 and of 128 entries
             dim3 hgrid(n_tokens, (heads + 2 * per_block - 1) / (2 * per_block));
 #define OXR_PREP_HEADS(LPH) \
-    head_prep_heads_kernel<LPH, 2><<<hgrid, 128, 0, stream>>>((__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, (const __nv_bfloat16*)proj, a)
+    oxr_launch_small(head_prep_heads_kernel<LPH, 2>, dim3(hgrid), dim3(128), 0, stream, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, (const __nv_bfloat16*)proj, a)
             if (lph == 8) OXR_PREP_HEADS(8);
             else OXR_PREP_HEADS(16);
 #undef OXR_PREP_HEADS
             return oxr_launch_status();
         }
-        head_prep_bf16x8_kernel<<<vgrid, 128, 0, stream>>>((__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, (const __nv_bfloat16*)proj, a, lph, hpw);
-    } else if (dtype == 0) head_prep_kernel<float><<<grid, 32 * warps, smem, stream>>>((float*)q_out, (float*)k_pool, (float*)v_pool, (const float*)proj, a);
-    else head_prep_kernel<__nv_bfloat16><<<grid, 32 * warps, smem, stream>>>((__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool,
+        oxr_launch_small(head_prep_bf16x8_kernel, dim3(vgrid), dim3(128), 0, stream, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, (const __nv_bfloat16*)proj, a, lph, hpw);
+    } else if (dtype == 0) oxr_launch_small(head_prep_kernel<float>, dim3(grid), dim3(32 * warps), smem, stream, (float*)q_out, (float*)k_pool, (float*)v_pool, (const float*)proj, a);
+    else oxr_launch_small(head_prep_kernel<__nv_bfloat16>, dim3(grid), dim3(32 * warps), smem, stream, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool,
                                                                             (const __nv_bfloat16*)proj, a);
     if (a.taps != nullptr && a.n_taps > 1) {
         const int channels = a.channels;
         const int total = n_requests * channels;
-        if (dtype == 0) prep_tail_kernel<float><<<(total + 127) / 128, 128, 0, stream>>>((const float*)proj, a, channels, n_requests);
-        else prep_tail_kernel<__nv_bfloat16><<<(total + 127) / 128, 128, 0, stream>>>((const __nv_bfloat16*)proj, a, channels, n_requests);
+        if (dtype == 0) oxr_launch_small(prep_tail_kernel<float>, dim3((total + 127) / 128), dim3(128), 0, stream, (const float*)proj, a, channels, n_requests);
+        else oxr_launch_small(prep_tail_kernel<__nv_bfloat16>, dim3((total + 127) / 128), dim3(128), 0, stream, (const __nv_bfloat16*)proj, a, channels, n_requests);
     }
     return oxr_launch_status();
 }
@@ -447,6 +455,8 @@ OXR_API int oxr_head_prep(void* q_out, void* k_pool, void* v_pool, const void* p
 // o[t, h DV + d] *= sigmoid(g[t, g_col0 + (per_head ? h : h DV + d)]) in place; the sigmoid in fp32.
 template <typename T>
 __global__ void sigmoid_gate_kernel(T* __restrict__ o, const T* __restrict__ g, int g_stride, int g_col0, int inner, int DV, int per_head, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t t = i / inner;
@@ -458,6 +468,8 @@ __global__ void sigmoid_gate_kernel(T* __restrict__ o, const T* __restrict__ g, 
 // The same for bf16 rows of whole 16-byte words: eight entries per thread (a head's entries share their gate when it is per head).
 __global__ void sigmoid_gate_bf16x8_kernel(__nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ g, int g_stride, int g_col0, int inner, int DV,
                                            int per_head, size_t words) {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= words) return;
     const int per_row = inner / 8;
@@ -485,11 +497,11 @@ OXR_API int oxr_sigmoid_gate(void* o, const void* g, int n_tokens, int g_stride,
     const unsigned blocks = (unsigned)((total + 255) / 256);
     if (dtype == 1 && inner % 8 == 0 && DV % 8 == 0 && (per_head || (g_stride % 8 == 0 && g_col0 % 8 == 0 && (uintptr_t)g % 16 == 0)) && (uintptr_t)o % 16 == 0) {
         const size_t words = total / 8;
-        sigmoid_gate_bf16x8_kernel<<<(unsigned)((words + 255) / 256), 256, 0, stream>>>((__nv_bfloat16*)o, (const __nv_bfloat16*)g, g_stride, g_col0, inner, DV,
+        oxr_launch_small(sigmoid_gate_bf16x8_kernel, dim3((unsigned)((words + 255) / 256)), dim3(256), 0, stream, (__nv_bfloat16*)o, (const __nv_bfloat16*)g, g_stride, g_col0, inner, DV,
                                                                                         per_head, words);
         return oxr_launch_status();
     }
-    if (dtype == 0) sigmoid_gate_kernel<float><<<blocks, 256, 0, stream>>>((float*)o, (const float*)g, g_stride, g_col0, inner, DV, per_head, total);
-    else sigmoid_gate_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((__nv_bfloat16*)o, (const __nv_bfloat16*)g, g_stride, g_col0, inner, DV, per_head, total);
+    if (dtype == 0) oxr_launch_small(sigmoid_gate_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)o, (const float*)g, g_stride, g_col0, inner, DV, per_head, total);
+    else oxr_launch_small(sigmoid_gate_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (__nv_bfloat16*)o, (const __nv_bfloat16*)g, g_stride, g_col0, inner, DV, per_head, total);
     return oxr_launch_status();
 }

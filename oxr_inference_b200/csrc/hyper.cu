@@ -55,6 +55,8 @@ __device__ __forceinline__ void hy_store(__nv_bfloat16* p, const float (&v)[8]) 
 // Rows of whole 8-entry words, VPT words per thread.
 template <typename T, int S, int VPT>
 __global__ void __launch_bounds__(VPT <= 2 ? 512 : 1024) hyper_words_kernel(T* __restrict__ h, const T* __restrict__ y, const HyperArgs a) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const size_t row = blockIdx.x;
     const int hidden = a.hidden, nvec = hidden / 8;
@@ -123,6 +125,8 @@ __global__ void __launch_bounds__(VPT <= 2 ? 512 : 1024) hyper_words_kernel(T* _
 // Any width and number of streams, entry by entry; u of the row stands in shared memory between the two passes.
 template <typename T>
 __global__ void __launch_bounds__(256) hyper_kernel(T* __restrict__ h, const T* __restrict__ y, const HyperArgs a, int S) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ float hy_u[];
     __shared__ float red[32];
     const size_t row = blockIdx.x;
@@ -167,9 +171,9 @@ static int hyper_launch(T* h, const T* y, const HyperArgs& a, int S, int n, cuda
         const int threads = ((nvec + vpt - 1) / vpt + 31) / 32 * 32;
 #define OXR_HY(NS) \
     do { \
-        if (vpt == 1) hyper_words_kernel<T, NS, 1><<<n, threads, 0, stream>>>(h, y, a); \
-        else if (vpt == 2) hyper_words_kernel<T, NS, 2><<<n, threads, 0, stream>>>(h, y, a); \
-        else hyper_words_kernel<T, NS, 4><<<n, threads, 0, stream>>>(h, y, a); \
+        if (vpt == 1) oxr_launch_small(hyper_words_kernel<T, NS, 1>, dim3(n), dim3(threads), 0, stream, h, y, a); \
+        else if (vpt == 2) oxr_launch_small(hyper_words_kernel<T, NS, 2>, dim3(n), dim3(threads), 0, stream, h, y, a); \
+        else oxr_launch_small(hyper_words_kernel<T, NS, 4>, dim3(n), dim3(threads), 0, stream, h, y, a); \
     } while (0)
         if (S == 1) OXR_HY(1);
         else if (S == 2) OXR_HY(2);
@@ -184,7 +188,7 @@ static int hyper_launch(T* h, const T* y, const HyperArgs& a, int S, int n, cuda
         cudaError_t e = cudaFuncSetAttribute(hyper_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return 1000 + (int)e;
     }
-    hyper_kernel<T><<<n, a.hidden >= 1024 ? 256 : 128, smem, stream>>>(h, y, a, S);
+    oxr_launch_small(hyper_kernel<T>, dim3(n), dim3(a.hidden >= 1024 ? 256 : 128), smem, stream, h, y, a, S);
     return oxr_launch_status();
 }
 

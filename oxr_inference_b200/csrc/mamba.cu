@@ -21,6 +21,8 @@ __global__ void causal_conv_silu_kernel(T* __restrict__ out, const T* __restrict
                                         const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ state,
                                         long long slot_stride, const int* __restrict__ req_of_token, const int* __restrict__ cu_q,
                                         const int* __restrict__ state_slots) {
+    pdl_wait();
+    pdl_trigger();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = blockIdx.y;
     if (c >= channels) return;
@@ -50,6 +52,8 @@ __global__ void __launch_bounds__(CONV_THREADS) causal_conv4_silu_words_kernel(_
                                                                                const float* __restrict__ bias, const float* __restrict__ state,
                                                                                long long slot_stride, const int* __restrict__ req_of_token,
                                                                                const int* __restrict__ cu_q, const int* __restrict__ state_slots) {
+    pdl_wait();
+    pdl_trigger();
     const int c = (blockIdx.x * CONV_THREADS + threadIdx.x) * 8;
     if (c >= channels) return;
     float wt[8][4], b[8];
@@ -101,6 +105,8 @@ __global__ void __launch_bounds__(CONV_THREADS) causal_conv4_silu_words_kernel(_
 template <typename T>
 __global__ void conv_tail_roll_kernel(float* __restrict__ state, long long slot_stride, const T* __restrict__ proj, int proj_stride, int col0,
                                       int channels, int taps, const int* __restrict__ cu_q, const int* __restrict__ state_slots) {
+    pdl_wait();
+    pdl_trigger();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y;
     if (c >= channels) return;
@@ -128,6 +134,7 @@ __global__ void __launch_bounds__(32 * NW) ssm_scan_kernel(
     float* __restrict__ y, const T* __restrict__ xbc, const T* __restrict__ proj, int proj_stride, int dt_col0, int heads, int vdim, int N,
     int groups, const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip, float* __restrict__ state,
     long long slot_stride, const int* __restrict__ cu_q, const int* __restrict__ state_slots) {
+    pdl_wait();
     constexpr int NP = 32 * NW;                       // N rounded up to whole warps
     extern __shared__ __align__(16) float scan_smem[];
     float* Bs = scan_smem;                            // [TT][NP]
@@ -239,6 +246,8 @@ __global__ void __launch_bounds__(32 * NW) ssm_scan_kernel(
 template <typename T>
 __global__ void gated_group_norm_kernel(T* __restrict__ out, const float* __restrict__ y, const T* __restrict__ proj, int proj_stride, int z_col0,
                                         const float* __restrict__ weight, int inner, int part, float eps) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const int t = blockIdx.y, lo = blockIdx.x * part;
     float ss = 0.f;
@@ -260,6 +269,8 @@ __global__ void gated_group_norm_kernel(T* __restrict__ out, const float* __rest
 // twice, an entry at a time, and works the silu out twice. 2,048 tokens x 8,192 in 8 parts: 75 -> 32 us (20 us of bytes).
 __global__ void gated_group_norm_words_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ y, const __nv_bfloat16* __restrict__ proj, int proj_stride,
                                               int z_col0, const float* __restrict__ weight, int inner, int part, float eps) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const int t = blockIdx.y, at = blockIdx.x * part + 8 * threadIdx.x;
     const bool ok = 8 * (int)threadIdx.x < part;
@@ -296,16 +307,16 @@ static int mamba_conv(void* out, const void* proj, int n_tokens, int n_requests,
     // the 16-byte form wants whole words and, to fill the chip with a thread per eight channels of 16 tokens, more than a decode step's rows
     const auto words = [](const void* p) { return (uintptr_t)p % 16 == 0; };
     if (sizeof(T) == 2 && taps == 4 && n_tokens > CONV_RUN && channels % 8 == 0 && proj_stride % 8 == 0 && col0 % 8 == 0 && words(out) && words(proj) && words(w))
-        causal_conv4_silu_words_kernel<<<dim3((channels / 8 + CONV_THREADS - 1) / CONV_THREADS, (n_tokens + CONV_RUN - 1) / CONV_RUN), CONV_THREADS, 0, stream>>>(
+        oxr_launch_small(causal_conv4_silu_words_kernel, dim3((channels / 8 + CONV_THREADS - 1) / CONV_THREADS, (n_tokens + CONV_RUN - 1) / CONV_RUN), dim3(CONV_THREADS), 0, stream, 
             (__nv_bfloat16*)out, (const __nv_bfloat16*)proj, proj_stride, col0, channels, n_tokens, w, bias, state, slot_stride, req_of_token, cu_q, state_slots);
     else {
         dim3 grid((channels + 127) / 128, n_tokens);
-        causal_conv_silu_kernel<T><<<grid, 128, 0, stream>>>((T*)out, (const T*)proj, proj_stride, col0, channels, taps, w, bias, state, slot_stride,
+        oxr_launch_small(causal_conv_silu_kernel<T>, dim3(grid), dim3(128), 0, stream, (T*)out, (const T*)proj, proj_stride, col0, channels, taps, w, bias, state, slot_stride,
                                                             req_of_token, cu_q, state_slots);
     }
     if (taps > 1) {
         dim3 grid2((channels + 127) / 128, n_requests);
-        conv_tail_roll_kernel<T><<<grid2, 128, 0, stream>>>(state, slot_stride, (const T*)proj, proj_stride, col0, channels, taps, cu_q, state_slots);
+        oxr_launch_small(conv_tail_roll_kernel<T>, dim3(grid2), dim3(128), 0, stream, state, slot_stride, (const T*)proj, proj_stride, col0, channels, taps, cu_q, state_slots);
     }
     return oxr_launch_status();
 }
@@ -330,7 +341,7 @@ static void mamba_scan(float* y, const void* xbc, const void* proj, int n_reques
     constexpr size_t smem = (size_t)(TT * (2 * 32 * NW + 32 + NW * 32 + 2)) * sizeof(float);
     static_assert(smem <= 48 * 1024, "the tile fits the default shared memory");
     dim3 grid((vdim + 31) / 32, heads, n_requests);
-    ssm_scan_kernel<T, NW, TT><<<grid, 32 * NW, smem, stream>>>(y, (const T*)xbc, (const T*)proj, proj_stride, dt_col0, heads, vdim, N, groups, dt_bias,
+    oxr_launch(ssm_scan_kernel<T, NW, TT>, dim3(grid), dim3(32 * NW), smem, stream, false, y, (const T*)xbc, (const T*)proj, proj_stride, dt_col0, heads, vdim, N, groups, dt_bias,
                                                                 a_log, d_skip, state, slot_stride, cu_q, state_slots);
 }
 
@@ -380,12 +391,12 @@ OXR_API int oxr_gated_group_norm(void* out, const float* y, const void* proj, in
     dim3 grid(parts, n_tokens);
     const auto words = [](const void* p) { return (uintptr_t)p % 16 == 0; };
     if (dtype == 1 && part % 8 == 0 && part <= 8192 && proj_stride % 8 == 0 && z_col0 % 8 == 0 && words(out) && words(y) && words(proj)) {
-        gated_group_norm_words_kernel<<<grid, (part / 8 + 31) / 32 * 32, 0, stream>>>((__nv_bfloat16*)out, y, (const __nv_bfloat16*)proj, proj_stride, z_col0, weight,
+        oxr_launch_small(gated_group_norm_words_kernel, dim3(grid), dim3((part / 8 + 31) / 32 * 32), 0, stream, (__nv_bfloat16*)out, y, (const __nv_bfloat16*)proj, proj_stride, z_col0, weight,
                                                                                      inner, part, eps);
         return oxr_launch_status();
     }
-    if (dtype == 0) gated_group_norm_kernel<float><<<grid, threads, 0, stream>>>((float*)out, y, (const float*)proj, proj_stride, z_col0, weight, inner, part, eps);
-    else gated_group_norm_kernel<__nv_bfloat16><<<grid, threads, 0, stream>>>((__nv_bfloat16*)out, y, (const __nv_bfloat16*)proj, proj_stride, z_col0, weight,
+    if (dtype == 0) oxr_launch_small(gated_group_norm_kernel<float>, dim3(grid), dim3(threads), 0, stream, (float*)out, y, (const float*)proj, proj_stride, z_col0, weight, inner, part, eps);
+    else oxr_launch_small(gated_group_norm_kernel<__nv_bfloat16>, dim3(grid), dim3(threads), 0, stream, (__nv_bfloat16*)out, y, (const __nv_bfloat16*)proj, proj_stride, z_col0, weight,
                                                                               inner, part, eps);
     return oxr_launch_status();
 }

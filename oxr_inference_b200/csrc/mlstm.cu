@@ -27,6 +27,8 @@ __device__ __forceinline__ float log_sigmoid_f32(float v) { return fminf(v, 0.f)
 __global__ void __launch_bounds__(32) mlstm_gates_kernel(float* __restrict__ coef, const float* __restrict__ gates, const float* __restrict__ gate_bias,
                                                         int heads, int DK, int DV, float cap, float* __restrict__ state, long long slot_stride,
                                                         const int* __restrict__ cu_q, const int* __restrict__ state_slots) {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x, h = blockIdx.x, r = blockIdx.y;
     const int t0 = cu_q[r], t1 = cu_q[r + 1];
     if (t1 <= t0) return;
@@ -68,6 +70,7 @@ __global__ void __launch_bounds__(32 * NW) mlstm_scan_kernel(
     float* __restrict__ y, const T* __restrict__ proj, int proj_stride, int q_col0, int k_col0, int v_col0, const float* __restrict__ coef,
     int heads, int DK, int DV, float q_scale, float* __restrict__ state, long long slot_stride, const int* __restrict__ cu_q,
     const int* __restrict__ state_slots) {
+    pdl_wait();
     constexpr int KPT = 32, DKP = KPT * NW, NT = 32 * NW;
     __shared__ __align__(16) float ks[TT][DKP];
     __shared__ __align__(16) float qs[TT][DKP];
@@ -180,11 +183,11 @@ OXR_API int oxr_mlstm_scan(float* y, float* coef, const void* proj, int n_reques
                            long long slot_stride, const int* cu_q, const int* state_slots, int dtype, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (heads <= 0 || DK <= 0 || DK > 256 || DV <= 0 || heads > 65535 || n_requests > 65535 || !(cap > 0.f)) return OXR_BAD_ARGUMENT;
-    mlstm_gates_kernel<<<dim3(heads, n_requests), 32, 0, stream>>>(coef, gates, gate_bias, heads, DK, DV, cap, state, slot_stride, cu_q, state_slots);
+    oxr_launch_small(mlstm_gates_kernel, dim3(heads, n_requests), dim3(32), 0, stream, coef, gates, gate_bias, heads, DK, DV, cap, state, slot_stride, cu_q, state_slots);
     dim3 grid((DV + 31) / 32, heads, n_requests);
     const int nw = (DK + 31) / 32;
 #define OXR_MLSTM(T, NW) \
-    mlstm_scan_kernel<T, NW, 8><<<grid, 32 * NW, 0, stream>>>(y, (const T*)proj, proj_stride, q_col0, k_col0, v_col0, coef, heads, DK, DV, q_scale, \
+    oxr_launch(mlstm_scan_kernel<T, NW, 8>, dim3(grid), dim3(32 * NW), 0, stream, false, y, (const T*)proj, proj_stride, q_col0, k_col0, v_col0, coef, heads, DK, DV, q_scale, \
                                                              state, slot_stride, cu_q, state_slots)
 #define OXR_MLSTM_T(T) \
     do { \
@@ -205,6 +208,8 @@ OXR_API int oxr_mlstm_scan(float* y, float* coef, const void* proj, int n_reques
 template <typename T>
 __global__ void head_norm_gate_kernel(T* __restrict__ out, const float* __restrict__ y, const T* __restrict__ gate, int gate_stride, int gate_col0,
                                       const float* __restrict__ weight, int heads, int DV, float eps, int silu) {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int t = blockIdx.x, h = blockIdx.y * warps + (threadIdx.x >> 5);
     if (h >= heads) return;
@@ -225,7 +230,7 @@ OXR_API int oxr_head_norm_gate(void* out, const float* y, const void* gate, int 
     const int warps = heads >= 4 ? 4 : heads;
     dim3 grid(n_tokens, (heads + warps - 1) / warps);
     if (grid.y > 65535) return OXR_BAD_ARGUMENT;
-    if (dtype == 0) head_norm_gate_kernel<float><<<grid, 32 * warps, 0, stream>>>((float*)out, y, (const float*)gate, gate_stride, gate_col0, weight, heads, DV, eps, silu);
-    else head_norm_gate_kernel<__nv_bfloat16><<<grid, 32 * warps, 0, stream>>>((__nv_bfloat16*)out, y, (const __nv_bfloat16*)gate, gate_stride, gate_col0, weight, heads, DV, eps, silu);
+    if (dtype == 0) oxr_launch_small(head_norm_gate_kernel<float>, dim3(grid), dim3(32 * warps), 0, stream, (float*)out, y, (const float*)gate, gate_stride, gate_col0, weight, heads, DV, eps, silu);
+    else oxr_launch_small(head_norm_gate_kernel<__nv_bfloat16>, dim3(grid), dim3(32 * warps), 0, stream, (__nv_bfloat16*)out, y, (const __nv_bfloat16*)gate, gate_stride, gate_col0, weight, heads, DV, eps, silu);
     return oxr_launch_status();
 }

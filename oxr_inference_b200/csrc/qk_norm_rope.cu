@@ -18,6 +18,8 @@ __global__ void qk_norm_rope_store_kernel(
     const float* __restrict__ sin_table, const int* __restrict__ positions, const int* __restrict__ slots,
     int n_tokens, int H, int KV, int D, float eps, int max_positions, long long num_slots, int norm_q, int norm_k,
     int rotate, int* status) {
+    pdl_wait();
+    pdl_trigger();
     const int warps_per_block = blockDim.x >> 5;
     const int lane = threadIdx.x & 31;
     const long long unit = (long long)blockIdx.x * warps_per_block + (threadIdx.x >> 5);
@@ -382,7 +384,7 @@ OXR_API int oxr_qk_norm_rope_store(void* q_out, void* k_cache, void* v_cache, co
     }
     const int pairs = (D / 2 + 31) / 32;  // 1..8
 #define LAUNCH(T, P)                                                                                               \
-    qk_norm_rope_store_kernel<T, P><<<blocks, warps * 32, 0, stream>>>(                                              \
+    oxr_launch_small(qk_norm_rope_store_kernel<T, P>, dim3(blocks), dim3(warps * 32), 0, stream,                                               \
         (T*)q_out, (T*)k_cache, (T*)v_cache, (const T*)qkv, q_weight, k_weight, cos_table, sin_table, positions, slots, \
         n_tokens, H, KV, D, eps, max_positions, num_slots, norm_q, norm_k, rotate, status)
 #define DISPATCH(T)                                   \

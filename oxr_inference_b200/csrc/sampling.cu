@@ -46,6 +46,8 @@ __device__ __forceinline__ void block_argmax(float& v, int& i, float* sval, int*
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_partial_kernel(float* __restrict__ part_max, int* __restrict__ part_idx, float* __restrict__ part_sum,
                       const float* __restrict__ logits, int vocab, const float* __restrict__ temperature) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float sval[SAMPLE_THREADS];
     __shared__ int sidx[SAMPLE_THREADS];
     const int r = blockIdx.y, chunks = gridDim.x, c = blockIdx.x;
@@ -80,6 +82,8 @@ sample_final_kernel(int* __restrict__ out, const float* __restrict__ part_max, c
                     const float* __restrict__ part_sum, int chunks, const float* __restrict__ logits, int vocab,
                     const float* __restrict__ temperature, const int* __restrict__ seed_lo, const int* __restrict__ seed_hi,
                     const int* __restrict__ counter) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float sval[SAMPLE_THREADS];
     __shared__ int sidx[SAMPLE_THREADS];
     __shared__ float s_target;
@@ -157,6 +161,8 @@ sample_final_kernel(int* __restrict__ out, const float* __restrict__ part_max, c
 
 __global__ void repetition_penalty_kernel(float* __restrict__ logits, const unsigned char* __restrict__ seen,
                                           const int* __restrict__ row_slot, const float* __restrict__ penalty, int vocab) {
+    pdl_wait();
+    pdl_trigger();
     const int r = blockIdx.y;
     const float p = penalty[r];
     if (p == 1.f) return;
@@ -172,6 +178,8 @@ __global__ void repetition_penalty_kernel(float* __restrict__ logits, const unsi
 
 __global__ void mark_seen_kernel(unsigned char* __restrict__ seen, const int* __restrict__ slots,
                                  const int* __restrict__ tokens, int n, int vocab) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         const int tok = tokens[i];
@@ -192,10 +200,10 @@ OXR_API int oxr_sample(int* out, const float* logits, int rows, int vocab, const
     float* part_max = (float*)scratch;
     int* part_idx = (int*)scratch + (size_t)rows * chunks;
     float* part_sum = (float*)scratch + 2 * (size_t)rows * chunks;
-    sample_partial_kernel<<<dim3(chunks, rows), SAMPLE_THREADS, 0, stream>>>(part_max, part_idx, part_sum, logits, vocab, temperature);
+    oxr_launch_small(sample_partial_kernel, dim3(chunks, rows), dim3(SAMPLE_THREADS), 0, stream, part_max, part_idx, part_sum, logits, vocab, temperature);
     int rc = oxr_launch_status();
     if (rc) return rc;
-    sample_final_kernel<<<rows, SAMPLE_THREADS, 0, stream>>>(out, part_max, part_idx, part_sum, chunks, logits, vocab, temperature,
+    oxr_launch_small(sample_final_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, stream, out, part_max, part_idx, part_sum, chunks, logits, vocab, temperature,
                                                             seed_lo, seed_hi, counter);
     return oxr_launch_status();
 }
@@ -204,13 +212,13 @@ OXR_API int oxr_repetition_penalty(float* logits, const unsigned char* seen, con
                                    int rows, int vocab, cudaStream_t stream) {
     if (rows <= 0) return 0;
     dim3 grid((vocab + 1023) / 1024 < 64 ? (vocab + 1023) / 1024 : 64, rows);
-    repetition_penalty_kernel<<<grid, 256, 0, stream>>>(logits, seen, row_slot, penalty, vocab);
+    oxr_launch_small(repetition_penalty_kernel, dim3(grid), dim3(256), 0, stream, logits, seen, row_slot, penalty, vocab);
     return oxr_launch_status();
 }
 
 OXR_API int oxr_mark_seen(unsigned char* seen, const int* slots, const int* tokens, int n, int vocab, cudaStream_t stream) {
     if (n <= 0) return 0;
-    mark_seen_kernel<<<(n + 255) / 256, 256, 0, stream>>>(seen, slots, tokens, n, vocab);
+    oxr_launch_small(mark_seen_kernel, dim3((n + 255) / 256), dim3(256), 0, stream, seen, slots, tokens, n, vocab);
     return oxr_launch_status();
 }
 
@@ -276,11 +284,11 @@ int oxr_sample_static(int* out_tokens, const float* logits, int rows, int vocab,
     float* part_max = (float*)scratch;
     int* part_idx = (int*)scratch + (size_t)rows * chunks;
     float* part_sum = (float*)scratch + 2 * (size_t)rows * chunks;
-    sample_partial_kernel<<<dim3((unsigned)chunks, rows), SAMPLE_THREADS, 0, stream>>>(part_max, part_idx, part_sum, logits, vocab,
+    oxr_launch_small(sample_partial_kernel, dim3((unsigned)chunks, rows), dim3(SAMPLE_THREADS), 0, stream, part_max, part_idx, part_sum, logits, vocab,
                                                                                         temperature);
     e = cudaGetLastError();
     if (e == cudaSuccess) {
-        sample_final_kernel<<<rows, SAMPLE_THREADS, 0, stream>>>(out_tokens, part_max, part_idx, part_sum, (int)chunks, logits, vocab,
+        oxr_launch_small(sample_final_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, stream, out_tokens, part_max, part_idx, part_sum, (int)chunks, logits, vocab,
                                                                 temperature, seed_lo, seed_hi, counter);
         e = cudaGetLastError();
     }

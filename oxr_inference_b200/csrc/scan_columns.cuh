@@ -111,6 +111,7 @@ __device__ __forceinline__ void scan_four(const __nv_bfloat16* at, float (&v)[4]
 // grid (ceil(DV / COLS), heads, requests). Row pieces are whole 16-byte words (scan_fits).
 template <typename T, int J, int E, bool VECTOR>
 __global__ void __launch_bounds__(ScanShape<T, J, E, VECTOR>::THREADS) column_scan_kernel(const ScanArgs a) {
+    pdl_wait();
     using Sh = ScanShape<T, J, E, VECTOR>;
     constexpr int TT = SCAN_TT, TPG = J / 8, P = E / 2, W = 16 / (int)sizeof(T);      // tokens whose sums meet in one butterfly; entries of a 16-byte word
     extern __shared__ __align__(16) unsigned char column_smem[];
@@ -278,7 +279,7 @@ int scan_launch_j(const ScanArgs& a, cudaStream_t stream) {
         cudaError_t e = cudaFuncSetAttribute(column_scan_kernel<T, J, E, VECTOR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM);
         if (e != cudaSuccess) return 1000 + (int)e;
     }
-    column_scan_kernel<T, J, E, VECTOR><<<dim3((a.DV + Sh::COLS - 1) / Sh::COLS, a.heads, a.n_requests), Sh::THREADS, Sh::SMEM, stream>>>(a);
+    oxr_launch(column_scan_kernel<T, J, E, VECTOR>, dim3((a.DV + Sh::COLS - 1) / Sh::COLS, a.heads, a.n_requests), dim3(Sh::THREADS), Sh::SMEM, stream, false, a);
     return oxr_launch_status();
 }
 // Eight entries a lane where that makes warps enough to hide one another's latencies (a warp alone on its scheduler issues an instruction every 3.4

@@ -80,6 +80,8 @@ template <typename T, int VEC> __device__ __forceinline__ void sn_store(T* p, co
 
 template <typename T, int VEC, int VPT>
 __global__ void __launch_bounds__(VEC == 8 && VPT <= 2 ? 512 : 1024) shift_norm_kernel(T* __restrict__ out, const T* __restrict__ y, const ShiftNormArgs a, int rows_per_block) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const int hidden = a.hidden, nvec = hidden / VEC;
     float prev[VPT][VEC], h[VPT][VEC];
@@ -200,7 +202,7 @@ OXR_API int oxr_shift_norm(void* out, const float* stream, const void* y, float*
                        (uintptr_t)y % 16 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)w_post % 16 == 0 && (uintptr_t)w % 16 == 0 &&
                        (uintptr_t)mu % 16 == 0 && (uintptr_t)state % 16 == 0 && state_stride % 4 == 0;
 #define OXR_SN(T, VEC, VPT) \
-    shift_norm_kernel<T, VEC, VPT><<<blocks, ((hidden / VEC + VPT - 1) / VPT + 31) / 32 * 32, 0, stream_>>>((T*)out, (const T*)y, a, rows_per_block)
+    oxr_launch_small(shift_norm_kernel<T, VEC, VPT>, dim3(blocks), dim3(((hidden / VEC + VPT - 1) / VPT + 31) / 32 * 32), 0, stream_, (T*)out, (const T*)y, a, rows_per_block)
     if (words) {
         const int nvec = hidden / 8;
         if (nvec <= 512) OXR_SN(__nv_bfloat16, 8, 1);

@@ -10,6 +10,8 @@
 template <typename T>
 __global__ void stream_rms_norm_kernel(T* __restrict__ out, const float* __restrict__ stream, const float* __restrict__ weight,
                                        const int* __restrict__ rows, int hidden, float eps) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const int r = blockIdx.x;
     const float* x = stream + (size_t)(rows ? rows[r] : r) * hidden;
@@ -27,6 +29,8 @@ template <typename T>
 __global__ void norm_add_norm_kernel(float* __restrict__ stream, const T* __restrict__ y, const float* __restrict__ w_post,
                                      T* __restrict__ out, const float* __restrict__ w_next, int hidden, float eps_post, float eps_next,
                                      int row_floats_in_smem) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ float smem[];
     float* red = smem;
     float* rowbuf = smem + 32;
@@ -82,6 +86,8 @@ __device__ __forceinline__ uint4 f32_to_bf16x8(const float (&v)[8]) {
 template <int VPT>
 __global__ void stream_rms_norm_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ stream, const float* __restrict__ weight,
                                               const int* __restrict__ rows, int hidden, float eps) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const float* x = stream + (size_t)(rows ? rows[blockIdx.x] : blockIdx.x) * hidden;
     __nv_bfloat16* dst = out + (size_t)blockIdx.x * hidden;
@@ -118,6 +124,8 @@ template <int VPT>
 __global__ void norm_add_norm_bf16x8_kernel(float* __restrict__ stream, const __nv_bfloat16* __restrict__ y, const float* __restrict__ w_post,
                                             __nv_bfloat16* __restrict__ out, const float* __restrict__ w_next, int hidden, float eps_post,
                                             float eps_next) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const size_t at = (size_t)blockIdx.x * hidden;
     const int nvec = hidden / 8;
@@ -180,6 +188,8 @@ __global__ void norm_add_norm_bf16x8_kernel(float* __restrict__ stream, const __
 // out[r] = [ a[r] | b[r] ] rounded to T
 template <typename T>
 __global__ void concat2_cast_kernel(T* __restrict__ out, const float* __restrict__ a, const float* __restrict__ b, int hidden, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t r = i / (2 * hidden);
         const int c = (int)(i % (2 * hidden));
@@ -188,6 +198,8 @@ __global__ void concat2_cast_kernel(T* __restrict__ out, const float* __restrict
 }
 
 __global__ void add_row_f32_kernel(float* __restrict__ x, const float* __restrict__ row, int hidden, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) x[i] += row[i % hidden];
 }
 
@@ -197,6 +209,8 @@ __global__ void add_row_f32_kernel(float* __restrict__ x, const float* __restric
 template <typename T>
 __global__ void clamped_glu_kernel(T* __restrict__ out, const T* __restrict__ gate_up, int inter, int interleave, float alpha, float limit,
                                    size_t total) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t row = i / inter;
         const int col = (int)(i % inter);
@@ -216,6 +230,8 @@ __global__ void clamped_glu_kernel(T* __restrict__ out, const T* __restrict__ ga
 
 // bf16, [gate | up] side by side, `inter` a multiple of 8: 16-byte loads and stores. Grid (column words, rows).
 __global__ void clamped_glu_bf16x8_kernel(uint4* __restrict__ out, const uint4* __restrict__ gate_up, int inter8, float alpha, float limit) {
+    pdl_wait();
+    pdl_trigger();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= inter8) return;
     const size_t row = blockIdx.y;
@@ -236,6 +252,8 @@ __device__ __forceinline__ float gelu_tanh_of(float z) { return 0.5f * z * (1.f 
 
 template <typename T>
 __global__ void gelu_glu_kernel(T* __restrict__ out, const T* __restrict__ gate_up, int inter, int interleave, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t row = i / inter;
         const int col = (int)(i % inter);
@@ -248,6 +266,8 @@ __global__ void gelu_glu_kernel(T* __restrict__ out, const T* __restrict__ gate_
 // cos/sin [tokens, half] of position * freq[i], times `magnitude`: products and functions in fp64, rounded once to fp32.
 __global__ void rotary_angles_kernel(float* __restrict__ cos_out, float* __restrict__ sin_out, const int* __restrict__ positions,
                                      const double* __restrict__ freq, double magnitude, int half, int total) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     double s, c;
@@ -269,12 +289,12 @@ OXR_API int oxr_stream_rms_norm(void* out, const float* stream, const float* wei
     if (dtype == 1 && hidden % 8 == 0 && hidden <= 32768 && (uintptr_t)stream % 16 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)weight % 16 == 0) {
         const int nvec = hidden / 8, vpt = nvec <= 512 ? 1 : (nvec <= 2048 ? 2 : 4), words = ((nvec + vpt - 1) / vpt + 31) / 32 * 32;
         const auto kernel = vpt == 1 ? stream_rms_norm_bf16x8_kernel<1> : (vpt == 2 ? stream_rms_norm_bf16x8_kernel<2> : stream_rms_norm_bf16x8_kernel<4>);
-        kernel<<<n_out, words, 0, stream_>>>((__nv_bfloat16*)out, stream, weight, rows, hidden, eps);
+        oxr_launch_small(kernel, dim3(n_out), dim3(words), 0, stream_, (__nv_bfloat16*)out, stream, weight, rows, hidden, eps);
         return oxr_launch_status();
     }
     const int threads = hidden >= 1024 ? 256 : 128;
-    if (dtype == 0) stream_rms_norm_kernel<float><<<n_out, threads, 0, stream_>>>((float*)out, stream, weight, rows, hidden, eps);
-    else stream_rms_norm_kernel<__nv_bfloat16><<<n_out, threads, 0, stream_>>>((__nv_bfloat16*)out, stream, weight, rows, hidden, eps);
+    if (dtype == 0) oxr_launch_small(stream_rms_norm_kernel<float>, dim3(n_out), dim3(threads), 0, stream_, (float*)out, stream, weight, rows, hidden, eps);
+    else oxr_launch_small(stream_rms_norm_kernel<__nv_bfloat16>, dim3(n_out), dim3(threads), 0, stream_, (__nv_bfloat16*)out, stream, weight, rows, hidden, eps);
     return oxr_launch_status();
 }
 
@@ -289,18 +309,18 @@ OXR_API int oxr_norm_add_norm(float* stream, const void* y, const float* w_post,
         const int threads = ((nvec + vpt - 1) / vpt + 31) / 32 * 32;
         const __nv_bfloat16* yb = (const __nv_bfloat16*)y;
         __nv_bfloat16* ob = (__nv_bfloat16*)out;
-        if (vpt == 1) norm_add_norm_bf16x8_kernel<1><<<n, threads, 0, stream_>>>(stream, yb, w_post, ob, w_next, hidden, eps_post, eps_next);
-        else if (vpt == 2) norm_add_norm_bf16x8_kernel<2><<<n, threads, 0, stream_>>>(stream, yb, w_post, ob, w_next, hidden, eps_post, eps_next);
-        else norm_add_norm_bf16x8_kernel<4><<<n, threads, 0, stream_>>>(stream, yb, w_post, ob, w_next, hidden, eps_post, eps_next);
+        if (vpt == 1) oxr_launch_small(norm_add_norm_bf16x8_kernel<1>, dim3(n), dim3(threads), 0, stream_, stream, yb, w_post, ob, w_next, hidden, eps_post, eps_next);
+        else if (vpt == 2) oxr_launch_small(norm_add_norm_bf16x8_kernel<2>, dim3(n), dim3(threads), 0, stream_, stream, yb, w_post, ob, w_next, hidden, eps_post, eps_next);
+        else oxr_launch_small(norm_add_norm_bf16x8_kernel<4>, dim3(n), dim3(threads), 0, stream_, stream, yb, w_post, ob, w_next, hidden, eps_post, eps_next);
         return oxr_launch_status();
     }
     const int threads = hidden >= 1024 ? 256 : 128;
     const int keep = hidden <= 8192 ? hidden : 0;
     const size_t smem = (32 + keep) * sizeof(float);
     if (dtype == 0)
-        norm_add_norm_kernel<float><<<n, threads, smem, stream_>>>(stream, (const float*)y, w_post, (float*)out, w_next, hidden, eps_post, eps_next, keep);
+        oxr_launch_small(norm_add_norm_kernel<float>, dim3(n), dim3(threads), smem, stream_, stream, (const float*)y, w_post, (float*)out, w_next, hidden, eps_post, eps_next, keep);
     else
-        norm_add_norm_kernel<__nv_bfloat16><<<n, threads, smem, stream_>>>(stream, (const __nv_bfloat16*)y, w_post, (__nv_bfloat16*)out, w_next, hidden,
+        oxr_launch_small(norm_add_norm_kernel<__nv_bfloat16>, dim3(n), dim3(threads), smem, stream_, stream, (const __nv_bfloat16*)y, w_post, (__nv_bfloat16*)out, w_next, hidden,
                                                                           eps_post, eps_next, keep);
     return oxr_launch_status();
 }
@@ -308,15 +328,15 @@ OXR_API int oxr_norm_add_norm(float* stream, const void* y, const float* w_post,
 OXR_API int oxr_concat2_cast(void* out, const float* a, const float* b, int n, int hidden, int dtype, cudaStream_t stream_) {
     if (n <= 0) return 0;
     const size_t total = (size_t)n * 2 * hidden;
-    if (dtype == 0) concat2_cast_kernel<float><<<grid_for(total, 256), 256, 0, stream_>>>((float*)out, a, b, hidden, total);
-    else concat2_cast_kernel<__nv_bfloat16><<<grid_for(total, 256), 256, 0, stream_>>>((__nv_bfloat16*)out, a, b, hidden, total);
+    if (dtype == 0) oxr_launch_small(concat2_cast_kernel<float>, dim3(grid_for(total, 256)), dim3(256), 0, stream_, (float*)out, a, b, hidden, total);
+    else oxr_launch_small(concat2_cast_kernel<__nv_bfloat16>, dim3(grid_for(total, 256)), dim3(256), 0, stream_, (__nv_bfloat16*)out, a, b, hidden, total);
     return oxr_launch_status();
 }
 
 OXR_API int oxr_add_row_f32(float* x, const float* row, int n, int hidden, cudaStream_t stream_) {
     if (n <= 0) return 0;
     const size_t total = (size_t)n * hidden;
-    add_row_f32_kernel<<<grid_for(total, 256), 256, 0, stream_>>>(x, row, hidden, total);
+    oxr_launch_small(add_row_f32_kernel, dim3(grid_for(total, 256)), dim3(256), 0, stream_, x, row, hidden, total);
     return oxr_launch_status();
 }
 
@@ -326,12 +346,12 @@ OXR_API int oxr_clamped_glu(void* out, const void* gate_up, int n, int inter, in
     if (inter <= 0 || interleave < 0 || (interleave && inter % interleave)) return OXR_BAD_ARGUMENT;
     if (dtype == 1 && interleave == 0 && inter % 8 == 0 && n <= 65535 && (uintptr_t)out % 16 == 0 && (uintptr_t)gate_up % 16 == 0) {
         dim3 grid((inter / 8 + 127) / 128, n);
-        clamped_glu_bf16x8_kernel<<<grid, 128, 0, stream_>>>((uint4*)out, (const uint4*)gate_up, inter / 8, alpha, limit);
+        oxr_launch_small(clamped_glu_bf16x8_kernel, dim3(grid), dim3(128), 0, stream_, (uint4*)out, (const uint4*)gate_up, inter / 8, alpha, limit);
         return oxr_launch_status();
     }
     const size_t total = (size_t)n * inter;
-    if (dtype == 0) clamped_glu_kernel<float><<<grid_for(total, 256), 256, 0, stream_>>>((float*)out, (const float*)gate_up, inter, interleave, alpha, limit, total);
-    else clamped_glu_kernel<__nv_bfloat16><<<grid_for(total, 256), 256, 0, stream_>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)gate_up, inter, interleave,
+    if (dtype == 0) oxr_launch_small(clamped_glu_kernel<float>, dim3(grid_for(total, 256)), dim3(256), 0, stream_, (float*)out, (const float*)gate_up, inter, interleave, alpha, limit, total);
+    else oxr_launch_small(clamped_glu_kernel<__nv_bfloat16>, dim3(grid_for(total, 256)), dim3(256), 0, stream_, (__nv_bfloat16*)out, (const __nv_bfloat16*)gate_up, inter, interleave,
                                                                                      alpha, limit, total);
     return oxr_launch_status();
 }
@@ -340,15 +360,15 @@ OXR_API int oxr_gelu_glu(void* out, const void* gate_up, int n, int inter, int i
     if (n <= 0) return 0;
     if (inter <= 0 || interleave < 0 || (interleave && inter % interleave)) return OXR_BAD_ARGUMENT;
     const size_t total = (size_t)n * inter;
-    if (dtype == 0) gelu_glu_kernel<float><<<grid_for(total, 256), 256, 0, stream_>>>((float*)out, (const float*)gate_up, inter, interleave, total);
-    else gelu_glu_kernel<__nv_bfloat16><<<grid_for(total, 256), 256, 0, stream_>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)gate_up, inter, interleave, total);
+    if (dtype == 0) oxr_launch_small(gelu_glu_kernel<float>, dim3(grid_for(total, 256)), dim3(256), 0, stream_, (float*)out, (const float*)gate_up, inter, interleave, total);
+    else oxr_launch_small(gelu_glu_kernel<__nv_bfloat16>, dim3(grid_for(total, 256)), dim3(256), 0, stream_, (__nv_bfloat16*)out, (const __nv_bfloat16*)gate_up, inter, interleave, total);
     return oxr_launch_status();
 }
 
 OXR_API int oxr_rotary_angles(float* cos_out, float* sin_out, const int* positions, const double* freq, double magnitude, int n, int half, cudaStream_t stream_) {
     if (n <= 0 || half <= 0) return 0;
     const int total = n * half;
-    rotary_angles_kernel<<<(total + 127) / 128, 128, 0, stream_>>>(cos_out, sin_out, positions, freq, magnitude, half, total);
+    oxr_launch_small(rotary_angles_kernel, dim3((total + 127) / 128), dim3(128), 0, stream_, cos_out, sin_out, positions, freq, magnitude, half, total);
     return oxr_launch_status();
 }
 
@@ -400,6 +420,8 @@ __device__ __forceinline__ void prefetch_row(const float* p, int hidden) {
 template <typename T>
 __global__ void stream_layer_norm_kernel(T* __restrict__ out, const float* __restrict__ stream, const float* __restrict__ weight,
                                          const float* __restrict__ bias, const int* __restrict__ rows, int hidden, float eps) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ __align__(16) float ln_row[];
     __shared__ float red[32];
     const int r = blockIdx.x;
@@ -441,10 +463,10 @@ OXR_API int oxr_stream_layer_norm(void* out, const float* stream, const float* w
     const size_t smem = (size_t)hidden * sizeof(float);
     if (dtype == 0) {
         if (int rc = with_row_smem(stream_layer_norm_kernel<float>, smem)) return rc;
-        stream_layer_norm_kernel<float><<<n_out, threads, smem, stream_>>>((float*)out, stream, weight, bias, rows, hidden, eps);
+        oxr_launch_small(stream_layer_norm_kernel<float>, dim3(n_out), dim3(threads), smem, stream_, (float*)out, stream, weight, bias, rows, hidden, eps);
     } else {
         if (int rc = with_row_smem(stream_layer_norm_kernel<__nv_bfloat16>, smem)) return rc;
-        stream_layer_norm_kernel<__nv_bfloat16><<<n_out, threads, smem, stream_>>>((__nv_bfloat16*)out, stream, weight, bias, rows, hidden, eps);
+        oxr_launch_small(stream_layer_norm_kernel<__nv_bfloat16>, dim3(n_out), dim3(threads), smem, stream_, (__nv_bfloat16*)out, stream, weight, bias, rows, hidden, eps);
     }
     return oxr_launch_status();
 }
@@ -506,6 +528,8 @@ template <typename T>
 __global__ void gated_residual_kernel(float* __restrict__ stream, const T* __restrict__ a, const float* __restrict__ ab, const T* __restrict__ f,
                                       const float* __restrict__ fb, const T* __restrict__ gates, int gates_stride, const float* __restrict__ gate_bias,
                                       float* __restrict__ history, int index, const float* __restrict__ mixw, int hidden, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t row = i / hidden;
         float x = stream[i] + gated_sum_at<T>(i, row, (int)(i - row * hidden), a, ab, f, fb, gates, gates_stride, gate_bias, hidden);
@@ -527,6 +551,8 @@ __global__ void gated_residual_norm_kernel(T* __restrict__ out, float* stream, c
                                            const T* __restrict__ f, const float* __restrict__ fb, const T* __restrict__ gates, int gates_stride,
                                            const float* __restrict__ gate_bias, float* history, int index, const float* __restrict__ mixw,
                                            int hidden, size_t total, const float* __restrict__ weight, const float* __restrict__ bias, float eps) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ __align__(16) float ln_row[];   // [hidden] the stream's new row, then [hidden] X
     __shared__ float red[32];
     float* x_row = ln_row + hidden;
@@ -563,12 +589,12 @@ OXR_API int oxr_gated_residual_norm(void* out, float* stream, const void* a, con
     const int threads = hidden >= 4096 ? 1024 : hidden >= 2048 ? 512 : hidden >= 1024 ? 256 : 128;   // every thread's loads of a row are in flight together
     if (dtype == 0) {
         if (int rc = with_row_smem(gated_residual_norm_kernel<float>, smem)) return rc;
-        gated_residual_norm_kernel<float><<<n, threads, smem, stream_>>>((float*)out, stream, (const float*)a, ab, (const float*)f, fb, (const float*)gates,
+        oxr_launch_small(gated_residual_norm_kernel<float>, dim3(n), dim3(threads), smem, stream_, (float*)out, stream, (const float*)a, ab, (const float*)f, fb, (const float*)gates,
                                                                         gates_stride, gate_bias, history, index, mixw, hidden, total, weight, bias, eps);
     } else {
         typedef __nv_bfloat16 B;
         if (int rc = with_row_smem(gated_residual_norm_kernel<B>, smem)) return rc;
-        gated_residual_norm_kernel<B><<<n, threads, smem, stream_>>>((B*)out, stream, (const B*)a, ab, (const B*)f, fb, (const B*)gates, gates_stride,
+        oxr_launch_small(gated_residual_norm_kernel<B>, dim3(n), dim3(threads), smem, stream_, (B*)out, stream, (const B*)a, ab, (const B*)f, fb, (const B*)gates, gates_stride,
                                                                     gate_bias, history, index, mixw, hidden, total, weight, bias, eps);
     }
     return oxr_launch_status();
@@ -581,10 +607,10 @@ OXR_API int oxr_gated_residual(float* stream, const void* a, const float* ab, co
     if (hidden <= 0 || a == nullptr || (history != nullptr && (mixw == nullptr || index < 0))) return OXR_BAD_ARGUMENT;
     const size_t total = (size_t)n * hidden;
     if (dtype == 0)
-        gated_residual_kernel<float><<<grid_for(total, 256), 256, 0, stream_>>>(stream, (const float*)a, ab, (const float*)f, fb, (const float*)gates,
+        oxr_launch_small(gated_residual_kernel<float>, dim3(grid_for(total, 256)), dim3(256), 0, stream_, stream, (const float*)a, ab, (const float*)f, fb, (const float*)gates,
                                                                                gates_stride, gate_bias, history, index, mixw, hidden, total);
     else
-        gated_residual_kernel<__nv_bfloat16><<<grid_for(total, 256), 256, 0, stream_>>>(stream, (const __nv_bfloat16*)a, ab, (const __nv_bfloat16*)f, fb,
+        oxr_launch_small(gated_residual_kernel<__nv_bfloat16>, dim3(grid_for(total, 256)), dim3(256), 0, stream_, stream, (const __nv_bfloat16*)a, ab, (const __nv_bfloat16*)f, fb,
                                                                                        (const __nv_bfloat16*)gates, gates_stride, gate_bias, history,
                                                                                        index, mixw, hidden, total);
     return oxr_launch_status();
@@ -594,6 +620,8 @@ OXR_API int oxr_gated_residual(float* stream, const void* a, const float* ab, co
 // out = 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3))), fp32 arithmetic, rounded once; out may be x itself.
 template <typename T>
 __global__ void gelu_tanh_kernel(T* __restrict__ out, const T* __restrict__ x, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const float z = Num<T>::to_f32(x[i]);
         out[i] = Num<T>::from_f32(0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))));
@@ -601,6 +629,8 @@ __global__ void gelu_tanh_kernel(T* __restrict__ out, const T* __restrict__ x, s
 }
 
 __global__ void gelu_tanh_bf16x8_kernel(uint4* __restrict__ out, const uint4* __restrict__ x, size_t total8) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total8; i += (size_t)gridDim.x * blockDim.x) {
         float z[8], o[8];
         bf16x8_to_f32(x[i], z);
@@ -613,25 +643,27 @@ __global__ void gelu_tanh_bf16x8_kernel(uint4* __restrict__ out, const uint4* __
 OXR_API int oxr_gelu_tanh(void* out, const void* x, long long total, int dtype, cudaStream_t stream_) {
     if (total <= 0) return 0;
     if (dtype == 1 && total % 8 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)x % 16 == 0) {
-        gelu_tanh_bf16x8_kernel<<<grid_for((size_t)total / 8, 256), 256, 0, stream_>>>((uint4*)out, (const uint4*)x, (size_t)total / 8);
+        oxr_launch_small(gelu_tanh_bf16x8_kernel, dim3(grid_for((size_t)total / 8, 256)), dim3(256), 0, stream_, (uint4*)out, (const uint4*)x, (size_t)total / 8);
         return oxr_launch_status();
     }
-    if (dtype == 0) gelu_tanh_kernel<float><<<grid_for((size_t)total, 256), 256, 0, stream_>>>((float*)out, (const float*)x, (size_t)total);
-    else gelu_tanh_kernel<__nv_bfloat16><<<grid_for((size_t)total, 256), 256, 0, stream_>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)x, (size_t)total);
+    if (dtype == 0) oxr_launch_small(gelu_tanh_kernel<float>, dim3(grid_for((size_t)total, 256)), dim3(256), 0, stream_, (float*)out, (const float*)x, (size_t)total);
+    else oxr_launch_small(gelu_tanh_kernel<__nv_bfloat16>, dim3(grid_for((size_t)total, 256)), dim3(256), 0, stream_, (__nv_bfloat16*)out, (const __nv_bfloat16*)x, (size_t)total);
     return oxr_launch_status();
 }
 
 // y += x element by element (the sum in fp32, rounded once)
 template <typename T>
 __global__ void add_inplace_kernel(T* __restrict__ y, const T* __restrict__ x, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
         y[i] = Num<T>::from_f32(Num<T>::to_f32(y[i]) + Num<T>::to_f32(x[i]));
 }
 
 OXR_API int oxr_add_inplace(void* y, const void* x, long long total, int dtype, cudaStream_t stream_) {
     if (total <= 0) return 0;
-    if (dtype == 0) add_inplace_kernel<float><<<grid_for((size_t)total, 256), 256, 0, stream_>>>((float*)y, (const float*)x, (size_t)total);
-    else add_inplace_kernel<__nv_bfloat16><<<grid_for((size_t)total, 256), 256, 0, stream_>>>((__nv_bfloat16*)y, (const __nv_bfloat16*)x, (size_t)total);
+    if (dtype == 0) oxr_launch_small(add_inplace_kernel<float>, dim3(grid_for((size_t)total, 256)), dim3(256), 0, stream_, (float*)y, (const float*)x, (size_t)total);
+    else oxr_launch_small(add_inplace_kernel<__nv_bfloat16>, dim3(grid_for((size_t)total, 256)), dim3(256), 0, stream_, (__nv_bfloat16*)y, (const __nv_bfloat16*)x, (size_t)total);
     return oxr_launch_status();
 }
 
@@ -641,6 +673,8 @@ OXR_API int oxr_add_inplace(void* y, const void* x, long long total, int dtype, 
 template <typename T>
 __global__ void pair_norm_mean_kernel(T* __restrict__ out, const T* __restrict__ a, const T* __restrict__ b, const float* __restrict__ wa,
                                       const float* __restrict__ wb, int hidden, float eps) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const size_t at = (size_t)blockIdx.x * hidden;
     float sa = 0.f, sb = 0.f;
@@ -660,6 +694,8 @@ __global__ void pair_norm_mean_kernel(T* __restrict__ out, const T* __restrict__
 template <int VPT>
 __global__ void pair_norm_mean_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                                              const float* __restrict__ wa, const float* __restrict__ wb, int hidden, float eps) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const size_t at = (size_t)blockIdx.x * hidden;
     const int nvec = hidden / 8;
@@ -706,39 +742,43 @@ OXR_API int oxr_pair_norm_mean(void* out, const void* a, const void* b, const fl
         const int vpt = nvec <= 512 ? 1 : (nvec <= 2048 ? 2 : 4);
         const int threads_v = ((nvec + vpt - 1) / vpt + 31) / 32 * 32;
         const __nv_bfloat16 *ab = (const __nv_bfloat16*)a, *bb = (const __nv_bfloat16*)b;
-        if (vpt == 1) pair_norm_mean_bf16x8_kernel<1><<<n, threads_v, 0, stream_>>>((__nv_bfloat16*)out, ab, bb, wa, wb, hidden, eps);
-        else if (vpt == 2) pair_norm_mean_bf16x8_kernel<2><<<n, threads_v, 0, stream_>>>((__nv_bfloat16*)out, ab, bb, wa, wb, hidden, eps);
-        else pair_norm_mean_bf16x8_kernel<4><<<n, threads_v, 0, stream_>>>((__nv_bfloat16*)out, ab, bb, wa, wb, hidden, eps);
+        if (vpt == 1) oxr_launch_small(pair_norm_mean_bf16x8_kernel<1>, dim3(n), dim3(threads_v), 0, stream_, (__nv_bfloat16*)out, ab, bb, wa, wb, hidden, eps);
+        else if (vpt == 2) oxr_launch_small(pair_norm_mean_bf16x8_kernel<2>, dim3(n), dim3(threads_v), 0, stream_, (__nv_bfloat16*)out, ab, bb, wa, wb, hidden, eps);
+        else oxr_launch_small(pair_norm_mean_bf16x8_kernel<4>, dim3(n), dim3(threads_v), 0, stream_, (__nv_bfloat16*)out, ab, bb, wa, wb, hidden, eps);
         return oxr_launch_status();
     }
     const int threads = hidden >= 2048 ? 256 : 128;
-    if (dtype == 0) pair_norm_mean_kernel<float><<<n, threads, 0, stream_>>>((float*)out, (const float*)a, (const float*)b, wa, wb, hidden, eps);
-    else pair_norm_mean_kernel<__nv_bfloat16><<<n, threads, 0, stream_>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, wa, wb, hidden, eps);
+    if (dtype == 0) oxr_launch_small(pair_norm_mean_kernel<float>, dim3(n), dim3(threads), 0, stream_, (float*)out, (const float*)a, (const float*)b, wa, wb, hidden, eps);
+    else oxr_launch_small(pair_norm_mean_kernel<__nv_bfloat16>, dim3(n), dim3(threads), 0, stream_, (__nv_bfloat16*)out, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, wa, wb, hidden, eps);
     return oxr_launch_status();
 }
 
 // out = fa * a + fb * b element by element (fp32, rounded once; out may be a): two mixers' results with a factor each.
 template <typename T>
 __global__ void scaled_sum_kernel(T* out, const T* a, const T* __restrict__ b, float fa, float fb, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
         out[i] = Num<T>::from_f32(fa * Num<T>::to_f32(a[i]) + fb * Num<T>::to_f32(b[i]));
 }
 
 OXR_API int oxr_scaled_sum(void* out, const void* a, const void* b, float fa, float fb, long long total, int dtype, cudaStream_t stream_) {
     if (total <= 0) return 0;
-    if (dtype == 0) scaled_sum_kernel<float><<<grid_for((size_t)total, 256), 256, 0, stream_>>>((float*)out, (const float*)a, (const float*)b, fa, fb, (size_t)total);
-    else scaled_sum_kernel<__nv_bfloat16><<<grid_for((size_t)total, 256), 256, 0, stream_>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, fa, fb, (size_t)total);
+    if (dtype == 0) oxr_launch_small(scaled_sum_kernel<float>, dim3(grid_for((size_t)total, 256)), dim3(256), 0, stream_, (float*)out, (const float*)a, (const float*)b, fa, fb, (size_t)total);
+    else oxr_launch_small(scaled_sum_kernel<__nv_bfloat16>, dim3(grid_for((size_t)total, 256)), dim3(256), 0, stream_, (__nv_bfloat16*)out, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, fa, fb, (size_t)total);
     return oxr_launch_status();
 }
 
 // x <- cap * tanh(x / cap), fp32, in place (capped logits).
 __global__ void tanh_cap_kernel(float* __restrict__ x, float cap, size_t total) {
+    pdl_wait();
+    pdl_trigger();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) x[i] = cap * tanhf(x[i] / cap);
 }
 
 OXR_API int oxr_tanh_cap(float* x, float cap, long long total, cudaStream_t stream_) {
     if (total <= 0) return 0;
     if (!(cap > 0.f)) return OXR_BAD_ARGUMENT;
-    tanh_cap_kernel<<<grid_for((size_t)total, 256), 256, 0, stream_>>>(x, cap, (size_t)total);
+    oxr_launch_small(tanh_cap_kernel, dim3(grid_for((size_t)total, 256)), dim3(256), 0, stream_, x, cap, (size_t)total);
     return oxr_launch_status();
 }
