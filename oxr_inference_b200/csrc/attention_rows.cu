@@ -24,6 +24,8 @@ __global__ void __launch_bounds__(128) attn_rows_kernel(
     const T* __restrict__ v_pool, long long v_slot_stride, int v_head_stride, int DK, int DV, int H, int KVH, const int* __restrict__ positions,
     const int* __restrict__ req_of_token, const int* __restrict__ block_table, int table_width, int page_size, int num_pages, float scale,
     int chunk, int window, int keep_first, const float* __restrict__ dist_bias, int bias_rows, const float* __restrict__ sink, int* status) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ float q_smem[];   // [warps, DK]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int t = blockIdx.x, h = blockIdx.y * warps + warp;
@@ -112,7 +114,7 @@ OXR_API int oxr_attention_rows(void* out, const void* q, int q_stride, const voi
     const size_t smem = (size_t)warps * DK * sizeof(float);
     if (smem > 48 * 1024) return OXR_BAD_ARGUMENT;
 #define OXR_ROWS(T, DVC) \
-    attn_rows_kernel<T, DVC><<<grid, 32 * warps, smem, stream>>>((T*)out, (const T*)q, q_stride, (const T*)k_pool, k_slot_stride, k_head_stride, \
+    oxr_launch(attn_rows_kernel<T, DVC>, dim3(grid), dim3(32 * warps), smem, stream, false, (T*)out, (const T*)q, q_stride, (const T*)k_pool, k_slot_stride, k_head_stride, \
                                                                 (const T*)v_pool, v_slot_stride, v_head_stride, DK, DV, H, KVH, positions, req_of_token, \
                                                                 block_table, table_width, page_size, num_pages, scale, chunk, window, keep_first, dist_bias, \
                                                                 bias_rows, sink, status)
@@ -135,6 +137,8 @@ OXR_API int oxr_attention_rows(void* out, const void* q, int q_stride, const voi
 template <typename T>
 __global__ void scatter_rows_kernel(T* __restrict__ pool, long long slot_stride, long long pool_slots, const T* __restrict__ src, int src_stride, int col0,
                                     int width, const int* __restrict__ slots, int* status, T* __restrict__ pool2, long long slot_stride2, int width2) {
+    pdl_wait();
+    pdl_trigger();
     const int t = blockIdx.x;
     const int slot = slots[t];
     if (slot < 0) return;
@@ -152,10 +156,10 @@ OXR_API int oxr_scatter_rows(void* pool, long long slot_stride, long long pool_s
                              cudaStream_t stream) {
     if (n_tokens <= 0 || width <= 0) return 0;
     if (dtype == 0)
-        scatter_rows_kernel<float><<<n_tokens, 128, 0, stream>>>((float*)pool, slot_stride, pool_slots, (const float*)src, src_stride, col0, width, slots, status,
+        oxr_launch_small(scatter_rows_kernel<float>, dim3(n_tokens), dim3(128), 0, stream, (float*)pool, slot_stride, pool_slots, (const float*)src, src_stride, col0, width, slots, status,
                                                                 (float*)pool2, slot_stride2, width2);
     else
-        scatter_rows_kernel<__nv_bfloat16><<<n_tokens, 128, 0, stream>>>((__nv_bfloat16*)pool, slot_stride, pool_slots, (const __nv_bfloat16*)src, src_stride, col0,
+        oxr_launch_small(scatter_rows_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(128), 0, stream, (__nv_bfloat16*)pool, slot_stride, pool_slots, (const __nv_bfloat16*)src, src_stride, col0,
                                                                         width, slots, status, (__nv_bfloat16*)pool2, slot_stride2, width2);
     return oxr_launch_status();
 }
@@ -169,6 +173,8 @@ template <typename T>
 __global__ void latent_prep_kernel(T* __restrict__ pool, long long slot_stride, long long pool_slots, const T* __restrict__ down, int down_stride, int rank, int rot,
                                    const float* __restrict__ weight, float eps, const T* q, int heads, int q_head_dim, int q_rot0, T* q_out,
                                    int qo_head_dim, int qo_rot0, const float* __restrict__ cos_t, const float* __restrict__ sin_t, int half, int halves, const int* __restrict__ slots, int* status) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const int t = blockIdx.x;
     const int step = halves ? 1 : 2, gap = halves ? half : 1;     // pair i: entries step * i and step * i + gap
@@ -269,6 +275,8 @@ __global__ void __launch_bounds__(128) latent_prep_words_kernel(__nv_bfloat16* _
                                                                 int q_head_dim, int q_rot0, __nv_bfloat16* q_out, int qo_head_dim, int qo_rot0,
                                                                 const float* __restrict__ cos_t, const float* __restrict__ sin_t, int half,
                                                                 const int* __restrict__ slots, int* status) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int A = HALVES ? 8 : 4;                                                       // angles of a piece
     const int t = blockIdx.x, lane = threadIdx.x & 31, slot = slots[t], per = half / A;     // pieces of a rotated part
     const __nv_bfloat16* row = down + (size_t)t * down_stride;
@@ -314,6 +322,8 @@ __global__ void __launch_bounds__(128) latent_prep_words_kernel(__nv_bfloat16* _
 
 __global__ void __launch_bounds__(128) cols_rms_norm_words_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ x, int stride, int width,
                                                                   const float* __restrict__ weight, float eps) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const __nv_bfloat16* row = x + (size_t)blockIdx.x * stride;
     constexpr int KEEP = 2;
@@ -359,16 +369,16 @@ OXR_API int oxr_latent_prep(void* pool, long long slot_stride, long long pool_sl
         q_head_dim % 8 == 0 && q_rot0 % 8 == 0 && qo_head_dim % 8 == 0 && qo_rot0 % 8 == 0 && (uintptr_t)pool % 16 == 0 && (uintptr_t)down % 16 == 0 &&
         (uintptr_t)q % 16 == 0 && (uintptr_t)q_out % 16 == 0 && (uintptr_t)weight % 16 == 0 && (uintptr_t)cos_t % 16 == 0 && (uintptr_t)sin_t % 16 == 0) {
         const auto kernel = halves ? latent_prep_words_kernel<true> : latent_prep_words_kernel<false>;
-        kernel<<<n_tokens, 128, 0, stream>>>((__nv_bfloat16*)pool, slot_stride, pool_slots, (const __nv_bfloat16*)down, down_stride, rank, weight, eps,
+        oxr_launch_small(kernel, dim3(n_tokens), dim3(128), 0, stream, (__nv_bfloat16*)pool, slot_stride, pool_slots, (const __nv_bfloat16*)down, down_stride, rank, weight, eps,
                                              (const __nv_bfloat16*)q, heads, q_head_dim, q_rot0, (__nv_bfloat16*)q_out, qo_head_dim, qo_rot0, cos_t, sin_t, half,
                                              slots, status);
         return oxr_launch_status();
     }
     if (dtype == 0)
-        latent_prep_kernel<float><<<n_tokens, 128, 0, stream>>>((float*)pool, slot_stride, pool_slots, (const float*)down, down_stride, rank, rot, weight, eps, (const float*)q, heads,
+        oxr_launch_small(latent_prep_kernel<float>, dim3(n_tokens), dim3(128), 0, stream, (float*)pool, slot_stride, pool_slots, (const float*)down, down_stride, rank, rot, weight, eps, (const float*)q, heads,
                                                                q_head_dim, q_rot0, (float*)q_out, qo_head_dim, qo_rot0, cos_t, sin_t, half, halves, slots, status);
     else
-        latent_prep_kernel<__nv_bfloat16><<<n_tokens, 128, 0, stream>>>((__nv_bfloat16*)pool, slot_stride, pool_slots, (const __nv_bfloat16*)down, down_stride, rank, rot, weight,
+        oxr_launch_small(latent_prep_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(128), 0, stream, (__nv_bfloat16*)pool, slot_stride, pool_slots, (const __nv_bfloat16*)down, down_stride, rank, rot, weight,
                                                                        eps, (const __nv_bfloat16*)q, heads, q_head_dim, q_rot0, (__nv_bfloat16*)q_out, qo_head_dim,
                                                                        qo_rot0, cos_t, sin_t, half, halves, slots, status);
     return oxr_launch_status();
@@ -377,6 +387,8 @@ OXR_API int oxr_latent_prep(void* pool, long long slot_stride, long long pool_sl
 // out[t] = x[t, 0:width] / rms * weight for rows `stride` apart (columns of a wider product): fp32 arithmetic, one rounding. One block per row.
 template <typename T>
 __global__ void cols_rms_norm_kernel(T* __restrict__ out, const T* __restrict__ x, int stride, int width, const float* __restrict__ weight, float eps) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[32];
     const T* row = x + (size_t)blockIdx.x * stride;
     float ss = 0.f;
@@ -392,12 +404,12 @@ OXR_API int oxr_cols_rms_norm(void* out, const void* x, int n, int stride, int w
     if (n <= 0) return 0;
     if (width <= 0 || stride < width) return OXR_BAD_ARGUMENT;
     if (dtype == 1 && width % 8 == 0 && stride % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)weight % 16 == 0) {
-        cols_rms_norm_words_kernel<<<n, 128, 0, stream>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)x, stride, width, weight, eps);
+        oxr_launch_small(cols_rms_norm_words_kernel, dim3(n), dim3(128), 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)x, stride, width, weight, eps);
         return oxr_launch_status();
     }
     const int threads = width >= 1024 ? 256 : 128;
-    if (dtype == 0) cols_rms_norm_kernel<float><<<n, threads, 0, stream>>>((float*)out, (const float*)x, stride, width, weight, eps);
-    else cols_rms_norm_kernel<__nv_bfloat16><<<n, threads, 0, stream>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)x, stride, width, weight, eps);
+    if (dtype == 0) oxr_launch_small(cols_rms_norm_kernel<float>, dim3(n), dim3(threads), 0, stream, (float*)out, (const float*)x, stride, width, weight, eps);
+    else oxr_launch_small(cols_rms_norm_kernel<__nv_bfloat16>, dim3(n), dim3(threads), 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)x, stride, width, weight, eps);
     return oxr_launch_status();
 }
 
@@ -407,6 +419,8 @@ OXR_API int oxr_cols_rms_norm(void* out, const void* x, int n, int stride, int w
 template <typename T, int TM>
 __global__ void __launch_bounds__(128) head_linear_kernel(T* __restrict__ out, int out_head_stride, int out0, const T* __restrict__ x, int x_head_stride,
                                                           int x0, const T* __restrict__ w, int n_in, int n_out, int heads, int n_tokens) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ float xs[];   // [TM, n_in]
     const int h = blockIdx.y, t0 = blockIdx.x * TM;
     for (int i = threadIdx.x; i < TM * n_in; i += blockDim.x) {
@@ -438,6 +452,8 @@ __device__ __forceinline__ float2 hl_load2(const __nv_bfloat16* p) { return __bf
 template <typename T, int TM>
 __global__ void __launch_bounds__(128) head_linear_few_kernel(T* __restrict__ out, int out_head_stride, int out0, const T* __restrict__ x, int x_head_stride,
                                                               int x0, const T* __restrict__ w, int n_in, int n_out, int heads, int n_tokens) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ float xs[];   // [TM, n_in], then [4][TM][64]
     float* part = xs + TM * n_in;
     const int h = blockIdx.y, t0 = blockIdx.x * TM, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.z * 64 + 2 * lane;
@@ -478,6 +494,65 @@ __global__ void __launch_bounds__(128) head_linear_few_kernel(T* __restrict__ ou
     }
 }
 
+// The same in bf16 with a warp's whole quarter of the matrix (at most KPW rows of 64 columns) in registers, asked for at once and before the wait for the
+// kernel that writes x (no kernel of a step writes weights). Eight rows at a time a block made four to six trips to memory one after the other: 13 tokens,
+// 32 heads of 128 x 192: 10.7 us, 5.2 here. The sums are the same, in the same order.
+template <int KPW>
+__global__ void __launch_bounds__(128) head_linear_few_words_kernel(__nv_bfloat16* __restrict__ out, int out_head_stride, int out0,
+                                                                    const __nv_bfloat16* __restrict__ x, int x_head_stride, int x0,
+                                                                    const __nv_bfloat16* __restrict__ w, int n_in, int n_out, int heads, int n_tokens) {
+    constexpr int TM = 8;
+    extern __shared__ __align__(16) float xs[];   // [TM, n_in], then [4][TM][64]
+    float* part = xs + TM * n_in;
+    const int h = blockIdx.y, t0 = blockIdx.x * TM, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.z * 64 + 2 * lane;
+    const int per = n_in / 4, k0 = warp * per;    // n_in a multiple of 16: whole quarters of whole 4-entry words
+    const __nv_bfloat16* wh = w + (size_t)h * n_in * n_out + (size_t)k0 * n_out + (c < n_out ? c : 0);
+    __nv_bfloat162 wr[KPW];
+#pragma unroll
+    for (int i = 0; i < KPW; ++i) wr[i] = i < per ? *reinterpret_cast<const __nv_bfloat162*>(wh + (size_t)i * n_out) : __floats2bfloat162_rn(0.f, 0.f);
+    pdl_wait();
+    pdl_trigger();
+    const int nk = n_in / 8;
+    for (int i = threadIdx.x; i < TM * nk; i += 128) {
+        const int m = i / nk, k = (i - m * nk) * 8;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (t0 + m < n_tokens) v = *reinterpret_cast<const uint4*>(x + ((size_t)(t0 + m) * heads + h) * x_head_stride + x0 + k);
+        float4* dst = reinterpret_cast<float4*>(xs + m * n_in + k);
+        dst[0] = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+        dst[1] = make_float4(__uint_as_float(v.z << 16), __uint_as_float(v.z & 0xffff0000u), __uint_as_float(v.w << 16), __uint_as_float(v.w & 0xffff0000u));
+    }
+    __syncthreads();
+    float acc[TM][2];
+#pragma unroll
+    for (int m = 0; m < TM; ++m) acc[m][0] = acc[m][1] = 0.f;
+#pragma unroll
+    for (int i = 0; i < KPW; i += 4) {
+        if (i >= per) break;
+        float2 wv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) wv[j] = __bfloat1622float2(wr[i + j]);
+#pragma unroll
+        for (int m = 0; m < TM; ++m) {
+            const float4 xv = *reinterpret_cast<const float4*>(xs + m * n_in + k0 + i);
+            acc[m][0] = fmaf(xv.x, wv[0].x, acc[m][0]); acc[m][1] = fmaf(xv.x, wv[0].y, acc[m][1]);
+            acc[m][0] = fmaf(xv.y, wv[1].x, acc[m][0]); acc[m][1] = fmaf(xv.y, wv[1].y, acc[m][1]);
+            acc[m][0] = fmaf(xv.z, wv[2].x, acc[m][0]); acc[m][1] = fmaf(xv.z, wv[2].y, acc[m][1]);
+            acc[m][0] = fmaf(xv.w, wv[3].x, acc[m][0]); acc[m][1] = fmaf(xv.w, wv[3].y, acc[m][1]);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < TM; ++m) *reinterpret_cast<float2*>(part + (warp * TM + m) * 64 + 2 * lane) = make_float2(acc[m][0], acc[m][1]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < TM * 32; i += 128) {
+        const int m = i / 32, p = 2 * (i % 32), o = blockIdx.z * 64 + p, at = m * 64 + p;
+        if (t0 + m < n_tokens && o < n_out) {
+            const float a = ((part[at] + part[TM * 64 + at]) + part[2 * TM * 64 + at]) + part[3 * TM * 64 + at];
+            const float b = ((part[at + 1] + part[TM * 64 + at + 1]) + part[2 * TM * 64 + at + 1]) + part[3 * TM * 64 + at + 1];
+            *reinterpret_cast<__nv_bfloat162*>(out + ((size_t)(t0 + m) * heads + h) * out_head_stride + out0 + o) = __floats2bfloat162_rn(a, b);
+        }
+    }
+}
+
 // The same on the tensor cores (bf16, fp32 sums in k order per 16-wide step): a block takes 64 tokens of one head, a warp 16 of them;
 // x rows and the head's matrix, 64 output columns at a time, stand in shared memory. n_in a multiple of 16, n_out of 16.
 __device__ __forceinline__ void hl_ldsm_x4(uint32_t (&r)[4], const __nv_bfloat16* p) {
@@ -498,6 +573,8 @@ constexpr int HL_BM = 64, HL_BN = 64;
 __global__ void __launch_bounds__(128) head_linear_mma_kernel(__nv_bfloat16* __restrict__ out, int out_head_stride, int out0,
                                                               const __nv_bfloat16* __restrict__ x, int x_head_stride, int x0,
                                                               const __nv_bfloat16* __restrict__ w, int n_in, int n_out, int heads, int n_tokens, int words) {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ __align__(16) unsigned char hl_smem[];
     const int lda = n_in + 8, ldb = HL_BN + 8;
     __nv_bfloat16* As = reinterpret_cast<__nv_bfloat16*>(hl_smem);   // [64][n_in + 8]
@@ -581,7 +658,7 @@ OXR_API int oxr_head_linear(void* out, int out_head_stride, int out0, const void
         dim3 grid((n_tokens + HL_BM - 1) / HL_BM, heads);
         const int words = x_head_stride % 8 == 0 && x0 % 8 == 0 && out_head_stride % 2 == 0 && out0 % 2 == 0 && (uintptr_t)x % 16 == 0 &&
                           (uintptr_t)w % 16 == 0 && (uintptr_t)out % 4 == 0;
-        head_linear_mma_kernel<<<grid, 128, mma_smem, stream>>>((__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_head_stride, x0,
+        oxr_launch(head_linear_mma_kernel, dim3(grid), dim3(128), mma_smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_head_stride, x0,
                                                                (const __nv_bfloat16*)w, n_in, n_out, heads, n_tokens, words);
         return oxr_launch_status();
     }
@@ -589,11 +666,18 @@ OXR_API int oxr_head_linear(void* out, int out_head_stride, int out0, const void
     const size_t few_smem = (size_t)(FEW * n_in + 4 * FEW * 64) * sizeof(float);
     if (n_tokens <= 16 && n_out % 2 == 0 && few_smem <= 48 * 1024 && (uintptr_t)w % 8 == 0) {
         dim3 grid((n_tokens + FEW - 1) / FEW, heads, (n_out + 63) / 64);
+        if (dtype == 1 && n_in % 16 == 0 && n_in <= 256 && x_head_stride % 8 == 0 && x0 % 8 == 0 && out_head_stride % 2 == 0 && out0 % 2 == 0 &&
+            (uintptr_t)x % 16 == 0 && (uintptr_t)out % 4 == 0) {
+            const auto kernel = n_in <= 128 ? head_linear_few_words_kernel<32> : (n_in <= 192 ? head_linear_few_words_kernel<48> : head_linear_few_words_kernel<64>);
+            oxr_launch(kernel, grid, dim3(128), few_smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_head_stride, x0,
+                             (const __nv_bfloat16*)w, n_in, n_out, heads, n_tokens);
+            return oxr_launch_status();
+        }
         if (dtype == 0)
-            head_linear_few_kernel<float, FEW><<<grid, 128, few_smem, stream>>>((float*)out, out_head_stride, out0, (const float*)x, x_head_stride, x0, (const float*)w,
+            oxr_launch(head_linear_few_kernel<float, FEW>, dim3(grid), dim3(128), few_smem, stream, false, (float*)out, out_head_stride, out0, (const float*)x, x_head_stride, x0, (const float*)w,
                                                                                 n_in, n_out, heads, n_tokens);
         else
-            head_linear_few_kernel<__nv_bfloat16, FEW><<<grid, 128, few_smem, stream>>>((__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x,
+            oxr_launch(head_linear_few_kernel<__nv_bfloat16, FEW>, dim3(grid), dim3(128), few_smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x,
                                                                                         x_head_stride, x0, (const __nv_bfloat16*)w, n_in, n_out, heads, n_tokens);
         return oxr_launch_status();
     }
@@ -602,10 +686,10 @@ OXR_API int oxr_head_linear(void* out, int out_head_stride, int out0, const void
     if (smem > 48 * 1024) return OXR_BAD_ARGUMENT;
     dim3 grid((n_tokens + TM - 1) / TM, heads);
     if (dtype == 0)
-        head_linear_kernel<float, TM><<<grid, 128, smem, stream>>>((float*)out, out_head_stride, out0, (const float*)x, x_head_stride, x0, (const float*)w, n_in,
+        oxr_launch(head_linear_kernel<float, TM>, dim3(grid), dim3(128), smem, stream, false, (float*)out, out_head_stride, out0, (const float*)x, x_head_stride, x0, (const float*)w, n_in,
                                                                   n_out, heads, n_tokens);
     else
-        head_linear_kernel<__nv_bfloat16, TM><<<grid, 128, smem, stream>>>((__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_head_stride, x0,
+        oxr_launch(head_linear_kernel<__nv_bfloat16, TM>, dim3(grid), dim3(128), smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_head_stride, x0,
                                                                           (const __nv_bfloat16*)w, n_in, n_out, heads, n_tokens);
     return oxr_launch_status();
 }

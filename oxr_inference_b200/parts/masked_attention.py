@@ -198,6 +198,11 @@ class MaskedAttention(Mixer):
             if self.value_mix == "keep":
                 ctx.shared[self.value_mix_key] = kept
             q_width = q.shape[1]
+        elif self.tiled and self.DK == self.DV and qkv.dtype == torch.bfloat16:
+            # q apart, K and V into the cache: one kernel (without a norm and a rotation it copies)
+            q = ops.qk_norm_rope_store(qkv, None, None, None, None, ctx.positions, group.slots if cache.store else ctx.no_store_slots, k_pool, v_pool,
+                                       self.H, self.KV, self.DK, 0.0, ctx.status).view(ctx.n_tokens, self.cq)
+            q_width = self.cq
         else:
             if cache.store:
                 ops.scatter_rows(k_pool, qkv, self.cq, group.slots, ctx.status, pool2=v_pool)   # the k columns, then the v columns
