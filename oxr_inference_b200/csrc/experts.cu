@@ -392,10 +392,57 @@ __global__ void combine_rows_kernel(T* __restrict__ out, const T* __restrict__ y
     }
 }
 
+// The same on bf16 rows of whole 16-byte words, eight entries a thread, the rows of up to four choices asked for together. An entry at a time, each behind its
+// choice's place, 1,421 tokens of 4 x 4,096 took 29 us, 10.5 here (9 us of bytes).
+__global__ void __launch_bounds__(256) combine_rows_words_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ y, const int* __restrict__ place,
+                                                                 const float* __restrict__ weights, int top, int width, const __nv_bfloat16* __restrict__ x,
+                                                                 const float* __restrict__ kept) {
+    pdl_wait();
+    pdl_trigger();
+    const int t = blockIdx.x;
+    auto add = [](float (&acc)[8], float w, const uint4& v) {
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            acc[2 * i] = fmaf(w, __uint_as_float(u[i] << 16), acc[2 * i]);
+            acc[2 * i + 1] = fmaf(w, __uint_as_float(u[i] & 0xffff0000u), acc[2 * i + 1]);
+        }
+    };
+    for (int c = 8 * threadIdx.x; c < width; c += 8 * blockDim.x) {
+        float acc[8] = {};
+        for (int j0 = 0; j0 < top; j0 += 4) {
+            uint4 v[4];
+            float w[4];
+            bool ok[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int at = j0 + j < top ? place[(size_t)t * top + j0 + j] : -1;
+                ok[j] = at >= 0;
+                w[j] = ok[j] ? weights[(size_t)t * top + j0 + j] : 0.f;
+                v[j] = ok[j] ? *reinterpret_cast<const uint4*>(y + (size_t)at * width + c) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (ok[j]) add(acc, w[j], v[j]);
+        }
+        if (x != nullptr) add(acc, kept[t], *reinterpret_cast<const uint4*>(x + (size_t)t * width + c));
+        uint4 o;
+        __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
+        *reinterpret_cast<uint4*>(out + (size_t)t * width + c) = o;
+    }
+}
+
 OXR_API int oxr_combine_rows(void* out, const void* y, const int* place, const float* weights, int n_tokens, int top, int width, const void* x, const float* kept,
                              int dtype, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (top <= 0 || width <= 0) return OXR_BAD_ARGUMENT;
+    if (dtype == 1 && width % 8 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)x % 16 == 0) {
+        oxr_launch_small(combine_rows_words_kernel, dim3(n_tokens), dim3(width >= 2048 ? 256 : 128), 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)y, place,
+                         weights, top, width, (const __nv_bfloat16*)x, kept);
+        return oxr_launch_status();
+    }
     if (dtype == 0) oxr_launch_small(combine_rows_kernel<float>, dim3(n_tokens), dim3(256), 0, stream, (float*)out, (const float*)y, place, weights, top, width, (const float*)x, kept);
     else oxr_launch_small(combine_rows_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(256), 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)y, place, weights, top, width, (const __nv_bfloat16*)x, kept);
     return oxr_launch_status();
