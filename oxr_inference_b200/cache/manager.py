@@ -98,8 +98,10 @@ class CacheManager:
             # TMA maps serve the kernels of plain grouped-query attention: keys and values of one size, causal or windowed
             self.kv_maps = [ops.make_kv_maps(k, v, page_size) if (g.need.value_dim is None and g.need.chunk == 0) else None
                             for g, k, v in zip(plan.groups, self.k_pools, self.v_pools)]
-            # masked groups, and groups whose key rows are the values, use them for their long tiles
-            self.long_maps = [own or (ops.make_kv_maps(k, k if v is None else v, page_size) if g.need.v_dim in (0, g.need.head_dim) else None)
+            # masked groups, and groups whose key rows are the values, use them for their long tiles, where the tiled kernels take their rows at all (wider
+            # ones, such as a latent row of 512 + 64 entries, have no library of kernels that could make a map)
+            self.long_maps = [own or (ops.make_kv_maps(k, k if v is None else v, page_size)
+                                      if ops.tiled_attention_takes(g.need.head_dim, g.need.v_dim or g.need.head_dim, dtype) else None)
                               for own, g, k, v in zip(self.kv_maps, plan.groups, self.k_pools, self.v_pools)]
 
     # ---- sizes

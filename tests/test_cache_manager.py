@@ -3,6 +3,7 @@
 import random
 
 import pytest
+import torch
 
 from oxr_inference_b200.cache import RELEASED, CacheManager, PagePool, make_cache_plan, pages_for
 from oxr_inference_b200.parts.base import PagedKVNeed, StateNeed
@@ -178,3 +179,27 @@ def test_room_is_what_the_held_pages_can_take():
     m.close(r)
     assert r.room == 0 and r.released == [0, 0]
     m.check()
+
+
+@pytest.mark.parametrize("head,value,chunk", [(576, 0, 0), (320, 0, 0), (320, 320, 24), (320, 64, 0), (576, 576, 24)])
+def test_rows_wider_than_the_tiled_kernels_get_no_maps(monkeypatch, head, value, chunk):
+    """Latent and masked groups whose rows are a multiple of 64 above 256 are served by the kernel that takes any row; a map of their pool would need a
+    library that does not exist. Narrower rows still get theirs."""
+    from oxr_inference_b200 import ops
+    from oxr_inference_b200.ops.build import check_head_dim
+
+    made = []
+
+    def make(k, v, page_size):   # what the real one does with a pool on the device
+        if k.shape[-1] % 64 == 0:
+            check_head_dim(k.shape[-1])
+        made.append(k.shape[-1])
+        return object()
+
+    monkeypatch.setattr(ops, "make_kv_maps", make)
+    zeros = torch.zeros
+    monkeypatch.setattr(torch, "zeros", lambda *a, device=None, **kw: zeros(*a, device="meta", **kw))
+    needs = [PagedKVNeed(1, head, value_dim=value, chunk=chunk), PagedKVNeed(1, 256, value_dim=0), PagedKVNeed(2, 128, value_dim=128, chunk=24)]
+    cache = CacheManager(make_cache_plan(needs, [None] * 3), page_size=16, num_pages=4, max_requests=2, device=torch.device("cuda"), dtype=torch.bfloat16)
+    assert cache.long_maps[0] is None and cache.long_maps[1] is not None and cache.long_maps[2] is not None
+    assert made == [256, 128]

@@ -87,6 +87,19 @@ def test_one_mechanism(name, dtype, tmp_path):
     close(run_cut(r, ids, [2, 3, 2, 11, 2, 17, 1, 2, 21]), want, dtype, f"{name}, portions")
 
 
+@pytest.mark.parametrize("name,layer", [("latent_512_and_64", RU.latent_layer(heads=3, dim=16, rot_dim=64, rot_dims=64, vdim=16, kv_rank=512, mlp=None)),
+                                        ("chunked_320", RU.attention_layer(heads=2, kv_heads=1, dim=320, vdim=320, mlp=None))])
+def test_rows_of_whole_words_wider_than_the_tiled_kernels(name, layer, tmp_path):
+    """Cache rows of 576 and 320 entries in pages of 16: sizes a tensor map could describe, but that no tiled kernel takes."""
+    cfg = RU.model_config([layer])
+    folder = RU.make_folder(tmp_path, cfg, name, seed=5)
+    ids = RU.tokens(cfg, 61, seed=1)
+    want = RU.plain_logits(folder, ids)
+    r = runner_for(folder, "bfloat16", page_size=16)
+    close(run_cut(r, ids, [61]), want, "bfloat16", f"{name}, whole prompt")
+    close(run_cut(r, ids, [2, 3, 2, 11, 2, 17, 1, 2, 21]), want, "bfloat16", f"{name}, portions")
+
+
 # ------------------------------------------------------------------------------------------------ whole models, every cutting
 MODELS = {"X": RU.MODEL_X, "Y": RU.MODEL_Y, "Z": RU.MODEL_Z}
 
