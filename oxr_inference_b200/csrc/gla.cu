@@ -6,21 +6,24 @@
 //   S_t = diag(alpha_t) S_(t-1) + k_t v_t^T          o_t = S_t^T q_t          q_t already scaled
 //
 // The decay (log-sigmoid, division by tau, exponential), S and every sum over it are fp32; T is the activation type of the q|k|v
-// projections; z is fp32. The recurrence runs token by token in the order of the sequence whatever the cut, so a position's result does
-// not depend on how a prompt was cut into steps. Columns of S (one value dimension each) are independent: a block takes 32 columns of one
-// head of one request.
+// projections; z is fp32. The recurrence runs token by token in the order of the sequence whatever the cut, and every kernel for it (the ones
+// below, and the one of scan_columns.cuh) adds up o in one order, so a position's result does not depend on how a prompt was cut into steps nor on
+// what else is in the batch. Columns of S (one value dimension each) are independent: a block takes 32 columns of one head of one request.
 //
 // grid (ceil(DV / 32), heads, requests); block = 32 * NW threads with NW = ceil(DK / KPT). Lane l owns the value column p = 32 blockIdx.x + l,
-// warp w the key entries KPT w .. KPT w + KPT - 1: a thread keeps KPT = 32 or 16 entries of S in registers (16: twice the warps for the same
+// warp w the key entries 4 (w + NW m) .. + 3 for m = 0 .. KPT / 4 - 1: a thread keeps KPT = 32 or 16 entries of S in registers (16: twice the warps for the same
 // state, which is what hides the loop's latencies when a step brings many tokens of a request; keys of up to 128). A tile of TT tokens goes through shared memory at
 // a time (thread d brings entry d of k, q and the decay of each token; the next tile's loads are in flight while this one is computed); the
-// warps' partial sums of S^T q meet in shared memory and are added in the order of the warps after the tile.
+// warps' partial sums of S^T q meet in shared memory and are added after the tile. Every NW-th four entries to a warp, so that a thread's sums are the
+// first ones of the order in scan_columns.cuh.
 #include "scan_columns.cuh"
 
 __device__ __forceinline__ float gla_log_sigmoid(float v) { return fminf(v, 0.f) - log1pf(expf(-fabsf(v))); }
 
+// The bound on registers: twelve warps an SM (16 with eight warps of 16 entries), without it the compiler takes registers for eight. Single tokens of 48
+// requests, 16 heads of 128 x 256: 59 us, 80 without the bound.
 template <typename T, int NW, int TT, int KPT>
-__global__ void __launch_bounds__(32 * NW) gla_scan_kernel(
+__global__ void __launch_bounds__(32 * NW, NW == 8 ? (KPT == 32 ? 1 : 2) : 12 / NW) gla_scan_kernel(
     float* __restrict__ y, const T* __restrict__ proj, int proj_stride, int q_col0, int k_col0, int v_col0, const float* __restrict__ z,
     const float* __restrict__ z_bias, float inv_tau, int heads, int DK, int DV, float q_scale, float* __restrict__ state, long long slot_stride,
     const int* __restrict__ cu_q, const int* __restrict__ state_slots) {
@@ -35,10 +38,11 @@ __global__ void __launch_bounds__(32 * NW) gla_scan_kernel(
     const int t0 = cu_q[r], t1 = cu_q[r + 1];
     if (t1 <= t0) return;
     float* S = state + (long long)state_slots[r] * slot_stride + (long long)h * DK * DV;
-    const int n0 = KPT * warp;
-    float s[KPT];
+    f32x2 s[KPT / 2];                                // pair i: entries entry(i) and entry(i) + 1
+    auto entry = [&](int i) { return 4 * (warp + NW * (i >> 1)) + 2 * (i & 1); };
+    auto stored = [&](int e) { return (e < DK && p < DV) ? S[(size_t)e * DV + p] : 0.f; };
 #pragma unroll
-    for (int k = 0; k < KPT; ++k) s[k] = (n0 + k < DK && p < DV) ? S[(size_t)(n0 + k) * DV + p] : 0.f;
+    for (int i = 0; i < KPT / 2; ++i) s[i] = pack2(stored(entry(i)), stored(entry(i) + 1));
     const float zb = n < DK ? z_bias[h * DK + n] : 0.f;
 
     constexpr int VPT = (TT * 32 + NT - 1) / NT;      // v values per thread and tile
@@ -66,7 +70,7 @@ __global__ void __launch_bounds__(32 * NW) gla_scan_kernel(
         for (int t = 0; t < TT; ++t) {
             if (n < DKP) {
                 ks[t][n] = Num<T>::to_f32(kreg[t]);
-                qs[t][n] = Num<T>::to_f32(qreg[t]) * q_scale;
+                qs[t][n] = Num<T>::to_f32(qreg[t]);
                 as[t][n] = expf(gla_log_sigmoid(zreg[t] + zb) * inv_tau);
             }
         }
@@ -85,32 +89,27 @@ __global__ void __launch_bounds__(32 * NW) gla_scan_kernel(
         if (more) fetch(tile + TT);
         for (int t = 0; t < nt; ++t) {
             const float tv = vs[t][lane];
-            const float4* k4 = reinterpret_cast<const float4*>(&ks[t][n0]);
-            const float4* q4 = reinterpret_cast<const float4*>(&qs[t][n0]);
-            const float4* a4 = reinterpret_cast<const float4*>(&as[t][n0]);
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};   // four chains, added in a fixed order
+            const f32x2 tv2 = pack2(tv, tv);
+            float four[KPT / 4];
 #pragma unroll
-            for (int j = 0; j < KPT / 4; ++j) {
-                const float4 kk = k4[j], qq = q4[j], aa = a4[j];
-                s[4 * j] = fmaf(aa.x, s[4 * j], tv * kk.x);
-                sum[0] = fmaf(s[4 * j], qq.x, sum[0]);
-                s[4 * j + 1] = fmaf(aa.y, s[4 * j + 1], tv * kk.y);
-                sum[1] = fmaf(s[4 * j + 1], qq.y, sum[1]);
-                s[4 * j + 2] = fmaf(aa.z, s[4 * j + 2], tv * kk.z);
-                sum[2] = fmaf(s[4 * j + 2], qq.z, sum[2]);
-                s[4 * j + 3] = fmaf(aa.w, s[4 * j + 3], tv * kk.w);
-                sum[3] = fmaf(s[4 * j + 3], qq.w, sum[3]);
+            for (int m = 0; m < KPT / 4; ++m) {
+                const int e = entry(2 * m);
+                const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(&ks[t][e]), qq = *reinterpret_cast<const ulonglong2*>(&qs[t][e]),
+                                 aa = *reinterpret_cast<const ulonglong2*>(&as[t][e]);
+                s[2 * m] = fma2(aa.x, s[2 * m], mul2(kk.x, tv2));
+                s[2 * m + 1] = fma2(aa.y, s[2 * m + 1], mul2(kk.y, tv2));
+                four[m] = scan_sum_four(s[2 * m], s[2 * m + 1], qq.x, qq.y);
             }
-            part[t][warp][lane] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            part[t][warp][lane] = scan_halve<KPT / 4>(four);
         }
         __syncthreads();
         for (int i = n; i < nt * 32; i += NT) {
             const int t = i >> 5, c = i & 31;
             if (p0 + c < DV) {
-                float num = 0.f;
+                float v[NW];
 #pragma unroll
-                for (int w = 0; w < NW; ++w) num += part[t][w][c];
-                y[(size_t)(tile + t) * heads * DV + h * DV + p0 + c] = num;
+                for (int w = 0; w < NW; ++w) v[w] = part[t][w][c];
+                y[(size_t)(tile + t) * heads * DV + h * DV + p0 + c] = scan_halve<NW>(v) * q_scale;
             }
         }
         if (more) {
@@ -119,9 +118,15 @@ __global__ void __launch_bounds__(32 * NW) gla_scan_kernel(
             __syncthreads();
         }
     }
+    if (p < DV) {
 #pragma unroll
-    for (int k = 0; k < KPT; ++k)
-        if (n0 + k < DK && p < DV) S[(size_t)(n0 + k) * DV + p] = s[k];
+        for (int i = 0; i < KPT / 2; ++i) {
+            float lo, hi;
+            unpack2(s[i], lo, hi);
+            if (entry(i) < DK) S[(size_t)entry(i) * DV + p] = lo;
+            if (entry(i) + 1 < DK) S[(size_t)(entry(i) + 1) * DV + p] = hi;
+        }
+    }
 }
 
 // decay[t, i] = sigmoid(z[t, i] + bias[i])^(1 / tau), four entries a thread: once per token and key channel, where the recurrence's blocks (one per 32 value

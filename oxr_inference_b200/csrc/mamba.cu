@@ -8,9 +8,10 @@
 //
 //   S_t = decay_t S_(t-1) + dt_t B_t x_t^T          y_t = S_t^T C_t + D x_t
 //
-// The recurrence runs token by token in the order of the sequence whatever the cut, so a position's result does not
-// depend on how the prompt was cut into steps. Columns of S (one value dimension p each) are independent: a block takes
-// 32 columns of one head of one request.
+// The recurrence runs token by token in the order of the sequence whatever the cut, and both kernels for it (the one below, and the one of
+// scan_columns.cuh for steps that bring many tokens) add up y in one order, so a position's result does not depend on how the prompt was cut
+// into steps nor on what else is in the batch. Columns of S (one value dimension p each) are independent: a block takes 32 columns of one head of
+// one request.
 #include "scan_columns.cuh"
 
 // ---------------------------------------------------------------------------------------------- convolution
@@ -120,17 +121,16 @@ __global__ void conv_tail_roll_kernel(float* __restrict__ state, long long slot_
 }
 
 // ---------------------------------------------------------------------------------------------- recurrence
-__device__ __forceinline__ float softplus_f32(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
-
 // grid (ceil(vdim / 32), heads, requests); block = 32 * NW threads with NW = ceil(N / 32). Lane l owns the value column
-// p = 32 blockIdx.x + l, warp w the state entries n = 32 w .. 32 w + 31, so a thread keeps 32 entries of S in registers and
-// updates them with plain multiply-adds: B and C of a token are the same for all lanes and come from shared memory as
+// p = 32 blockIdx.x + l, warp w the state entries 4 (w + NW m) .. + 3 for m = 0 .. 7, so a thread keeps 32 entries of S in registers and
+// updates them with plain multiply-adds in pairs: B and C of a token are the same for all lanes and come from shared memory as
 // broadcast 16-byte loads, no shuffles. The step's tokens go through shared memory TT at a time (B, C, x, softplus and decay,
 // each computed once per token and block; the next tile is fetched while this one is computed); the warps' partial sums of y
-// meet there too and are added in the order of the warps.
+// meet there too. Every NW-th four entries to a warp, so that a thread's sums are the first ones of the order in scan_columns.cuh.
 // S is stored [heads, N, vdim]: the lanes of a warp read and write 128 contiguous bytes per state entry.
+// The bound on registers: a step of single tokens is the state's way through them, and three blocks of four warps on an SM are what it took before.
 template <typename T, int NW, int TT>
-__global__ void __launch_bounds__(32 * NW) ssm_scan_kernel(
+__global__ void __launch_bounds__(32 * NW, NW == 4 ? 3 : 1) ssm_scan_kernel(
     float* __restrict__ y, const T* __restrict__ xbc, const T* __restrict__ proj, int proj_stride, int dt_col0, int heads, int vdim, int N,
     int groups, const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip, float* __restrict__ state,
     long long slot_stride, const int* __restrict__ cu_q, const int* __restrict__ state_slots) {
@@ -148,11 +148,13 @@ __global__ void __launch_bounds__(32 * NW) ssm_scan_kernel(
     const int t0 = cu_q[r], t1 = cu_q[r + 1];
     if (t1 <= t0) return;
     const int inner = heads * vdim, channels = inner + 2 * groups * N, g = h / (heads / groups);
-    const int b_col = inner + g * N, c_col = inner + groups * N + g * N, n0 = 32 * warp;
+    const int b_col = inner + g * N, c_col = inner + groups * N + g * N;
     float* S = state + (long long)state_slots[r] * slot_stride + (long long)h * N * vdim;
-    float s[32];
+    f32x2 s[16];                                      // pair i: entries entry(i) and entry(i) + 1
+    auto entry = [&](int i) { return 4 * (warp + NW * (i >> 1)) + 2 * (i & 1); };
+    auto stored = [&](int e) { return (e < N && p < vdim) ? S[(size_t)e * vdim + p] : 0.f; };
 #pragma unroll
-    for (int k = 0; k < 32; ++k) s[k] = (n0 + k < N && p < vdim) ? S[(size_t)(n0 + k) * vdim + p] : 0.f;
+    for (int i = 0; i < 16; ++i) s[i] = pack2(stored(entry(i)), stored(entry(i) + 1));
     const float neg_a = -expf(a_log[h]), bias = dt_bias[h], skip = d_skip[h];
 
     // A tile's inputs are fetched into registers while the tile before it is computed (all loads of a tile are issued back to
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(32 * NW) ssm_scan_kernel(
             if (i < TT * 32) xs[i] = Num<T>::to_f32(xv[j]);
         }
         if ((int)threadIdx.x < nt) {
-            const float dt = softplus_f32(Num<T>::to_f32(dtv) + bias);
+            const float dt = scan_softplus(Num<T>::to_f32(dtv) + bias);
             dts[threadIdx.x] = dt;
             decays[threadIdx.x] = expf(neg_a * dt);
         }
@@ -203,31 +205,25 @@ __global__ void __launch_bounds__(32 * NW) ssm_scan_kernel(
         if (more) fetch(tile + TT);
         for (int t = 0; t < nt; ++t) {
             const float decay = decays[t], dx = dts[t] * xs[t * 32 + lane];
-            const float4* b4 = reinterpret_cast<const float4*>(Bs + t * NP + n0);
-            const float4* c4 = reinterpret_cast<const float4*>(Cs + t * NP + n0);
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};   // four chains instead of one of 32 dependent multiply-adds; added in a fixed order
+            const f32x2 decay2 = pack2(decay, decay), dx2 = pack2(dx, dx);
+            float four[8];
 #pragma unroll
-            for (int k4 = 0; k4 < 8; ++k4) {
-                const float4 b = b4[k4], c = c4[k4];
-                s[4 * k4] = fmaf(decay, s[4 * k4], dx * b.x);
-                sum[0] = fmaf(s[4 * k4], c.x, sum[0]);
-                s[4 * k4 + 1] = fmaf(decay, s[4 * k4 + 1], dx * b.y);
-                sum[1] = fmaf(s[4 * k4 + 1], c.y, sum[1]);
-                s[4 * k4 + 2] = fmaf(decay, s[4 * k4 + 2], dx * b.z);
-                sum[2] = fmaf(s[4 * k4 + 2], c.z, sum[2]);
-                s[4 * k4 + 3] = fmaf(decay, s[4 * k4 + 3], dx * b.w);
-                sum[3] = fmaf(s[4 * k4 + 3], c.w, sum[3]);
+            for (int m = 0; m < 8; ++m) {
+                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(Bs + t * NP + entry(2 * m)), c = *reinterpret_cast<const ulonglong2*>(Cs + t * NP + entry(2 * m));
+                s[2 * m] = fma2(decay2, s[2 * m], mul2(b.x, dx2));
+                s[2 * m + 1] = fma2(decay2, s[2 * m + 1], mul2(b.y, dx2));
+                four[m] = scan_sum_four(s[2 * m], s[2 * m + 1], c.x, c.y);
             }
-            part[(t * NW + warp) * 32 + lane] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            part[(t * NW + warp) * 32 + lane] = scan_halve<8>(four);
         }
         __syncthreads();
         for (int i = threadIdx.x; i < nt * 32; i += 32 * NW) {
             const int t = i >> 5, c = i & 31;
             if (p0 + c >= vdim) continue;
-            float v = 0.f;
+            float v[NW];
 #pragma unroll
-            for (int w = 0; w < NW; ++w) v += part[(t * NW + w) * 32 + c];
-            y[(size_t)(tile + t) * inner + h * vdim + p0 + c] = fmaf(skip, xs[i], v);
+            for (int w = 0; w < NW; ++w) v[w] = part[(t * NW + w) * 32 + c];
+            y[(size_t)(tile + t) * inner + h * vdim + p0 + c] = fmaf(skip, xs[i], scan_halve<NW>(v));
         }
         if (!more) break;
         __syncthreads();   // everyone has read this tile's buffers
@@ -236,8 +232,12 @@ __global__ void __launch_bounds__(32 * NW) ssm_scan_kernel(
     }
     if (p < vdim) {
 #pragma unroll
-        for (int k = 0; k < 32; ++k)
-            if (n0 + k < N) S[(size_t)(n0 + k) * vdim + p] = s[k];
+        for (int i = 0; i < 16; ++i) {
+            float lo, hi;
+            unpack2(s[i], lo, hi);
+            if (entry(i) < N) S[(size_t)entry(i) * vdim + p] = lo;
+            if (entry(i) + 1 < N) S[(size_t)(entry(i) + 1) * vdim + p] = hi;
+        }
     }
 }
 

@@ -2,8 +2,10 @@
 //
 //   S_t = decay_t * S_(t-1) + k_t x_t^T          o_t = S_t^T q_t          S [DK, DV] per request and head, fp32
 //
-// with a decay per key entry (VECTOR) or one per token and head. Token by token in the order of the sequence whatever the cut, so a position's
-// result does not depend on how a prompt was cut into steps. Columns of S are independent.
+// with a decay per key entry (VECTOR) or one per token and head. Columns of S are independent. Token by token in the order of the sequence, and with one
+// order of the sum S^T q in every kernel that takes these recurrences (this one with four or eight entries a lane, and the two for few tokens a
+// request in gla.cu and mamba.cu): four neighbouring entries first, then the upper half of the fours onto the lower half until one is left. So a position's result has
+// the same bits however a prompt was cut into steps and whatever else is in the batch.
 //
 // What bounds it: a thread that owns one column reads 4 bytes of k, q and decay from shared memory for every entry it updates, and shared memory returns
 // 64 bytes a cycle to an SM's registers (measured), so the loads took several times as long as the multiply-adds they fed. Here a thread owns E = 4 or 8
@@ -12,8 +14,8 @@
 // activations' type until they are in registers. The dot products of J / 8 tokens meet in one butterfly that halves their number with every
 // step (lane j ends with number j / 2 of them). What is left is issue slots: about 100 (E = 4) or 157 (E = 8) a token and warp.
 // Raw values come by cp.async, tiles of TT tokens, STAGES - 1 tiles ahead; one barrier per tile. 32 / E warps a block.
-// 2,048 tokens on a B200: 16 heads of 128 x 256 with a decay per entry 409 us (one column a thread: 739); 128 heads of 128 x 64 with one per token 637
-// (704), prompts of 700 and 700 tokens 341 (473), 16 of 64 224 (272).
+// 2,048 tokens on a B200, L2 flushed before: 16 heads of 128 x 256 with a decay per entry 402 us (one column a thread: 774); 128 heads of 128 x 64 with one per
+// token 614 (705), prompts of 700 and 700 tokens 356 (506).
 #pragma once
 
 #include <type_traits>
@@ -39,6 +41,29 @@ template <int N> __device__ __forceinline__ float group_reduce(float (&v)[N], in
             half[i] = keep + __shfl_xor_sync(0xffffffffu, send, N);
         }
         return group_reduce<N / 2>(half, lane);
+    }
+}
+
+// The first step of every sum S^T q: the products of four neighbouring entries (two pairs), the second pair's added to the first's, then the halves
+__device__ __forceinline__ float scan_sum_four(f32x2 s01, f32x2 s23, f32x2 q01, f32x2 q23) {
+    float lo, hi;
+    unpack2(fma2(s23, q23, mul2(s01, q01)), lo, hi);
+    return lo + hi;
+}
+
+// The others: the upper half onto the lower until one is left (N a power of two; else one after the other, for sizes that one kernel alone takes)
+template <int N> __device__ __forceinline__ float scan_halve(const float (&v)[N]) {
+    if constexpr (N == 1) return v[0];
+    else if constexpr (N % 2 == 0) {
+        float half[N / 2];
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) half[i] = v[i] + v[N / 2 + i];
+        return scan_halve<N / 2>(half);
+    } else {
+        float sum = v[0];
+#pragma unroll
+        for (int i = 1; i < N; ++i) sum += v[i];
+        return sum;
     }
 }
 
@@ -222,18 +247,15 @@ __global__ void __launch_bounds__(ScanShape<T, J, E, VECTOR>::THREADS) column_sc
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const f32x2 xx = pack2(x[c], x[c]);
-                        f32x2 sum = 0, sum1 = 0;      // two chains of pairs, added in a fixed order
+                        float four[P / 2];
 #pragma unroll
                         for (int i = 0; i < P; i += 2) {
                             s[c][i] = fma2(aa[i], s[c][i], mul2(kk[i], xx));
                             s[c][i + 1] = fma2(aa[i + 1], s[c][i + 1], mul2(kk[i + 1], xx));
-                            sum = i == 0 ? mul2(s[c][i], qq[i]) : fma2(s[c][i], qq[i], sum);
-                            sum1 = i == 0 ? mul2(s[c][i + 1], qq[i + 1]) : fma2(s[c][i + 1], qq[i + 1], sum1);
+                            four[i / 2] = scan_sum_four(s[c][i], s[c][i + 1], qq[i], qq[i + 1]);
                         }
-                        float lo, hi, lo1, hi1;
-                        unpack2(sum, lo, hi);
-                        unpack2(sum1, lo1, hi1);
-                        d[4 * k + c] = (lo + hi) + (lo1 + hi1);
+                        if constexpr (E == 8) d[4 * k + c] = four[0] + four[1];
+                        else d[4 * k + c] = four[0];
                     }
                 }
                 float o = group_reduce<4 * TPG>(d, lane);

@@ -2020,7 +2020,7 @@ def gla_scan(proj: torch.Tensor, q_col0: int, k_col0: int, v_col0: int, z: torch
     decay = None
     if not key_entries_per_thread:
         # portions of prompts: the kernel whose threads hold several columns, where it takes the sizes, else twice the warps per head (2,048 tokens of
-        # 16 heads of 128 x 256: 409 against 739 us); single tokens: the state's trip through the registers is all there is, and fewer
+        # 16 heads of 128 x 256: 402 against 774 us); single tokens: the state's trip through the registers is all there is, and fewer
         # partial sums are cheaper (20.5 against 24.6 us)
         many = n > 2 * n_requests
         key_entries_per_thread = 16 if many else 32

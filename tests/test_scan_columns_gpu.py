@@ -79,3 +79,48 @@ def test_decay_per_token(ops, H, N, P, G, lengths, dtype):
             want[t] = torch.einsum("hnp,hn->hp", S, c[t]) + skip.double()[:, None] * x[t]
     close(got, want.view(n, -1))
     close(left, after)
+
+
+def tokens_of(kind, n, H, DK, DV, dtype, g):
+    """One request's inputs, a row per token."""
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    if kind == "entry":
+        return rnd(n, H * (2 * DK + DV)).to(dtype), rnd(n, H * DK) * 2
+    return rnd(n, H * DV + 2 * 2 * DK).to(dtype), rnd(n, 8 + H).to(dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kind,H,DK,DV", [("entry", 16, 128, 128), ("entry", 64, 64, 72), ("entry", 2, 256, 40), ("entry", 2, 48, 64), ("entry", 3, 16, 24), ("entry", 1, 20, 8),
+                                          ("token", 32, 128, 64), ("token", 64, 64, 72), ("token", 2, 256, 40), ("token", 2, 40, 64), ("token", 4, 100, 36)])
+def test_same_bits_however_cut_and_whatever_else_is_in_the_batch(ops, kind, H, DK, DV, dtype):
+    """One sequence in a step of its own, in portions with single tokens between, and beside others: few requests and many (from 2,048 warps of eight
+    entries on, a lane of the kernel for many tokens holds eight entries instead of four), single tokens and portions."""
+    g = torch.Generator(device=DEV).manual_seed(7)
+    per_head = torch.randn(3, H * (DK if kind == "entry" else 1), generator=g, device=DEV) * 0.5
+    mine = tokens_of(kind, 61, H, DK, DV, dtype, g)
+    start = torch.randn(H * DK * DV, generator=g, device=DEV)
+
+    def step(requests, state, slots):
+        cu, cu_q, _ = split([len(r[0]) for r in requests])
+        rows, extra = (torch.cat([r[i] for r in requests]) for i in (0, 1))
+        common = dict(heads=H, cu_q=cu_q, state_slots=torch.tensor(slots, dtype=torch.int32, device=DEV), n_requests=len(requests))
+        if kind == "entry":
+            return ops.gla_scan(rows, 0, H * DK, 2 * H * DK, extra, per_head[0], key_dim=DK, value_dim=DV, tau=4.0, q_scale=0.3, state=state, **common), cu
+        return ops.mamba_scan(rows, extra, 8, vdim=DV, state=DK, groups=2, dt_bias=per_head[0], a_log=per_head[1] - 2, d_skip=per_head[2],
+                              ssm=state, **common), cu
+
+    alone = start.repeat(1, 1)
+    want, _ = step([mine], alone, [0])
+    cut, rows, at = start.repeat(1, 1), [], 0
+    for n in (1, 2, 1, 5, 17, 3, 1, 1, 30):
+        rows.append(step([[t[at:at + n] for t in mine]], cut, [0])[0])
+        at += n
+    assert at == 61 and torch.equal(torch.cat(rows), want) and torch.equal(cut, alone)
+    for others in ([1], [1] * 8, [40, 1, 3, 70, 1, 1, 9, 2], [1] * 70):
+        states = torch.randn(len(others) + 1, H * DK * DV, generator=g, device=DEV)
+        states[len(others) // 2] = start
+        step_of = [tokens_of(kind, n, H, DK, DV, dtype, g) for n in others]
+        step_of.insert(len(others) // 2, mine)
+        got, cu = step(step_of, states, list(range(len(others) + 1)))
+        first = cu[len(others) // 2]
+        assert torch.equal(got[first:first + 61], want) and torch.equal(states[len(others) // 2], alone[0])
