@@ -44,11 +44,14 @@ template <int N> __device__ __forceinline__ float group_reduce(float (&v)[N], in
     }
 }
 
+__device__ __forceinline__ float add_halves(f32x2 v) {
+    float lo, hi;
+    unpack2(v, lo, hi);
+    return lo + hi;
+}
 // The first step of every sum S^T q: the products of four neighbouring entries (two pairs), the second pair's added to the first's, then the halves
 __device__ __forceinline__ float scan_sum_four(f32x2 s01, f32x2 s23, f32x2 q01, f32x2 q23) {
-    float lo, hi;
-    unpack2(fma2(s23, q23, mul2(s01, q01)), lo, hi);
-    return lo + hi;
+    return add_halves(fma2(s23, q23, mul2(s01, q01)));
 }
 
 // The others: the upper half onto the lower until one is left (N a power of two; else one after the other, for sizes that one kernel alone takes)
@@ -247,15 +250,29 @@ __global__ void __launch_bounds__(ScanShape<T, J, E, VECTOR>::THREADS) column_sc
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const f32x2 xx = pack2(x[c], x[c]);
-                        float four[P / 2];
+                        if constexpr (E == 8 && !VECTOR) {
+                            // the same sums, the first pairs of both fours before the second ones: 6 to 12 % less time (Mamba-2, 128 heads of 128 x 64, 3 prompts
+                            // of 700 tokens: 569 and 508 us), where four entries a lane or a decay per entry take more
+                            f32x2 pairs[2];
 #pragma unroll
-                        for (int i = 0; i < P; i += 2) {
-                            s[c][i] = fma2(aa[i], s[c][i], mul2(kk[i], xx));
-                            s[c][i + 1] = fma2(aa[i + 1], s[c][i + 1], mul2(kk[i + 1], xx));
-                            four[i / 2] = scan_sum_four(s[c][i], s[c][i + 1], qq[i], qq[i + 1]);
+                            for (int half = 0; half < 2; ++half)
+#pragma unroll
+                                for (int i = half; i < P; i += 2) {
+                                    s[c][i] = fma2(aa[i], s[c][i], mul2(kk[i], xx));
+                                    pairs[i / 2] = half == 0 ? mul2(s[c][i], qq[i]) : fma2(s[c][i], qq[i], pairs[i / 2]);
+                                }
+                            d[4 * k + c] = add_halves(pairs[0]) + add_halves(pairs[1]);
+                        } else {
+                            float four[P / 2];
+#pragma unroll
+                            for (int i = 0; i < P; i += 2) {
+                                s[c][i] = fma2(aa[i], s[c][i], mul2(kk[i], xx));
+                                s[c][i + 1] = fma2(aa[i + 1], s[c][i + 1], mul2(kk[i + 1], xx));
+                                four[i / 2] = scan_sum_four(s[c][i], s[c][i + 1], qq[i], qq[i + 1]);
+                            }
+                            d[4 * k + c] = four[0];
+                            if constexpr (E == 8) d[4 * k + c] += four[1];
                         }
-                        if constexpr (E == 8) d[4 * k + c] = four[0] + four[1];
-                        else d[4 * k + c] = four[0];
                     }
                 }
                 float o = group_reduce<4 * TPG>(d, lane);
