@@ -38,6 +38,7 @@ struct DeltaArgs {
     const int* cu_q;
     const int* state_slots;
     int async;                                // every row piece is whole 16-byte words: copied ahead by cp.async
+    RequestOrder order = {nullptr, 0};        // the requests in the order of their blocks
 };
 
 constexpr int DELTA_TT = 8, DELTA_COLS = 32, DELTA_WARPS = 4, DELTA_PREP_WARPS = DELTA_TT,      // tokens per tile; columns per block; computing warps; preparing warps, one per token
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delt
     constexpr int DKP = Sh::DKP, CPT = Sh::CPT, KL = (DKP + 31) / 32;      // KL: key entries per lane when a warp prepares a token
     extern __shared__ __align__(16) float dsm[];      // [2][TILE], then the results [2][TT][COLS]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int p0 = blockIdx.x * DELTA_COLS, h = blockIdx.y, r = longest_first(a.cu_q, gridDim.z, blockIdx.z);
+    const int p0 = blockIdx.x * DELTA_COLS, h = blockIdx.y, r = request_of(a.order, gridDim.z, blockIdx.z);
     const int t0 = a.cu_q[r], t1 = a.cu_q[r + 1];
     if (t1 <= t0) return;
     const int DK = a.DK, DV = a.DV, n_tiles = (t1 - t0 + DELTA_TT - 1) / DELTA_TT;
@@ -456,13 +457,14 @@ static int delta_launch_j(float* y, const T* proj, const DeltaArgs& a, int n_req
 OXR_API int oxr_delta_scan(float* y, const void* proj, int n_requests, int stride, int r_col0, int k_col0, int v_col0, const float* zw, int zw_stride,
                            const float* w0, const float* za, int za_stride, const float* ab, float rate, float len_eps, int heads, int DK, int DV,
                            float* state, long long slot_stride, const int* cu_q, const int* state_slots, int single, int dtype,
-                           cudaStream_t stream) {
+                           const int* order, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (heads <= 0 || DK <= 0 || DK > 256 || DV <= 0 || heads > 65535 || n_requests > 65535 || !(rate > 0.f) || !(len_eps > 0.f)) return OXR_BAD_ARGUMENT;
     DeltaArgs a;
     a.stride = stride; a.r_col0 = r_col0; a.k_col0 = k_col0; a.v_col0 = v_col0; a.zw = zw; a.zw_stride = zw_stride; a.w0 = w0; a.za = za;
     a.za_stride = za_stride; a.ab = ab; a.rate = rate; a.len_eps = len_eps; a.heads = heads; a.DK = DK; a.DV = DV; a.state = state;
     a.slot_stride = slot_stride; a.cu_q = cu_q; a.state_slots = state_slots;
+    a.order = RequestOrder(order, n_requests);
     const int word = dtype == 0 ? 4 : 8;      // elements of the projections per 16 bytes
     a.async = DK % word == 0 && DK % 4 == 0 && DV % word == 0 && stride % word == 0 && r_col0 % word == 0 && k_col0 % word == 0 && v_col0 % word == 0 &&
               zw_stride % 4 == 0 && za_stride % 4 == 0 && (uintptr_t)proj % 16 == 0 && (uintptr_t)zw % 16 == 0 && (uintptr_t)za % 16 == 0;

@@ -16,6 +16,8 @@
 // a time (thread d brings entry d of k, q and the decay of each token; the next tile's loads are in flight while this one is computed); the
 // warps' partial sums of S^T q meet in shared memory and are added after the tile. Every NW-th four entries to a warp, so that a thread's sums are the
 // first ones of the order in scan_columns.cuh.
+#include <climits>
+
 #include "scan_columns.cuh"
 
 __device__ __forceinline__ float gla_log_sigmoid(float v) { return fminf(v, 0.f) - log1pf(expf(-fabsf(v))); }
@@ -26,7 +28,7 @@ template <typename T, int NW, int TT, int KPT>
 __global__ void __launch_bounds__(32 * NW, NW == 8 ? (KPT == 32 ? 1 : 2) : 12 / NW) gla_scan_kernel(
     float* __restrict__ y, const T* __restrict__ proj, int proj_stride, int q_col0, int k_col0, int v_col0, const float* __restrict__ z,
     const float* __restrict__ z_bias, float inv_tau, int heads, int DK, int DV, float q_scale, float* __restrict__ state, long long slot_stride,
-    const int* __restrict__ cu_q, const int* __restrict__ state_slots) {
+    const int* __restrict__ cu_q, const int* __restrict__ state_slots, int most) {
     pdl_wait();
     constexpr int DKP = KPT * NW, NT = 32 * NW;      // NT >= DKP: thread d brings key entry d of every token
     __shared__ __align__(16) float ks[TT][DKP];
@@ -36,7 +38,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? (KPT == 32 ? 1 : 2) : 12 / 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = threadIdx.x;
     const int p0 = blockIdx.x * 32, p = p0 + lane, h = blockIdx.y, r = blockIdx.z;
     const int t0 = cu_q[r], t1 = cu_q[r + 1];
-    if (t1 <= t0) return;
+    if (t1 <= t0 || t1 - t0 > most) return;          // requests of more tokens are the other kernel's of this step
     float* S = state + (long long)state_slots[r] * slot_stride + (long long)h * DK * DV;
     f32x2 s[KPT / 2];                                // pair i: entries entry(i) and entry(i) + 1
     auto entry = [&](int i) { return 4 * (warp + NW * (i >> 1)) + 2 * (i & 1); };
@@ -141,38 +143,46 @@ __global__ void gla_decay_kernel(float4* __restrict__ decay, const float4* __res
                            expf(gla_log_sigmoid(v.w + b.w) * inv_tau));
 }
 
-// decay: fp32 scratch [n_tokens, heads * DK] for steps of many tokens per request, which the kernel of scan_columns.cuh takes where the sizes are its own; null:
-// the kernel above.
+// n_long requests bring at least long_from tokens; long_list (host memory, may be null) names them, the longest first. With `decay` (fp32 scratch
+// [n_tokens, heads * DK]) they go to the kernel of scan_columns.cuh, where that takes the sizes, all others to the kernel above, in a launch of its own.
+// Which kernel takes a request changes no result.
 OXR_API int oxr_gla_scan(float* y, const void* proj, int n_requests, int proj_stride, int q_col0, int k_col0, int v_col0, const float* z,
                          const float* z_bias, float tau, int heads, int DK, int DV, float q_scale, float* state, long long slot_stride, const int* cu_q,
-                         const int* state_slots, int dtype, int key_entries_per_thread, float* decay, int n_tokens, cudaStream_t stream) {
+                         const int* state_slots, int dtype, int key_entries_per_thread, float* decay, int n_tokens,
+                         const int* long_list, int n_long, int long_from, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (heads <= 0 || DK <= 0 || DK > 256 || DV <= 0 || heads > 65535 || n_requests > 65535 || !(tau > 0.f)) return OXR_BAD_ARGUMENT;
-    if (decay != nullptr && n_tokens > 0) {
+    int most = INT_MAX;
+    if (decay != nullptr && n_tokens > 0 && n_long > 0) {
         const size_t size = dtype == 0 ? 4 : 2;
         ScanArgs a = {};
         a.k = (const char*)proj + k_col0 * size; a.q = (const char*)proj + q_col0 * size; a.x = (const char*)proj + v_col0 * size;
         a.stride = proj_stride; a.k_group = 1; a.decay = decay; a.q_scale = q_scale; a.y = y; a.state = state; a.slot_stride = slot_stride; a.cu_q = cu_q;
         a.state_slots = state_slots; a.heads = heads; a.DV = DV; a.n_requests = n_requests;
+        a.least = n_long < n_requests ? long_from : 0;
+        a.order = RequestOrder(long_list, n_long);
         if ((dtype == 0 ? scan_fits<float>(a, DK) : scan_fits<__nv_bfloat16>(a, DK)) && (uintptr_t)z % 16 == 0 && (uintptr_t)z_bias % 16 == 0) {
             const size_t total = (size_t)n_tokens * heads * DK / 4;
             oxr_launch_small(gla_decay_kernel, dim3((unsigned)((total + 127) / 128)), dim3(128), 0, stream, (float4*)decay, (const float4*)z, (const float4*)z_bias, 1.f / tau,
                                                                                  heads * DK / 4, total);
             int rc = oxr_launch_status();
             if (rc) return rc;
-            return dtype == 0 ? scan_launch<float, true>(a, DK, stream) : scan_launch<__nv_bfloat16, true>(a, DK, stream);
+            rc = dtype == 0 ? scan_launch<float, true>(a, DK, n_long, stream) : scan_launch<__nv_bfloat16, true>(a, DK, n_long, stream);
+            if (rc || n_long >= n_requests) return rc;
+            most = long_from - 1;
         }
     }
     dim3 grid((DV + 31) / 32, heads, n_requests);
-    // 16 key entries a thread (twice the warps per head) where that still fits a block of 8 warps; key_entries_per_thread 16 or 32 forces one
-    const bool narrow = key_entries_per_thread == 16 ? DK <= 128 : (key_entries_per_thread == 32 ? false : DK <= 128);
+    // key_entries_per_thread 16 or 32 forces a split. Else 16 (twice the warps per head) for portions of prompts, where that still fits a block of 8 warps; for few
+    // tokens the state's trip through the registers is all there is, and fewer partial sums are cheaper (8 single tokens: 20.5 against 24.6 us)
+    const bool narrow = DK <= 128 && (key_entries_per_thread ? key_entries_per_thread == 16 : n_long > 0 && most == INT_MAX);
     const int nw = narrow ? (DK + 15) / 16 : (DK + 31) / 32;
 #define OXR_GLA(T, NW) \
     do { \
         if (narrow) oxr_launch(gla_scan_kernel<T, NW, 8, 16>, dim3(grid), dim3(32 * NW), 0, stream, false, y, (const T*)proj, proj_stride, q_col0, k_col0, v_col0, z, z_bias, 1.f / tau, \
-                                                                                heads, DK, DV, q_scale, state, slot_stride, cu_q, state_slots); \
+                                                                                heads, DK, DV, q_scale, state, slot_stride, cu_q, state_slots, most); \
         else oxr_launch(gla_scan_kernel<T, NW, 8, 32>, dim3(grid), dim3(32 * NW), 0, stream, false, y, (const T*)proj, proj_stride, q_col0, k_col0, v_col0, z, z_bias, 1.f / tau, heads, \
-                                                                         DK, DV, q_scale, state, slot_stride, cu_q, state_slots); \
+                                                                         DK, DV, q_scale, state, slot_stride, cu_q, state_slots, most); \
     } while (0)
 #define OXR_GLA_T(T) \
     do { \

@@ -12,6 +12,8 @@
 // scan_columns.cuh for steps that bring many tokens) add up y in one order, so a position's result does not depend on how the prompt was cut
 // into steps nor on what else is in the batch. Columns of S (one value dimension p each) are independent: a block takes 32 columns of one head of
 // one request.
+#include <climits>
+
 #include "scan_columns.cuh"
 
 // ---------------------------------------------------------------------------------------------- convolution
@@ -133,7 +135,7 @@ template <typename T, int NW, int TT>
 __global__ void __launch_bounds__(32 * NW, NW == 4 ? 3 : 1) ssm_scan_kernel(
     float* __restrict__ y, const T* __restrict__ xbc, const T* __restrict__ proj, int proj_stride, int dt_col0, int heads, int vdim, int N,
     int groups, const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip, float* __restrict__ state,
-    long long slot_stride, const int* __restrict__ cu_q, const int* __restrict__ state_slots) {
+    long long slot_stride, const int* __restrict__ cu_q, const int* __restrict__ state_slots, int most) {
     pdl_wait();
     constexpr int NP = 32 * NW;                       // N rounded up to whole warps
     extern __shared__ __align__(16) float scan_smem[];
@@ -146,7 +148,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 3 : 1) ssm_scan_kernel(
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int p0 = blockIdx.x * 32, p = p0 + lane, h = blockIdx.y, r = blockIdx.z;
     const int t0 = cu_q[r], t1 = cu_q[r + 1];
-    if (t1 <= t0) return;
+    if (t1 <= t0 || t1 - t0 > most) return;          // requests of more tokens are the other kernel's of this step
     const int inner = heads * vdim, channels = inner + 2 * groups * N, g = h / (heads / groups);
     const int b_col = inner + g * N, c_col = inner + groups * N + g * N;
     float* S = state + (long long)state_slots[r] * slot_stride + (long long)h * N * vdim;
@@ -336,22 +338,24 @@ OXR_API int oxr_mamba_conv(void* out, const void* proj, int n_tokens, int n_requ
 template <typename T, int NW>
 static void mamba_scan(float* y, const void* xbc, const void* proj, int n_requests, int proj_stride, int dt_col0, int heads, int vdim, int N, int groups,
                        const float* dt_bias, const float* a_log, const float* d_skip, float* state, long long slot_stride, const int* cu_q,
-                       const int* state_slots, cudaStream_t stream) {
+                       const int* state_slots, int most, cudaStream_t stream) {
     constexpr int TT = NW <= 4 ? 16 : 8;
     constexpr size_t smem = (size_t)(TT * (2 * 32 * NW + 32 + NW * 32 + 2)) * sizeof(float);
     static_assert(smem <= 48 * 1024, "the tile fits the default shared memory");
     dim3 grid((vdim + 31) / 32, heads, n_requests);
     oxr_launch(ssm_scan_kernel<T, NW, TT>, dim3(grid), dim3(32 * NW), smem, stream, false, y, (const T*)xbc, (const T*)proj, proj_stride, dt_col0, heads, vdim, N, groups, dt_bias,
-                                                                a_log, d_skip, state, slot_stride, cu_q, state_slots);
+                                                                a_log, d_skip, state, slot_stride, cu_q, state_slots, most);
 }
 
+// n_long requests bring at least long_from tokens; long_list (host memory, may be null) names them, the longest first. They go to the kernel of
+// scan_columns.cuh, where that takes the sizes, all others to the kernel above, in a launch of its own. Which kernel takes a request changes no result.
 OXR_API int oxr_mamba_scan(float* y, const void* xbc, const void* proj, int n_requests, int proj_stride, int dt_col0, int heads, int vdim, int N, int groups,
                            const float* dt_bias, const float* a_log, const float* d_skip, float* state, long long slot_stride, const int* cu_q,
-                           const int* state_slots, int dtype, int n_tokens, cudaStream_t stream) {
+                           const int* state_slots, int dtype, const int* long_list, int n_long, int long_from, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (heads <= 0 || vdim <= 0 || N <= 0 || N > 256 || groups <= 0 || heads % groups || n_requests > 65535 || heads > 65535) return OXR_BAD_ARGUMENT;
-    // Many tokens of a request (not decode steps, whose cost is the state's way through the registers): the kernel of scan_columns.cuh
-    if (n_tokens > 2 * n_requests) {
+    int most = INT_MAX;
+    if (n_long > 0) {
         const size_t size = dtype == 0 ? 4 : 2;
         const int inner = heads * vdim;
         ScanArgs a = {};
@@ -359,15 +363,20 @@ OXR_API int oxr_mamba_scan(float* y, const void* xbc, const void* proj, int n_re
         a.stride = inner + 2 * groups * N; a.k_group = heads / groups; a.dt = (const char*)proj + dt_col0 * size; a.dt_stride = proj_stride;
         a.dt_bias = dt_bias; a.a_log = a_log; a.skip = d_skip; a.y = y; a.state = state; a.slot_stride = slot_stride; a.cu_q = cu_q; a.state_slots = state_slots;
         a.heads = heads; a.DV = vdim; a.n_requests = n_requests;
-        if (dtype == 0 ? scan_fits<float>(a, N) : scan_fits<__nv_bfloat16>(a, N))
-            return dtype == 0 ? scan_launch<float, false>(a, N, stream) : scan_launch<__nv_bfloat16, false>(a, N, stream);
+        a.least = n_long < n_requests ? long_from : 0;
+        a.order = RequestOrder(long_list, n_long);
+        if (dtype == 0 ? scan_fits<float>(a, N) : scan_fits<__nv_bfloat16>(a, N)) {
+            const int rc = dtype == 0 ? scan_launch<float, false>(a, N, n_long, stream) : scan_launch<__nv_bfloat16, false>(a, N, n_long, stream);
+            if (rc || n_long >= n_requests) return rc;
+            most = long_from - 1;
+        }
     }
     const int nw = (N + 31) / 32;
 #define OXR_SCAN(NW) \
     (dtype == 0 ? mamba_scan<float, NW>(y, xbc, proj, n_requests, proj_stride, dt_col0, heads, vdim, N, groups, dt_bias, a_log, d_skip, state, \
-                                        slot_stride, cu_q, state_slots, stream) \
+                                        slot_stride, cu_q, state_slots, most, stream) \
                 : mamba_scan<__nv_bfloat16, NW>(y, xbc, proj, n_requests, proj_stride, dt_col0, heads, vdim, N, groups, dt_bias, a_log, d_skip, state, \
-                                                slot_stride, cu_q, state_slots, stream))
+                                                slot_stride, cu_q, state_slots, most, stream))
     switch (nw) {
         case 1: OXR_SCAN(1); break;
         case 2: OXR_SCAN(2); break;

@@ -70,20 +70,22 @@ template <int N> __device__ __forceinline__ float scan_halve(const float (&v)[N]
     }
 }
 
-// The request that blocks with index z of a one-block-per-request axis take: the z-th longest of the step (whole warps ask). Blocks start in the order
-// of their index, and a recurrence runs as long as its longest request: started last, that one would run alone at the end. Of more
-// than 32 requests each is as good as another.
-__device__ __forceinline__ int longest_first(const int* __restrict__ cu_q, int n, int z) {
-    if (n < 2 || n > 32) return z;
-    const int lane = threadIdx.x & 31;
-    const int len = lane < n ? cu_q[lane + 1] - cu_q[lane] : -1;
-    int rank = 0;
-    for (int k = 0; k < n; ++k) {
-        const int other = __shfl_sync(0xffffffffu, len, k);
-        rank += other > len || (other == len && k < lane);
+// The requests of a launch in the order of their blocks. Blocks start in the order of their index, and a recurrence runs as long as its longest request: started
+// last, that one would run alone at the end. The host knows the lengths and names up to 32 requests, the longest first (an index out of the kernel's arguments
+// is the same for a whole warp to the compiler too; ranking the lengths on the device cost the delta rule's chain of one prompt 2 %). Else all of the
+// step, the last first: the scheduler puts portions of prompts behind the requests that decode.
+constexpr int LISTED_MAX = 32;
+struct RequestOrder {
+    int n = 0;                       // 0: none named
+    int r[LISTED_MAX];
+    RequestOrder(const int* list, int count) {
+        if (list == nullptr || count > LISTED_MAX) return;
+        n = count;
+        for (int i = 0; i < n; ++i) r[i] = list[i];
     }
-    return __ffs(__ballot_sync(0xffffffffu, lane < n && rank == z)) - 1;
-}
+    int blocks(int n_requests) const { return n > 0 ? n : n_requests; }
+};
+__device__ __forceinline__ int request_of(const RequestOrder& o, int n_blocks, int z) { return o.n > 0 ? o.r[z] : n_blocks - 1 - z; }
 
 struct ScanArgs {
     const void *k, *q, *x;           // row 0, head 0: rows of `stride` entries, heads (or, k and q, groups of heads) side by side
@@ -98,6 +100,8 @@ struct ScanArgs {
     long long slot_stride;
     const int *cu_q, *state_slots;
     int heads, DV, n_requests;
+    int least;                       // of the launch's requests those of fewer tokens are the other kernel's
+    RequestOrder order = {nullptr, 0};
 };
 
 constexpr int SCAN_TT = 8, SCAN_STAGES = 4;
@@ -136,7 +140,7 @@ __device__ __forceinline__ void scan_four(const __nv_bfloat16* at, float (&v)[4]
     v[2] = __uint_as_float(a.y << 16); v[3] = __uint_as_float(a.y & 0xffff0000u);
 }
 
-// grid (ceil(DV / COLS), heads, requests). Row pieces are whole 16-byte words (scan_fits).
+// grid (ceil(DV / COLS), heads, requests of this launch). Row pieces are whole 16-byte words (scan_fits).
 template <typename T, int J, int E, bool VECTOR>
 __global__ void __launch_bounds__(ScanShape<T, J, E, VECTOR>::THREADS) column_scan_kernel(const ScanArgs a) {
     pdl_wait();
@@ -145,10 +149,10 @@ __global__ void __launch_bounds__(ScanShape<T, J, E, VECTOR>::THREADS) column_sc
     extern __shared__ __align__(16) unsigned char column_smem[];
     __shared__ float scalars[SCAN_STAGES][2][TT];                             // dt and decay of a token, where a token has one
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, j = lane % J;
-    const int h = blockIdx.y, r = longest_first(a.cu_q, a.n_requests, blockIdx.z);
+    const int h = blockIdx.y, r = request_of(a.order, gridDim.z, blockIdx.z);
     const int p0 = blockIdx.x * Sh::COLS, c0 = (warp * Sh::GROUPS + lane / J) * 4;   // this thread's first column of the block
     const int t0 = a.cu_q[r], t1 = a.cu_q[r + 1], DV = a.DV;
-    if (t1 <= t0) return;
+    if (t1 <= t0 || t1 - t0 < a.least) return;
     const int n_tiles = (t1 - t0 + TT - 1) / TT;
     const T* kp = (const T*)a.k + (size_t)(h / a.k_group) * Sh::DK;
     const T* qp = (const T*)a.q + (size_t)(h / a.k_group) * Sh::DK;
@@ -318,16 +322,20 @@ int scan_launch_j(const ScanArgs& a, cudaStream_t stream) {
         cudaError_t e = cudaFuncSetAttribute(column_scan_kernel<T, J, E, VECTOR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM);
         if (e != cudaSuccess) return 1000 + (int)e;
     }
-    oxr_launch(column_scan_kernel<T, J, E, VECTOR>, dim3((a.DV + Sh::COLS - 1) / Sh::COLS, a.heads, a.n_requests), dim3(Sh::THREADS), Sh::SMEM, stream, false, a);
+    oxr_launch(column_scan_kernel<T, J, E, VECTOR>, dim3((a.DV + Sh::COLS - 1) / Sh::COLS, a.heads, a.order.blocks(a.n_requests)), dim3(Sh::THREADS), Sh::SMEM, stream, false, a);
     return oxr_launch_status();
 }
 // Eight entries a lane where that makes warps enough to hide one another's latencies (a warp alone on its scheduler issues an instruction every 3.4
-// cycles), else four: twice the warps, each with half the work and almost the same overhead. Measured on a B200, four against eight: 512 warps of
-// eight entries (16 heads of 128 x 256, one request of 2,048 tokens) 409 against 549 us, 1,024 (two of 700) 219 and 244, 1,536 388 and 424; 2,048 (128
-// heads of 128 x 64, two of 700) 396 and 341, 8,192 143 and 132.
+// cycles), else four: twice the warps, each with half the work and almost the same overhead. Measured on a B200 by the warps that eight entries make, four against
+// eight, us: a decay per entry 512 (16 heads of 128 x 256, 2,048 tokens) 400 and 574, 1,024 (two prompts of 700) 218 and 251, 1,536 304 and 318, 2,048 402
+// and 390, 8,192 (16 of 100) 226 and 200; one per token 512 (64 heads of 128 x 64, 2,048 tokens) 465 and 549, 1,024 (two of 700) 219 and 217, 1,536 299 and 277, 2,048
+// 404 and 338.
+// Only the n_long requests that this kernel takes count, and only they get blocks: one prompt beside 20 single tokens is one request's warps, and a grid with blocks for the
+// others too, more than are resident at once, was dealt out with three of the prompt's blocks to an SM instead of one (1,200 tokens of gated linear
+// attention alone 239 us, beside three single tokens 361).
 template <typename T, bool VECTOR>
-int scan_launch(const ScanArgs& a, int DK, cudaStream_t stream) {
-    const bool wide = (long long)a.heads * a.DV * DK / 1024 * a.n_requests >= 2048;
+int scan_launch(const ScanArgs& a, int DK, int n_long, cudaStream_t stream) {
+    const bool wide = (long long)a.heads * a.DV * DK / 1024 * n_long >= (VECTOR ? 2048 : 1536);
     if (DK == 256) return scan_launch_j<T, 32, 8, VECTOR>(a, stream);
     if (DK == 128) return wide ? scan_launch_j<T, 16, 8, VECTOR>(a, stream) : scan_launch_j<T, 32, 4, VECTOR>(a, stream);
     return wide ? scan_launch_j<T, 8, 8, VECTOR>(a, stream) : scan_launch_j<T, 16, 4, VECTOR>(a, stream);

@@ -15,7 +15,9 @@ from __future__ import annotations
 import ctypes
 import functools
 import os
+from collections.abc import Sequence
 from ctypes import c_double, c_float, c_int, c_longlong, c_size_t, c_void_p
+from typing import NamedTuple
 
 import torch
 
@@ -140,7 +142,7 @@ def _lib():
         lib.oxr_clamped_glu.argtypes = [p, p, i, i, i, f, f, i, p]
         lib.oxr_rotary_angles.argtypes = [p, p, p, p, c_double, i, i, p]
         lib.oxr_mamba_conv.argtypes = [p, p, i, i, i, i, i, i, p, p, p, ll, p, p, p, i, p]
-        lib.oxr_mamba_scan.argtypes = [p, p, p, i, i, i, i, i, i, i, p, p, p, p, ll, p, p, i, i, p]
+        lib.oxr_mamba_scan.argtypes = [p, p, p, i, i, i, i, i, i, i, p, p, p, p, ll, p, p, i, p, i, i, p]
         lib.oxr_gated_group_norm.argtypes = [p, p, p, i, i, i, p, i, i, f, i, p]
         lib.oxr_attention_rows.argtypes = [p, p, i, p, ll, i, p, ll, i, i, i, i, i, i, p, p, p, i, i, i, f, i, i, i, p, i, p, i, p, p]
         lib.oxr_scatter_rows.argtypes = [p, ll, ll, p, i, i, i, p, i, i, p, p, ll, i, p]
@@ -173,7 +175,7 @@ def _lib():
         lib.oxr_expert_clamped_glu.argtypes = [p, p, p, i, i, i, f, f, i, p]
         lib.oxr_head_prep.argtypes = [p, p, p, p, i, i, i, i, i, i, i, i, i, i, i, i, p, p, p, i, p, ll, i, i, p, p, p, f, p, p, i, p, ll, p, p, p, i, p, p]
         lib.oxr_sigmoid_gate.argtypes = [p, p, i, i, i, i, i, i, i, p]
-        lib.oxr_gla_scan.argtypes = [p, p, i, i, i, i, i, p, p, f, i, i, i, f, p, ll, p, p, i, i, p, i, p]
+        lib.oxr_gla_scan.argtypes = [p, p, i, i, i, i, i, p, p, f, i, i, i, f, p, ll, p, p, i, i, p, i, p, i, i, p]
         lib.oxr_pair_norm_mean.argtypes = [p, p, p, p, p, i, i, f, i, p]
         lib.oxr_tanh_cap.argtypes = [p, f, ll, p]
         lib.oxr_expert_silu_glu.argtypes = [p, p, p, i, i, i, i, i, p]
@@ -182,7 +184,7 @@ def _lib():
         lib.oxr_gelu_glu.argtypes = [p, p, i, i, i, i, p]
         lib.oxr_scaled_sum.argtypes = [p, p, p, f, f, ll, i, p]
         lib.oxr_shift_norm.argtypes = [p, p, p, p, p, f, p, f, p, p, ll, p, p, p, i, i, i, i, p]
-        lib.oxr_delta_scan.argtypes = [p, p, i, i, i, i, i, p, i, p, p, i, p, f, f, i, i, i, p, ll, p, p, i, i, p]
+        lib.oxr_delta_scan.argtypes = [p, p, i, i, i, i, i, p, i, p, p, i, p, f, f, i, i, i, p, ll, p, p, i, i, p, p]
         lib.oxr_tanh_cols.argtypes = [p, p, i, i, i, i, i, p]
         lib.oxr_diff_prep.argtypes = [p, p, p, p, i, i, i, i, i, i, i, i, i, i, i, p, p, ll, i, p, p]
         lib.oxr_diff_combine.argtypes = [p, p, i, i, i, i, p, f, f, i, p]
@@ -1492,10 +1494,62 @@ def mamba_conv(proj: torch.Tensor, col0: int, channels: int, weight: torch.Tenso
     return out
 
 
+class ScanRule(NamedTuple):
+    """Which requests of a step go to the recurrence's kernel for portions of prompts (``scan_columns.cuh``), the others to the one for few tokens."""
+
+    least: int
+    """A request of this many tokens is a portion."""
+    beside: int
+    """More than 32 requests, or a portion longer than ``overlap`` tokens for each of fewer: portions beside others get a launch of their own
+    from this length of the longest on, else the kernel for few tokens takes all."""
+    overlap: int
+    """Up to 32 requests whose longest portion has no more than this many tokens for each of them: the kernel for portions takes all, so that the others run beside it."""
+
+
+MAMBA_RULE, GLA_RULE = ScanRule(17, 64, 16), ScanRule(12, 32, 4)
+"""Measured on a B200, us, kernel for few tokens / for portions / each its own. Mamba-2 (128 heads of 128 x 64): 1 request of 16 tokens 14 / 16, 8 of 12 45 / 43, 32 of
+16 167 / 164, 8 of 24 68 / 61; beside 8 single tokens a portion of 64 53 / 43 / 54, of 128 78 / 68 / 73; beside 20 of 128 104 / 82 / 99, of 1,200
+520 / 504 / 415; beside 48 of 32 127 / - / 132, of 96 152 / 172 / 150. Gated linear attention (16 heads of 128 x 256): 1 of 12 14 / 15, 8 of 8 27 / 32, 32 of 8 70 / 73, 32 of 12
+98 / 87; beside 8 of 24 31 / 30 / 32, of 64 53 / 42 / 40; beside 20 of 64 66 / 50 / 52, of 1,200 692 / 413 / 267; beside 48 of 24 74 / 86 / 75."""
+
+
+def _long_requests(q_lens: Sequence[int] | None, n_tokens: int, n_requests: int, rule: ScanRule) -> tuple[ctypes.Array | None, int]:
+    """The requests that the kernel for portions takes, the longest first, and their number; without the lengths all or none, by the average."""
+    if q_lens is None:
+        return None, n_requests if n_tokens >= rule.least * n_requests else 0
+    _need_lengths(q_lens, n_requests)
+    longest = max(q_lens, default=0)
+    if longest < rule.least:
+        return None, 0
+    least = rule.least
+    if min(q_lens) < least:
+        if n_requests <= 32 and longest <= rule.overlap * n_requests:
+            least = 0
+        elif longest < rule.beside:
+            return None, 0
+    found = sorted((r for r, n in enumerate(q_lens) if n >= least), key=q_lens.__getitem__, reverse=True)
+    return (c_int * len(found))(*found), len(found)
+
+
+def _longest_first(q_lens: Sequence[int] | None, n_requests: int) -> ctypes.Array | None:
+    """All requests, the longest first, where their lengths are known and a launch can name them all."""
+    if q_lens is None or not 1 < n_requests <= 32:
+        return None
+    _need_lengths(q_lens, n_requests)
+    return (c_int * n_requests)(*sorted(range(n_requests), key=q_lens.__getitem__, reverse=True))
+
+
+def _need_lengths(q_lens: Sequence[int], n_requests: int) -> None:
+    if len(q_lens) != n_requests:
+        raise KernelError(f"{len(q_lens)} request lengths for {n_requests} requests")
+
+
 def mamba_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col0: int, *, heads: int, vdim: int, state: int, groups: int, dt_bias: torch.Tensor,
-               a_log: torch.Tensor, d_skip: torch.Tensor, ssm: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor, n_requests: int) -> torch.Tensor:
+               a_log: torch.Tensor, d_skip: torch.Tensor, ssm: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor, n_requests: int,
+               q_lens: Sequence[int] | None = None) -> torch.Tensor:
     """The selective-state recurrence over a packed step: fp32 ``y [tokens, heads * vdim]``; ``ssm`` (fp32 view, first axis the slot, each
-    slot ``[heads, state, vdim]``) is read and left at the state after each request's last token."""
+    slot ``[heads, state, vdim]``) is read and left at the state after each request's last token. ``q_lens``: the host's copy of the requests' tokens
+    of this step, which picks kernels and changes no result."""
     _need(xbc, "xbc")
     _need(proj, "proj")
     if ssm.dtype != torch.float32 or ssm.stride(-1) != 1:
@@ -1504,7 +1558,8 @@ def mamba_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col0: int, *, heads: in
     y = torch.empty((n, heads * vdim), dtype=torch.float32, device=xbc.device)
     _done(_lib().oxr_mamba_scan(y.data_ptr(), xbc.data_ptr(), proj.data_ptr(), n_requests, proj.shape[1], dt_col0, heads, vdim, state, groups,
                                 dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), ssm.data_ptr(), ssm.stride(0), cu_q.data_ptr(),
-                                state_slots.data_ptr(), _dtype_code(xbc), n, _stream()), "mamba_scan")
+                                state_slots.data_ptr(), _dtype_code(xbc), *_long_requests(q_lens, n, n_requests, MAMBA_RULE), MAMBA_RULE.least,
+                                _stream()), "mamba_scan")
     return y
 
 
@@ -2002,12 +2057,13 @@ def sigmoid_gate_(o: torch.Tensor, proj: torch.Tensor, gate_col0: int, value_dim
 
 def gla_scan(proj: torch.Tensor, q_col0: int, k_col0: int, v_col0: int, z: torch.Tensor, z_bias: torch.Tensor, *, heads: int, key_dim: int,
              value_dim: int, tau: float, q_scale: float, state: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor, n_requests: int,
-             key_entries_per_thread: int = 0) -> torch.Tensor:
+             key_entries_per_thread: int = 0, q_lens: Sequence[int] | None = None) -> torch.Tensor:
     """Gated linear attention over a packed step: per head ``S_t = diag(alpha_t) S_(t-1) + k_t v_t^T``, ``o_t = S_t^T (q_t * q_scale)`` with the decay
     ``alpha_t = sigmoid(z_t + z_bias)^(1 / tau)`` per key channel. ``proj`` holds q, k and v head by head from the given columns; ``z [tokens, heads *
     key_dim]`` is fp32; ``state`` (fp32, first axis the slot: S ``[heads, key_dim, value_dim]``) is read and left at the state after each request's
     last token. Returns fp32 ``o [tokens, heads * value_dim]``. ``key_entries_per_thread`` (16 or 32) forces the kernel's split of a head's
-    key channels over threads; 0 chooses the kernel and the split by the step's shape."""
+    key channels over threads; 0 chooses the kernel and the split by the step's shape. ``q_lens``: the host's copy of the requests' tokens of this step, which
+    picks kernels and changes no result."""
     _need(proj, "proj")
     _need(z, "z", torch.float32)
     _need(z_bias, "z_bias", torch.float32)
@@ -2017,17 +2073,14 @@ def gla_scan(proj: torch.Tensor, q_col0: int, k_col0: int, v_col0: int, z: torch
     if z.shape != (n, heads * key_dim) or z_bias.numel() != heads * key_dim:
         raise KernelError("gla_scan: the decay logits must be [tokens, heads * key_dim] with one bias each")
     y = torch.empty((n, heads * value_dim), dtype=torch.float32, device=proj.device)
-    decay = None
-    if not key_entries_per_thread:
-        # portions of prompts: the kernel whose threads hold several columns, where it takes the sizes, else twice the warps per head (2,048 tokens of
-        # 16 heads of 128 x 256: 402 against 774 us); single tokens: the state's trip through the registers is all there is, and fewer
-        # partial sums are cheaper (20.5 against 24.6 us)
-        many = n > 2 * n_requests
-        key_entries_per_thread = 16 if many else 32
-        decay = torch.empty_like(z) if many else None
+    # portions of prompts: the kernel whose threads hold several columns, where it takes the sizes, else twice the warps per head (2,048 tokens of
+    # 16 heads of 128 x 256: 402 against 774 us)
+    long_list, n_long = (None, 0) if key_entries_per_thread else _long_requests(q_lens, n, n_requests, GLA_RULE)
+    decay = torch.empty_like(z) if n_long else None
     _done(_lib().oxr_gla_scan(y.data_ptr(), proj.data_ptr(), int(n_requests), proj.shape[1], int(q_col0), int(k_col0), int(v_col0), z.data_ptr(),
                               z_bias.data_ptr(), float(tau), int(heads), int(key_dim), int(value_dim), float(q_scale), state.data_ptr(), state.stride(0),
-                              cu_q.data_ptr(), state_slots.data_ptr(), _dtype_code(proj), int(key_entries_per_thread), _ptr(decay), n, _stream()), "gla_scan")
+                              cu_q.data_ptr(), state_slots.data_ptr(), _dtype_code(proj), int(key_entries_per_thread), _ptr(decay), n, long_list, n_long,
+                              GLA_RULE.least, _stream()), "gla_scan")
     return y
 
 
@@ -2199,7 +2252,7 @@ def tanh_cols(z: torch.Tensor, col0: int, width: int, out_dtype: torch.dtype) ->
 
 def delta_scan(proj: torch.Tensor, r_col0: int, k_col0: int, v_col0: int, zw: torch.Tensor, w_bias: torch.Tensor, za: torch.Tensor, a_bias: torch.Tensor, *,
                heads: int, key_dim: int, value_dim: int, rate: float, len_eps: float, state: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor,
-               n_requests: int, single_tokens: bool = False) -> torch.Tensor:
+               n_requests: int, single_tokens: bool = False, q_lens: Sequence[int] | None = None) -> torch.Tensor:
     """The delta rule with a decay per key channel over a packed step: per head, with ``u = k / sqrt(sum k^2 + len_eps)``, ``w = exp(-rate *
     sigmoid(zw + w_bias))`` and ``a = sigmoid(za + a_bias)``,
 
@@ -2207,8 +2260,8 @@ def delta_scan(proj: torch.Tensor, r_col0: int, k_col0: int, v_col0: int, zw: to
 
     ``proj`` holds r, k and v head by head from the given columns; ``zw`` and ``za`` (fp32 ``[tokens, >= heads * key_dim]``, the first columns) are the
     logits of decay and removal rate; ``state`` (fp32, first axis the slot: S transposed, ``[heads, value_dim, key_dim]``) is read and left at the
-    state after each request's last token. ``single_tokens``: every request brings exactly one token (a decode step has a kernel of its own).
-    Returns fp32 ``o [tokens, heads * value_dim]``."""
+    state after each request's last token. ``single_tokens``: every request brings exactly one token (a decode step has a kernel of its own). ``q_lens``: the host's copy
+    of the requests' tokens of this step: the longest start first. Returns fp32 ``o [tokens, heads * value_dim]``."""
     _need(proj, "proj")
     _need(zw, "zw", torch.float32)
     _need(za, "za", torch.float32)
@@ -2226,7 +2279,7 @@ def delta_scan(proj: torch.Tensor, r_col0: int, k_col0: int, v_col0: int, zw: to
     _done(_lib().oxr_delta_scan(y.data_ptr(), proj.data_ptr(), int(n_requests), proj.shape[1], int(r_col0), int(k_col0), int(v_col0), zw.data_ptr(),
                                 zw.shape[1], w_bias.data_ptr(), za.data_ptr(), za.shape[1], a_bias.data_ptr(), float(rate), float(len_eps), int(heads),
                                 int(key_dim), int(value_dim), state.data_ptr(), state.stride(0), cu_q.data_ptr(), state_slots.data_ptr(),
-                                int(bool(single_tokens)), _dtype_code(proj), _stream()), "delta_scan")
+                                int(bool(single_tokens)), _dtype_code(proj), None if single_tokens else _longest_first(q_lens, n_requests), _stream()), "delta_scan")
     return y
 
 

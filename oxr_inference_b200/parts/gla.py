@@ -64,5 +64,6 @@ class GatedLinearAttention(Mixer):
         a1_col0 = 2 * self.keys + 2 * self.inner
         z = self.decay(proj[:, a1_col0:].contiguous(), torch.float32)   # [tokens, heads * key_dim], kept in fp32
         o = ops.gla_scan(proj, 0, self.keys, 2 * self.keys, z, self.vectors["a2.b"], heads=self.H, key_dim=self.DK, value_dim=self.DV, tau=self.tau,
-                         q_scale=self.DK ** -0.5, state=cache.state, cu_q=ctx.cu_q, state_slots=ctx.state_slots, n_requests=ctx.n_requests)
+                         q_scale=self.DK ** -0.5, state=cache.state, cu_q=ctx.cu_q, state_slots=ctx.state_slots, n_requests=ctx.n_requests,
+                         q_lens=ctx.q_lens)
         return self.out(ops.head_norm_gate(o, proj, 2 * self.keys + self.inner, self.head_norm, self.H, self.eps, silu=True))

@@ -68,5 +68,6 @@ class Mamba2(Mixer):
         xbc = ops.mamba_conv(proj, self.inner, self.channels, v["conv"], v["conv.b"], tail, req_of_token=ctx.req_of_token, cu_q=ctx.cu_q,
                              state_slots=ctx.state_slots, n_requests=ctx.n_requests)
         y = ops.mamba_scan(xbc, proj, self.inner + self.channels, heads=self.H, vdim=self.P, state=self.N, groups=self.G, dt_bias=v["dt_bias"],
-                           a_log=v["A_log"], d_skip=v["D"], ssm=state, cu_q=ctx.cu_q, state_slots=ctx.state_slots, n_requests=ctx.n_requests)
+                           a_log=v["A_log"], d_skip=v["D"], ssm=state, cu_q=ctx.cu_q, state_slots=ctx.state_slots, n_requests=ctx.n_requests,
+                           q_lens=ctx.q_lens)
         return self.out(ops.gated_group_norm(y, proj, 0, v["norm"], self.norm_groups, self.eps))

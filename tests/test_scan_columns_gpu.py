@@ -100,10 +100,11 @@ def test_same_bits_however_cut_and_whatever_else_is_in_the_batch(ops, kind, H, D
     mine = tokens_of(kind, 61, H, DK, DV, dtype, g)
     start = torch.randn(H * DK * DV, generator=g, device=DEV)
 
-    def step(requests, state, slots):
+    def step(requests, state, slots, named=False):
         cu, cu_q, _ = split([len(r[0]) for r in requests])
         rows, extra = (torch.cat([r[i] for r in requests]) for i in (0, 1))
-        common = dict(heads=H, cu_q=cu_q, state_slots=torch.tensor(slots, dtype=torch.int32, device=DEV), n_requests=len(requests))
+        common = dict(heads=H, cu_q=cu_q, state_slots=torch.tensor(slots, dtype=torch.int32, device=DEV), n_requests=len(requests),
+                      q_lens=[len(r[0]) for r in requests] if named else None)
         if kind == "entry":
             return ops.gla_scan(rows, 0, H * DK, 2 * H * DK, extra, per_head[0], key_dim=DK, value_dim=DV, tau=4.0, q_scale=0.3, state=state, **common), cu
         return ops.mamba_scan(rows, extra, 8, vdim=DV, state=DK, groups=2, dt_bias=per_head[0], a_log=per_head[1] - 2, d_skip=per_head[2],
@@ -116,11 +117,12 @@ def test_same_bits_however_cut_and_whatever_else_is_in_the_batch(ops, kind, H, D
         rows.append(step([[t[at:at + n] for t in mine]], cut, [0])[0])
         at += n
     assert at == 61 and torch.equal(torch.cat(rows), want) and torch.equal(cut, alone)
-    for others in ([1], [1] * 8, [40, 1, 3, 70, 1, 1, 9, 2], [1] * 70):
+    # without and with the lengths on the host, which name the requests of the kernel for many tokens (up to 32 of them); 40 such requests; 70 single tokens
+    for others, named in [(o, named) for o in ([1], [1] * 8, [40, 1, 3, 70, 1, 1, 9, 2], [1] * 70, [18, 1] * 40) for named in (False, True)]:
         states = torch.randn(len(others) + 1, H * DK * DV, generator=g, device=DEV)
         states[len(others) // 2] = start
         step_of = [tokens_of(kind, n, H, DK, DV, dtype, g) for n in others]
         step_of.insert(len(others) // 2, mine)
-        got, cu = step(step_of, states, list(range(len(others) + 1)))
+        got, cu = step(step_of, states, list(range(len(others) + 1)), named)
         first = cu[len(others) // 2]
         assert torch.equal(got[first:first + 61], want) and torch.equal(states[len(others) // 2], alone[0])
