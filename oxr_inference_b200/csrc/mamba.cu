@@ -306,9 +306,12 @@ template <typename T>
 static int mamba_conv(void* out, const void* proj, int n_tokens, int n_requests, int proj_stride, int col0, int channels, int taps,
                       const float* w, const float* bias, float* state, long long slot_stride, const int* req_of_token, const int* cu_q,
                       const int* state_slots, cudaStream_t stream) {
-    // the 16-byte form wants whole words and, to fill the chip with a thread per eight channels of 16 tokens, more than a decode step's rows
+    // The 16-byte form wants whole words and work enough for a thread per eight channels of 16 tokens, behind the first token of each request (which brings a
+    // tail to fetch, an entry at a time). 10,240 channels, us, the general form and this one: 150 tokens 22 and 26, 256 28 and 28, 320 32 and 28, 2,048 138
+    // and 67; single tokens of 17, 48 and 256 requests 13 and 34, 17 and 38, 48 and 58; 48 of them beside 200, 300 and 400 tokens 32 and
+    // 38, 38 and 38, 44 and 40. 5,120 channels: 200 tokens 20 and 26, 400 26 and 26, 600 32 and 28.
     const auto words = [](const void* p) { return (uintptr_t)p % 16 == 0; };
-    if (sizeof(T) == 2 && taps == 4 && n_tokens > CONV_RUN && channels % 8 == 0 && proj_stride % 8 == 0 && col0 % 8 == 0 && words(out) && words(proj) && words(w))
+    if (sizeof(T) == 2 && taps == 4 && (long long)(n_tokens - n_requests) * channels >= 3000000 && channels % 8 == 0 && proj_stride % 8 == 0 && col0 % 8 == 0 && words(out) && words(proj) && words(w))
         oxr_launch_small(causal_conv4_silu_words_kernel, dim3((channels / 8 + CONV_THREADS - 1) / CONV_THREADS, (n_tokens + CONV_RUN - 1) / CONV_RUN), dim3(CONV_THREADS), 0, stream, 
             (__nv_bfloat16*)out, (const __nv_bfloat16*)proj, proj_stride, col0, channels, n_tokens, w, bias, state, slot_stride, req_of_token, cu_q, state_slots);
     else {

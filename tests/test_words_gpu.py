@@ -41,8 +41,14 @@ def test_mamba_conv(ops, lengths, channels, taps):
         assert torch.equal(state[slot, :channels * (taps - 1)].view(channels, taps - 1), x[:, -(taps - 1):].float())
 
 
+@pytest.mark.parametrize("lengths,channels", [([1, 15, 1, 33, 2, 1500], 2056), ([1] * 40 + [1461], 2056), ([300, 1, 17, 16], 10248), ([293, 1], 10240)])
+def test_mamba_conv_of_many_tokens(ops, lengths, channels):
+    """From three million entries behind the requests' first tokens on the 16-byte form takes the step; below, the general one."""
+    test_mamba_conv(ops, lengths, channels, 4)
+
+
 @pytest.mark.parametrize("n", [1, 19])
-@pytest.mark.parametrize("inner,parts", [(8, 1), (1032, 3), (8192, 8), (16384, 1), (60, 3)])
+@pytest.mark.parametrize("inner,parts", [(8, 1), (1032, 3), (8192, 8), (16384, 1), (60, 3), (8192, 1), (8184, 1), (8200, 1)])
 def test_gated_group_norm(ops, n, inner, parts):
     torch.manual_seed(2)
     y, w = torch.randn(n, inner, device=DEV), torch.rand(inner, device=DEV) + 0.5
