@@ -24,7 +24,6 @@ __global__ void __launch_bounds__(128) attn_rows_kernel(
     const T* __restrict__ v_pool, long long v_slot_stride, int v_head_stride, int DK, int DV, int H, int KVH, const int* __restrict__ positions,
     const int* __restrict__ req_of_token, const int* __restrict__ block_table, int table_width, int page_size, int num_pages, float scale,
     int chunk, int window, int keep_first, const float* __restrict__ dist_bias, int bias_rows, const float* __restrict__ sink, int* status) {
-    pdl_wait();
     pdl_trigger();
     extern __shared__ float q_smem[];   // [warps, DK]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -419,7 +418,6 @@ OXR_API int oxr_cols_rms_norm(void* out, const void* x, int n, int stride, int w
 template <typename T, int TM>
 __global__ void __launch_bounds__(128) head_linear_kernel(T* __restrict__ out, int out_head_stride, int out0, const T* __restrict__ x, int x_head_stride,
                                                           int x0, const T* __restrict__ w, int n_in, int n_out, int heads, int n_tokens) {
-    pdl_wait();
     pdl_trigger();
     extern __shared__ float xs[];   // [TM, n_in]
     const int h = blockIdx.y, t0 = blockIdx.x * TM;
@@ -452,7 +450,6 @@ __device__ __forceinline__ float2 hl_load2(const __nv_bfloat16* p) { return __bf
 template <typename T, int TM>
 __global__ void __launch_bounds__(128) head_linear_few_kernel(T* __restrict__ out, int out_head_stride, int out0, const T* __restrict__ x, int x_head_stride,
                                                               int x0, const T* __restrict__ w, int n_in, int n_out, int heads, int n_tokens) {
-    pdl_wait();
     pdl_trigger();
     extern __shared__ float xs[];   // [TM, n_in], then [4][TM][64]
     float* part = xs + TM * n_in;
@@ -494,8 +491,7 @@ __global__ void __launch_bounds__(128) head_linear_few_kernel(T* __restrict__ ou
     }
 }
 
-// The same in bf16 with a warp's whole quarter of the matrix (at most KPW rows of 64 columns) in registers, asked for at once and before the wait for the
-// kernel that writes x (no kernel of a step writes weights). Eight rows at a time a block made four to six trips to memory one after the other: 13 tokens,
+// The same in bf16 with a warp's whole quarter of the matrix (at most KPW rows of 64 columns) in registers, asked for at once. Eight rows at a time a block made four to six trips to memory one after the other: 13 tokens,
 // 32 heads of 128 x 192: 10.7 us, 5.2 here. The sums are the same, in the same order.
 template <int KPW>
 __global__ void __launch_bounds__(128) head_linear_few_words_kernel(__nv_bfloat16* __restrict__ out, int out_head_stride, int out0,
@@ -510,7 +506,6 @@ __global__ void __launch_bounds__(128) head_linear_few_words_kernel(__nv_bfloat1
     __nv_bfloat162 wr[KPW];
 #pragma unroll
     for (int i = 0; i < KPW; ++i) wr[i] = i < per ? *reinterpret_cast<const __nv_bfloat162*>(wh + (size_t)i * n_out) : __floats2bfloat162_rn(0.f, 0.f);
-    pdl_wait();
     pdl_trigger();
     const int nk = n_in / 8;
     for (int i = threadIdx.x; i < TM * nk; i += 128) {
@@ -573,7 +568,6 @@ constexpr int HL_BM = 64, HL_BN = 64;
 __global__ void __launch_bounds__(128) head_linear_mma_kernel(__nv_bfloat16* __restrict__ out, int out_head_stride, int out0,
                                                               const __nv_bfloat16* __restrict__ x, int x_head_stride, int x0,
                                                               const __nv_bfloat16* __restrict__ w, int n_in, int n_out, int heads, int n_tokens, int words) {
-    pdl_wait();
     pdl_trigger();
     extern __shared__ __align__(16) unsigned char hl_smem[];
     const int lda = n_in + 8, ldb = HL_BN + 8;

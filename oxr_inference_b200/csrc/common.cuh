@@ -153,7 +153,7 @@ static inline void oxr_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 
 // The element-wise kernels and norms between a step's products and attention: chained while there is at most a block an SM, as in a decode step, where the
 // launch itself is what they cost (a Radapel decode step of 95 launches 1,064 -> 1,010 us). Such a kernel waits first thing and
-// then triggers, so that at most two kernels are under way. Not chained: larger grids, a prompt's, where a launch is nothing; and whatever
+// then triggers, so that at most two kernels are under way. Not chained (such kernels trigger, for a chained one behind them, and have nothing to wait for): larger grids, a prompt's, where a launch is nothing; and whatever
 // needs its blocks spread over the SMs (recurrences, split-KV attention, the per-head maps): blocks that start while the kernel before still holds
 // part of the chip end up side by side on the rest of it (128 blocks of a gated linear attention 896 us instead of 409).
 template <typename... KArgs, typename... Args>

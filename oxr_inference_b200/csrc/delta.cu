@@ -72,7 +72,6 @@ template <int N> __device__ __forceinline__ void delta_columns(const float* p, f
 
 template <typename T, int J, int KW>
 __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delta_scan_kernel(float* __restrict__ y, const T* __restrict__ proj, const DeltaArgs a) {
-    pdl_wait();
     using Sh = DeltaShape<J, KW>;
     constexpr int DKP = Sh::DKP, CPT = Sh::CPT, KL = (DKP + 31) / 32;      // KL: key entries per lane when a warp prepares a token
     extern __shared__ __align__(16) float dsm[];      // [2][TILE], then the results [2][TT][COLS]
@@ -337,7 +336,6 @@ __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delt
 // shared memory; every group of lanes prepares the token's vectors for its own key entries. grid (columns / 32, heads, requests).
 template <typename T, int J, int KW>
 __global__ void __launch_bounds__(32 * DELTA_WARPS) delta_step_kernel(float* __restrict__ y, const T* __restrict__ proj, const DeltaArgs a) {
-    pdl_wait();
     pdl_trigger();
     constexpr int CPT = DeltaShape<J, KW>::CPT;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane % J, c0 = (warp * (32 / J) + lane / J) * CPT;

@@ -11,7 +11,6 @@ OXR_TL_DEFINE(oxr_tl_read_elem)
 template <typename TT, typename TO>
 __global__ void embedding_kernel(TO* __restrict__ out, const TT* __restrict__ table, const int* __restrict__ ids,
                                  int hidden, int vocab, float scale, int* status) {
-    pdl_wait();
     pdl_trigger();
     const int t = blockIdx.x;
     const int id = ids[t];
@@ -29,7 +28,6 @@ __global__ void embedding_kernel(TO* __restrict__ out, const TT* __restrict__ ta
 template <typename T>
 __global__ void embedding_vec_kernel(T* __restrict__ out, const T* __restrict__ table, const int* __restrict__ ids,
                                      int words_per_row, int vocab, int* status) {
-    pdl_wait();
     pdl_trigger();
     const int t = blockIdx.x;
     const int id = ids[t];
@@ -47,7 +45,6 @@ __global__ void embedding_vec_kernel(T* __restrict__ out, const T* __restrict__ 
 // 2,048 rows 19; here 2.6 and 12.
 __global__ void embedding_widen_kernel(float* __restrict__ out, const uint4* __restrict__ table, const int* __restrict__ ids, int words_per_row, int vocab,
                                        float scale, int* status) {
-    pdl_wait();
     pdl_trigger();
     const int t = blockIdx.x;
     const int id = ids[t];

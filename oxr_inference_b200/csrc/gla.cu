@@ -29,7 +29,6 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? (KPT == 32 ? 1 : 2) : 12 / 
     float* __restrict__ y, const T* __restrict__ proj, int proj_stride, int q_col0, int k_col0, int v_col0, const float* __restrict__ z,
     const float* __restrict__ z_bias, float inv_tau, int heads, int DK, int DV, float q_scale, float* __restrict__ state, long long slot_stride,
     const int* __restrict__ cu_q, const int* __restrict__ state_slots, int most) {
-    pdl_wait();
     constexpr int DKP = KPT * NW, NT = 32 * NW;      // NT >= DKP: thread d brings key entry d of every token
     __shared__ __align__(16) float ks[TT][DKP];
     __shared__ __align__(16) float qs[TT][DKP];

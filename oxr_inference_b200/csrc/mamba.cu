@@ -136,7 +136,6 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 ? 3 : 1) ssm_scan_kernel(
     float* __restrict__ y, const T* __restrict__ xbc, const T* __restrict__ proj, int proj_stride, int dt_col0, int heads, int vdim, int N,
     int groups, const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip, float* __restrict__ state,
     long long slot_stride, const int* __restrict__ cu_q, const int* __restrict__ state_slots, int most) {
-    pdl_wait();
     constexpr int NP = 32 * NW;                       // N rounded up to whole warps
     extern __shared__ __align__(16) float scan_smem[];
     float* Bs = scan_smem;                            // [TT][NP]

@@ -70,7 +70,6 @@ __global__ void __launch_bounds__(32 * NW) mlstm_scan_kernel(
     float* __restrict__ y, const T* __restrict__ proj, int proj_stride, int q_col0, int k_col0, int v_col0, const float* __restrict__ coef,
     int heads, int DK, int DV, float q_scale, float* __restrict__ state, long long slot_stride, const int* __restrict__ cu_q,
     const int* __restrict__ state_slots) {
-    pdl_wait();
     constexpr int KPT = 32, DKP = KPT * NW, NT = 32 * NW;
     __shared__ __align__(16) float ks[TT][DKP];
     __shared__ __align__(16) float qs[TT][DKP];

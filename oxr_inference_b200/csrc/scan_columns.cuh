@@ -143,7 +143,6 @@ __device__ __forceinline__ void scan_four(const __nv_bfloat16* at, float (&v)[4]
 // grid (ceil(DV / COLS), heads, requests of this launch). Row pieces are whole 16-byte words (scan_fits).
 template <typename T, int J, int E, bool VECTOR>
 __global__ void __launch_bounds__(ScanShape<T, J, E, VECTOR>::THREADS) column_scan_kernel(const ScanArgs a) {
-    pdl_wait();
     using Sh = ScanShape<T, J, E, VECTOR>;
     constexpr int TT = SCAN_TT, TPG = J / 8, P = E / 2, W = 16 / (int)sizeof(T);      // tokens whose sums meet in one butterfly; entries of a 16-byte word
     extern __shared__ __align__(16) unsigned char column_smem[];

@@ -497,8 +497,8 @@ LONG_MASK_BYTES = 35328
 def masked_long_rows(num_heads: int, num_kv_heads: int, head_dim: int, dtype: torch.dtype, page_size: int, *, shared: bool = False,
                      bias_rows: int = 0, scale: float = 1.0) -> int:
     """Rows of a long tile for attention under the masks and extras of :func:`paged_attention`, or with keys that are the values (``shared``):
-    256 for the tcgen05 kernel at head sizes 64 and 128 (a bias table has to fit beside its operands: two bytes short of 35 KB for the heads of one
-    KV head), 128 for the tcgen05 kernel over shared rows at 192 and 256, else 64 for the mma.sync kernel, which takes everything (a scale
+    256 for the tcgen05 kernel at head sizes 64 and 128 (a bias table has to fit beside its operands: 34.5 KB for the heads of one KV
+    head, what head size 128 leaves; 64 leaves more, unused), 128 for the tcgen05 kernel over shared rows at 192 and 256, else 64 for the mma.sync kernel, which takes everything (a scale
     that is not positive too: the tcgen05 kernels scale a row's maximum, not its scores)."""
     if not tma_gathers_possible(head_dim, page_size, dtype) or not scale > 0:
         return PREFILL_ROWS
