@@ -43,8 +43,8 @@ __global__ void causal_conv_silu_kernel(T* __restrict__ out, const T* __restrict
 
 // Four taps on bf16 rows of whole 16-byte words: a thread takes eight channels of CONV_RUN tokens, one word a token, and keeps the last three inputs and the
 // weights in registers. Element by element the kernel above fetched every input four times and its weight row 16 bytes apart: 2,048 tokens of
-// 10,240 channels took 131 to 142 us, 56 to 62 here (reading and writing each value once takes 13 us). The arithmetic is that of the kernel above, entry by entry.
-constexpr int CONV_RUN = 16, CONV_THREADS = 128;
+// 10,240 channels took 131 to 142 us, 56 to 62 a word at a time, 47 to 52 here (reading and writing each value once takes 13 us). The arithmetic is that of the kernel above, entry by entry.
+constexpr int CONV_RUN = 16, CONV_THREADS = 128, CONV_AHEAD = 4;
 __device__ __forceinline__ void conv_widen(const uint4& w, float (&v)[8]) {
     const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
@@ -69,38 +69,49 @@ __global__ void __launch_bounds__(CONV_THREADS) causal_conv4_silu_words_kernel(_
     const int first = blockIdx.y * CONV_RUN, last = min(first + CONV_RUN, n_tokens);
     float past[3][8];      // the inputs of the tokens three, two and one back
     int r = -1;
-#pragma unroll 4
-    for (int t = first; t < last; ++t) {
-        const int rt = req_of_token[t];
-        if (rt != r) {     // the run's first token or a request's: what lies before it comes from the rows before, or from the request's tail
-            r = rt;
-            const int i = t - cu_q[r];
-            const float* tail = state + (long long)state_slots[r] * slot_stride + (long long)c * 3;
+    for (int t0 = first; t0 < last; t0 += CONV_AHEAD) {
+        uint4 words[CONV_AHEAD];       // asked for together: one behind the other's request, each waited for its trip to memory
+        int requests[CONV_AHEAD];
 #pragma unroll
-            for (int back = 3; back >= 1; --back) {
-                if (i - back >= 0) conv_widen(*reinterpret_cast<const uint4*>(proj + (size_t)(t - back) * proj_stride + col0 + c), past[3 - back]);
-                else {
+        for (int k = 0; k < CONV_AHEAD; ++k) {
+            const int t = min(t0 + k, last - 1);
+            words[k] = *reinterpret_cast<const uint4*>(proj + (size_t)t * proj_stride + col0 + c);
+            requests[k] = req_of_token[t];
+        }
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) past[3 - back][e] = tail[e * 3 + 3 + (i - back)];
+        for (int k = 0; k < CONV_AHEAD; ++k) {
+            const int t = t0 + k;
+            if (t >= last) break;
+            if (requests[k] != r) {     // the run's first token or a request's: what lies before it comes from the rows before, or from the request's tail
+                r = requests[k];
+                const int i = t - cu_q[r];
+                const float* tail = state + (long long)state_slots[r] * slot_stride + (long long)c * 3;
+#pragma unroll
+                for (int back = 3; back >= 1; --back) {
+                    if (i - back >= 0) conv_widen(*reinterpret_cast<const uint4*>(proj + (size_t)(t - back) * proj_stride + col0 + c), past[3 - back]);
+                    else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) past[3 - back][e] = tail[e * 3 + 3 + (i - back)];
+                    }
                 }
             }
-        }
-        float now[8], o[8];
-        conv_widen(*reinterpret_cast<const uint4*>(proj + (size_t)t * proj_stride + col0 + c), now);
+            float now[8], o[8];
+            conv_widen(words[k], now);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            float acc = fmaf(wt[e][0], past[0][e], b[e]);
-            acc = fmaf(wt[e][1], past[1][e], acc);
-            acc = fmaf(wt[e][2], past[2][e], acc);
-            acc = fmaf(wt[e][3], now[e], acc);
-            o[e] = acc / (1.f + expf(-acc));
-            past[0][e] = past[1][e]; past[1][e] = past[2][e]; past[2][e] = now[e];
-        }
-        uint4 word;
-        __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&word);
+            for (int e = 0; e < 8; ++e) {
+                float acc = fmaf(wt[e][0], past[0][e], b[e]);
+                acc = fmaf(wt[e][1], past[1][e], acc);
+                acc = fmaf(wt[e][2], past[2][e], acc);
+                acc = fmaf(wt[e][3], now[e], acc);
+                o[e] = acc / (1.f + expf(-acc));
+                past[0][e] = past[1][e]; past[1][e] = past[2][e]; past[2][e] = now[e];
+            }
+            uint4 word;
+            __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&word);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) p[e] = __floats2bfloat162_rn(o[2 * e], o[2 * e + 1]);
-        *reinterpret_cast<uint4*>(out + (size_t)t * channels + c) = word;
+            for (int e = 0; e < 4; ++e) p[e] = __floats2bfloat162_rn(o[2 * e], o[2 * e + 1]);
+            *reinterpret_cast<uint4*>(out + (size_t)t * channels + c) = word;
+        }
     }
 }
 
