@@ -12,11 +12,12 @@
 //
 // so a token has ONE sum over the key channels to wait for (both dot products of a column together), and o does not wait for the update.
 //
-// Columns of S (one value entry each) are independent: a block takes 32 of them of one head of one request, 8 per computing warp. J lanes share
-// a group of CPT = J / 4 columns: lane j holds the key entries 4 (j + J i) .. + 3, i < KW, of each (J = DK / 4 rounded up to a power of two, 4 to
+// Columns of S (one value entry each) are independent: a block takes 32 of them of one head of one request, 4 or 8 per computing warp (two warps of 4 on a scheduler
+// hide some of one another's latencies: 2,048 tokens of 32 heads of 128 x 128 608 us with one warp of 8, 588 with two). J lanes share
+// a group of CPT = J / 8 columns (J / 4 for the shorter keys): lane j holds the key entries 4 (j + J i) .. + 3, i < KW, of each (J = DK / 4 rounded up to a power of two, 4 to
 // 32; KW = 2 for keys of more than 128 entries), as pairs for the packed fp32 multiply-add; entries from DK on are zero. So every vector read
 // from shared memory is read once per group, and the 2 CPT dot products of a token meet in a butterfly that halves their number with every
-// step: lane j ends with number j / 2 of them, and a column's d1 goes back to the group by one shuffle. In memory the state lies column by
+// step until one is left: lane j ends with number j / SPREAD of them, and a column's d1 goes back to the group by one shuffle. In memory the state lies column by
 // column ([DV, DK] per head), which makes a column's lanes neighbours there, too.
 // A warp per token of a tile prepares it (unit key, decay, rate, the two scalar products), a tile of TT tokens ahead of the computing warps in a
 // second buffer, from raw values that cp.async brings in two more tiles ahead, and writes the finished tile's results out. A step of single tokens runs a
@@ -38,23 +39,45 @@ struct DeltaArgs {
     const int* cu_q;
     const int* state_slots;
     int async;                                // every row piece is whole 16-byte words: copied ahead by cp.async
+    int beside;                               // two blocks may share an SM (see `delta_launch`)
     RequestOrder order = {nullptr, 0};        // the requests in the order of their blocks
 };
 
-constexpr int DELTA_TT = 8, DELTA_COLS = 32, DELTA_WARPS = 4, DELTA_PREP_WARPS = DELTA_TT,      // tokens per tile; columns per block; computing warps; preparing warps, one per token
+constexpr int DELTA_TT = 8, DELTA_COLS = 32, DELTA_PREP_WARPS = DELTA_TT, DELTA_STEP_WARPS = 4,      // tokens per tile; columns per block; preparing warps, one per token; warps of the kernel for single tokens
               DELTA_STAGES = 4;                                                           // tiles of raw values on their way or waiting
 
 __device__ __forceinline__ float delta_sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
 
 template <int J, int KW> struct DeltaShape {
-    static constexpr int DKP = 4 * J * KW, CPT = J / 4, NV = 2 * CPT;
+    static constexpr int DKP = 4 * J * KW, CPT = J >= 16 ? J / 8 : J / 4, SPREAD = J / (2 * CPT);     // SPREAD: lanes that end with the same sum
+    static constexpr int WARPS = DELTA_COLS / (32 / J * CPT), THREADS = 32 * (WARPS + DELTA_PREP_WARPS);   // computing warps; all threads
+    static constexpr int BLOCKS = J == 32 && KW == 1 ? 2 : 1;                              // that an SM's registers are to hold
     static constexpr int VEC = DELTA_TT * DKP;                                            // one vector of every token of a tile
     static constexpr int TILE = 5 * VEC + DELTA_TT * DELTA_COLS + 2 * DELTA_TT;           // floats of a tile's buffer
     template <typename T> static constexpr int TOKEN = (2 * DKP + DELTA_COLS) * (int)sizeof(T) + 8 * DKP;      // bytes of a token's raw values
     template <typename T> static constexpr size_t SMEM =
         (size_t)(2 * TILE + 2 * DELTA_TT * DELTA_COLS) * sizeof(float) + (size_t)DELTA_STAGES * DELTA_TT * TOKEN<T>;
-    static_assert(DELTA_WARPS * (32 / J) * CPT == DELTA_COLS, "the warps hold the block's columns");
+    static_assert(WARPS * (32 / J) * CPT == DELTA_COLS, "the warps hold the block's columns");
 };
+
+// The sums of v[0 .. N - 1] over a group of 2 D neighbouring lanes, number j / (2 D / N) of them for lane j of the group: the lanes D, D / 2, ... 1 away add
+// up in that order, and while there are several numbers left, each of two lanes goes on with half of them.
+template <int N, int D> __device__ __forceinline__ float delta_sums(float (&v)[N], int lane) {
+    if constexpr (D == 0) return v[0];
+    else if constexpr (N == 1) {
+        float one[1] = {v[0] + __shfl_xor_sync(0xffffffffu, v[0], D)};
+        return delta_sums<1, D / 2>(one, lane);
+    } else {
+        float half[N / 2];
+        const bool up = (lane & D) != 0;       // this lane keeps the upper half of the numbers
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+            const float send = up ? v[i] : v[N / 2 + i], keep = up ? v[N / 2 + i] : v[i];
+            half[i] = keep + __shfl_xor_sync(0xffffffffu, send, D);
+        }
+        return delta_sums<N / 2, D / 2>(half, lane);
+    }
+}
 
 // N neighbouring floats from an address that is a multiple of N
 template <int N> __device__ __forceinline__ void delta_columns(const float* p, float (&v)[N]) {
@@ -71,7 +94,7 @@ template <int N> __device__ __forceinline__ void delta_columns(const float* p, f
 }
 
 template <typename T, int J, int KW>
-__global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delta_scan_kernel(float* __restrict__ y, const T* __restrict__ proj, const DeltaArgs a) {
+__global__ void __launch_bounds__(DeltaShape<J, KW>::THREADS, DeltaShape<J, KW>::BLOCKS) delta_scan_kernel(float* __restrict__ y, const T* __restrict__ proj, const DeltaArgs a) {
     using Sh = DeltaShape<J, KW>;
     constexpr int DKP = Sh::DKP, CPT = Sh::CPT, KL = (DKP + 31) / 32;      // KL: key entries per lane when a warp prepares a token
     extern __shared__ __align__(16) float dsm[];      // [2][TILE], then the results [2][TT][COLS]
@@ -82,9 +105,9 @@ __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delt
     const int DK = a.DK, DV = a.DV, n_tiles = (t1 - t0 + DELTA_TT - 1) / DELTA_TT;
     float* results = dsm + 2 * Sh::TILE;
 
-    if (warp >= DELTA_WARPS) {
+    if (warp >= Sh::WARPS) {
         // ---- preparing warps: token `slot` of every tile
-        const int slot = warp - DELTA_WARPS;
+        const int slot = warp - Sh::WARPS;
         float w0[KL], ab[KL];
 #pragma unroll
         for (int i = 0; i < KL; ++i) {
@@ -234,8 +257,8 @@ __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delt
             s[c][2 * i] = pack2(v.x, v.y);
             s[c][2 * i + 1] = pack2(v.z, v.w);
         }
-    const int mine = j >> 1;                                   // which of the 2 CPT sums this lane ends with: d1 of column mine, or d2 of column mine - CPT
-    const bool writes = mine >= CPT && (j & 1) == 0;
+    const int mine = j / Sh::SPREAD;                           // which of the 2 CPT sums this lane ends with: d1 of column mine, or d2 of column mine - CPT
+    const bool writes = mine >= CPT && j % Sh::SPREAD == 0;
     const int out_col = c0 + mine - CPT;
     __syncthreads();
     for (int tile = 0; tile < n_tiles; ++tile) {
@@ -283,7 +306,7 @@ __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delt
                 uu[i] = vec[DKP / 4 + J * i];
                 wr[i] = vec[Sh::VEC / 4 + DKP / 4 + J * i];
             }
-            const float sum = group_reduce<2 * CPT>(d, lane);
+            const float sum = delta_sums<2 * CPT, J / 2>(d, lane);
             // the part of the update that does not wait for the sums
 #pragma unroll
             for (int c = 0; c < CPT; ++c) {
@@ -297,7 +320,7 @@ __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delt
             const float held = __shfl_xor_sync(0xffffffffu, sum, J / 2);      // d1 of the column whose d2 this lane has
 #pragma unroll
             for (int c = 0; c < CPT; ++c) {
-                const float a1 = __shfl_sync(0xffffffffu, sum, 2 * c, J);
+                const float a1 = __shfl_sync(0xffffffffu, sum, Sh::SPREAD * c, J);
                 const f32x2 h2 = pack2(a1, a1);
 #pragma unroll
                 for (int i = 0; i < KW; ++i) {
@@ -335,9 +358,9 @@ __global__ void __launch_bounds__(32 * (DELTA_WARPS + DELTA_PREP_WARPS), 1) delt
 // One token per request (a decode step), where a step is its state's way through the registers: the same layout of columns over lanes without
 // shared memory; every group of lanes prepares the token's vectors for its own key entries. grid (columns / 32, heads, requests).
 template <typename T, int J, int KW>
-__global__ void __launch_bounds__(32 * DELTA_WARPS) delta_step_kernel(float* __restrict__ y, const T* __restrict__ proj, const DeltaArgs a) {
+__global__ void __launch_bounds__(32 * DELTA_STEP_WARPS) delta_step_kernel(float* __restrict__ y, const T* __restrict__ proj, const DeltaArgs a) {
     pdl_trigger();
-    constexpr int CPT = DeltaShape<J, KW>::CPT;
+    constexpr int CPT = J / 4;         // columns a thread
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane % J, c0 = (warp * (32 / J) + lane / J) * CPT;
     const int p0 = blockIdx.x * DELTA_COLS + c0, h = blockIdx.y, r = blockIdx.z, DK = a.DK, DV = a.DV;
     const int t = a.cu_q[r];
@@ -430,16 +453,19 @@ static int delta_launch(float* y, const T* proj, const DeltaArgs& a, int n_reque
     using Sh = DeltaShape<J, KW>;
     const dim3 grid((a.DV + DELTA_COLS - 1) / DELTA_COLS, a.heads, n_requests);
     if (single) {
-        oxr_launch(delta_step_kernel<T, J, KW>, dim3(grid), dim3(32 * DELTA_WARPS), 0, stream, false, y, proj, a);
+        oxr_launch(delta_step_kernel<T, J, KW>, dim3(grid), dim3(32 * DELTA_STEP_WARPS), 0, stream, false, y, proj, a);
         return oxr_launch_status();
     }
-    constexpr size_t SMEM = Sh::template SMEM<T>;
+    // Two blocks on an SM take a token each in about 0.47 us where one alone takes 0.29: better for several requests of like lengths, worse for a long one (blocks are dealt
+    // out two to an SM also while SMs are free). A block that is to be alone asks for more than half of the shared memory. 32 heads of 128 x 128, us, alone and
+    // beside: 700, 700, 700 tokens 609 and 537, 1,000 and 900: 550 and 477, 16 of 100: 441 and 355, 1,200 beside 40 single tokens 475 and 674.
+    constexpr size_t SMEM = Sh::template SMEM<T>, ALONE = Sh::BLOCKS > 1 && SMEM < 116 * 1024 ? 116 * 1024 : SMEM;
     static_assert(SMEM <= 227 * 1024, "fits a block");
-    if constexpr (SMEM > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<T, J, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    if constexpr (ALONE > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<T, J, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ALONE);
         if (e != cudaSuccess) return 1000 + (int)e;
     }
-    oxr_launch(delta_scan_kernel<T, J, KW>, dim3(grid), dim3(32 * (DELTA_WARPS + DELTA_PREP_WARPS)), SMEM, stream, false, y, proj, a);
+    oxr_launch(delta_scan_kernel<T, J, KW>, dim3(grid), dim3(Sh::THREADS), a.beside ? SMEM : ALONE, stream, false, y, proj, a);
     return oxr_launch_status();
 }
 
@@ -455,13 +481,14 @@ static int delta_launch_j(float* y, const T* proj, const DeltaArgs& a, int n_req
 OXR_API int oxr_delta_scan(float* y, const void* proj, int n_requests, int stride, int r_col0, int k_col0, int v_col0, const float* zw, int zw_stride,
                            const float* w0, const float* za, int za_stride, const float* ab, float rate, float len_eps, int heads, int DK, int DV,
                            float* state, long long slot_stride, const int* cu_q, const int* state_slots, int single, int dtype,
-                           const int* order, cudaStream_t stream) {
+                           const int* order, int beside, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (heads <= 0 || DK <= 0 || DK > 256 || DV <= 0 || heads > 65535 || n_requests > 65535 || !(rate > 0.f) || !(len_eps > 0.f)) return OXR_BAD_ARGUMENT;
     DeltaArgs a;
     a.stride = stride; a.r_col0 = r_col0; a.k_col0 = k_col0; a.v_col0 = v_col0; a.zw = zw; a.zw_stride = zw_stride; a.w0 = w0; a.za = za;
     a.za_stride = za_stride; a.ab = ab; a.rate = rate; a.len_eps = len_eps; a.heads = heads; a.DK = DK; a.DV = DV; a.state = state;
     a.slot_stride = slot_stride; a.cu_q = cu_q; a.state_slots = state_slots;
+    a.beside = beside;
     a.order = RequestOrder(order, n_requests);
     const int word = dtype == 0 ? 4 : 8;      // elements of the projections per 16 bytes
     a.async = DK % word == 0 && DK % 4 == 0 && DV % word == 0 && stride % word == 0 && r_col0 % word == 0 && k_col0 % word == 0 && v_col0 % word == 0 &&

@@ -184,7 +184,7 @@ def _lib():
         lib.oxr_gelu_glu.argtypes = [p, p, i, i, i, i, p]
         lib.oxr_scaled_sum.argtypes = [p, p, p, f, f, ll, i, p]
         lib.oxr_shift_norm.argtypes = [p, p, p, p, p, f, p, f, p, p, ll, p, p, p, i, i, i, i, p]
-        lib.oxr_delta_scan.argtypes = [p, p, i, i, i, i, i, p, i, p, p, i, p, f, f, i, i, i, p, ll, p, p, i, i, p, p]
+        lib.oxr_delta_scan.argtypes = [p, p, i, i, i, i, i, p, i, p, p, i, p, f, f, i, i, i, p, ll, p, p, i, i, p, i, p]
         lib.oxr_tanh_cols.argtypes = [p, p, i, i, i, i, i, p]
         lib.oxr_diff_prep.argtypes = [p, p, p, p, i, i, i, i, i, i, i, i, i, i, i, p, p, ll, i, p, p]
         lib.oxr_diff_combine.argtypes = [p, p, i, i, i, i, p, f, f, i, p]
@@ -1539,6 +1539,15 @@ def _longest_first(q_lens: Sequence[int] | None, n_requests: int) -> ctypes.Arra
     return (c_int * n_requests)(*sorted(range(n_requests), key=q_lens.__getitem__, reverse=True))
 
 
+def _delta_beside(q_lens: Sequence[int] | None, heads: int, value_dim: int) -> bool:
+    """Whether two blocks of the delta rule are to share an SM: each then takes 1.63 times as long for a token, and twice as many run. Alone the blocks take as long as the
+    longest request, or as all of them dealt out over the SMs."""
+    if q_lens is None or len(q_lens) < 2:
+        return False
+    longest = max(q_lens)
+    return 1.63 * longest < max(longest, sum(q_lens) * heads * -(-value_dim // 32) / num_sms())
+
+
 def _need_lengths(q_lens: Sequence[int], n_requests: int) -> None:
     if len(q_lens) != n_requests:
         raise KernelError(f"{len(q_lens)} request lengths for {n_requests} requests")
@@ -2279,7 +2288,8 @@ def delta_scan(proj: torch.Tensor, r_col0: int, k_col0: int, v_col0: int, zw: to
     _done(_lib().oxr_delta_scan(y.data_ptr(), proj.data_ptr(), int(n_requests), proj.shape[1], int(r_col0), int(k_col0), int(v_col0), zw.data_ptr(),
                                 zw.shape[1], w_bias.data_ptr(), za.data_ptr(), za.shape[1], a_bias.data_ptr(), float(rate), float(len_eps), int(heads),
                                 int(key_dim), int(value_dim), state.data_ptr(), state.stride(0), cu_q.data_ptr(), state_slots.data_ptr(),
-                                int(bool(single_tokens)), _dtype_code(proj), None if single_tokens else _longest_first(q_lens, n_requests), _stream()), "delta_scan")
+                                int(bool(single_tokens)), _dtype_code(proj), None if single_tokens else _longest_first(q_lens, n_requests),
+                                int(_delta_beside(q_lens, heads, value_dim)), _stream()), "delta_scan")
     return y
 
 
