@@ -112,7 +112,8 @@ def _lib():
         lib.oxr_silu_mul.argtypes = [p, p, i, i, i, i, p]
         lib.oxr_cast.argtypes = [p, p, c_size_t, i, i, p]
         lib.oxr_qk_norm_rope_store.argtypes = [p, p, p, p, p, p, p, p, p, p, i, i, i, i, f, i, c_longlong, i, i, i, i, p, p]
-        lib.oxr_gemm_f32_nt.argtypes = [p, p, p, i, i, i, p]
+        lib.oxr_gemm_f32_nt.argtypes = [p, p, p, p, i, i, i, i, i, p, p]
+        lib.oxr_gemm_f32_segments.argtypes = [i]
         lib.oxr_gemm_skinny_bf16.argtypes = [p, p, p, i, i, i, i, p]
         lib.oxr_gemm_skinny_gated_bf16.argtypes = [p, p, p, i, i, i, p]
         lib.oxr_gemm_stream_bf16.argtypes = [p, p, p, i, i, i, i, i, p, p]
@@ -203,7 +204,7 @@ def _lib():
                      "oxr_gated_relu2", "oxr_expert_sort", "oxr_gather_rows", "oxr_combine_rows", "oxr_gemm_tcgen05_grouped_bf16"):
             getattr(lib, name).restype = c_int
         for name in ("oxr_embedding", "oxr_add_rms_norm", "oxr_silu_mul", "oxr_cast", "oxr_qk_norm_rope_store",
-                     "oxr_gemm_f32_nt", "oxr_gemm_skinny_bf16", "oxr_gemm_skinny_gated_bf16", "oxr_gemm_stream_bf16", "oxr_gemm_stream_gated_bf16", "oxr_gemm_tcgen05_bf16", "oxr_gemm_tcgen05_pair_bf16", "oxr_gemm_tcgen05_gated_bf16", "oxr_gemm_few_rows_cluster_bf16", "oxr_gemm_few_rows_max_clusters",
+                     "oxr_gemm_f32_nt", "oxr_gemm_f32_segments", "oxr_gemm_skinny_bf16", "oxr_gemm_skinny_gated_bf16", "oxr_gemm_stream_bf16", "oxr_gemm_stream_gated_bf16", "oxr_gemm_tcgen05_bf16", "oxr_gemm_tcgen05_pair_bf16", "oxr_gemm_tcgen05_gated_bf16", "oxr_gemm_few_rows_cluster_bf16", "oxr_gemm_few_rows_max_clusters",
                      "oxr_gemm_tcgen05_pair_gated_bf16", "oxr_sample", "oxr_repetition_penalty", "oxr_mark_seen"):
             getattr(lib, name).restype = c_int
         lib.oxr_set_chain.argtypes = [c_int]
@@ -862,6 +863,27 @@ def _gemm_plan(m: int, n: int, k: int, may_split: bool = True) -> tuple[int, int
     return best
 
 
+F32_MAX_TILE = 128
+
+
+@functools.lru_cache(maxsize=None)
+def _gemm_f32_plan(m: int, n: int, k: int) -> tuple[int, bool]:
+    """(rows of x per block, whether the segments of k go to the blocks of a cluster) of the 32-bit product: the least rounds of blocks times what a block
+    takes, 1.15 + 0.0065 * rows microseconds per 64 k and 4 at its ends. Measured on a B200 with 1 to 1,000 rows and 2,048 to 16,384 columns, the formula is within 15 % of it:
+    333 rows x 16,384 x 2,048 in three tiles of 112 rows 190 us (a fourth of 96: 238), 333 x 2,048 x 8,192 206 us in one block a tile, 100 in clusters of four."""
+    best, best_cost = (16, False), None
+    segments = _lib().oxr_gemm_f32_segments(k)
+    for tiles in range(-(-m // F32_MAX_TILE), -(-m // 16) + 1):
+        tile = -(-(-(-m // tiles)) // 16) * 16
+        blocks = -(-m // tile) * -(-n // 128)
+        for parts in {1, segments}:
+            rounds = -(-blocks // (_few_rows_clusters(parts) if parts > 1 else num_sms()))
+            cost = rounds * (k / 64 / parts * (1.15 + 0.0065 * tile) + 4)
+            if best_cost is None or cost < best_cost - 1e-9:
+                best, best_cost = (tile, parts > 1), cost
+    return best
+
+
 GEMM_FEW_ROWS = 256          # the widest tile of a tcgen05 product
 GEMM_FEW_ROWS_ANY_SHARES = 192
 
@@ -937,7 +959,7 @@ def _gemm_split_buffers(device: torch.device) -> tuple[torch.Tensor, torch.Tenso
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """``x @ weight.T`` for ``weight [out, in]``, no bias (oxr_runtime/language.py:223-231), fp32 accumulation.
 
-    float32 x float32 runs the fp32 CUDA-core kernel (no TF32). bfloat16 x bfloat16 runs the skinny kernel up to
+    float32 x float32 runs the tensor-core kernel on parts of eight bits, whose error is that of fewer 32-bit roundings than K (no TF32). bfloat16 x bfloat16 runs the skinny kernel up to
     ``SKINNY_MAX_ROWS`` rows and the TMA + tcgen05 kernel beyond (cuBLAS only when a row is not a whole number of
     16-byte words). A weight kept in float32 under bfloat16 activations is multiplied in fp32 and the result
     rounded once. ``out`` (contiguous ``[rows, out]`` of the output dtype) receives the product instead of a new tensor.
@@ -963,7 +985,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     if weight.dtype == torch.float32:
         x32 = cast(x, torch.float32)
         out = given if given is not None and out_dtype == torch.float32 else torch.empty((m, n), dtype=torch.float32, device=x.device)
-        _done(lib.oxr_gemm_f32_nt(out.data_ptr(), x32.data_ptr(), weight.data_ptr(), m, n, k, _stream()), "gemm_f32")
+        tile, shared = _gemm_f32_plan(m, n, k)
+        parts = torch.empty((3, m, -(-k // 8) * 8), dtype=torch.bfloat16, device=x.device)
+        _done(lib.oxr_gemm_f32_nt(out.data_ptr(), x32.data_ptr(), weight.data_ptr(), parts.data_ptr(), m, n, k, tile, int(shared),
+                                  new_status(x.device).data_ptr(), _stream()), "gemm_f32")
         if given is not None and out_dtype != torch.float32:
             given.copy_(out)
             return given

@@ -1,0 +1,54 @@
+"""The 32-bit product on parts of eight bits, at the sizes where it can go wrong."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from oxr_inference_b200 import ops
+
+    return ops
+
+
+def randn(*shape, seed):
+    return torch.randn(*shape, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV)
+
+
+@pytest.mark.parametrize("widened", [False, True], ids=["24bit", "widened"])
+@pytest.mark.parametrize("K", [60, 64, 1028, 2048, 4100, 8190])
+def test_sums_in_segments_are_the_same_however_dealt_out(ops, K, widened):
+    """One, two and four segments of k, whole and ragged chunks, rows of whole 16-byte words and others; blocks that take one segment and blocks that take
+    all, tiles of every width. W of 24-bit numbers, of bf16 numbers, and with a few 24-bit numbers among these (a chunk then takes all six products)."""
+    x, w = randn(130, K, seed=1), randn(300, K, seed=2)
+    if widened:
+        w = w.bfloat16().float()
+        w[70, K // 2] += 2 ** -20
+        w[299, K - 1] = 1 / 3
+    want = x.double() @ w.double().T
+    lib, status = ops._lib(), ops.new_status(DEV)
+    got = []
+    for tile in (16, 48, 112, 128):
+        for shared in (0, 1):
+            out = torch.full((130, 300), float("nan"), device=DEV)
+            parts = torch.empty(3, 130, -(-K // 8) * 8, dtype=torch.bfloat16, device=DEV)
+            assert lib.oxr_gemm_f32_nt(out.data_ptr(), x.data_ptr(), w.data_ptr(), parts.data_ptr(), 130, 300, K, tile, shared, status.data_ptr(), ops._stream()) == 0
+            got.append(out)
+    ops.check_status(status)
+    # a chunk's four times sixteen products, each time at most 2^-23 of what is there, and the parts left out; then K / 64 + 4 roundings of 2^-24
+    assert ((got[0].double() - want).abs() <= (16 + K / 64) * 2 ** -24 * (x.double().abs() @ w.double().abs().T)).all()
+    assert all(torch.equal(got[0], other) for other in got[1:])
+    assert torch.equal(ops.linear(x[7:8].contiguous(), w), got[0][7:8])
+
+
+def test_infinities_and_what_rounds_to_one(ops):
+    x, w = randn(20, 300, seed=3), randn(140, 300, seed=4)
+    x[3, 5], x[4, 7], x[6, 20] = float("inf"), float("nan"), 3.4e38
+    w[10, 5], w[11, 9], w[12, 20] = 0.0, -float("inf"), 0.5
+    got, want = ops.linear(x, w), (x.double() @ w.double().T).float()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()], want[want.isinf()])
+    assert got[6, 12].isfinite() and abs(got[6, 12] / want[6, 12] - 1) < 1e-6
