@@ -27,7 +27,7 @@ constexpr int BN = 32;
 constexpr int SIMT_WARPS = 4;
 constexpr int ROWS_PER_WARP = BM / SIMT_WARPS;
 constexpr int DCHUNKS = (D + 31) / 32;
-constexpr int KS_STRIDE = D + 1;
+constexpr int KS_STRIDE = D + 4;   // rows of whole 16-byte words, eight neighbouring ones on different banks
 
 struct AttnArgs {
     const int* tile_req;     // [tiles] request of each tile
@@ -114,14 +114,46 @@ template <> struct Vec<__nv_bfloat16> {
     }
 };
 
+// Rows of one K or V block on their way into shared memory: fp32 rows as they are by cp.async, others widened. Zeros for keys outside [k_lo, k_end).
+template <typename T>
+__device__ __forceinline__ void simt_load(float* dst, int stride, const T* __restrict__ cache, int kt, int k_lo, int k_end, int req, int kvh, bool say, const AttnArgs& a) {
+    constexpr int VE = Vec<T>::N, VPK = D / VE;                                       // vectors per key
+    for (int v = threadIdx.x; v < BN * VPK; v += SIMT_WARPS * 32) {
+        const int j = v / VPK, part = v % VPK, kp = kt + j;
+        bool ok = kp >= k_lo && kp < k_end;
+        size_t base = 0;
+        if (ok) {
+            const int page = a.block_table[(size_t)req * a.table_width + (a.page_shift >= 0 ? kp >> a.page_shift : kp / a.page_size)];
+            ok = page >= 0 && page < a.num_pages;
+            if (ok) base = (((size_t)page * a.page_size + (a.page_shift >= 0 ? kp & (a.page_size - 1) : kp % a.page_size)) * a.KV + kvh) * D + part * VE;
+            else if (say && part == 0) oxr_report(a.status, OXR_BAD_PAGE, req);
+        }
+        float* at = dst + j * stride + part * VE;
+        if constexpr (sizeof(T) == 4) {
+            const int bytes = ok ? 16 : 0;   // 0: the 16 bytes are zero-filled and the cache is not read
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(at)), "l"(cache + base), "r"(bytes) : "memory");
+        } else {
+            float f[VE];
+#pragma unroll
+            for (int e = 0; e < VE; ++e) f[e] = 0.f;
+            if (ok) Vec<T>::load(cache + base, f);
+#pragma unroll
+            for (int e = 0; e < VE; e += 4) *reinterpret_cast<float4*>(at + e) = make_float4(f[e], f[e + 1], f[e + 2], f[e + 3]);
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// What bounds it is the multiply-adds' issue and, in a short prompt, the chain of blocks of the last rows: rows and weights come out of shared memory four
+// entries at a time (a word read per three multiply-adds instead of one each), the next block's keys and this block's values arrive meanwhile.
 template <typename T>
 __global__ void __launch_bounds__(SIMT_WARPS * 32)
 attn_simt_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restrict__ k_cache,
                  const T* __restrict__ v_cache, const AttnArgs a) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     float* Qs = smem;                       // [BM][D]
-    float* Ks = Qs + BM * D;                // [BN][D + 1]
-    float* Vs = Ks + BN * KS_STRIDE;        // [BN][D]
+    float* Ks = Qs + BM * D;                // [2][BN][D + 4]
+    float* Vs = Ks + 2 * BN * KS_STRIDE;    // [BN][D]
     float* Ps = Vs + BN * D;                // [BM][BN]
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -164,44 +196,33 @@ attn_simt_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restri
     const int k_end = pos0 + tok_end;                                                  // exclusive, causal bound
     const int k_lo = a.window > 0 ? max(0, pos0 + tok0 - a.window + 1) : 0;            // first key any row sees
     const int k_first = (k_lo / BN) * BN;
-    constexpr int VE = Vec<T>::N, VPK = D / VE;                                       // vectors per key
 
-    for (int kt = k_first; kt < k_end; kt += BN) {
-        __syncthreads();   // previous tile fully consumed (also orders the Q store before the first use)
-        for (int v = tid; v < BN * VPK; v += SIMT_WARPS * 32) {
-            const int j = v / VPK, part = v % VPK;
-            const int kp = kt + j;
-            float kf[VE], vf[VE];
-#pragma unroll
-            for (int e = 0; e < VE; ++e) kf[e] = vf[e] = 0.f;
-            if (kp >= k_lo && kp < k_end) {
-                const int page = a.block_table[(size_t)req * a.table_width + kp / a.page_size];
-                if (page < 0 || page >= a.num_pages) {
-                    if (part == 0) oxr_report(a.status, OXR_BAD_PAGE, req);
-                } else {
-                    const size_t base = (((size_t)page * a.page_size + kp % a.page_size) * a.KV + kvh) * D + part * VE;
-                    Vec<T>::load(k_cache + base, kf);
-                    Vec<T>::load(v_cache + base, vf);
-                }
-            }
-#pragma unroll
-            for (int e = 0; e < VE; ++e) {
-                Ks[j * KS_STRIDE + part * VE + e] = kf[e];
-                Vs[j * D + part * VE + e] = vf[e];
-            }
-        }
-        __syncthreads();
+    if (k_first < k_end) simt_load<T>(Ks, KS_STRIDE, k_cache, k_first, k_lo, k_end, req, kvh, true, a);
+    for (int kt = k_first, buf = 0; kt < k_end; kt += BN, buf ^= 1) {
+        __syncthreads();   // the block before is fully consumed
+        simt_load<T>(Vs, D, v_cache, kt, k_lo, k_end, req, kvh, false, a);
+        // (behind the last block: keys from k_end on, all zeros, never used)
+        simt_load<T>(Ks + (buf ^ 1) * BN * KS_STRIDE, KS_STRIDE, k_cache, kt + BN, k_lo, k_end, req, kvh, true, a);
+        asm volatile("cp.async.wait_group 2;" ::: "memory");
+        __syncthreads();   // this block's keys are there (and, in the first, Q is)
 
         // ---- scores: lane = key, this warp's rows
         float s[ROWS_PER_WARP];
 #pragma unroll
         for (int i = 0; i < ROWS_PER_WARP; ++i) s[i] = 0.f;
-        const float* krow = Ks + lane * KS_STRIDE;
-#pragma unroll 8
-        for (int d = 0; d < D; ++d) {
-            const float kv = krow[d];
+        const float* krow = Ks + (buf * BN + lane) * KS_STRIDE;
+        const float* qrow = Qs + warp * ROWS_PER_WARP * D;
+#pragma unroll 4
+        for (int d = 0; d < D; d += 4) {
+            const float4 kv = *reinterpret_cast<const float4*>(krow + d);
 #pragma unroll
-            for (int i = 0; i < ROWS_PER_WARP; ++i) s[i] = fmaf(Qs[(warp * ROWS_PER_WARP + i) * D + d], kv, s[i]);
+            for (int i = 0; i < ROWS_PER_WARP; ++i) {
+                const float4 qv = *reinterpret_cast<const float4*>(qrow + i * D + d);
+                s[i] = fmaf(qv.x, kv.x, s[i]);
+                s[i] = fmaf(qv.y, kv.y, s[i]);
+                s[i] = fmaf(qv.z, kv.z, s[i]);
+                s[i] = fmaf(qv.w, kv.w, s[i]);
+            }
         }
         const int kp = kt + lane;
         float alpha[ROWS_PER_WARP];
@@ -220,29 +241,37 @@ attn_simt_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restri
             m[i] = m_new;
             Ps[(warp * ROWS_PER_WARP + i) * BN + lane] = p;
         }
-        __syncwarp();
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();   // this block's values are there
 
         // ---- O += P V: lane = column of V
 #pragma unroll
         for (int i = 0; i < ROWS_PER_WARP; ++i)
 #pragma unroll
             for (int c = 0; c < DCHUNKS; ++c) o[i][c] *= alpha[i];
-        for (int j = 0; j < BN; ++j) {
-            float pv[ROWS_PER_WARP];
+#pragma unroll 2
+        for (int j0 = 0; j0 < BN; j0 += 4) {
+            float pv[ROWS_PER_WARP][4];
 #pragma unroll
-            for (int i = 0; i < ROWS_PER_WARP; ++i) pv[i] = Ps[(warp * ROWS_PER_WARP + i) * BN + j];
+            for (int i = 0; i < ROWS_PER_WARP; ++i) {
+                const float4 p4 = *reinterpret_cast<const float4*>(Ps + (warp * ROWS_PER_WARP + i) * BN + j0);
+                pv[i][0] = p4.x; pv[i][1] = p4.y; pv[i][2] = p4.z; pv[i][3] = p4.w;
+            }
 #pragma unroll
-            for (int c = 0; c < DCHUNKS; ++c) {
-                const int d = lane + 32 * c;
-                if (d < D) {
-                    const float vv = Vs[j * D + d];
+            for (int j = 0; j < 4; ++j) {
 #pragma unroll
-                    for (int i = 0; i < ROWS_PER_WARP; ++i) o[i][c] = fmaf(pv[i], vv, o[i][c]);
+                for (int c = 0; c < DCHUNKS; ++c) {
+                    const int d = lane + 32 * c;
+                    if (d < D) {
+                        const float vv = Vs[(j0 + j) * D + d];
+#pragma unroll
+                        for (int i = 0; i < ROWS_PER_WARP; ++i) o[i][c] = fmaf(pv[i][j], vv, o[i][c]);
+                    }
                 }
             }
         }
-        __syncwarp();
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 
 #pragma unroll
     for (int i = 0; i < ROWS_PER_WARP; ++i) {
@@ -259,7 +288,7 @@ attn_simt_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restri
     }
 }
 
-constexpr size_t SIMT_SMEM = (size_t)(BM * D + BN * KS_STRIDE + BN * D + BM * BN) * sizeof(float);
+constexpr size_t SIMT_SMEM = (size_t)(BM * D + 2 * BN * KS_STRIDE + BN * D + BM * BN) * sizeof(float);
 
 template <typename T>
 int launch_simt(void* out, const void* q, const void* k_cache, const void* v_cache, const AttnArgs& a, int num_tiles,
