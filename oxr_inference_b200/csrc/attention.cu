@@ -562,6 +562,30 @@ __device__ __forceinline__ TileGeometry tile_geometry(const AttnArgs& a, int row
 }
 
 // Q rows [row0, row0 + nrows) of the tile -> shared memory (zeros for rows without a token/head).
+// The same for rows of 32 chunks (head size 256), in two steps: warp w copies the rows w, w + 4, ..., and its lane l looks row w + 4 (l % 16) up: one trip to the
+// block table for all of them, where a lookup behind each row's bounds check made sixteen, one after the other. -1: no key there.
+constexpr bool ROW_PER_WARP = D == 256;
+__device__ __forceinline__ int lookup_kv_row(const int* __restrict__ table_row, const AttnArgs& a, int k0, int k_lo, int k_end, int req) {
+    const int kp = k0 + (threadIdx.x >> 5) + 4 * (threadIdx.x & 15);
+    if (kp < k_lo || kp >= k_end) return -1;
+    const int page = table_row[a.page_shift >= 0 ? kp >> a.page_shift : kp / a.page_size];
+    if (page < 0 || page >= a.num_pages) {
+        oxr_report(a.status, OXR_BAD_PAGE, req);
+        return -1;
+    }
+    return a.page_shift >= 0 ? (page << a.page_shift) + (kp & (a.page_size - 1)) : page * a.page_size + kp % a.page_size;
+}
+__device__ __forceinline__ void copy_kv_rows(bf16* Ks, bf16* Vs, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache, const AttnArgs& a, int kvh, int rows) {
+    const size_t row_elems = (size_t)a.KV * D, col = (size_t)kvh * D + (threadIdx.x & 31) * 8;
+    const int at = (threadIdx.x >> 5) * LDS + (threadIdx.x & 31) * 8;
+#pragma unroll 4
+    for (int i = 0; i < MMA_BN / 4; ++i) {
+        const int row = __shfl_sync(0xffffffffu, rows, i);
+        const size_t base = row >= 0 ? (size_t)row * row_elems + col : 0;
+        cp_async_16(Ks + at + 4 * i * LDS, k_cache + base, row >= 0);
+        if (Vs != nullptr) cp_async_16(Vs + at + 4 * i * LDS, v_cache + base, row >= 0);
+    }
+}
 __device__ __forceinline__ void load_q_rows(bf16* Qs, const bf16* __restrict__ q, const AttnArgs& a, const TileGeometry& g,
                                             int nrows) {
     constexpr int CPR = D / 8;
@@ -745,10 +769,10 @@ __device__ __forceinline__ void merge_warps(const float* mo, int nrows, int spli
 constexpr int MERGE_ITEMS = D > 128 ? 4 : 1;     // two at head size 128 cost a short context's decode step 1 us a layer
 template <int NI>
 __device__ __forceinline__ void merge_pieces(bf16* __restrict__ out, const float* __restrict__ all_ml, const float* __restrict__ all_o,
-                                             int splits, int rows_live, const TileGeometry& g, const AttnArgs& a) {
+                                             int splits, int rows_live, const TileGeometry& g, const AttnArgs& a, int row0 = 0) {
     constexpr int CHUNK = 8, DV = D / 4;
     const int total = rows_live * DV;
-    for (int idx0 = threadIdx.x; idx0 < total; idx0 += MMA_THREADS * NI) {
+    for (int idx0 = row0 * DV + threadIdx.x; idx0 < total; idx0 += MMA_THREADS * NI) {
         float M[NI], L[NI];
         float4 O[NI];
         int row[NI], d[NI];
@@ -827,7 +851,8 @@ attn_mma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float
                        int* __restrict__ counters, const bf16* __restrict__ q, const bf16* __restrict__ k_cache,
                        const bf16* __restrict__ v_cache, const AttnArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_ticket;
+    [[maybe_unused]] __shared__ int s_ticket;
+    if constexpr (SHARED) pdl_trigger();      // the merging kernel's blocks may wait beside this one's
     bf16* Qs = reinterpret_cast<bf16*>(smem_raw);
     bf16* Ks = Qs + DECODE_ROWS * LDS;                      // DECODE_STAGES stages
     bf16* Vs = SHARED ? Ks : Ks + DECODE_STAGES * MMA_BN * LDS;   // DECODE_STAGES stages
@@ -853,12 +878,19 @@ attn_mma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float
 
     if (count > 0) {
         const int* table_row = a.block_table + (size_t)g.req * a.table_width;
+        auto lookup = [&](int b) { return lookup_kv_row(table_row, a, kw.key0(first + b, MMA_BN), kw.lo(first + b), kw.end(first + b, k_end), g.req); };
+        auto load = [&](int b, int rows) {      // block b of the piece into its stage; rows: its lookup, where there is one
+            bf16 *ks = Ks + (b % DECODE_STAGES) * MMA_BN * LDS, *vs = SHARED ? nullptr : Vs + (b % DECODE_STAGES) * MMA_BN * LDS;
+            if constexpr (ROW_PER_WARP) copy_kv_rows(ks, vs, k_cache, v_cache, a, g.kvh, rows);
+            else load_kv_block(ks, vs, k_cache, v_cache, table_row, a, g.kvh, kw.key0(first + b, MMA_BN), kw.lo(first + b), kw.end(first + b, k_end), g.req);
+        };
+        int rows[DECODE_STAGES - 1];
+#pragma unroll
+        for (int st = 0; st < DECODE_STAGES - 1; ++st) rows[st] = ROW_PER_WARP && st < count ? lookup(st) : -1;
         load_q_rows(Qs, q, a, g, DECODE_ROWS);
 #pragma unroll
         for (int st = 0; st < DECODE_STAGES - 1; ++st) {
-            if (st < count)
-                load_kv_block(Ks + st * MMA_BN * LDS, SHARED ? nullptr : Vs + st * MMA_BN * LDS, k_cache, v_cache, table_row, a, g.kvh,
-                              kw.key0(first + st, MMA_BN), kw.lo(first + st), kw.end(first + st, k_end), g.req);
+            if (st < count) load(st, rows[st]);
             cp_async_commit();
         }
         int row_pos[2], row_lo[2];
@@ -885,9 +917,7 @@ attn_mma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float
             // block b + STAGES - 1 goes into the stage that block b - 1 used; the barrier at the end of the previous
             // iteration made it free
             const int nb = b + DECODE_STAGES - 1;
-            if (nb < count)
-                load_kv_block(Ks + (nb % DECODE_STAGES) * MMA_BN * LDS, SHARED ? nullptr : Vs + (nb % DECODE_STAGES) * MMA_BN * LDS, k_cache, v_cache,
-                              table_row, a, g.kvh, kw.key0(first + nb, MMA_BN), kw.lo(first + nb), kw.end(first + nb, k_end), g.req);
+            if (nb < count) load(nb, ROW_PER_WARP ? lookup(nb) : -1);
             cp_async_commit();
             cp_async_wait<DECODE_STAGES - 1>();
             __syncthreads();
@@ -938,17 +968,34 @@ attn_mma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float
     }
     if (splits == 1) return;
 
-    // ---- ticket: the last piece to finish merges them all
-    __threadfence();          // this block's partial is visible device-wide before its ticket is
-    __syncthreads();
-    if (threadIdx.x == 0) s_ticket = atomicAdd(&counters[unit], 1);
-    __syncthreads();
-    if (s_ticket != splits - 1) return;
-    __threadfence();          // order the reads below after the tickets of the other pieces
-    if (threadIdx.x == 0) counters[unit] = 0;   // ready for the next launch (nobody else touches it any more)
-    const float* all_ml = part_ml + unit * splits * DECODE_ROWS * 2;
-    const float* all_o = part_o + unit * splits * DECODE_ROWS * D;
-    merge_pieces<MERGE_ITEMS>(out, all_ml, all_o, splits, rows_live, g, a);
+    if constexpr (!SHARED) {
+        // ---- ticket: the last piece to finish merges them all
+        __threadfence();          // this block's partial is visible device-wide before its ticket is
+        __syncthreads();
+        if (threadIdx.x == 0) s_ticket = atomicAdd(&counters[unit], 1);
+        __syncthreads();
+        if (s_ticket != splits - 1) return;
+        __threadfence();          // order the reads below after the tickets of the other pieces
+        if (threadIdx.x == 0) counters[unit] = 0;   // ready for the next launch (nobody else touches it any more)
+        const float* all_ml = part_ml + unit * splits * DECODE_ROWS * 2;
+        const float* all_o = part_o + unit * splits * DECODE_ROWS * D;
+        merge_pieces<MERGE_ITEMS>(out, all_ml, all_o, splits, rows_live, g, a);
+    }
+}
+
+// The pieces of the shared form (one key/value head, a unit per 16 query rows) merged by a block per two rows: few units of many pieces are what a compressed cache's
+// decode step makes, and the last block of each took 15 to 19 of a launch's 34 to 39 us for its 290 KB of partial results (8 requests of 2,048 keys, 18
+// pieces of 16 rows of 256). The same sums in the same order.
+constexpr int COMBINE_ROWS = 2;
+__global__ void __launch_bounds__(MMA_THREADS) attn_combine_kernel(bf16* __restrict__ out, const float* __restrict__ part_o, const float* __restrict__ part_ml, int splits,
+                                                                   const AttnArgs a) {
+    pdl_wait();
+    pdl_trigger();
+    const TileGeometry g = tile_geometry(a, DECODE_ROWS);
+    const int rows_live = g.tok0 < g.tok_end ? (g.tok_end - g.tok0) * g.heads_per_tile : 0, row0 = blockIdx.z * COMBINE_ROWS;
+    if (row0 >= rows_live) return;
+    const size_t unit = (size_t)blockIdx.x * gridDim.y + blockIdx.y;
+    merge_pieces<1>(out, part_ml + unit * splits * DECODE_ROWS * 2, part_o + unit * splits * DECODE_ROWS * D, splits, min(row0 + COMBINE_ROWS, rows_live), g, a, row0);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -2889,10 +2936,13 @@ static int paged_attention_bf16(void* out, const void* q, const void* k_cache, c
         if (TMA_OK && kv_maps != nullptr && a.page_shift >= 3)
             return launch_tma_decode<false>(out, q, n_short, KV * groups, splits, part_o, part_ml, counters, kv_maps, pool_row0, cut, a, FuseQkv{}, stream);
         oxr_last_short_kernel = 1;
-        if (k_cache == v_cache)
+        if (k_cache == v_cache) {
             attn_mma_decode_kernel<true><<<dim3(n_short, KV * groups, splits), MMA_THREADS, decode_smem(true), stream>>>(
                 (bf16*)out, part_o, part_ml, counters, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, a);
-        else
+            if (splits > 1)
+                oxr_launch(attn_combine_kernel, dim3(n_short, KV * groups, (DECODE_ROWS + COMBINE_ROWS - 1) / COMBINE_ROWS), dim3(MMA_THREADS), 0, stream, true,
+                           (bf16*)out, part_o, part_ml, splits, a);
+        } else
             attn_mma_decode_kernel<false><<<dim3(n_short, KV * groups, splits), MMA_THREADS, decode_smem(false), stream>>>(
                 (bf16*)out, part_o, part_ml, counters, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, a);
         int rc = oxr_launch_status();

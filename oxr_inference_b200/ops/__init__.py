@@ -676,7 +676,7 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
                                                    status.data_ptr(), _stream())
         global launch_count
         _done(code, "paged_attention_masked_bf16")
-        launch_count += 1 if n_long and n_short else 0
+        launch_count += (1 if n_long and n_short else 0) + (1 if n_short and splits > 1 and v_cache.data_ptr() == k_cache.data_ptr() else 0)
         return out
     code = lib.oxr_paged_attention_bf16(out.data_ptr(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), s_req.data_ptr(),
                                         s_tok.data_ptr(), n_short, l_req.data_ptr(), l_tok.data_ptr(), n_long, *common, splits,
