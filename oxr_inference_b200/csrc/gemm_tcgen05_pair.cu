@@ -13,6 +13,9 @@
 //     with a cluster mask frees a stage in both blocks and hands the accumulator to both blocks' epilogue warps,
 //     which give it back by arriving on the leader's barrier;
 //   * tiles are walked persistently by the pairs, two accumulators in tensor memory overlap epilogue and MMA.
+// ACROSS has W along the 256-row side of the tile and the rows of X as its width, any multiple of 32: the same products transposed, for numbers of rows that fill
+// tiles of 256 badly (1,562 rows x 24,576 x 4,096 gated 262 us in 7 x 256 rows, 226 in 10 x 160; 1,421 x 4,096 x 12,288 135 and 112). Its epilogue costs 4 to 9 us
+// a product more (the accumulator comes out column by column), so where the rows do fill the tiles the plain form stays.
 // No TMA copy is multicast. Every wait on an mbarrier is bounded as in the one-SM kernel; both blocks meet at a
 // cluster barrier before tensor memory is freed, so neither leaves while the other may still touch its memory.
 #include "umma.cuh"
@@ -59,18 +62,84 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                  ::"r"(smem_addr(bar)), "h"((uint16_t)3) : "memory");
 }
 
-// Tile order as in the one-SM kernel, with 256-row tiles: pairs that run at the same time share few W tiles.
-__device__ __forceinline__ void pair_tile_origin(int tile, int M, int N, int bn, int& m0, int& n0) {
+struct PairTile { int m0, n0; };   // rows of X from m0, rows of W from n0
+
+// Tile order as in the one-SM kernel, with 256-row tiles: pairs that run at the same time share few W tiles. ACROSS: tiles of 256 rows of W by
+// bn rows of X, all tiles of rows of X for one W tile and then the next.
+template <bool ACROSS>
+__device__ __forceinline__ PairTile pair_tile(int tile, int M, int N, int bn) {
+    if constexpr (ACROSS) {
+        const int tiles_x = (M + bn - 1) / bn;
+        return {tile % tiles_x * bn, tile / tiles_x * 2 * BM};
+    }
     constexpr int GROUP_M = 16;
     const int tiles_m = (M + 2 * BM - 1) / (2 * BM), tiles_n = (N + bn - 1) / bn;
     const int per_group = GROUP_M * tiles_n;
     const int group = tile / per_group, within = tile % per_group;
     const int group_rows = min(GROUP_M, tiles_m - group * GROUP_M);
-    m0 = (group * GROUP_M + within % group_rows) * 2 * BM;
-    n0 = (within / group_rows) * bn;
+    return {(group * GROUP_M + within % group_rows) * 2 * BM, (within / group_rows) * bn};
 }
 
+// ACROSS: the four epilogue warps of a block have a column of C per lane, 128 in all, and turn a piece of up to 32 rows over in shared memory: rows of 128 columns
+// (GATED 64) and 16 bytes against bank conflicts, which then leave in whole 16-byte words, 256 (128) bytes of a row side by side. (Stored from the registers, two bytes
+// a lane and 32 or 64 bytes of a row at a time, a gated product of 1,562 x 24,576 x 4,096 in tiles of 160 took 317 us instead of 226.)
+template <typename TO, bool GATED> struct Turned {
+    static constexpr int COLS = GATED ? 64 : 128, PITCH = COLS * (int)sizeof(TO) + 16, BYTES = 2 * 32 * PITCH;   // two pieces: one barrier each
+};
 template <typename TO, bool GATED>
+__device__ __forceinline__ void turn_piece(unsigned char* buf, const uint32_t (&v)[32], int count, int col, const GateForm& gate) {   // col: 0 .. 127
+    using T = Turned<TO, GATED>;
+    if constexpr (!GATED) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            if (j < count) *reinterpret_cast<TO*>(buf + j * T::PITCH + col * (int)sizeof(TO)) = Num<TO>::from_f32(__uint_as_float(v[j]));
+    } else {
+        // gate and up columns alternate in eights: lanes 0..7 and 16..23 have gates, the lanes eight behind them their ups. A gate's lane keeps every even row and gets
+        // its up, an up's lane gets the gates of the odd ones.
+        const bool up = col & 8;
+        TO* at = reinterpret_cast<TO*>(buf + (up ? T::PITCH : 0)) + col / 16 * 8 + col % 8;
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+            const float mine = __uint_as_float(up ? v[j + 1] : v[j]);
+            const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(up ? v[j] : v[j + 1]), 8);
+            if (j < count) *reinterpret_cast<TO*>(reinterpret_cast<unsigned char*>(at) + j * T::PITCH) = Num<TO>::from_f32(gate_apply(gate, up ? other : mine, up ? mine : other));
+        }
+    }
+}
+// rows row0 .. of C, columns from col0 on, `width` columns of C in all
+template <typename TO, bool GATED>
+__device__ __forceinline__ void store_turned(TO* __restrict__ C, const unsigned char* buf, int rows, int row0, int col0, int width) {
+    using T = Turned<TO, GATED>;
+    constexpr int PER = 16 / (int)sizeof(TO), WORDS = T::COLS / PER;
+    const bool whole = width % PER == 0 && (uintptr_t)C % 16 == 0;
+    for (int i = threadIdx.x - 64; i < rows * WORDS; i += 128) {
+        const int r = i / WORDS, c = i % WORDS * PER;
+        if (col0 + c >= width) continue;
+        const uint4 word = *reinterpret_cast<const uint4*>(buf + r * T::PITCH + c * (int)sizeof(TO));
+        TO* at = C + (size_t)(row0 + r) * width + col0 + c;
+        if (whole) *reinterpret_cast<uint4*>(at) = word;
+        else {
+            const TO* e = reinterpret_cast<const TO*>(&word);
+#pragma unroll
+            for (int k = 0; k < PER; ++k)
+                if (col0 + c + k < width) at[k] = e[k];
+        }
+    }
+}
+// Barrier 1 is the epilogue warps' own (128 threads).
+__device__ __forceinline__ void turn_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ bool turn_all(bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 q, %1, 0;\n\t"
+        "bar.red.and.pred p, 1, 128, q;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(r) : "r"((uint32_t)v) : "memory");
+    return r != 0;
+}
+
+template <typename TO, bool GATED, bool ACROSS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_tcgen05_pair_kernel(TO* __restrict__ C, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                          int M, int N, int K, int bn, int stages, int tmem_cols, int num_tiles, int* status, const GateForm gate) {
@@ -115,31 +184,37 @@ gemm_tcgen05_pair_kernel(TO* __restrict__ C, const __grid_constant__ CUtensorMap
             // No kernel writes the weights: this block's halves of W's tiles for the first ring of stages are requested
             // before the kernel (when it is launched dependent on the one before) waits for that one; the rows of X for
             // the same stages follow after the wait. The leader arms each of these stages for both blocks' bytes.
+            auto load_w = [&](int stage, int kb, const PairTile& t, uint32_t bar) {
+                unsigned char* dst = tiles + (size_t)stage * stage_size;
+                if constexpr (ACROSS) tma_load_2d_pair(dst, &map_w, kb * BK, t.n0 + (int)rank * BM, bar);
+                else tma_load_2d_pair(dst + A_BYTES, &map_w, kb * BK, t.n0 + (int)rank * (bn / 2), bar);
+            };
+            auto load_x = [&](int stage, int kb, const PairTile& t, uint32_t bar) {
+                unsigned char* dst = tiles + (size_t)stage * stage_size;
+                if constexpr (ACROSS) tma_load_2d_pair(dst + A_BYTES, &map_x, kb * BK, t.m0 + (int)rank * (bn / 2), bar);
+                else tma_load_2d_pair(dst, &map_x, kb * BK, t.m0 + (int)rank * BM, bar);
+            };
             int early = 0;
             for (int tile = pair; tile < num_tiles && early < stages; tile += num_pairs) {
-                int m0, n0;
-                pair_tile_origin(tile, M, N, bn, m0, n0);
+                const PairTile t = pair_tile<ACROSS>(tile, M, N, bn);
                 for (int kb = 0; kb < num_kb && early < stages; ++kb, ++early) {
                     if (rank == 0) mbar_expect_tx(full + early, 2u * (uint32_t)stage_size);
-                    tma_load_2d_pair(tiles + (size_t)early * stage_size + A_BYTES, &map_w, kb * BK, n0 + (int)rank * (bn / 2),
-                                     in_block(smem_addr(full + early), 0));
+                    load_w(early, kb, t, in_block(smem_addr(full + early), 0));
                 }
             }
             pdl_wait();
             int step = 0;
             for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-                int m0, n0;
-                pair_tile_origin(tile, M, N, bn, m0, n0);
+                const PairTile t = pair_tile<ACROSS>(tile, M, N, bn);
                 for (int kb = 0; kb < num_kb; ++kb, ++step) {
-                    unsigned char* a_dst = tiles + (size_t)s * stage_size;
                     const uint32_t leader_full = in_block(smem_addr(full + s), 0);
-                    if (step < early) {   // first ring: the stage is free and armed, its half of W's tile is on its way
-                        tma_load_2d_pair(a_dst, &map_x, kb * BK, m0 + (int)rank * BM, leader_full);
+                    if (step < early) {   // first ring: the stage is free and armed, its part of W's tile is on its way
+                        load_x(s, kb, t, leader_full);
                     } else {
                         if (!mbar_wait(empty + s, phase ^ 1)) { atomicExch(gave_up, 1u); oxr_report(status, OXR_WAIT_EXPIRED, 10); ok = false; break; }
                         if (rank == 0) mbar_expect_tx(full + s, 2u * (uint32_t)stage_size);   // both blocks' bytes
-                        tma_load_2d_pair(a_dst, &map_x, kb * BK, m0 + (int)rank * BM, leader_full);
-                        tma_load_2d_pair(a_dst + A_BYTES, &map_w, kb * BK, n0 + (int)rank * (bn / 2), leader_full);
+                        load_x(s, kb, t, leader_full);
+                        load_w(s, kb, t, leader_full);
                     }
                     if (++s == stages) { s = 0; phase ^= 1; }
                 }
@@ -178,18 +253,20 @@ gemm_tcgen05_pair_kernel(TO* __restrict__ C, const __grid_constant__ CUtensorMap
         // ------------------------------------------------------------------ epilogue: this block's 128 rows
         pdl_wait();   // C may still be read by the kernels before this one
         const int quarter = warp & 3;
+        [[maybe_unused]] unsigned char* turned = reinterpret_cast<unsigned char*>(full) + BARRIER_BYTES;
+        [[maybe_unused]] int piece = 0;
         int it = 0;
         for (int tile = pair; tile < num_tiles; tile += num_pairs, ++it) {
-            int m0, n0;
-            pair_tile_origin(tile, M, N, bn, m0, n0);
+            const PairTile t = pair_tile<ACROSS>(tile, M, N, bn);
             const int acc = it & 1;
             const uint32_t acc_phase = (it >> 1) & 1;
-            const int row = m0 + (int)rank * BM + quarter * 32 + lane;
+            [[maybe_unused]] const int row = t.m0 + (int)rank * BM + quarter * 32 + lane;
             bool ok = mbar_wait(accum_full + acc, acc_phase);
             if (!ok) { atomicExch(gave_up, 1u); if (lane == 0) oxr_report(status, OXR_WAIT_EXPIRED, 12); }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             ok = ok && (*reinterpret_cast<volatile uint32_t*>(gave_up) == 0);
-            ok = __all_sync(0xffffffffu, ok);
+            if constexpr (ACROSS) ok = turn_all(ok);          // the four warps meet at barriers below: they leave together
+            else ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             const uint32_t acc_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * acc_stride;
 #pragma unroll 1
@@ -198,11 +275,19 @@ gemm_tcgen05_pair_kernel(TO* __restrict__ C, const __grid_constant__ CUtensorMap
                 const int count = min(32, bn - c0);
                 if (count == 32) tmem_ld_32x32(acc_addr + (uint32_t)c0, v);
                 else tmem_ld_32x16(acc_addr + (uint32_t)c0, v);
-                if (row < M && n0 + c0 < N) {
-                    if constexpr (GATED) store_row_piece_gated<TO>(C + (size_t)row * (N / 2) + (n0 + c0) / 2, v, count, n0 + c0, N, gate);
+                if constexpr (ACROSS) {
+                    unsigned char* buf = turned + (piece & 1) * 32 * Turned<TO, GATED>::PITCH;   // last read before the barrier of the piece between
+                    ++piece;
+                    if (!GATED && gate.kind == 2) relu2_piece(v);
+                    turn_piece<TO, GATED>(buf, v, count, quarter * 32 + lane, gate);
+                    turn_sync();
+                    const int col0 = t.n0 + (int)rank * BM;
+                    store_turned<TO, GATED>(C, buf, min(count, M - t.m0 - c0), t.m0 + c0, GATED ? col0 / 2 : col0, GATED ? N / 2 : N);
+                } else if (row < M && t.n0 + c0 < N) {
+                    if constexpr (GATED) store_row_piece_gated<TO>(C + (size_t)row * (N / 2) + (t.n0 + c0) / 2, v, count, t.n0 + c0, N, gate);
                     else {
                         if (gate.kind == 2) relu2_piece(v);   // the plain product's optional activation
-                        store_row_piece<TO>(C + (size_t)row * N + n0 + c0, v, count, n0 + c0, N);
+                        store_row_piece<TO>(C + (size_t)row * N + t.n0 + c0, v, count, t.n0 + c0, N);
                     }
                 }
             }
@@ -219,11 +304,11 @@ gemm_tcgen05_pair_kernel(TO* __restrict__ C, const __grid_constant__ CUtensorMap
     }
 }
 
-template <typename TO, bool GATED = false>
+template <typename TO, bool GATED, bool ACROSS>
 int launch_pair(void* C, const void* X, const void* W, int M, int N, int K, int bn, int* status, cudaStream_t stream, int act = 0) {
     static int max_pairs = 0;   // per instantiation
     if (max_pairs == 0) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<TO, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<TO, GATED, ACROSS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
         if (e != cudaSuccess) return 1000 + (int)e;
         int dev = 0, sms = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 2) sms = 148;
@@ -240,46 +325,49 @@ int launch_pair(void* C, const void* X, const void* W, int M, int N, int K, int 
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, gemm_tcgen05_pair_kernel<TO, GATED>, &cfg) != cudaSuccess || clusters <= 0) {
+        if (cudaOccupancyMaxActiveClusters(&clusters, gemm_tcgen05_pair_kernel<TO, GATED, ACROSS>, &cfg) != cudaSuccess || clusters <= 0) {
             (void)cudaGetLastError();
             clusters = sms / 2;
         }
         max_pairs = clusters < sms / 2 ? clusters : sms / 2;
     }
     CUtensorMap map_x, map_w;
-    if (!oxr_make_map_bf16(&map_x, X, M, K, BM) || !oxr_make_map_bf16(&map_w, W, N, K, bn / 2)) return OXR_BAD_ARGUMENT;
-    const long long tiles = (long long)((N + bn - 1) / bn) * ((M + 2 * BM - 1) / (2 * BM));
+    if (!oxr_make_map_bf16(&map_x, X, M, K, ACROSS ? bn / 2 : BM) || !oxr_make_map_bf16(&map_w, W, N, K, ACROSS ? BM : bn / 2)) return OXR_BAD_ARGUMENT;
+    const long long tiles = ACROSS ? (long long)((N + 2 * BM - 1) / (2 * BM)) * ((M + bn - 1) / bn) : (long long)((N + bn - 1) / bn) * ((M + 2 * BM - 1) / (2 * BM));
     if (tiles > 0x7fffffffLL) return OXR_BAD_ARGUMENT;
-    int stages = RING_BYTES / pair_stage_bytes(bn);
+    int stages = (RING_BYTES - (ACROSS ? Turned<TO, GATED>::BYTES : 0)) / pair_stage_bytes(bn);
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     int tmem_cols = 32;
     while (tmem_cols < 2 * bn) tmem_cols *= 2;
     const unsigned pairs = (unsigned)(tiles < max_pairs ? tiles : max_pairs);
-    oxr_launch(gemm_tcgen05_pair_kernel<TO, GATED>, dim3(2 * pairs), dim3(PAIR_THREADS), SMEM_BYTES, stream, true, (TO*)C, map_x, map_w, M, N, K,
+    oxr_launch(gemm_tcgen05_pair_kernel<TO, GATED, ACROSS>, dim3(2 * pairs), dim3(PAIR_THREADS), SMEM_BYTES, stream, true, (TO*)C, map_x, map_w, M, N, K,
                bn, stages, tmem_cols, (int)tiles, status, act == 1 ? RELU2_FORM : (GATED ? oxr_gate_form : PLAIN_FORM));
     return oxr_launch_status();
 }
 }  // namespace
 
-// out_dtype: 0 = float32, 1 = bfloat16. Requires K % 8 == 0 and 16-byte aligned X, W. tile_n: columns of the output
-// per pair of blocks, a multiple of 32 from 32 to 256 (each block stages half of them). act 1: the output is relu(x)^2 of the fp32 sums.
-OXR_API int oxr_gemm_tcgen05_pair_bf16(void* C, const void* X, const void* W, int M, int N, int K, int out_dtype, int tile_n, int act, int* status,
+// out_dtype: 0 = float32, 1 = bfloat16. Requires K % 8 == 0 and 16-byte aligned X, W. tile: the size, a multiple of 32 from 32 to 256, of a pair's tile along
+// the side that is not 256 long: columns of the output (each block stages half of them), or, with `across`, rows. act 1: the output is relu(x)^2 of the fp32 sums.
+OXR_API int oxr_gemm_tcgen05_pair_bf16(void* C, const void* X, const void* W, int M, int N, int K, int out_dtype, int tile, int across, int act, int* status,
                                        cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (act != 0 && act != 1) return OXR_BAD_ARGUMENT;
     if (K <= 0 || K % 8 != 0 || (uintptr_t)X % 16 != 0 || (uintptr_t)W % 16 != 0) return OXR_BAD_ARGUMENT;
-    if (tile_n < 32 || tile_n > MAX_BN || tile_n % 32 != 0) return OXR_BAD_ARGUMENT;
-    if (out_dtype == 1) return launch_pair<__nv_bfloat16>(C, X, W, M, N, K, tile_n, status, stream, act);
-    if (out_dtype == 0) return launch_pair<float>(C, X, W, M, N, K, tile_n, status, stream, act);
+    if (tile < 32 || tile > MAX_BN || tile % 32 != 0) return OXR_BAD_ARGUMENT;
+    if (out_dtype == 1 && across) return launch_pair<__nv_bfloat16, false, true>(C, X, W, M, N, K, tile, status, stream, act);
+    if (out_dtype == 1) return launch_pair<__nv_bfloat16, false, false>(C, X, W, M, N, K, tile, status, stream, act);
+    if (out_dtype == 0 && across) return launch_pair<float, false, true>(C, X, W, M, N, K, tile, status, stream, act);
+    if (out_dtype == 0) return launch_pair<float, false, false>(C, X, W, M, N, K, tile, status, stream, act);
     return OXR_BAD_ARGUMENT;
 }
 
 // C [M, N / 2] = silu(X Wg^T) * (X Wu^T) in bf16 for W [N, K] whose gate and up rows alternate in groups of 8 (N a
 // multiple of 16): the pair kernel with the gated epilogue.
-OXR_API int oxr_gemm_tcgen05_pair_gated_bf16(void* C, const void* X, const void* W, int M, int N, int K, int tile_n, int* status,
+OXR_API int oxr_gemm_tcgen05_pair_gated_bf16(void* C, const void* X, const void* W, int M, int N, int K, int tile, int across, int* status,
                                              cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (N % 16 != 0 || K <= 0 || K % 8 != 0 || (uintptr_t)X % 16 != 0 || (uintptr_t)W % 16 != 0 || (uintptr_t)C % 16 != 0) return OXR_BAD_ARGUMENT;
-    if (tile_n < 32 || tile_n > MAX_BN || tile_n % 32 != 0) return OXR_BAD_ARGUMENT;
-    return launch_pair<__nv_bfloat16, true>(C, X, W, M, N, K, tile_n, status, stream);
+    if (tile < 32 || tile > MAX_BN || tile % 32 != 0) return OXR_BAD_ARGUMENT;
+    if (across) return launch_pair<__nv_bfloat16, true, true>(C, X, W, M, N, K, tile, status, stream);
+    return launch_pair<__nv_bfloat16, true, false>(C, X, W, M, N, K, tile, status, stream);
 }

@@ -125,11 +125,11 @@ def _lib():
         lib.oxr_gemm_stream_blocks.argtypes = [i]
         lib.oxr_gemm_stream_blocks.restype = c_int
         lib.oxr_gemm_tcgen05_bf16.argtypes = [p, p, p, i, i, i, i, i, i, p, p, i, p, p]
-        lib.oxr_gemm_tcgen05_pair_bf16.argtypes = [p, p, p, i, i, i, i, i, i, p, p]
+        lib.oxr_gemm_tcgen05_pair_bf16.argtypes = [p, p, p, i, i, i, i, i, i, i, p, p]
         lib.oxr_gemm_tcgen05_gated_bf16.argtypes = [p, p, p, i, i, i, i, p, p]
         lib.oxr_gemm_few_rows_cluster_bf16.argtypes = [p, p, p, i, i, i, i, i, p, p]
         lib.oxr_gemm_few_rows_max_clusters.argtypes = [i]
-        lib.oxr_gemm_tcgen05_pair_gated_bf16.argtypes = [p, p, p, i, i, i, i, p, p]
+        lib.oxr_gemm_tcgen05_pair_gated_bf16.argtypes = [p, p, p, i, i, i, i, i, p, p]
         lib.oxr_sample.argtypes = [p, p, i, i, p, p, p, p, p, p]
         lib.oxr_sample_chunks.argtypes = [i]
         lib.oxr_sample_chunks.restype = c_int
@@ -399,7 +399,7 @@ def gated_linear(x: torch.Tensor, weight: torch.Tensor, interleave: int = 0, *, 
         elif m <= SKINNY_MAX_ROWS:
             _done(lib.oxr_gemm_skinny_gated_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, _stream()), "gemm_skinny_gated")
         elif _gemm_pair_plan(m, n, k):
-            _done(lib.oxr_gemm_tcgen05_pair_gated_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, _gemm_pair_plan(m, n, k),
+            _done(lib.oxr_gemm_tcgen05_pair_gated_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, *_gemm_pair_tiles(m, n, k),
                                                        new_status(x.device).data_ptr(), _stream()), "gemm_tcgen05_pair_gated")
         else:
             tile_n, _ = _gemm_plan(m, n, k, False)   # the gated epilogue has no shares of k
@@ -941,6 +941,24 @@ def _gemm_pair_plan(m: int, n: int, k: int) -> int:
     return best
 
 
+@functools.lru_cache(maxsize=None)
+def _gemm_pair_tiles(m: int, n: int, k: int) -> tuple[int, int]:
+    """(tile, across) of a product that the two-SM kernel takes: tiles of 256 rows of x by the ``tile`` columns of ``_gemm_pair_plan``, or ``across``: 256 columns by ``tile``
+    rows of x, where that promises 4 %. Rounds of pairs times what a tile takes, fitted to 504 timings of products in turn on a B200 (520 to 2,048 rows, 2,048 to 24,576
+    columns, k 2,048 to 12,288, 96 to 256 wide): a 64-wide k step takes 0.00163 us a column and no less than 0.235, a product 0.0143 us a column of its tile beside; across
+    0.00169 and 0.23, 4.9 us a product, and a tile no less than the 0.085 us a row of its epilogue. 1,562 rows x 24,576 x 4,096 262 -> 226 us, 1,421 x 4,096 x 12,288
+    135 -> 112, 2,011 x 4,096 x 12,288 175 -> 164."""
+    pairs, steps = num_sms() // 2, -(-k // 64)
+    tile = _gemm_pair_plan(m, n, k)
+    best = (tile, 0)
+    best_cost = 0.96 * (-(-(-(-m // 256) * -(-n // tile)) // pairs) * steps * max(0.235, 0.00163 * tile) + 0.0143 * tile)
+    for tile in (256, 224, 192, 160, 128, 96):
+        cost = -(-(-(-m // tile) * -(-n // 256)) // pairs) * max(steps * max(0.23, 0.00169 * tile), 0.085 * tile) + 4.9
+        if cost < best_cost - 1e-9:
+            best, best_cost = (tile, 1), cost
+    return best
+
+
 GEMM_MAX_SPLIT_TILES = GEMM_WORKSPACE_BYTES // (2 * 128 * 16 * 4)   # the most tiles a split product can have
 
 
@@ -1012,9 +1030,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
             _done(lib.oxr_gemm_few_rows_cluster_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, _DT[out_dtype], few,
                                                      new_status(x.device).data_ptr(), _stream()), "gemm_few_rows_cluster")
             return out
-        pair_tile = _gemm_pair_plan(m, n, k)
-        if pair_tile:
-            _done(lib.oxr_gemm_tcgen05_pair_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, _DT[out_dtype], pair_tile, 0,
+        if _gemm_pair_plan(m, n, k):
+            _done(lib.oxr_gemm_tcgen05_pair_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, _DT[out_dtype], *_gemm_pair_tiles(m, n, k), 0,
                                                  new_status(x.device).data_ptr(), _stream()), "gemm_tcgen05_pair")
             return out
         tile_n, splits = _gemm_plan(m, n, k)
@@ -1047,14 +1064,13 @@ def relu2_linear(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
         raise KernelError(f"relu2_linear: x has {k} columns, weight has {weight.shape[1]}")
     if x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and k % 8 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0:
         lib, status = _lib(), new_status(x.device).data_ptr()
-        pair_tile = _gemm_pair_plan(m, n, k)
         if m <= STREAM_MAX_ROWS and STREAM_GEMM:
             out = torch.empty((m, n), dtype=x.dtype, device=x.device)
             _done(lib.oxr_gemm_stream_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, 1, 1, status, _stream()), "gemm_stream")
             return out
-        if pair_tile:
+        if _gemm_pair_plan(m, n, k):
             out = torch.empty((m, n), dtype=x.dtype, device=x.device)
-            _done(lib.oxr_gemm_tcgen05_pair_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, 1, pair_tile, 1, status, _stream()),
+            _done(lib.oxr_gemm_tcgen05_pair_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, 1, *_gemm_pair_tiles(m, n, k), 1, status, _stream()),
                   "gemm_tcgen05_pair")
             return out
         if m > SKINNY_MAX_ROWS and not _gemm_few_rows_plan(m, n, k):
