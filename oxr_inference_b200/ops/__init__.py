@@ -159,6 +159,7 @@ def _lib():
         lib.oxr_gated_relu2.argtypes = [p, p, p, i, i, i, i, p]
         lib.oxr_expert_sort.argtypes = [p, p, p, p, p, i, i, i, i, p]
         lib.oxr_gemm_tcgen05_grouped_bf16.argtypes = [p, p, p, i, i, i, i, p, i, i, i, p, p]
+        lib.oxr_gemm_tcgen05_grouped_gated_bf16.argtypes = [p, p, p, i, i, i, i, p, i, p, p]
         lib.oxr_gather_rows.argtypes = [p, p, p, i, i, i, i, p]
         lib.oxr_combine_rows.argtypes = [p, p, p, p, i, i, i, p, p, i, p]
         lib.oxr_stream_layer_norm.argtypes = [p, p, p, p, p, i, i, f, i, p]
@@ -201,7 +202,7 @@ def _lib():
         for name in ("oxr_stream_rms_norm", "oxr_norm_add_norm", "oxr_concat2_cast", "oxr_add_row_f32", "oxr_clamped_glu", "oxr_rotary_angles",
                      "oxr_mamba_conv", "oxr_mamba_scan", "oxr_gated_group_norm", "oxr_attention_rows", "oxr_scatter_rows", "oxr_latent_prep",
                      "oxr_head_linear", "oxr_conv_qkv_store", "oxr_add_bias", "oxr_scale_f32", "oxr_mlstm_scan", "oxr_head_norm_gate", "oxr_route",
-                     "oxr_gated_relu2", "oxr_expert_sort", "oxr_gather_rows", "oxr_combine_rows", "oxr_gemm_tcgen05_grouped_bf16"):
+                     "oxr_gated_relu2", "oxr_expert_sort", "oxr_gather_rows", "oxr_combine_rows", "oxr_gemm_tcgen05_grouped_bf16", "oxr_gemm_tcgen05_grouped_gated_bf16"):
             getattr(lib, name).restype = c_int
         for name in ("oxr_embedding", "oxr_add_rms_norm", "oxr_silu_mul", "oxr_cast", "oxr_qk_norm_rope_store",
                      "oxr_gemm_f32_nt", "oxr_gemm_f32_segments", "oxr_gemm_skinny_bf16", "oxr_gemm_skinny_gated_bf16", "oxr_gemm_stream_bf16", "oxr_gemm_stream_gated_bf16", "oxr_gemm_tcgen05_bf16", "oxr_gemm_tcgen05_pair_bf16", "oxr_gemm_tcgen05_gated_bf16", "oxr_gemm_few_rows_cluster_bf16", "oxr_gemm_few_rows_max_clusters",
@@ -1963,23 +1964,46 @@ def grouped_linear_takes(x_dtype: torch.dtype, weight: torch.Tensor, k: int) -> 
     return x_dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and k % 8 == 0 and weight.data_ptr() % 16 == 0
 
 
-def grouped_linear(x: torch.Tensor, weight: torch.Tensor, tile_group: torch.Tensor, n: int, out_dtype: torch.dtype | None = None,
-                   relu2: bool = False) -> torch.Tensor:
-    """``out[r] = x[r] @ weight[g n : (g + 1) n].T`` with ``g = tile_group[r // GROUP_TILE_ROWS]``: rows ordered by the matrix they multiply (each
-    group padded to whole tiles of rows), ``weight [groups * n, k]`` the matrices stacked. One launch of the TMA + tcgen05 kernel, whatever
-    the groups' sizes, which stay on the device. A tile whose group is -1 is not computed (its rows of ``out`` are left unwritten: nobody
-    may read them). ``relu2``: the epilogue writes ``relu(out)^2`` of the fp32 sums."""
+def _grouped_tile(x: torch.Tensor, weight: torch.Tensor, tile_group: torch.Tensor, n: int) -> int:
+    """Checks the operands of a grouped product and picks its tile width."""
     _need(x, "x", torch.bfloat16)
     _need(weight, "weight", torch.bfloat16)
     _need(tile_group, "tile_group", torch.int32)
     m, k = x.shape
     if weight.shape[1] != k or weight.shape[0] % n or m % GROUP_TILE_ROWS or tile_group.numel() != m // GROUP_TILE_ROWS or k % 8:
         raise KernelError("grouped_linear: sizes do not fit")
+    # of the list's tiles about half a tile a group is not used (see `expert_sort`), and the kernel leaves those out
+    return _gemm_plan(max(GROUP_TILE_ROWS, m - weight.shape[0] // n * (GROUP_TILE_ROWS // 2)), n, k, False)[0]
+
+
+def grouped_linear(x: torch.Tensor, weight: torch.Tensor, tile_group: torch.Tensor, n: int, out_dtype: torch.dtype | None = None,
+                   relu2: bool = False) -> torch.Tensor:
+    """``out[r] = x[r] @ weight[g n : (g + 1) n].T`` with ``g = tile_group[r // GROUP_TILE_ROWS]``: rows ordered by the matrix they multiply (each
+    group padded to whole tiles of rows), ``weight [groups * n, k]`` the matrices stacked. One launch of the TMA + tcgen05 kernel, whatever
+    the groups' sizes, which stay on the device. A tile whose group is -1 is not computed (its rows of ``out`` are left unwritten: nobody
+    may read them). ``relu2``: the epilogue writes ``relu(out)^2`` of the fp32 sums."""
+    tile_n = _grouped_tile(x, weight, tile_group, n)
+    m, k = x.shape
     out_dtype = out_dtype or x.dtype
     out = torch.empty((m, n), dtype=out_dtype, device=x.device)
-    tile_n, _ = _gemm_plan(m, n, k, False)
     _done(_lib().oxr_gemm_tcgen05_grouped_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, weight.shape[0] // n, tile_group.data_ptr(),
                                                _DT[out_dtype], tile_n, int(relu2), new_status(x.device).data_ptr(), _stream()), "gemm_tcgen05_grouped")
+    return out
+
+
+def grouped_gated_linear(x: torch.Tensor, weight: torch.Tensor, tile_group: torch.Tensor, n: int, *, kind: str = "silu", alpha: float = 1.0,
+                         limit: float = 0.0) -> torch.Tensor:
+    """:func:`grouped_linear` for matrices of ``n / 2`` gates' rows and then their ups', with the activation of :func:`gated_linear` in the epilogue, on the
+    fp32 sums: ``[rows, n / 2]``."""
+    tile_n = max(32, _grouped_tile(x, weight, tile_group, n) // 32 * 32)
+    m, k = x.shape
+    if n % 2:
+        raise KernelError("grouped_gated_linear: as many gates as ups")
+    lib = _lib()
+    lib.oxr_set_gate_form(GATE_KINDS[kind], float(alpha), float(limit))   # read by the launcher below, handed to its kernel by value
+    out = torch.empty((m, n // 2), dtype=x.dtype, device=x.device)
+    _done(lib.oxr_gemm_tcgen05_grouped_gated_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, weight.shape[0] // n, tile_group.data_ptr(),
+                                                  tile_n, new_status(x.device).data_ptr(), _stream()), "gemm_tcgen05_grouped_gated")
     return out
 
 

@@ -181,11 +181,11 @@ class RoutedExperts(FeedForward):
                 ops.scale_placed_rows_(x, place, weights)
                 weights = torch.ones_like(weights)
             if self.activation == "silu_glu":
-                a = ops.silu_mul(ops.grouped_linear(x, self.up, tile_group, self.up_rows))
+                a = ops.grouped_gated_linear(x, self.up, tile_group, self.up_rows)      # the activation in the product's epilogue
             elif self.gated:
-                a = ops.clamped_glu(ops.grouped_linear(x, self.up, tile_group, self.up_rows), alpha=self.alpha, limit=self.limit)
+                a = ops.grouped_gated_linear(x, self.up, tile_group, self.up_rows, kind="clamped", alpha=self.alpha, limit=self.limit)
             else:
-                a = ops.grouped_linear(x, self.up, tile_group, self.ff, relu2=True)     # the activation in the product's epilogue
+                a = ops.grouped_linear(x, self.up, tile_group, self.ff, relu2=True)
             y = ops.grouped_linear(a, self.down_by_expert.view(self.E * self.hidden, self.ff), tile_group, self.hidden)
             return ops.combine_rows(y, place, weights, same, kept)
         counts, order, place, _ = ops.expert_sort(ids, self.E)

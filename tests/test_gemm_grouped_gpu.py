@@ -1,0 +1,56 @@
+"""Grouped products: tiles of no group, and the activation behind the product."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from oxr_inference_b200 import ops
+
+    return ops
+
+
+def randn(*shape, seed):
+    return torch.randn(*shape, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV)
+
+
+@pytest.mark.parametrize("groups", [[0, 0, 2, -1, 1, -1, -1], [-1, -1], [3], [1, 1, 1, 0] + [-1] * 40])
+def test_grouped_product_with_tiles_of_no_group(ops, groups):
+    """Tiles of no group at the end (the usual case) and between others; none used at all."""
+    m, n, k = 128 * len(groups), 272, 136
+    x, w = randn(m, k, seed=9).bfloat16(), (randn(4 * n, k, seed=10) * 0.1).bfloat16()
+    status = ops.new_status(DEV)
+    got = ops.grouped_linear(x, w, torch.tensor(groups, dtype=torch.int32, device=DEV), n, torch.float32)
+    ops.check_status(status)
+    for i, g in enumerate(groups):
+        if g >= 0:
+            rows = slice(128 * i, 128 * i + 128)
+            torch.testing.assert_close(got[rows], x[rows].float() @ w[g * n:(g + 1) * n].float().T, atol=1e-4, rtol=1e-5)
+
+
+@pytest.mark.parametrize("ff", [16, 136, 200])
+@pytest.mark.parametrize("kind", ["silu", "clamped"])
+def test_grouped_product_with_the_activation_behind_it(ops, ff, kind):
+    """Gates' rows first, then the ups': halves of a tile that reach beyond the gates and beyond the matrix."""
+    groups, k = [2, 0, 0, -1, 1, -1], 136
+    m, n = 128 * len(groups), 2 * ff
+    x, w = randn(m, k, seed=11).bfloat16(), (randn(3 * n, k, seed=12) * 0.1).bfloat16()
+    status = ops.new_status(DEV)
+    got = ops.grouped_gated_linear(x, w, torch.tensor(groups, dtype=torch.int32, device=DEV), n, kind=kind, alpha=1.7, limit=1.5)
+    ops.check_status(status)
+    assert got.shape == (m, ff) and got.dtype == torch.bfloat16
+    for i, e in enumerate(groups):
+        if e >= 0:
+            rows = slice(128 * i, 128 * i + 128)
+            g, u = (x[rows].float() @ w[e * n:(e + 1) * n].float().T).split(ff, 1)
+            if kind == "silu":
+                want = torch.nn.functional.silu(g) * u
+            else:
+                g = g.clamp(max=1.5)
+                want = g * torch.sigmoid(1.7 * g) * (u.clamp(-1.5, 1.5) + 1)
+            # one rounding to 16 bits, the fast exponential's and division's few steps of 32 bits, sums in another order
+            torch.testing.assert_close(got[rows].float(), want, rtol=2 ** -7, atol=1e-3)
