@@ -170,7 +170,7 @@ OXR_API int oxr_scatter_rows(void* pool, long long slot_stride, long long pool_s
 // the rest pass unchanged. `down` rows are down_stride apart (columns of a wider product).
 template <typename T>
 __global__ void latent_prep_kernel(T* __restrict__ pool, long long slot_stride, long long pool_slots, const T* __restrict__ down, int down_stride, int rank, int rot,
-                                   const float* __restrict__ weight, float eps, const T* q, int heads, int q_head_dim, int q_rot0, T* q_out,
+                                   const float* __restrict__ weight, float eps, const T* q, int q_stride, int heads, int q_head_dim, int q_rot0, T* q_out,
                                    int qo_head_dim, int qo_rot0, const float* __restrict__ cos_t, const float* __restrict__ sin_t, int half, int halves, const int* __restrict__ slots, int* status) {
     pdl_wait();
     pdl_trigger();
@@ -202,7 +202,7 @@ __global__ void latent_prep_kernel(T* __restrict__ pool, long long slot_stride, 
     }
     for (int i = threadIdx.x; i < heads * half; i += blockDim.x) {
         const int h = i / half, k = i % half;
-        const T* qr = q + ((size_t)t * heads + h) * q_head_dim + q_rot0;
+        const T* qr = q + (size_t)t * q_stride + (size_t)h * q_head_dim + q_rot0;
         T* qo = q_out + ((size_t)t * heads + h) * qo_head_dim + qo_rot0;
         const float u = Num<T>::to_f32(qr[step * k]), v = Num<T>::to_f32(qr[step * k + gap]);
         qo[step * k] = Num<T>::from_f32(u * c[k] - v * s[k]);
@@ -212,7 +212,7 @@ __global__ void latent_prep_kernel(T* __restrict__ pool, long long slot_stride, 
     if (rest > 0 && q_out != q)
         for (int i = threadIdx.x; i < heads * rest; i += blockDim.x) {
             const int h = i / rest, k = 2 * half + i % rest;
-            q_out[((size_t)t * heads + h) * qo_head_dim + qo_rot0 + k] = q[((size_t)t * heads + h) * q_head_dim + q_rot0 + k];
+            q_out[((size_t)t * heads + h) * qo_head_dim + qo_rot0 + k] = q[(size_t)t * q_stride + (size_t)h * q_head_dim + q_rot0 + k];
         }
 }
 
@@ -270,7 +270,7 @@ __device__ __forceinline__ void lp_turn(__nv_bfloat16* dst, const __nv_bfloat16*
 template <bool HALVES>
 __global__ void __launch_bounds__(128) latent_prep_words_kernel(__nv_bfloat16* __restrict__ pool, long long slot_stride, long long pool_slots,
                                                                 const __nv_bfloat16* __restrict__ down, int down_stride, int rank,
-                                                                const float* __restrict__ weight, float eps, const __nv_bfloat16* q, int heads,
+                                                                const float* __restrict__ weight, float eps, const __nv_bfloat16* q, int q_stride, int heads,
                                                                 int q_head_dim, int q_rot0, __nv_bfloat16* q_out, int qo_head_dim, int qo_rot0,
                                                                 const float* __restrict__ cos_t, const float* __restrict__ sin_t, int half,
                                                                 const int* __restrict__ slots, int* status) {
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(128) latent_prep_words_kernel(__nv_bfloat16* _
         lp_load(ct + A * w, c);
         lp_load(st + A * w, s);
         for (int h = threadIdx.x / per; h < heads; h += stride)
-            lp_turn(q_out + ((size_t)t * heads + h) * qo_head_dim + qo_rot0 + 8 * w, q + ((size_t)t * heads + h) * q_head_dim + q_rot0 + 8 * w, half, c, s);
+            lp_turn(q_out + ((size_t)t * heads + h) * qo_head_dim + qo_rot0 + 8 * w, q + (size_t)t * q_stride + (size_t)h * q_head_dim + q_rot0 + 8 * w, half, c, s);
     }
 }
 
@@ -360,25 +360,25 @@ __global__ void __launch_bounds__(128) cols_rms_norm_words_kernel(__nv_bfloat16*
 }
 
 OXR_API int oxr_latent_prep(void* pool, long long slot_stride, long long pool_slots, const void* down, int down_stride, int rank, int rot, const float* weight, float eps,
-                            const void* q, int heads, int q_head_dim, int q_rot0, void* q_out, int qo_head_dim, int qo_rot0, const float* cos_t,
+                            const void* q, int q_stride, int heads, int q_head_dim, int q_rot0, void* q_out, int qo_head_dim, int qo_rot0, const float* cos_t,
                             const float* sin_t, int half, int halves, const int* slots, int n_tokens, int dtype, int* status, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
-    if (rank <= 0 || down_stride < rank + rot || rot < 0 || 2 * half > rot || q_rot0 + rot > q_head_dim || qo_rot0 + rot > qo_head_dim) return OXR_BAD_ARGUMENT;
+    if (rank <= 0 || down_stride < rank + rot || rot < 0 || 2 * half > rot || q_rot0 + rot > q_head_dim || q_stride < heads * q_head_dim || qo_rot0 + rot > qo_head_dim) return OXR_BAD_ARGUMENT;
     if (dtype == 1 && half > 0 && half % (halves ? 8 : 4) == 0 && half <= (halves ? 1024 : 512) && rot == 2 * half && rank % 8 == 0 && slot_stride % 8 == 0 && down_stride % 8 == 0 &&
-        q_head_dim % 8 == 0 && q_rot0 % 8 == 0 && qo_head_dim % 8 == 0 && qo_rot0 % 8 == 0 && (uintptr_t)pool % 16 == 0 && (uintptr_t)down % 16 == 0 &&
+        q_stride % 8 == 0 && q_head_dim % 8 == 0 && q_rot0 % 8 == 0 && qo_head_dim % 8 == 0 && qo_rot0 % 8 == 0 && (uintptr_t)pool % 16 == 0 && (uintptr_t)down % 16 == 0 &&
         (uintptr_t)q % 16 == 0 && (uintptr_t)q_out % 16 == 0 && (uintptr_t)weight % 16 == 0 && (uintptr_t)cos_t % 16 == 0 && (uintptr_t)sin_t % 16 == 0) {
         const auto kernel = halves ? latent_prep_words_kernel<true> : latent_prep_words_kernel<false>;
         oxr_launch_small(kernel, dim3(n_tokens), dim3(128), 0, stream, (__nv_bfloat16*)pool, slot_stride, pool_slots, (const __nv_bfloat16*)down, down_stride, rank, weight, eps,
-                                             (const __nv_bfloat16*)q, heads, q_head_dim, q_rot0, (__nv_bfloat16*)q_out, qo_head_dim, qo_rot0, cos_t, sin_t, half,
+                                             (const __nv_bfloat16*)q, q_stride, heads, q_head_dim, q_rot0, (__nv_bfloat16*)q_out, qo_head_dim, qo_rot0, cos_t, sin_t, half,
                                              slots, status);
         return oxr_launch_status();
     }
     if (dtype == 0)
-        oxr_launch_small(latent_prep_kernel<float>, dim3(n_tokens), dim3(128), 0, stream, (float*)pool, slot_stride, pool_slots, (const float*)down, down_stride, rank, rot, weight, eps, (const float*)q, heads,
+        oxr_launch_small(latent_prep_kernel<float>, dim3(n_tokens), dim3(128), 0, stream, (float*)pool, slot_stride, pool_slots, (const float*)down, down_stride, rank, rot, weight, eps, (const float*)q, q_stride, heads,
                                                                q_head_dim, q_rot0, (float*)q_out, qo_head_dim, qo_rot0, cos_t, sin_t, half, halves, slots, status);
     else
         oxr_launch_small(latent_prep_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(128), 0, stream, (__nv_bfloat16*)pool, slot_stride, pool_slots, (const __nv_bfloat16*)down, down_stride, rank, rot, weight,
-                                                                       eps, (const __nv_bfloat16*)q, heads, q_head_dim, q_rot0, (__nv_bfloat16*)q_out, qo_head_dim,
+                                                                       eps, (const __nv_bfloat16*)q, q_stride, heads, q_head_dim, q_rot0, (__nv_bfloat16*)q_out, qo_head_dim,
                                                                        qo_rot0, cos_t, sin_t, half, halves, slots, status);
     return oxr_launch_status();
 }
@@ -416,14 +416,14 @@ OXR_API int oxr_cols_rms_norm(void* out, const void* x, int n, int stride, int w
 // out[t, h, out0 + o] = sum_i x[t, h, x0 + i] * w[h, i, o]   (w stored input-major per head: [heads, n_in, n_out]); fp32 sums in the
 // order i = 0, 1, 2, ...; entries of out outside [out0, out0 + n_out) are left alone. grid (token tiles, heads).
 template <typename T, int TM>
-__global__ void __launch_bounds__(128) head_linear_kernel(T* __restrict__ out, int out_head_stride, int out0, const T* __restrict__ x, int x_head_stride,
+__global__ void __launch_bounds__(128) head_linear_kernel(T* __restrict__ out, int out_head_stride, int out0, const T* __restrict__ x, int x_stride, int x_head_stride,
                                                           int x0, const T* __restrict__ w, int n_in, int n_out, int heads, int n_tokens) {
     pdl_trigger();
     extern __shared__ float xs[];   // [TM, n_in]
     const int h = blockIdx.y, t0 = blockIdx.x * TM;
     for (int i = threadIdx.x; i < TM * n_in; i += blockDim.x) {
         const int m = i / n_in, k = i % n_in;
-        xs[i] = (t0 + m < n_tokens) ? Num<T>::to_f32(x[((size_t)(t0 + m) * heads + h) * x_head_stride + x0 + k]) : 0.f;
+        xs[i] = (t0 + m < n_tokens) ? Num<T>::to_f32(x[(size_t)(t0 + m) * x_stride + (size_t)h * x_head_stride + x0 + k]) : 0.f;
     }
     __syncthreads();
     const T* wh = w + (size_t)h * n_in * n_out;
@@ -448,7 +448,7 @@ __device__ __forceinline__ float2 hl_load2(const float* p) { return *reinterpret
 __device__ __forceinline__ float2 hl_load2(const __nv_bfloat16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
 
 template <typename T, int TM>
-__global__ void __launch_bounds__(128) head_linear_few_kernel(T* __restrict__ out, int out_head_stride, int out0, const T* __restrict__ x, int x_head_stride,
+__global__ void __launch_bounds__(128) head_linear_few_kernel(T* __restrict__ out, int out_head_stride, int out0, const T* __restrict__ x, int x_stride, int x_head_stride,
                                                               int x0, const T* __restrict__ w, int n_in, int n_out, int heads, int n_tokens) {
     pdl_trigger();
     extern __shared__ float xs[];   // [TM, n_in], then [4][TM][64]
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(128) head_linear_few_kernel(T* __restrict__ ou
     const int h = blockIdx.y, t0 = blockIdx.x * TM, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.z * 64 + 2 * lane;
     for (int i = threadIdx.x; i < TM * n_in; i += 128) {
         const int m = i / n_in, k = i - m * n_in;
-        xs[i] = (t0 + m < n_tokens) ? Num<T>::to_f32(x[((size_t)(t0 + m) * heads + h) * x_head_stride + x0 + k]) : 0.f;
+        xs[i] = (t0 + m < n_tokens) ? Num<T>::to_f32(x[(size_t)(t0 + m) * x_stride + (size_t)h * x_head_stride + x0 + k]) : 0.f;
     }
     __syncthreads();
     const int per = (n_in + 3) / 4, k0 = min(n_in, warp * per), k1 = min(n_in, k0 + per);
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(128) head_linear_few_kernel(T* __restrict__ ou
 // 32 heads of 128 x 192: 10.7 us, 5.2 here. The sums are the same, in the same order.
 template <int KPW>
 __global__ void __launch_bounds__(128) head_linear_few_words_kernel(__nv_bfloat16* __restrict__ out, int out_head_stride, int out0,
-                                                                    const __nv_bfloat16* __restrict__ x, int x_head_stride, int x0,
+                                                                    const __nv_bfloat16* __restrict__ x, int x_stride, int x_head_stride, int x0,
                                                                     const __nv_bfloat16* __restrict__ w, int n_in, int n_out, int heads, int n_tokens) {
     constexpr int TM = 8;
     extern __shared__ __align__(16) float xs[];   // [TM, n_in], then [4][TM][64]
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(128) head_linear_few_words_kernel(__nv_bfloat1
     for (int i = threadIdx.x; i < TM * nk; i += 128) {
         const int m = i / nk, k = (i - m * nk) * 8;
         uint4 v = make_uint4(0, 0, 0, 0);
-        if (t0 + m < n_tokens) v = *reinterpret_cast<const uint4*>(x + ((size_t)(t0 + m) * heads + h) * x_head_stride + x0 + k);
+        if (t0 + m < n_tokens) v = *reinterpret_cast<const uint4*>(x + (size_t)(t0 + m) * x_stride + (size_t)h * x_head_stride + x0 + k);
         float4* dst = reinterpret_cast<float4*>(xs + m * n_in + k);
         dst[0] = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
         dst[1] = make_float4(__uint_as_float(v.z << 16), __uint_as_float(v.z & 0xffff0000u), __uint_as_float(v.w << 16), __uint_as_float(v.w & 0xffff0000u));
@@ -566,7 +566,7 @@ __device__ __forceinline__ void hl_mma16816(float (&c)[4], const uint32_t (&a)[4
 constexpr int HL_BM = 64, HL_BN = 64;
 
 __global__ void __launch_bounds__(128) head_linear_mma_kernel(__nv_bfloat16* __restrict__ out, int out_head_stride, int out0,
-                                                              const __nv_bfloat16* __restrict__ x, int x_head_stride, int x0,
+                                                              const __nv_bfloat16* __restrict__ x, int x_stride, int x_head_stride, int x0,
                                                               const __nv_bfloat16* __restrict__ w, int n_in, int n_out, int heads, int n_tokens, int words) {
     pdl_trigger();
     extern __shared__ __align__(16) unsigned char hl_smem[];
@@ -580,12 +580,12 @@ __global__ void __launch_bounds__(128) head_linear_mma_kernel(__nv_bfloat16* __r
         for (int i = threadIdx.x; i < HL_BM * nk; i += 128) {
             const int m = i / nk, k = (i - m * nk) * 8;
             *reinterpret_cast<uint4*>(As + m * lda + k) =
-                (t0 + m < n_tokens) ? *reinterpret_cast<const uint4*>(x + ((size_t)(t0 + m) * heads + h) * x_head_stride + x0 + k) : zero;
+                (t0 + m < n_tokens) ? *reinterpret_cast<const uint4*>(x + (size_t)(t0 + m) * x_stride + (size_t)h * x_head_stride + x0 + k) : zero;
         }
     } else {
         for (int i = threadIdx.x; i < HL_BM * n_in; i += 128) {
             const int m = i / n_in, k = i % n_in;
-            As[m * lda + k] = (t0 + m < n_tokens) ? x[((size_t)(t0 + m) * heads + h) * x_head_stride + x0 + k] : __float2bfloat16_rn(0.f);
+            As[m * lda + k] = (t0 + m < n_tokens) ? x[(size_t)(t0 + m) * x_stride + (size_t)h * x_head_stride + x0 + k] : __float2bfloat16_rn(0.f);
         }
     }
     const __nv_bfloat16* wh = w + (size_t)h * n_in * n_out;
@@ -637,10 +637,10 @@ __global__ void __launch_bounds__(128) head_linear_mma_kernel(__nv_bfloat16* __r
     }
 }
 
-OXR_API int oxr_head_linear(void* out, int out_head_stride, int out0, const void* x, int x_head_stride, int x0, const void* w, int n_in, int n_out,
+OXR_API int oxr_head_linear(void* out, int out_head_stride, int out0, const void* x, int x_stride, int x_head_stride, int x0, const void* w, int n_in, int n_out,
                             int heads, int n_tokens, int dtype, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
-    if (n_in <= 0 || n_out <= 0 || heads <= 0 || heads > 65535) return OXR_BAD_ARGUMENT;
+    if (n_in <= 0 || n_out <= 0 || heads <= 0 || heads > 65535 || x_stride < (heads - 1) * x_head_stride + x0 + n_in) return OXR_BAD_ARGUMENT;
     const size_t mma_smem = ((size_t)HL_BM * (n_in + 8) + (size_t)n_in * (HL_BN + 8)) * sizeof(__nv_bfloat16);
     if (dtype == 1 && n_tokens > 16 && n_in % 16 == 0 && n_out % 16 == 0 && mma_smem <= 200 * 1024) {
         static size_t configured = 0;
@@ -650,9 +650,9 @@ OXR_API int oxr_head_linear(void* out, int out_head_stride, int out0, const void
             configured = mma_smem;
         }
         dim3 grid((n_tokens + HL_BM - 1) / HL_BM, heads);
-        const int words = x_head_stride % 8 == 0 && x0 % 8 == 0 && out_head_stride % 2 == 0 && out0 % 2 == 0 && (uintptr_t)x % 16 == 0 &&
+        const int words = x_stride % 8 == 0 && x_head_stride % 8 == 0 && x0 % 8 == 0 && out_head_stride % 2 == 0 && out0 % 2 == 0 && (uintptr_t)x % 16 == 0 &&
                           (uintptr_t)w % 16 == 0 && (uintptr_t)out % 4 == 0;
-        oxr_launch(head_linear_mma_kernel, dim3(grid), dim3(128), mma_smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_head_stride, x0,
+        oxr_launch(head_linear_mma_kernel, dim3(grid), dim3(128), mma_smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_stride, x_head_stride, x0,
                                                                (const __nv_bfloat16*)w, n_in, n_out, heads, n_tokens, words);
         return oxr_launch_status();
     }
@@ -660,19 +660,19 @@ OXR_API int oxr_head_linear(void* out, int out_head_stride, int out0, const void
     const size_t few_smem = (size_t)(FEW * n_in + 4 * FEW * 64) * sizeof(float);
     if (n_tokens <= 16 && n_out % 2 == 0 && few_smem <= 48 * 1024 && (uintptr_t)w % 8 == 0) {
         dim3 grid((n_tokens + FEW - 1) / FEW, heads, (n_out + 63) / 64);
-        if (dtype == 1 && n_in % 16 == 0 && n_in <= 256 && x_head_stride % 8 == 0 && x0 % 8 == 0 && out_head_stride % 2 == 0 && out0 % 2 == 0 &&
+        if (dtype == 1 && n_in % 16 == 0 && n_in <= 256 && x_stride % 8 == 0 && x_head_stride % 8 == 0 && x0 % 8 == 0 && out_head_stride % 2 == 0 && out0 % 2 == 0 &&
             (uintptr_t)x % 16 == 0 && (uintptr_t)out % 4 == 0) {
             const auto kernel = n_in <= 128 ? head_linear_few_words_kernel<32> : (n_in <= 192 ? head_linear_few_words_kernel<48> : head_linear_few_words_kernel<64>);
-            oxr_launch(kernel, grid, dim3(128), few_smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_head_stride, x0,
+            oxr_launch(kernel, grid, dim3(128), few_smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_stride, x_head_stride, x0,
                              (const __nv_bfloat16*)w, n_in, n_out, heads, n_tokens);
             return oxr_launch_status();
         }
         if (dtype == 0)
-            oxr_launch(head_linear_few_kernel<float, FEW>, dim3(grid), dim3(128), few_smem, stream, false, (float*)out, out_head_stride, out0, (const float*)x, x_head_stride, x0, (const float*)w,
+            oxr_launch(head_linear_few_kernel<float, FEW>, dim3(grid), dim3(128), few_smem, stream, false, (float*)out, out_head_stride, out0, (const float*)x, x_stride, x_head_stride, x0, (const float*)w,
                                                                                 n_in, n_out, heads, n_tokens);
         else
             oxr_launch(head_linear_few_kernel<__nv_bfloat16, FEW>, dim3(grid), dim3(128), few_smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x,
-                                                                                        x_head_stride, x0, (const __nv_bfloat16*)w, n_in, n_out, heads, n_tokens);
+                                                                                        x_stride, x_head_stride, x0, (const __nv_bfloat16*)w, n_in, n_out, heads, n_tokens);
         return oxr_launch_status();
     }
     constexpr int TM = 8;
@@ -680,10 +680,10 @@ OXR_API int oxr_head_linear(void* out, int out_head_stride, int out0, const void
     if (smem > 48 * 1024) return OXR_BAD_ARGUMENT;
     dim3 grid((n_tokens + TM - 1) / TM, heads);
     if (dtype == 0)
-        oxr_launch(head_linear_kernel<float, TM>, dim3(grid), dim3(128), smem, stream, false, (float*)out, out_head_stride, out0, (const float*)x, x_head_stride, x0, (const float*)w, n_in,
+        oxr_launch(head_linear_kernel<float, TM>, dim3(grid), dim3(128), smem, stream, false, (float*)out, out_head_stride, out0, (const float*)x, x_stride, x_head_stride, x0, (const float*)w, n_in,
                                                                   n_out, heads, n_tokens);
     else
-        oxr_launch(head_linear_kernel<__nv_bfloat16, TM>, dim3(grid), dim3(128), smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_head_stride, x0,
+        oxr_launch(head_linear_kernel<__nv_bfloat16, TM>, dim3(grid), dim3(128), smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_stride, x_head_stride, x0,
                                                                           (const __nv_bfloat16*)w, n_in, n_out, heads, n_tokens);
     return oxr_launch_status();
 }

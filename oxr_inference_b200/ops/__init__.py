@@ -78,6 +78,19 @@ def _need_rows(t: torch.Tensor, name: str, dtype: torch.dtype | None = None) -> 
         raise KernelError(f"{name}: {t.dtype} {tuple(t.shape)} with strides {t.stride()} is not rows of {dtype or 'one dtype'}")
 
 
+def _need_heads(t: torch.Tensor, name: str, dtype: torch.dtype) -> int:
+    """Like :func:`_need` for ``[tokens, heads, size]`` whose tokens may lie apart (columns of a wider product); a token's heads lie side by side. Returns the
+    entries from token to token."""
+    if t.dim() != 3 or t.is_contiguous():
+        _need(t, name, dtype)
+        return t.shape[1] * t.shape[2] if t.dim() == 3 else t.shape[-1]
+    if not t.is_cuda:
+        raise KernelError(f"{name} is on {t.device}; the kernels run on a CUDA device only (there is no CPU path)")
+    if t.stride(2) != 1 or t.stride(1) != t.shape[2] or t.stride(0) < t.shape[1] * t.shape[2] or t.dtype != dtype:
+        raise KernelError(f"{name}: {t.dtype} {tuple(t.shape)} with strides {t.stride()} is not heads of {dtype}")
+    return t.stride(0)
+
+
 def _stream() -> int:
     """Handle of the current CUDA stream. The raw getter costs a fraction of a microsecond; `torch.cuda.current_stream()`
     builds a Stream object per call (several microseconds, per kernel launch of an eager step)."""
@@ -147,9 +160,9 @@ def _lib():
         lib.oxr_gated_group_norm.argtypes = [p, p, p, i, i, i, p, i, i, f, i, p]
         lib.oxr_attention_rows.argtypes = [p, p, i, p, ll, i, p, ll, i, i, i, i, i, i, p, p, p, i, i, i, f, i, i, i, p, i, p, i, p, p]
         lib.oxr_scatter_rows.argtypes = [p, ll, ll, p, i, i, i, p, i, i, p, p, ll, i, p]
-        lib.oxr_latent_prep.argtypes = [p, ll, ll, p, i, i, i, p, f, p, i, i, i, p, i, i, p, p, i, i, p, i, i, p, p]
+        lib.oxr_latent_prep.argtypes = [p, ll, ll, p, i, i, i, p, f, p, i, i, i, i, p, i, i, p, p, i, i, p, i, i, p, p]
         lib.oxr_cols_rms_norm.argtypes = [p, p, i, i, i, p, f, i, p]
-        lib.oxr_head_linear.argtypes = [p, i, i, p, i, i, p, i, i, i, i, i, p]
+        lib.oxr_head_linear.argtypes = [p, i, i, p, i, i, i, p, i, i, i, i, i, p]
         lib.oxr_conv_qkv_store.argtypes = [p, p, p, i, i, i, i, i, i, i, p, p, p, p, ll, p, p, p, p, f, i, p, p, p, p, p, ll, i, i, i, i, i, i, i, p, p]
         lib.oxr_add_bias.argtypes = [p, p, i, i, i, p]
         lib.oxr_scale_f32.argtypes = [p, f, ll, p]
@@ -1651,19 +1664,21 @@ def latent_prep(pool: torch.Tensor, down: torch.Tensor, rank: int, rot: int, wei
                 q_head_dim: int, q_rot0: int, q_out: torch.Tensor, qo_head_dim: int, qo_rot0: int, cos: torch.Tensor, sin: torch.Tensor,
                 slots: torch.Tensor, status: torch.Tensor, halves: bool = False) -> None:
     """Per token: the latent cache row ``[rmsnorm(down[:rank]) * weight | rotate(down[rank:])]`` goes to ``pool[slot]`` (slot -1: not stored), and
-    every head's rotated query part ``rotate(q[h, q_rot0 : q_rot0 + rot])`` to ``q_out[h, qo_rot0 : ...]``. ``rotate`` turns entry pairs (2i, 2i+1),
+    every head's rotated query part ``rotate(q[h, q_rot0 : q_rot0 + rot])`` (``q [tokens, heads, *]`` may be columns of a wider product) to ``q_out[h, qo_rot0 : ...]``. ``rotate`` turns entry pairs (2i, 2i+1),
     or with ``halves`` the pairs (i, i + half), by the token's angle i (``cos``/``sin`` ``[tokens, half]``); entries past ``2 * half`` pass
     unchanged. ``down`` may be columns of a wider product (rows apart, entries of a row side by side)."""
     _need(pool, "pool")
     _need_rows(down, "down", pool.dtype)
-    _need(q, "q", pool.dtype)
+    q_stride = _need_heads(q, "q", pool.dtype) if q.dim() == 3 else heads * q_head_dim
+    if q.dim() != 3:
+        _need(q, "q", pool.dtype)
     _need(q_out, "q_out", pool.dtype)
     _need(cos, "cos", torch.float32)
     n = down.shape[0]
     if down.shape[1] != rank + rot or pool[0, 0].numel() != rank + rot:
         raise KernelError("latent_prep: sizes of the down projection and the pool do not fit")
     _done(_lib().oxr_latent_prep(pool.data_ptr(), rank + rot, pool.shape[0] * pool.shape[1], down.data_ptr(), down.stride(0), rank, rot, weight.data_ptr(), float(eps),
-                                 q.data_ptr(), heads, q_head_dim, q_rot0, q_out.data_ptr(), qo_head_dim, qo_rot0, cos.data_ptr(), sin.data_ptr(),
+                                 q.data_ptr(), q_stride, heads, q_head_dim, q_rot0, q_out.data_ptr(), qo_head_dim, qo_rot0, cos.data_ptr(), sin.data_ptr(),
                                  cos.shape[1], int(bool(halves)), slots.data_ptr(), n, _dtype_code(down), status.data_ptr(), _stream()), "latent_prep")
 
 
@@ -1682,15 +1697,15 @@ def cols_rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Te
 
 def head_linear(out: torch.Tensor, out0: int, x: torch.Tensor, x0: int, weight: torch.Tensor) -> torch.Tensor:
     """``out[t, h, out0 : out0 + n_out] = x[t, h, x0 : x0 + n_in] @ weight[h]`` for ``weight [heads, n_in, n_out]``; ``x`` and ``out`` are
-    ``[tokens, heads, *]``; fp32 sums."""
+    ``[tokens, heads, *]``, ``x`` perhaps columns of a wider product; fp32 sums."""
     _need(out, "out")
-    _need(x, "x", out.dtype)
+    x_stride = _need_heads(x, "x", out.dtype)
     _need(weight, "weight", out.dtype)
     heads, n_in, n_out = weight.shape
     n = x.shape[0]
     if x.shape[1] != heads or out.shape[1] != heads or x0 + n_in > x.shape[2] or out0 + n_out > out.shape[2]:
         raise KernelError("head_linear: sizes do not fit")
-    _done(_lib().oxr_head_linear(out.data_ptr(), out.shape[2], out0, x.data_ptr(), x.shape[2], x0, weight.data_ptr(), n_in, n_out, heads, n,
+    _done(_lib().oxr_head_linear(out.data_ptr(), out.shape[2], out0, x.data_ptr(), x_stride, x.shape[2], x0, weight.data_ptr(), n_in, n_out, heads, n,
                                  _dtype_code(x), _stream()), "head_linear")
     return out
 

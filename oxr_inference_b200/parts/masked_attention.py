@@ -326,7 +326,7 @@ class LatentAttention(Mixer):
             down = both[:, self.QL:]
         else:
             q_cols = H * (D + R)
-            q = both[:, :q_cols].contiguous().view(n, H, D + R)
+            q = both[:, :q_cols].unflatten(1, (H, D + R))      # columns of the product: no copy
             down = both[:, q_cols:]
         if self.position is not None:
             cos, sin = self.position.step_angles(ctx)
