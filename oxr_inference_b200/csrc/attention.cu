@@ -24,7 +24,7 @@ namespace {
 constexpr int D = HEAD_DIM;
 constexpr int BM = 16;
 constexpr int BN = 32;
-constexpr int SIMT_WARPS = 4;
+constexpr int SIMT_WARPS = 8;
 constexpr int ROWS_PER_WARP = BM / SIMT_WARPS;
 constexpr int DCHUNKS = (D + 31) / 32;
 constexpr int KS_STRIDE = D + 4;   // rows of whole 16-byte words, eight neighbouring ones on different banks
@@ -114,29 +114,38 @@ template <> struct Vec<__nv_bfloat16> {
     }
 };
 
-// Rows of one K or V block on their way into shared memory: fp32 rows as they are by cp.async, others widened. Zeros for keys outside [k_lo, k_end).
+// The cache row of key kt + lane, for every warp (BN is a warp's lanes): one trip to the block table for a block of keys, where a lookup per 16 bytes, behind its
+// bounds check, made eight, one after the other. -1: no key there (outside [k_lo, k_end)), or a page outside the pool.
+static_assert(BN == 32, "a lane looks up a key");
+__device__ __forceinline__ int simt_rows(int kt, int k_lo, int k_end, int req, const AttnArgs& a) {
+    const int kp = kt + (threadIdx.x & 31);
+    if (kp < k_lo || kp >= k_end) return -1;
+    const int page = a.block_table[(size_t)req * a.table_width + (a.page_shift >= 0 ? kp >> a.page_shift : kp / a.page_size)];
+    if (page < 0 || page >= a.num_pages) {
+        oxr_report(a.status, OXR_BAD_PAGE, req);
+        return -1;
+    }
+    return a.page_shift >= 0 ? (page << a.page_shift) + (kp & (a.page_size - 1)) : page * a.page_size + kp % a.page_size;
+}
+// Rows of one K or V block on their way into shared memory: fp32 rows as they are by cp.async, others widened. Zeros where there is no key.
 template <typename T>
-__device__ __forceinline__ void simt_load(float* dst, int stride, const T* __restrict__ cache, int kt, int k_lo, int k_end, int req, int kvh, bool say, const AttnArgs& a) {
-    constexpr int VE = Vec<T>::N, VPK = D / VE;                                       // vectors per key
-    for (int v = threadIdx.x; v < BN * VPK; v += SIMT_WARPS * 32) {
-        const int j = v / VPK, part = v % VPK, kp = kt + j;
-        bool ok = kp >= k_lo && kp < k_end;
-        size_t base = 0;
-        if (ok) {
-            const int page = a.block_table[(size_t)req * a.table_width + (a.page_shift >= 0 ? kp >> a.page_shift : kp / a.page_size)];
-            ok = page >= 0 && page < a.num_pages;
-            if (ok) base = (((size_t)page * a.page_size + (a.page_shift >= 0 ? kp & (a.page_size - 1) : kp % a.page_size)) * a.KV + kvh) * D + part * VE;
-            else if (say && part == 0) oxr_report(a.status, OXR_BAD_PAGE, req);
-        }
+__device__ __forceinline__ void simt_load(float* dst, int stride, const T* __restrict__ cache, int rows, int kvh, const AttnArgs& a) {
+    constexpr int VE = Vec<T>::N, VPK = D / VE, TOTAL = BN * VPK;                     // vectors per key and in all
+#pragma unroll 4
+    for (int v0 = 0; v0 < TOTAL; v0 += SIMT_WARPS * 32) {
+        const int v = v0 + threadIdx.x, j = min(v / VPK, BN - 1), part = v % VPK;
+        const int row = __shfl_sync(0xffffffffu, rows, j);
+        if (v >= TOTAL) continue;
+        const size_t base = row >= 0 ? ((size_t)row * a.KV + kvh) * D + part * VE : 0;
         float* at = dst + j * stride + part * VE;
         if constexpr (sizeof(T) == 4) {
-            const int bytes = ok ? 16 : 0;   // 0: the 16 bytes are zero-filled and the cache is not read
+            const int bytes = row >= 0 ? 16 : 0;   // 0: the 16 bytes are zero-filled and the cache is not read
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(at)), "l"(cache + base), "r"(bytes) : "memory");
         } else {
             float f[VE];
 #pragma unroll
             for (int e = 0; e < VE; ++e) f[e] = 0.f;
-            if (ok) Vec<T>::load(cache + base, f);
+            if (row >= 0) Vec<T>::load(cache + base, f);
 #pragma unroll
             for (int e = 0; e < VE; e += 4) *reinterpret_cast<float4*>(at + e) = make_float4(f[e], f[e + 1], f[e + 2], f[e + 3]);
         }
@@ -197,12 +206,14 @@ attn_simt_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restri
     const int k_lo = a.window > 0 ? max(0, pos0 + tok0 - a.window + 1) : 0;            // first key any row sees
     const int k_first = (k_lo / BN) * BN;
 
-    if (k_first < k_end) simt_load<T>(Ks, KS_STRIDE, k_cache, k_first, k_lo, k_end, req, kvh, true, a);
+    int rows = simt_rows(k_first, k_lo, k_end, req, a);
+    simt_load<T>(Ks, KS_STRIDE, k_cache, rows, kvh, a);
     for (int kt = k_first, buf = 0; kt < k_end; kt += BN, buf ^= 1) {
+        const int next = simt_rows(kt + BN, k_lo, k_end, req, a);   // behind the last block: no keys, zeros that nobody reads
         __syncthreads();   // the block before is fully consumed
-        simt_load<T>(Vs, D, v_cache, kt, k_lo, k_end, req, kvh, false, a);
-        // (behind the last block: keys from k_end on, all zeros, never used)
-        simt_load<T>(Ks + (buf ^ 1) * BN * KS_STRIDE, KS_STRIDE, k_cache, kt + BN, k_lo, k_end, req, kvh, true, a);
+        simt_load<T>(Vs, D, v_cache, rows, kvh, a);
+        simt_load<T>(Ks + (buf ^ 1) * BN * KS_STRIDE, KS_STRIDE, k_cache, next, kvh, a);
+        rows = next;
         asm volatile("cp.async.wait_group 2;" ::: "memory");
         __syncthreads();   // this block's keys are there (and, in the first, Q is)
 
