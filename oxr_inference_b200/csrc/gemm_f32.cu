@@ -15,10 +15,10 @@
 // (split on the way from global to shared memory) and the rows of A as the tile's width, any multiple of 16, so that a trace's few hundred rows waste none.
 // Relative error (2-norms) against 64 bits, normal inputs, here and of K fused multiply-adds in the order of k: K = 2,048 1.1e-7 and 8.1e-7, 8,192 1.3e-7 and 1.6e-6,
 // all positive 1.0e-7 and 7.0e-7.
-// What bounds it: a chunk's way through a block, 1.2 us and 0.0067 for each row of the tile: W's trip to the splitters and, beside it, the adders' reads of tensor memory,
-// eight columns at a time for want of registers; its products take 0.4 us. 333 rows, graph of products with other weights each, against 8 x 8 register tiles of fused
-// multiply-adds (42 TFLOP/s at best): 3,072 x 2,048 34 us (124), 2,048 x 2,048 32 (107), 16,384 x 2,048 188 (527), 2,048 x 8,192 104 (431); 40 rows 16,384 x
-// 2,048 61 (117); one row 16,384 x 2,048 53 (330), 3,072 x 2,048 24 (316).
+// What bounds it: a chunk's way through a block, 1.0 us and 0.006 for each row of the tile: the issuing thread's waits, W's trip to the splitters and the adders' reads
+// of tensor memory, eight columns at a time for want of registers; its products take 0.4 us. 333 rows, a graph of products with other weights each, against 8 x 8 register
+// tiles of fused multiply-adds (42 TFLOP/s at best): 3,072 x 2,048 31 us (124), 2,048 x 2,048 29 (107), 16,384 x 2,048 169 (527), 2,048 x 8,192 88 (431); 40 rows 16,384 x
+// 2,048 57 (117); one row 16,384 x 2,048 51 (330), 3,072 x 2,048 24 (316).
 #include "umma.cuh"
 
 namespace {
@@ -27,6 +27,7 @@ constexpr int F32_ADDERS = 8, F32_WORKERS = 16;   // warps 0..7 add the accumula
 constexpr int F32_THREADS = (F32_WORKERS + 2) * 32;
 constexpr int F32_W_PART = 128 * F32_CHUNK * 2, F32_W_STAGE = 3 * F32_W_PART;
 constexpr int F32_AHEAD = 8;           // chunks that one prefetch of a row of W covers (2 KB: 6 to 10 % faster than none, 4 chunks in between)
+constexpr int F32_CHUNKS = 8;          // chunks with barriers of their own
 constexpr int F32_MAX_TILE = 128, F32_MAX_SLOTS = 8, F32_MAX_SEGMENTS = 4, F32_MIN_SEGMENT = 1024;
 
 struct Parts { uint32_t p0, p1, p2; };     // two neighbouring values' parts, packed
@@ -141,16 +142,16 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
     unsigned char* w_stages = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);   // swizzle atoms are 1024 B
     unsigned char* a_slots = w_stages + 2 * F32_W_STAGE;
     const int part_bytes = bn * F32_CHUNK * 2, slot_bytes = 3 * part_bytes;
-    uint64_t* w_full = reinterpret_cast<uint64_t*>(a_slots + (size_t)slots * slot_bytes);   // [2]
-    uint64_t* w_empty = w_full + 2;
-    uint64_t* acc_full = w_empty + 2;     // [2]
-    uint64_t* acc_empty = acc_full + 2;
-    uint64_t* a_full = acc_empty + 2;     // [F32_MAX_SLOTS]
-    uint64_t* a_empty = a_full + F32_MAX_SLOTS;
-    unsigned char* w_more = reinterpret_cast<unsigned char*>(a_empty + F32_MAX_SLOTS);   // [2][4]: a warp's share of the chunk is not all bf16 numbers
+    // Chunk i's two barriers are i % F32_CHUNKS of each: `ready`, when its W is split, its A is here and its accumulators are drained of chunk i - 2; `done`, when its
+    // MMAs are: its stage of W and its slot of A are free and its accumulators full. One wait and one commit a chunk: with a barrier for each of these the issuing thread
+    // spent 2,800 cycles a chunk, half of them in waits for what was there already, and in three commits (16,384 x 2,048 188 us, 2,048 x 8,192 104).
+    uint64_t* ready = reinterpret_cast<uint64_t*>(a_slots + (size_t)slots * slot_bytes);
+    uint64_t* done = ready + F32_CHUNKS;
+    unsigned char* w_more = reinterpret_cast<unsigned char*>(done + F32_CHUNKS);   // [2][4]: a warp's share of the chunk is not all bf16 numbers
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(w_more + 8);
     uint32_t* gave_up = tmem_slot + 1;
-    static_assert((8 + 2 * F32_MAX_SLOTS) * 8 + 8 + 8 <= BARRIER_BYTES, "barriers outgrow their space");
+    static_assert(2 * F32_CHUNKS * 8 + 8 + 8 <= BARRIER_BYTES, "barriers outgrow their space");
+    static_assert(F32_MAX_SLOTS <= F32_CHUNKS, "nobody is a whole round of barriers behind");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n0 = blockIdx.y * 128, m0 = blockIdx.x * bn;
@@ -159,11 +160,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
     const int begin = shared ? (int)blockIdx.z * segment : 0, end = shared ? min(chunks_all, begin + segment) : chunks_all;
 
     if (tid == 0) {
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(w_full + i, (F32_WORKERS - F32_ADDERS) / 2); mbar_init(w_empty + i, 1);
-            mbar_init(acc_full + i, 1); mbar_init(acc_empty + i, F32_ADDERS);
-        }
-        for (int i = 0; i < slots; ++i) { mbar_init(a_full + i, 1); mbar_init(a_empty + i, 1); }
+        for (int i = 0; i < F32_CHUNKS; ++i) { mbar_init(ready + i, (F32_WORKERS - F32_ADDERS) / 2 + 1 + F32_ADDERS); mbar_init(done + i, 1); }
         *gave_up = 0;
         mbar_fence_init();
     }
@@ -175,6 +172,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    auto is_done = [&](int i) { return mbar_wait(done + i % F32_CHUNKS, (i / F32_CHUNKS) & 1); };
     auto expired = [&](int where) { atomicExch(gave_up, 1u); oxr_report(status, OXR_WAIT_EXPIRED, where); };
 
     if (warp == F32_WORKERS + 1) {
@@ -183,10 +181,10 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
             pdl_wait();
             for (int i = 0; i < end - begin; ++i) {
                 const int s = i % slots;
-                if (!mbar_wait(a_empty + s, ((i / slots) & 1) ^ 1)) { expired(60); break; }
-                mbar_expect_tx(a_full + s, (uint32_t)slot_bytes);
+                if (i >= slots && !is_done(i - slots)) { expired(60); break; }
+                mbar_expect_tx(ready + i % F32_CHUNKS, (uint32_t)slot_bytes);
                 for (int p = 0; p < 3; ++p)
-                    tma_load_2d(a_slots + (size_t)s * slot_bytes + (size_t)p * part_bytes, &map_a, (begin + i) * F32_CHUNK, p * M + m0, a_full + s);
+                    tma_load_2d(a_slots + (size_t)s * slot_bytes + (size_t)p * part_bytes, &map_a, (begin + i) * F32_CHUNK, p * M + m0, ready + i % F32_CHUNKS);
             }
         }
         __syncwarp();
@@ -196,8 +194,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
             const uint32_t idesc = umma_idesc(128, bn);
             for (int i = 0; i < end - begin; ++i) {
                 const int s = i & 1, as = i % slots;
-                const uint32_t use = (i >> 1) & 1;
-                if (!mbar_wait(acc_empty + s, use ^ 1) || !mbar_wait(a_full + as, (i / slots) & 1) || !mbar_wait(w_full + s, use)) { expired(61); break; }
+                if (!mbar_wait(ready + i % F32_CHUNKS, (i / F32_CHUNKS) & 1)) { expired(61); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const bool whole = *reinterpret_cast<const volatile uint32_t*>(w_more + 4 * s) != 0;
                 const uint32_t w_addr = smem_addr(w_stages + (size_t)s * F32_W_STAGE), a_addr = smem_addr(a_slots + (size_t)as * slot_bytes);
@@ -212,9 +209,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
                 product(rest, 0, 1, false);
                 if (whole) product(rest, 1, 0, false);
                 product(head, 0, 0, true);
-                umma_commit(w_empty + s);
-                umma_commit(a_empty + as);
-                umma_commit(acc_full + s);
+                umma_commit(done + i % F32_CHUNKS);
             }
         }
         __syncwarp();
@@ -223,6 +218,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
         const int quarter = warp & 3, half = warp >> 2;
         const int col = n0 + quarter * 32 + lane;                    // this lane's row of W: a column of C
         bool ok = true, odd = false;
+        if (lane == 0) { mbar_arrive(ready); mbar_arrive(ready + 1); }      // nothing to drain before the first two chunks
         for (int from = 0; from < end - begin && ok; from += segment) {
             const int to = min(end - begin, from + segment);
             float sum[4][16];
@@ -233,7 +229,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
 #pragma unroll 1
             for (int i = from; i < to; ++i) {
                 const int s = i & 1;
-                if (!mbar_wait(acc_full + s, (i >> 1) & 1)) { expired(62); ok = false; }
+                if (!is_done(i)) { expired(62); ok = false; }
                 ok = __all_sync(0xffffffffu, ok && *reinterpret_cast<volatile uint32_t*>(gave_up) == 0);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -253,7 +249,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(acc_empty + s);
+                if (lane == 0) mbar_arrive(ready + (i + 2) % F32_CHUNKS);
             }
             if (!ok) break;
             if (shared) {   // every MMA of the block is done: the ring holds the segment's sums now, [bn][128]
@@ -307,7 +303,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
         };
         fetch(begin + turn);
         for (int i = turn; begin + i < end; i += 2) {
-            bool ok = mbar_wait(w_empty + turn, ((i >> 1) & 1) ^ 1);
+            bool ok = i < 2 || is_done(i - 2);
             if (!ok) expired(63);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -340,7 +336,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
             if (lane == 0) w_more[4 * turn + (warp & 3)] = more;
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(w_full + turn);
+            if (lane == 0) mbar_arrive(ready + i % F32_CHUNKS);
             fetch(begin + i + 2);   // behind the fence, which would wait for loads on their way
         }
     }

@@ -883,8 +883,8 @@ F32_MAX_TILE = 128
 @functools.lru_cache(maxsize=None)
 def _gemm_f32_plan(m: int, n: int, k: int) -> tuple[int, bool]:
     """(rows of x per block, whether the segments of k go to the blocks of a cluster) of the 32-bit product: the least rounds of blocks times what a block
-    takes, 1.15 + 0.0065 * rows microseconds per 64 k and 4 at its ends. Measured on a B200 with 1 to 1,000 rows and 2,048 to 16,384 columns, the formula is within 15 % of it:
-    333 rows x 16,384 x 2,048 in three tiles of 112 rows 190 us (a fourth of 96: 238), 333 x 2,048 x 8,192 206 us in one block a tile, 100 in clusters of four."""
+    takes, 1 + 0.006 * rows microseconds per 64 k and 4 at its ends. Measured on a B200 with 1 to 1,000 rows and 2,048 to 16,384 columns, the formula is within 15 % of it:
+    333 rows x 16,384 x 2,048 in three tiles of 112 rows 169 us (in four of 96: 209), 333 x 2,048 x 8,192 183 us in one block a tile, 91 in clusters of four."""
     best, best_cost = (16, False), None
     segments = _lib().oxr_gemm_f32_segments(k)
     for tiles in range(-(-m // F32_MAX_TILE), -(-m // 16) + 1):
@@ -892,7 +892,7 @@ def _gemm_f32_plan(m: int, n: int, k: int) -> tuple[int, bool]:
         blocks = -(-m // tile) * -(-n // 128)
         for parts in {1, segments}:
             rounds = -(-blocks // (_few_rows_clusters(parts) if parts > 1 else num_sms()))
-            cost = rounds * (k / 64 / parts * (1.15 + 0.0065 * tile) + 4)
+            cost = rounds * (k / 64 / parts * (1 + 0.006 * tile) + 4)
             if best_cost is None or cost < best_cost - 1e-9:
                 best, best_cost = (tile, parts > 1), cost
     return best
