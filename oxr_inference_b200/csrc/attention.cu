@@ -1359,8 +1359,7 @@ attn_tma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float
             const bool full_block = key0 + 15 <= tile_first_pos && key0 >= k_lo && (a.window <= 0 || key0 > tile_last_pos - a.window);
             warp_block<16, true>(qf, Qs, Kst + warp * 16 * 64, Vst + warp * 16 * 64, key0, row_pos, row_ok, a.window, full_block,
                                  scale_log2, m, l, o);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty + st);   // this warp is done with the stage
+            mbar_release_stage(empty + st, lane);   // this warp is done with the stage
         }
         tl_streamed = OXR_TL_NOW();
 #pragma unroll
@@ -1706,8 +1705,7 @@ attn_tma_decode_walk_kernel(bf16* __restrict__ out, float* __restrict__ part_o, 
                 const bool full_block = key0 + 15 <= tile_first_pos && key0 >= p.k_lo && (a.window <= 0 || key0 > tile_last_pos - a.window);
                 warp_block<16, true>(qf, Qs, Kst + warp * 16 * 64, Vst + warp * 16 * 64, key0, row_pos, row_ok, a.window, full_block,
                                      scale_log2, m, l, o);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(empty + st);
+                mbar_release_stage(empty + st, lane);
             }
 #pragma unroll
             for (int r = 0; r < 2; ++r) {

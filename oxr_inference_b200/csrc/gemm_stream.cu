@@ -57,7 +57,7 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t b
 }
 __device__ __forceinline__ uint4 lds_16(const void* p) {
     uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_addr(p)));
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_addr(p)) : "memory");
     return v;
 }
 __device__ __forceinline__ uint4 ldg_16(const void* p) {   // an ordinary cached load: X stays in what the ring leaves of L1
@@ -249,8 +249,7 @@ gemm_stream_kernel(TO* __restrict__ C, const __nv_bfloat16* __restrict__ X, cons
                     mma_16816(acc[i], fa.z, fb.z, fa.w, fb.w, xr[j][c][i].z, xr[j][c][i].w);
                 }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty + st);
+            mbar_release_stage(empty + st, lane);
             if (q + X_AHEAD < total) load_x((sl + X_AHEAD) % slices, xr[j]);
             if (++sl < slices) continue;
             sl = 0;

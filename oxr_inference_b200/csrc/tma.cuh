@@ -50,8 +50,15 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
         ::"r"(smem_addr(dst)), "l"(map), "r"(smem_addr(bar)), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
-// Orders earlier ordinary shared-memory writes before later writes by TMA to the same addresses.
+// Orders earlier ordinary shared-memory accesses, reads too, before later accesses by TMA or bulk copies to the same addresses.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// A warp has read its part of a stage with ordinary loads, and the stage may be filled again. Without the fence the arrival did not wait for reads still on their
+// way: where a decode step's products started behind an attention kernel, the next slice's copy landed under a warp's last 64 bytes of a weight row.
+__device__ __forceinline__ void mbar_release_stage(uint64_t* bar, int lane) {
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
 
 // ---------------------------------------------------------------------------------------------------- host side
 typedef CUresult (*OxrEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
