@@ -3,8 +3,10 @@
 // This is the matrix product of the 32-bit path of the whole model (the reference multiplies through
 // nn.Linear, oxr_runtime/language.py:223-244; in fp32 only on the CPU in its tests).
 //
-// A 24-bit significand is three of 8 bits: x = x0 + x1 + x2 exactly, each part x less the parts before it, rounded to bf16 (below 2^-108 the last
-// ones run into bf16's smallest numbers). Products of two parts are exact in fp32, so a product of A and W is w0 a0 + (w0 a1 + w1 a0) + (w0 a2 + w1 a1 +
+// A 24-bit significand is three of 8 bits (the split into bf16 parts is that of Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for
+// higher-precision computations", 2019): x = x0 + x1 + x2, each part x less the parts before it, rounded to bf16. Both operands are first multiplied by 2^16 and their
+// sums by 2^-32: bf16's smallest number is then fp32's, 2^-149, and the parts of every fp32 number add up to it exactly, those of the smallest too
+// (unscaled, a third part fell out of bf16's range below 2^-108, and operands of 2^-126 kept 9 bits). Products of two parts are exact in fp32, so a product of A and W is w0 a0 + (w0 a1 + w1 a0) + (w0 a2 + w1 a1 +
 // w2 a0) up to 2^-24 of it (the size of one rounding, of either sign), and a W whose values are bf16 numbers, as a widened checkpoint's are, has
 // w1 = w2 = 0: three products, exact. Sums: over each chunk of 64 k the head products w0 a0 go into one accumulator in tensor memory and the others into a second one;
 // the two are added, and then to a sum in registers, rounded to nearest; each segment of k (1,024 of them or more, by K alone) has a sum of its own, and
@@ -32,11 +34,15 @@ constexpr int F32_MAX_TILE = 128, F32_MAX_SLOTS = 8, F32_MAX_SEGMENTS = 4, F32_M
 
 struct Parts { uint32_t p0, p1, p2; };     // two neighbouring values' parts, packed
 
+constexpr float F32_SCALE = 65536.f, F32_UNSCALE = 0x1p-32f;     // what both operands are multiplied by, and their sums
+
 __device__ __forceinline__ uint32_t bits2(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
 
-// v = hi + mid + lo. An infinite hi (also one that a finite v rounds to) or a NaN stands alone: the epilogue sees to such results.
+// F32_SCALE v = hi + mid + lo. An infinite hi (also one that a finite v makes, from 2^111 on) or a NaN stands alone: the epilogue sees to such results.
 __device__ __forceinline__ Parts split2(float a, float b) {
     Parts r;
+    a *= F32_SCALE;
+    b *= F32_SCALE;
     r.p0 = bits2(__floats2bfloat162_rn(a, b));
     const float a0 = __uint_as_float(r.p0 << 16), b0 = __uint_as_float(r.p0 & 0xffff0000u);
     float a1 = a - a0, b1 = b - b0;
@@ -112,7 +118,7 @@ __device__ __forceinline__ void f32_tmem_ld(uint32_t at, uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Where parts cannot hold a product (infinities, values that round to one) it is made as it is defined: fused multiply-adds in the order of k. A NaN stays one.
+// Where parts cannot hold a product (infinities, operands from 2^111 and sums from 2^95 on, which the scale takes out of range) it is made as it is defined: fused multiply-adds in the order of k. A NaN stays one.
 __device__ __forceinline__ bool f32_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
 __device__ __noinline__ void f32_again(float* c, const float* __restrict__ a, const float* __restrict__ w, int K) {
     if (f32_finite(*c)) return;
@@ -262,6 +268,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
                     }
             } else {        // one block for all segments: each segment's sum is added to what C holds of the ones before it
                 pdl_wait();
+                const float scale = to == end - begin ? F32_UNSCALE : 1.f;
                 int left = col < N ? min(bn, M - m0) - half * 16 : 0;      // rows from this warp's first on
                 float* at = C + (size_t)(m0 + half * 16) * N + col;
                 asm volatile("" : "+l"(at));   // or the compiler keeps all 64 addresses from segment to segment
@@ -270,7 +277,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         if (j < left) {
-                            const float t = from == 0 ? sum[g][j] : *at + sum[g][j];
+                            const float t = (from == 0 ? sum[g][j] : *at + sum[g][j]) * scale;
                             odd = odd || !f32_finite(t);
                             *at = t;
                         }
@@ -325,7 +332,8 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
                     *reinterpret_cast<uint2*>(at + F32_W_PART) = make_uint2(a.p1, b.p1);
                     *reinterpret_cast<uint2*>(at + 2 * F32_W_PART) = make_uint2(a.p2, b.p2);
                 } else {
-                    *reinterpret_cast<uint2*>(at) = make_uint2(__byte_perm(__float_as_uint(v[p].x), __float_as_uint(v[p].y), 0x7632), __byte_perm(__float_as_uint(v[p].z), __float_as_uint(v[p].w), 0x7632));
+                    *reinterpret_cast<uint2*>(at) = make_uint2(__byte_perm(__float_as_uint(F32_SCALE * v[p].x), __float_as_uint(F32_SCALE * v[p].y), 0x7632),
+                                                               __byte_perm(__float_as_uint(F32_SCALE * v[p].z), __float_as_uint(F32_SCALE * v[p].w), 0x7632));
                     if (stale) {
                         *reinterpret_cast<uint2*>(at + F32_W_PART) = make_uint2(0, 0);
                         *reinterpret_cast<uint2*>(at + 2 * F32_W_PART) = make_uint2(0, 0);
@@ -355,6 +363,7 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
                 asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(f32_in_block(mine, (uint32_t)r) + 4u * (uint32_t)e));
                 t = r == 0 ? v : t + v;
             }
+            t *= F32_UNSCALE;
             C[(size_t)m * N + n] = t;
             if (!f32_finite(t)) f32_again(C + (size_t)m * N + n, A + (size_t)m * K, W + (size_t)n * K, K);
         }

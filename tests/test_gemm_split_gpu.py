@@ -52,3 +52,24 @@ def test_infinities_and_what_rounds_to_one(ops):
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
     assert torch.equal(got[got.isinf()], want[want.isinf()])
     assert got[6, 12].isfinite() and abs(got[6, 12] / want[6, 12] - 1) < 1e-6
+
+
+@pytest.mark.parametrize("K", [300, 2050, 4100])
+@pytest.mark.parametrize("power", [-100, -112, -116, -120, -126, -130, -140, -146])
+def test_small_operands_keep_their_bits(ops, K, power):
+    """One, two and four segments; small rows of x and small rows of W, down to where an operand has three bits left; products that are themselves among the smallest numbers."""
+    small = (randn(40, K, seed=21).double() * 2.0 ** power).float()        # rounded to what fp32 has there
+    other = randn(150, K, seed=22)
+    lib, status = ops._lib(), ops.new_status(DEV)
+    for x, w in ((small, other * 2.0 ** 60), (other * 2.0 ** 60, small), (small, other)):
+        want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+        # as for operands of ordinary size; and half of the smallest number where the result is rounded to a multiple of it
+        room = (16 + K / 64) * 2 ** -24 * size + 2.0 ** -150
+        for shared in (0, 1):
+            out = torch.full(want.shape, float("nan"), device=DEV)
+            parts = torch.empty(3, x.shape[0], -(-K // 8) * 8, dtype=torch.bfloat16, device=DEV)
+            assert lib.oxr_gemm_f32_nt(out.data_ptr(), x.data_ptr(), w.data_ptr(), parts.data_ptr(), *want.shape, K, 48, shared, status.data_ptr(), ops._stream()) == 0
+            assert ((out.double() - want).abs() <= room).all()
+            if w.abs().max() > 1e3 or x.abs().max() > 1e3:                 # normal results: the error of ordinary operands
+                assert (out.double() - want).norm() <= 3e-7 * want.norm()
+    ops.check_status(status)
