@@ -442,3 +442,26 @@ OXR_API int oxr_gemm_f32_nt(float* C, const float* A, const float* W, void* part
 }
 
 OXR_API int oxr_gemm_f32_segments(int K) { return f32_segments(K); }
+
+// How many clusters of `segments` blocks of the product the GPU holds at a time (0 if such a cluster cannot be launched).
+OXR_API int oxr_gemm_f32_max_clusters(int segments) {
+    if (segments < 1 || segments > F32_MAX_SEGMENTS) return 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 64, (unsigned)segments);
+    cfg.blockDim = dim3(F32_THREADS);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 1;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = (unsigned)segments;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(gemm_f32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_f32_kernel<true>, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return n;
+}

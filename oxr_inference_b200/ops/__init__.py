@@ -127,6 +127,7 @@ def _lib():
         lib.oxr_qk_norm_rope_store.argtypes = [p, p, p, p, p, p, p, p, p, p, i, i, i, i, f, i, c_longlong, i, i, i, i, p, p]
         lib.oxr_gemm_f32_nt.argtypes = [p, p, p, p, i, i, i, i, i, p, p]
         lib.oxr_gemm_f32_segments.argtypes = [i]
+        lib.oxr_gemm_f32_max_clusters.argtypes = [i]
         lib.oxr_gemm_skinny_bf16.argtypes = [p, p, p, i, i, i, i, p]
         lib.oxr_gemm_skinny_gated_bf16.argtypes = [p, p, p, i, i, i, p]
         lib.oxr_gemm_stream_bf16.argtypes = [p, p, p, i, i, i, i, i, p, p]
@@ -218,7 +219,7 @@ def _lib():
                      "oxr_gated_relu2", "oxr_expert_sort", "oxr_gather_rows", "oxr_combine_rows", "oxr_gemm_tcgen05_grouped_bf16", "oxr_gemm_tcgen05_grouped_gated_bf16"):
             getattr(lib, name).restype = c_int
         for name in ("oxr_embedding", "oxr_add_rms_norm", "oxr_silu_mul", "oxr_cast", "oxr_qk_norm_rope_store",
-                     "oxr_gemm_f32_nt", "oxr_gemm_f32_segments", "oxr_gemm_skinny_bf16", "oxr_gemm_skinny_gated_bf16", "oxr_gemm_stream_bf16", "oxr_gemm_stream_gated_bf16", "oxr_gemm_tcgen05_bf16", "oxr_gemm_tcgen05_pair_bf16", "oxr_gemm_tcgen05_gated_bf16", "oxr_gemm_few_rows_cluster_bf16", "oxr_gemm_few_rows_max_clusters",
+                     "oxr_gemm_f32_nt", "oxr_gemm_f32_segments", "oxr_gemm_f32_max_clusters", "oxr_gemm_skinny_bf16", "oxr_gemm_skinny_gated_bf16", "oxr_gemm_stream_bf16", "oxr_gemm_stream_gated_bf16", "oxr_gemm_tcgen05_bf16", "oxr_gemm_tcgen05_pair_bf16", "oxr_gemm_tcgen05_gated_bf16", "oxr_gemm_few_rows_cluster_bf16", "oxr_gemm_few_rows_max_clusters",
                      "oxr_gemm_tcgen05_pair_gated_bf16", "oxr_sample", "oxr_repetition_penalty", "oxr_mark_seen"):
             getattr(lib, name).restype = c_int
         lib.oxr_set_chain.argtypes = [c_int]
@@ -881,17 +882,26 @@ F32_MAX_TILE = 128
 
 
 @functools.lru_cache(maxsize=None)
+def _f32_clusters(segments: int) -> int:
+    """Clusters of ``segments`` blocks of the 32-bit product that the GPU holds at a time; 0: none can be launched."""
+    return int(_lib().oxr_gemm_f32_max_clusters(segments))
+
+
+@functools.lru_cache(maxsize=None)
 def _gemm_f32_plan(m: int, n: int, k: int) -> tuple[int, bool]:
     """(rows of x per block, whether the segments of k go to the blocks of a cluster) of the 32-bit product: the least rounds of blocks times what a block
     takes, 1 + 0.006 * rows microseconds per 64 k and 4 at its ends. Measured on a B200 with 1 to 1,000 rows and 2,048 to 16,384 columns, the formula is within 15 % of it:
     333 rows x 16,384 x 2,048 in three tiles of 112 rows 169 us (in four of 96: 209), 333 x 2,048 x 8,192 183 us in one block a tile, 91 in clusters of four."""
     best, best_cost = (16, False), None
     segments = _lib().oxr_gemm_f32_segments(k)
-    for tiles in range(-(-m // F32_MAX_TILE), -(-m // 16) + 1):
+    for tiles in range(max(1, -(-m // F32_MAX_TILE)), -(-m // 16) + 1):
         tile = -(-(-(-m // tiles)) // 16) * 16
         blocks = -(-m // tile) * -(-n // 128)
         for parts in {1, segments}:
-            rounds = -(-blocks // (_few_rows_clusters(parts) if parts > 1 else num_sms()))
+            at_once = _f32_clusters(parts) if parts > 1 else num_sms()
+            if at_once == 0:
+                continue
+            rounds = -(-blocks // at_once)
             cost = rounds * (k / 64 / parts * (1 + 0.006 * tile) + 4)
             if best_cost is None or cost < best_cost - 1e-9:
                 best, best_cost = (tile, parts > 1), cost
@@ -1017,6 +1027,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     if weight.dtype == torch.float32:
         x32 = cast(x, torch.float32)
         out = given if given is not None and out_dtype == torch.float32 else torch.empty((m, n), dtype=torch.float32, device=x.device)
+        if m == 0 or n == 0:
+            return cast(out, out_dtype) if given is None else given
         tile, shared = _gemm_f32_plan(m, n, k)
         parts = torch.empty((3, m, -(-k // 8) * 8), dtype=torch.bfloat16, device=x.device)
         _done(lib.oxr_gemm_f32_nt(out.data_ptr(), x32.data_ptr(), weight.data_ptr(), parts.data_ptr(), m, n, k, tile, int(shared),

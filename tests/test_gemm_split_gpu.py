@@ -73,3 +73,12 @@ def test_small_operands_keep_their_bits(ops, K, power):
             if w.abs().max() > 1e3 or x.abs().max() > 1e3:                 # normal results: the error of ordinary operands
                 assert (out.double() - want).norm() <= 3e-7 * want.norm()
     ops.check_status(status)
+
+
+@pytest.mark.parametrize("M,N", [(0, 40), (3, 0), (0, 0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_products_without_rows_or_columns_are_empty(ops, M, N, dtype):
+    got = ops.linear(torch.empty(M, 2048, device=DEV, dtype=dtype), torch.empty(N, 2048, device=DEV))
+    assert got.shape == (M, N) and got.dtype == dtype
+    given = torch.empty(M, N, device=DEV, dtype=dtype)
+    assert ops.linear(torch.empty(M, 2048, device=DEV, dtype=dtype), torch.empty(N, 2048, device=DEV), out=given) is given

@@ -15,3 +15,11 @@ def test_rows_that_fill_tiles_badly_lie_across():
     assert ops._gemm_pair_tiles(1421, 4096, 12288) == (160, 1)
     assert ops._gemm_pair_tiles(1024, 24576, 4096)[1] == 0           # four tiles of 256 rows exactly
     assert ops._gemm_pair_tiles(1000, 8192, 2048)[1] == 0            # so short a k that the epilogue would not be hidden
+
+
+def test_32_bit_plans_without_rows_and_without_clusters(monkeypatch):
+    assert ops._gemm_f32_plan.__wrapped__(0, 2048, 4096) == (16, False)
+    monkeypatch.setattr(ops, "_f32_clusters", lambda segments: 0)           # what the library answers where no cluster can be launched
+    for m, n, k in ((1, 2048, 8192), (333, 16384, 2048), (5000, 300, 64)):
+        tile, shared = ops._gemm_f32_plan.__wrapped__(m, n, k)
+        assert tile % 16 == 0 and 16 <= tile <= ops.F32_MAX_TILE and not shared
