@@ -908,6 +908,15 @@ def _gemm_f32_plan(m: int, n: int, k: int) -> tuple[int, bool]:
     return best
 
 
+F32_PARTS_BYTES = 128 << 20
+
+
+def _gemm_f32_rows(m: int, k: int) -> int:
+    """Rows of x that one 32-bit product takes: its scratch, six bytes for each element of them, stays within ``F32_PARTS_BYTES`` (2,048 rows of 8,192 make 96 MB; 8,192 rows
+    of 12,288 made 576 MB). A row's result does not depend on the rows beside it."""
+    return min(m, max(1, F32_PARTS_BYTES // (6 * (-(-k // 8) * 8) * F32_MAX_TILE)) * F32_MAX_TILE)
+
+
 GEMM_FEW_ROWS = 256          # the widest tile of a tcgen05 product
 GEMM_FEW_ROWS_ANY_SHARES = 192
 
@@ -1004,7 +1013,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     float32 x float32 runs the tensor-core kernel on parts of eight bits, whose error is that of fewer 32-bit roundings than K (no TF32). bfloat16 x bfloat16 runs the skinny kernel up to
     ``SKINNY_MAX_ROWS`` rows and the TMA + tcgen05 kernel beyond (cuBLAS only when a row is not a whole number of
     16-byte words). A weight kept in float32 under bfloat16 activations is multiplied in fp32 and the result
-    rounded once. ``out`` (contiguous ``[rows, out]`` of the output dtype) receives the product instead of a new tensor.
+    rounded once; it takes up to ``F32_PARTS_BYTES`` of scratch for the parts of x. ``out`` (contiguous ``[rows, out]`` of the output dtype) receives the product instead of a new tensor.
     """
     if isinstance(x, NormedLazily):
         out = _scaled_linear(x, weight, gated=False) if out_dtype in (None, torch.bfloat16) else None
@@ -1029,12 +1038,15 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
         out = given if given is not None and out_dtype == torch.float32 else torch.empty((m, n), dtype=torch.float32, device=x.device)
         if m == 0 or n == 0:
             return cast(out, out_dtype) if given is None else given
-        tile, shared = _gemm_f32_plan(m, n, k)
-        parts = torch.empty((3, m, -(-k // 8) * 8), dtype=torch.bfloat16, device=x.device)
-        _done(lib.oxr_gemm_f32_nt(out.data_ptr(), x32.data_ptr(), weight.data_ptr(), parts.data_ptr(), m, n, k, tile, int(shared),
-                                  new_status(x.device).data_ptr(), _stream()), "gemm_f32")
+        rows = _gemm_f32_rows(m, k)
+        parts = torch.empty((3, rows, -(-k // 8) * 8), dtype=torch.bfloat16, device=x.device)
         global launch_count
-        launch_count += 1  # two kernels
+        for at in range(0, m, rows):
+            some = min(rows, m - at)
+            tile, shared = _gemm_f32_plan(some, n, k)
+            _done(lib.oxr_gemm_f32_nt(out[at:].data_ptr(), x32[at:].data_ptr(), weight.data_ptr(), parts.data_ptr(), some, n, k, tile, int(shared),
+                                      new_status(x.device).data_ptr(), _stream()), "gemm_f32")
+            launch_count += 1  # two kernels
         if given is not None and out_dtype != torch.float32:
             given.copy_(out)
             return given

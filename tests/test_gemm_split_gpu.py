@@ -82,3 +82,14 @@ def test_products_without_rows_or_columns_are_empty(ops, M, N, dtype):
     assert got.shape == (M, N) and got.dtype == dtype
     given = torch.empty(M, N, device=DEV, dtype=dtype)
     assert ops.linear(torch.empty(M, 2048, device=DEV, dtype=dtype), torch.empty(N, 2048, device=DEV), out=given) is given
+
+
+def test_products_cut_by_rows_keep_their_bits(ops, monkeypatch):
+    x, w = randn(700, 2052, seed=31), randn(96, 2052, seed=32)
+    whole = ops.linear(x, w)
+    monkeypatch.setattr(ops, "F32_PARTS_BYTES", 1)
+    before = ops.launch_count
+    assert ops._gemm_f32_rows(700, 2052) == 128 and torch.equal(ops.linear(x, w), whole)
+    assert ops.launch_count - before == 12          # six pieces of two kernels
+    given = torch.empty_like(whole)
+    assert ops.linear(x, w, out=given) is given and torch.equal(given, whole)

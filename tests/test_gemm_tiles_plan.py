@@ -23,3 +23,11 @@ def test_32_bit_plans_without_rows_and_without_clusters(monkeypatch):
     for m, n, k in ((1, 2048, 8192), (333, 16384, 2048), (5000, 300, 64)):
         tile, shared = ops._gemm_f32_plan.__wrapped__(m, n, k)
         assert tile % 16 == 0 and 16 <= tile <= ops.F32_MAX_TILE and not shared
+
+
+def test_32_bit_products_bound_their_scratch():
+    for m, k in ((1, 64), (333, 2048), (2048, 8192), (8192, 12288), (100000, 2047), (300, 1 << 20)):
+        rows = ops._gemm_f32_rows(m, k)
+        assert 0 < rows <= m and (rows == m or rows % ops.F32_MAX_TILE == 0)
+        assert rows <= ops.F32_MAX_TILE or 6 * rows * (-(-k // 8) * 8) <= ops.F32_PARTS_BYTES
+    assert ops._gemm_f32_rows(2048, 8192) == 2048
