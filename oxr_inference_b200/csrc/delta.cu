@@ -13,8 +13,8 @@
 // so a token has ONE sum over the key channels to wait for (both dot products of a column together), and o does not wait for the update.
 //
 // Columns of S (one value entry each) are independent: a block takes 32 of them of one head of one request, 4 or 8 per computing warp (two warps of 4 on a scheduler
-// hide some of one another's latencies: 2,048 tokens of 32 heads of 128 x 128 608 us with one warp of 8, 588 with two). J lanes share
-// a group of CPT = J / 8 columns (J / 4 for the shorter keys): lane j holds the key entries 4 (j + J i) .. + 3, i < KW, of each (J = DK / 4 rounded up to a power of two, 4 to
+// hide some of one another's latencies: 2,048 tokens of 32 heads of 128 x 128 608 us with one warp of 8, 588 with two, of 16 heads 609 and 590; with keys of 64 entries the
+// butterfly's extra shuffles cost more than that, 410 and 451). J lanes share a group of CPT = J / 8 columns (J / 4 up to 64 entries): lane j holds the key entries 4 (j + J i) .. + 3, i < KW, of each (J = DK / 4 rounded up to a power of two, 4 to
 // 32; KW = 2 for keys of more than 128 entries), as pairs for the packed fp32 multiply-add; entries from DK on are zero. So every vector read
 // from shared memory is read once per group, and the 2 CPT dot products of a token meet in a butterfly that halves their number with every
 // step until one is left: lane j ends with number j / SPREAD of them, and a column's d1 goes back to the group by one shuffle. In memory the state lies column by
@@ -49,7 +49,7 @@ constexpr int DELTA_TT = 8, DELTA_COLS = 32, DELTA_PREP_WARPS = DELTA_TT, DELTA_
 __device__ __forceinline__ float delta_sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
 
 template <int J, int KW> struct DeltaShape {
-    static constexpr int DKP = 4 * J * KW, CPT = J >= 16 ? J / 8 : J / 4, SPREAD = J / (2 * CPT);     // SPREAD: lanes that end with the same sum
+    static constexpr int DKP = 4 * J * KW, CPT = J >= 32 ? J / 8 : J / 4, SPREAD = J / (2 * CPT);     // SPREAD: lanes that end with the same sum
     static constexpr int WARPS = DELTA_COLS / (32 / J * CPT), THREADS = 32 * (WARPS + DELTA_PREP_WARPS);   // computing warps; all threads
     static constexpr int BLOCKS = J == 32 && KW == 1 ? 2 : 1;                              // that an SM's registers are to hold
     static constexpr int VEC = DELTA_TT * DKP;                                            // one vector of every token of a tile
