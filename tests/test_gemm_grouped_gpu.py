@@ -1,5 +1,7 @@
 """Grouped products: tiles of no group, and the activation behind the product."""
 
+import threading
+
 import pytest
 import torch
 
@@ -54,3 +56,28 @@ def test_grouped_product_with_the_activation_behind_it(ops, ff, kind):
                 want = g * torch.sigmoid(1.7 * g) * (u.clamp(-1.5, 1.5) + 1)
             # one rounding to 16 bits, the fast exponential's and division's few steps of 32 bits, sums in another order
             torch.testing.assert_close(got[rows].float(), want, rtol=2 ** -7, atol=1e-3)
+
+
+@pytest.mark.parametrize("grouped", [False, True])
+def test_another_thread_does_not_change_the_activation(ops, grouped):
+    """A second engine asks for its own form between this thread's two calls."""
+    m, n, k = 256, 64, 72
+    x, w = randn(m, k, seed=13).bfloat16(), (randn(2 * n, k, seed=14) * 0.1).bfloat16()
+    groups, lib, status = torch.tensor([1, 0], dtype=torch.int32, device=DEV), ops._lib(), ops.new_status(DEV)
+
+    def product(other):
+        out = torch.empty(m, n // 2, dtype=torch.bfloat16, device=DEV)
+        lib.oxr_set_gate_form(0, 1.0, 0.0)
+        if other:
+            t = threading.Thread(target=lib.oxr_set_gate_form, args=(1, 1.7, 0.01))
+            t.start()
+            t.join()
+        if grouped:
+            code = lib.oxr_gemm_tcgen05_grouped_gated_bf16(out.data_ptr(), x.data_ptr(), w.data_ptr(), m, n, k, 2, groups.data_ptr(), 64, status.data_ptr(), ops._stream())
+        else:
+            code = lib.oxr_gemm_tcgen05_gated_bf16(out.data_ptr(), x.data_ptr(), w.data_ptr(), m, n, k, 64, status.data_ptr(), ops._stream())
+        assert code == 0
+        ops.check_status(status)
+        return out
+
+    assert torch.equal(product(True), product(False))
