@@ -652,7 +652,12 @@ OXR_API int oxr_head_linear(void* out, int out_head_stride, int out0, const void
         // a block walks over all columns of its head, 64 at a time, or, where tiles of tokens and heads make fewer than two blocks an SM, takes 64 of them: 32 heads of 128 x 192, 300
         // tokens 19.8 -> 14.3 us, 100 tokens 18.4 -> 12.3; 1,421 tokens 24.6 and 28.7.
         dim3 grid((n_tokens + HL_BM - 1) / HL_BM, heads);
-        if (grid.x * grid.y <= 2 * 148) grid.z = (n_out + HL_BN - 1) / HL_BN;
+        static int sms = 0;
+        if (sms == 0) {
+            int dev = 0;
+            if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+        }
+        if (grid.x * grid.y <= 2u * (unsigned)sms) grid.z = (n_out + HL_BN - 1) / HL_BN;
         const int words = x_stride % 8 == 0 && x_head_stride % 8 == 0 && x0 % 8 == 0 && out_head_stride % 2 == 0 && out0 % 2 == 0 && (uintptr_t)x % 16 == 0 &&
                           (uintptr_t)w % 16 == 0 && (uintptr_t)out % 4 == 0;
         oxr_launch(head_linear_mma_kernel, dim3(grid), dim3(128), mma_smem, stream, false, (__nv_bfloat16*)out, out_head_stride, out0, (const __nv_bfloat16*)x, x_stride, x_head_stride, x0,
