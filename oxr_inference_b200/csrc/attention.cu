@@ -572,8 +572,7 @@ __device__ __forceinline__ TileGeometry tile_geometry(const AttnArgs& a, int row
     return g;
 }
 
-// Q rows [row0, row0 + nrows) of the tile -> shared memory (zeros for rows without a token/head).
-// The same for rows of 32 chunks (head size 256), in two steps: warp w copies the rows w, w + 4, ..., and its lane l looks row w + 4 (l % 16) up: one trip to the
+// `load_kv_block` for rows of 32 chunks (head size 256), in two steps: warp w copies the rows w, w + 4, ..., and its lane l looks row w + 4 (l % 16) up: one trip to the
 // block table for all of them, where a lookup behind each row's bounds check made sixteen, one after the other. -1: no key there.
 constexpr bool ROW_PER_WARP = D == 256;
 __device__ __forceinline__ int lookup_kv_row(const int* __restrict__ table_row, const AttnArgs& a, int k0, int k_lo, int k_end, int req) {
@@ -597,6 +596,7 @@ __device__ __forceinline__ void copy_kv_rows(bf16* Ks, bf16* Vs, const bf16* __r
         if (Vs != nullptr) cp_async_16(Vs + at + 4 * i * LDS, v_cache + base, row >= 0);
     }
 }
+// Q rows [row0, row0 + nrows) of the tile -> shared memory (zeros for rows without a token/head).
 __device__ __forceinline__ void load_q_rows(bf16* Qs, const bf16* __restrict__ q, const AttnArgs& a, const TileGeometry& g,
                                             int nrows) {
     constexpr int CPR = D / 8;
@@ -852,10 +852,10 @@ __device__ __forceinline__ void merge_pieces(bf16* __restrict__ out, const float
 //   part_o  [unit, split, 16, D] fp32 (unnormalised, relative to the partial maximum)
 //   part_ml [unit, split, 16, 2] = (maximum in log2 units, sum)
 // and takes a ticket from counters[unit]; the block that draws the last ticket merges all pieces and resets the
-// counter to zero for the next launch. Nobody waits for anybody.
+// counter to zero for the next launch (SHARED: `attn_combine_kernel` merges them). Nobody waits for anybody.
 // SHARED: the keys are the values (a compressed cache). Fetched once, a stage takes half the bytes, and at head size 256 two blocks fit an SM where
 // two copies left room for one (half a round of the pieces that `attention_splits` deals out): a decode step of
-// 13 requests of 225 to 1,800 keys, 32 heads, 48 -> 39 us a layer, and 37 with four items of the merge in flight
+// 13 requests of 225 to 1,800 keys, 32 heads, 48 -> 39 us a layer, with the merge by the last block
 template <bool SHARED>
 __global__ void __launch_bounds__(MMA_THREADS)
 attn_mma_decode_kernel(bf16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
