@@ -431,10 +431,15 @@ int launch_f32(float* C, const float* A, const float* W, __nv_bfloat16* parts, i
 }
 }  // namespace
 
-// parts: 3 * M * (K up to a multiple of 8) bf16 numbers of scratch, 16-byte aligned. tile: rows of A per block, a multiple of 16 from 16 to 128. shared: the
+// gemm_f32_short.cu
+OXR_API int oxr_gemm_f32_is_short(int N, int K);
+int oxr_gemm_f32_short(float* C, const float* A, const float* W, int M, int N, int K, cudaStream_t stream);
+
+// Short products (`oxr_gemm_f32_is_short`) run a kernel of their own, which uses none of the arguments after K. parts: 3 * M * (K up to a multiple of 8) bf16 numbers of scratch, 16-byte aligned. tile: rows of A per block, a multiple of 16 from 16 to 128. shared: the
 // segments of k go to the blocks of a cluster; the results are the same.
 OXR_API int oxr_gemm_f32_nt(float* C, const float* A, const float* W, void* parts, int M, int N, int K, int tile, int shared, int* status, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
+    if (K > 0 && oxr_gemm_f32_is_short(N, K)) return oxr_gemm_f32_short(C, A, W, M, N, K, stream);
     if (K <= 0 || tile < 16 || tile > F32_MAX_TILE || tile % 16 != 0 || (uintptr_t)parts % 16 != 0) return OXR_BAD_ARGUMENT;
     if (3ll * M > 0x7fffffffll) return OXR_BAD_ARGUMENT;
     if (K % 4 == 0 && (uintptr_t)W % 16 == 0) return launch_f32<true>(C, A, W, (__nv_bfloat16*)parts, M, N, K, tile, shared != 0, status, stream);

@@ -127,6 +127,7 @@ def _lib():
         lib.oxr_qk_norm_rope_store.argtypes = [p, p, p, p, p, p, p, p, p, p, i, i, i, i, f, i, c_longlong, i, i, i, i, p, p]
         lib.oxr_gemm_f32_nt.argtypes = [p, p, p, p, i, i, i, i, i, p, p]
         lib.oxr_gemm_f32_segments.argtypes = [i]
+        lib.oxr_gemm_f32_is_short.argtypes = [i, i]
         lib.oxr_gemm_f32_max_clusters.argtypes = [i]
         lib.oxr_gemm_skinny_bf16.argtypes = [p, p, p, i, i, i, i, p]
         lib.oxr_gemm_skinny_gated_bf16.argtypes = [p, p, p, i, i, i, p]
@@ -219,7 +220,7 @@ def _lib():
                      "oxr_gated_relu2", "oxr_expert_sort", "oxr_gather_rows", "oxr_combine_rows", "oxr_gemm_tcgen05_grouped_bf16", "oxr_gemm_tcgen05_grouped_gated_bf16"):
             getattr(lib, name).restype = c_int
         for name in ("oxr_embedding", "oxr_add_rms_norm", "oxr_silu_mul", "oxr_cast", "oxr_qk_norm_rope_store",
-                     "oxr_gemm_f32_nt", "oxr_gemm_f32_segments", "oxr_gemm_f32_max_clusters", "oxr_gemm_skinny_bf16", "oxr_gemm_skinny_gated_bf16", "oxr_gemm_stream_bf16", "oxr_gemm_stream_gated_bf16", "oxr_gemm_tcgen05_bf16", "oxr_gemm_tcgen05_pair_bf16", "oxr_gemm_tcgen05_gated_bf16", "oxr_gemm_few_rows_cluster_bf16", "oxr_gemm_few_rows_max_clusters",
+                     "oxr_gemm_f32_nt", "oxr_gemm_f32_segments", "oxr_gemm_f32_is_short", "oxr_gemm_f32_max_clusters", "oxr_gemm_skinny_bf16", "oxr_gemm_skinny_gated_bf16", "oxr_gemm_stream_bf16", "oxr_gemm_stream_gated_bf16", "oxr_gemm_tcgen05_bf16", "oxr_gemm_tcgen05_pair_bf16", "oxr_gemm_tcgen05_gated_bf16", "oxr_gemm_few_rows_cluster_bf16", "oxr_gemm_few_rows_max_clusters",
                      "oxr_gemm_tcgen05_pair_gated_bf16", "oxr_sample", "oxr_repetition_penalty", "oxr_mark_seen"):
             getattr(lib, name).restype = c_int
         lib.oxr_set_chain.argtypes = [c_int]
@@ -1038,15 +1039,16 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
         out = given if given is not None and out_dtype == torch.float32 else torch.empty((m, n), dtype=torch.float32, device=x.device)
         if m == 0 or n == 0:
             return cast(out, out_dtype) if given is None else given
-        rows = _gemm_f32_rows(m, k)
-        parts = torch.empty((3, rows, -(-k // 8) * 8), dtype=torch.bfloat16, device=x.device)
+        short = bool(lib.oxr_gemm_f32_is_short(n, k))
+        rows = m if short else _gemm_f32_rows(m, k)
+        parts = None if short else torch.empty((3, rows, -(-k // 8) * 8), dtype=torch.bfloat16, device=x.device)
         global launch_count
         for at in range(0, m, rows):
             some = min(rows, m - at)
-            tile, shared = _gemm_f32_plan(some, n, k)
-            _done(lib.oxr_gemm_f32_nt(out[at:].data_ptr(), x32[at:].data_ptr(), weight.data_ptr(), parts.data_ptr(), some, n, k, tile, int(shared),
+            tile, shared = (0, False) if short else _gemm_f32_plan(some, n, k)
+            _done(lib.oxr_gemm_f32_nt(out[at:].data_ptr(), x32[at:].data_ptr(), weight.data_ptr(), _ptr(parts), some, n, k, tile, int(shared),
                                       new_status(x.device).data_ptr(), _stream()), "gemm_f32")
-            launch_count += 1  # two kernels
+            launch_count += 0 if short else 1  # two kernels
         if given is not None and out_dtype != torch.float32:
             given.copy_(out)
             return given
