@@ -24,8 +24,6 @@ namespace {
 constexpr int D = HEAD_DIM;
 constexpr int BM = 16;
 constexpr int BN = 32;
-constexpr int SIMT_WARPS = 8;
-constexpr int ROWS_PER_WARP = BM / SIMT_WARPS;
 constexpr int DCHUNKS = (D + 31) / 32;
 constexpr int KS_STRIDE = D + 4;   // rows of whole 16-byte words, eight neighbouring ones on different banks
 
@@ -128,11 +126,11 @@ __device__ __forceinline__ int simt_rows(int kt, int k_lo, int k_end, int req, c
     return a.page_shift >= 0 ? (page << a.page_shift) + (kp & (a.page_size - 1)) : page * a.page_size + kp % a.page_size;
 }
 // Rows of one K or V block on their way into shared memory: fp32 rows as they are by cp.async, others widened. Zeros where there is no key.
-template <typename T>
+template <typename T, int WARPS>
 __device__ __forceinline__ void simt_load(float* dst, int stride, const T* __restrict__ cache, int rows, int kvh, const AttnArgs& a) {
     constexpr int VE = Vec<T>::N, VPK = D / VE, TOTAL = BN * VPK;                     // vectors per key and in all
 #pragma unroll 4
-    for (int v0 = 0; v0 < TOTAL; v0 += SIMT_WARPS * 32) {
+    for (int v0 = 0; v0 < TOTAL; v0 += WARPS * 32) {
         const int v = v0 + threadIdx.x, j = min(v / VPK, BN - 1), part = v % VPK;
         const int row = __shfl_sync(0xffffffffu, rows, j);
         if (v >= TOTAL) continue;
@@ -155,10 +153,11 @@ __device__ __forceinline__ void simt_load(float* dst, int stride, const T* __res
 
 // What bounds it is the multiply-adds' issue and, in a short prompt, the chain of blocks of the last rows: rows and weights come out of shared memory four
 // entries at a time (a word read per three multiply-adds instead of one each), the next block's keys and this block's values arrive meanwhile.
-template <typename T>
-__global__ void __launch_bounds__(SIMT_WARPS * 32)
+template <typename T, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 attn_simt_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restrict__ k_cache,
                  const T* __restrict__ v_cache, const AttnArgs a) {
+    constexpr int ROWS_PER_WARP = BM / WARPS;
     extern __shared__ __align__(16) float smem[];
     float* Qs = smem;                       // [BM][D]
     float* Ks = Qs + BM * D;                // [2][BN][D + 4]
@@ -178,7 +177,7 @@ attn_simt_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restri
     const int rows_used = a.tokens_per_tile * a.heads_per_tile;
 
     // ---- Q tile -> shared (fp32); rows without a (token, head) are zero
-    for (int i = tid; i < BM * D; i += SIMT_WARPS * 32) {
+    for (int i = tid; i < BM * D; i += WARPS * 32) {
         const int r = i / D, d = i % D;
         const int tok = tok0 + r / a.heads_per_tile, gh = hg * a.heads_per_tile + r % a.heads_per_tile;
         float v = 0.f;
@@ -207,12 +206,12 @@ attn_simt_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restri
     const int k_first = (k_lo / BN) * BN;
 
     int rows = simt_rows(k_first, k_lo, k_end, req, a);
-    simt_load<T>(Ks, KS_STRIDE, k_cache, rows, kvh, a);
+    simt_load<T, WARPS>(Ks, KS_STRIDE, k_cache, rows, kvh, a);
     for (int kt = k_first, buf = 0; kt < k_end; kt += BN, buf ^= 1) {
         const int next = simt_rows(kt + BN, k_lo, k_end, req, a);   // behind the last block: no keys, zeros that nobody reads
         __syncthreads();   // the block before is fully consumed
-        simt_load<T>(Vs, D, v_cache, rows, kvh, a);
-        simt_load<T>(Ks + (buf ^ 1) * BN * KS_STRIDE, KS_STRIDE, k_cache, next, kvh, a);
+        simt_load<T, WARPS>(Vs, D, v_cache, rows, kvh, a);
+        simt_load<T, WARPS>(Ks + (buf ^ 1) * BN * KS_STRIDE, KS_STRIDE, k_cache, next, kvh, a);
         rows = next;
         asm volatile("cp.async.wait_group 2;" ::: "memory");
         __syncthreads();   // this block's keys are there (and, in the first, Q is)
@@ -301,18 +300,33 @@ attn_simt_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restri
 
 constexpr size_t SIMT_SMEM = (size_t)(BM * D + 2 * BN * KS_STRIDE + BN * D + BM * BN) * sizeof(float);
 
-template <typename T>
-int launch_simt(void* out, const void* q, const void* k_cache, const void* v_cache, const AttnArgs& a, int num_tiles,
-                cudaStream_t stream) {
-    static bool configured = false;   // one attribute call per process and dtype
+template <typename T, int WARPS>
+int launch_simt_warps(void* out, const void* q, const void* k_cache, const void* v_cache, const AttnArgs& a, dim3 grid, cudaStream_t stream) {
+    static bool configured = false;   // one attribute call per process, dtype and number of warps
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_simt_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SIMT_SMEM);
+        cudaError_t e = cudaFuncSetAttribute(attn_simt_kernel<T, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SIMT_SMEM);
         if (e != cudaSuccess) return 1000 + (int)e;
         configured = true;
     }
-    dim3 grid(num_tiles, a.KV * a.head_groups);
-    attn_simt_kernel<T><<<grid, SIMT_WARPS * 32, SIMT_SMEM, stream>>>((T*)out, (const T*)q, (const T*)k_cache, (const T*)v_cache, a);
+    attn_simt_kernel<T, WARPS><<<grid, WARPS * 32, SIMT_SMEM, stream>>>((T*)out, (const T*)q, (const T*)k_cache, (const T*)v_cache, a);
     return oxr_launch_status();
+}
+// Eight warps of two rows each make a block's chain shorter, four of four read shared memory less often: with three blocks an SM or more the second counts, up to head size
+// 80 (16 heads on 4, us, eight and four: 1,500 tokens at 64 427 and 308, at 80 483 and 431, at 128 634 and 627; 333 tokens at 64 38 and 40, 8 x 2,048 keys 134 and 164). A row's
+// arithmetic is the same.
+template <typename T>
+int launch_simt(void* out, const void* q, const void* k_cache, const void* v_cache, const AttnArgs& a, int num_tiles,
+                cudaStream_t stream) {
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    }
+    const dim3 grid(num_tiles, a.KV * a.head_groups);
+    if constexpr (D <= 80) {
+        if ((long long)grid.x * grid.y >= 3 * sms) return launch_simt_warps<T, 4>(out, q, k_cache, v_cache, a, grid, stream);
+    }
+    return launch_simt_warps<T, 8>(out, q, k_cache, v_cache, a, grid, stream);
 }
 }  // namespace
 
