@@ -415,7 +415,7 @@ def gated_linear(x: torch.Tensor, weight: torch.Tensor, interleave: int = 0, *, 
         elif m <= SKINNY_MAX_ROWS:
             _done(lib.oxr_gemm_skinny_gated_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, _stream()), "gemm_skinny_gated")
         elif _gemm_pair_plan(m, n, k):
-            _done(lib.oxr_gemm_tcgen05_pair_gated_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, *_gemm_pair_tiles(m, n, k),
+            _done(lib.oxr_gemm_tcgen05_pair_gated_bf16(out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, *_gemm_pair_tiles(m, n, k, True),
                                                        new_status(x.device).data_ptr(), _stream()), "gemm_tcgen05_pair_gated")
         else:
             tile_n, _ = _gemm_plan(m, n, k, False)   # the gated epilogue has no shares of k
@@ -976,16 +976,17 @@ def _gemm_pair_plan(m: int, n: int, k: int) -> int:
 
 
 @functools.lru_cache(maxsize=None)
-def _gemm_pair_tiles(m: int, n: int, k: int) -> tuple[int, int]:
+def _gemm_pair_tiles(m: int, n: int, k: int, gated: bool = False) -> tuple[int, int]:
     """(tile, across) of a product that the two-SM kernel takes: tiles of 256 rows of x by the ``tile`` columns of ``_gemm_pair_plan``, or ``across``: 256 columns by ``tile``
-    rows of x, where that promises 4 %. Rounds of pairs times what a tile takes, fitted to 504 timings of products in turn on a B200 (520 to 2,048 rows, 2,048 to 24,576
+    rows of x, where that promises 5 %, or 8 for a gated product, whose turned epilogue costs more than the formula says (60 drawn sizes, both forms in turn: promises below
+    that came out at 0.94 to 1.09 times the speed, the others at 1.01 to 1.22). Rounds of pairs times what a tile takes, fitted to 504 timings of products in turn on a B200 (520 to 2,048 rows, 2,048 to 24,576
     columns, k 2,048 to 12,288, 96 to 256 wide): a 64-wide k step takes 0.00163 us a column and no less than 0.235, a product 0.0143 us a column of its tile beside; across
     0.00169 and 0.23, 4.9 us a product, and a tile no less than the 0.085 us a row of its epilogue. 1,562 rows x 24,576 x 4,096 262 -> 226 us, 1,421 x 4,096 x 12,288
     135 -> 112, 2,011 x 4,096 x 12,288 175 -> 164."""
     pairs, steps = num_sms() // 2, -(-k // 64)
     tile = _gemm_pair_plan(m, n, k)
     best = (tile, 0)
-    best_cost = 0.96 * (-(-(-(-m // 256) * -(-n // tile)) // pairs) * steps * max(0.235, 0.00163 * tile) + 0.0143 * tile)
+    best_cost = (0.92 if gated else 0.95) * (-(-(-(-m // 256) * -(-n // tile)) // pairs) * steps * max(0.235, 0.00163 * tile) + 0.0143 * tile)
     for tile in (256, 224, 192, 160, 128, 96):
         cost = -(-(-(-m // tile) * -(-n // 256)) // pairs) * max(steps * max(0.23, 0.00169 * tile), 0.085 * tile) + 4.9
         if cost < best_cost - 1e-9:

@@ -6,8 +6,9 @@ from oxr_inference_b200 import ops
 def test_every_plan_is_a_valid_launch():
     for m in (512, 513, 700, 1000, 1421, 1562, 2011, 2048, 5000):
         for n, k in ((576, 4096), (4096, 4096), (6144, 4096), (24576, 4096), (4096, 12288), (32768, 2048), (8192, 64)):
-            tile, across = ops._gemm_pair_tiles(m, n, k)
-            assert tile % 32 == 0 and 64 <= tile <= 256 and across in (0, 1)
+            for gated in (False, True):
+                tile, across = ops._gemm_pair_tiles(m, n, k, gated)
+                assert tile % 32 == 0 and 64 <= tile <= 256 and across in (0, 1)
 
 
 def test_rows_that_fill_tiles_badly_lie_across():
@@ -15,6 +16,10 @@ def test_rows_that_fill_tiles_badly_lie_across():
     assert ops._gemm_pair_tiles(1421, 4096, 12288) == (160, 1)
     assert ops._gemm_pair_tiles(1024, 24576, 4096)[1] == 0           # four tiles of 256 rows exactly
     assert ops._gemm_pair_tiles(1000, 8192, 2048)[1] == 0            # so short a k that the epilogue would not be hidden
+    # promises that measured slower: a few per cent, and gated products whose epilogue is the dearer one
+    assert ops._gemm_pair_tiles(1912, 2048, 4096)[1] == 0
+    assert ops._gemm_pair_tiles(1340, 12352, 4096, True)[1] == ops._gemm_pair_tiles(1430, 4096, 4096, True)[1] == 0
+    assert ops._gemm_pair_tiles(1599, 24576, 8192, True)[1] == 1
 
 
 def test_32_bit_plans_without_rows_and_without_clusters(monkeypatch):
