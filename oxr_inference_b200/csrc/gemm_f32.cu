@@ -1,4 +1,4 @@
-// True fp32 GEMM: C[M,N] = A[M,K] * W[N,K]^T with no less than fp32's precision, on the bf16 tensor cores (no TF32).
+// 32-bit GEMM: C[M,N] = A[M,K] * W[N,K]^T on the bf16 tensor cores, in parts of eight bits (no TF32). Short rows: gemm_f32_short.cu.
 //
 // This is the matrix product of the 32-bit path of the whole model (the reference multiplies through
 // nn.Linear, oxr_runtime/language.py:223-244; in fp32 only on the CPU in its tests).
@@ -6,21 +6,23 @@
 // A 24-bit significand is three of 8 bits (the split into bf16 parts is that of Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for
 // higher-precision computations", 2019): x = x0 + x1 + x2, each part x less the parts before it, rounded to bf16. Both operands are first multiplied by 2^16 and their
 // sums by 2^-32: bf16's smallest number is then fp32's, 2^-149, and the parts of every fp32 number add up to it exactly, those of the smallest too
-// (unscaled, a third part fell out of bf16's range below 2^-108, and operands of 2^-126 kept 9 bits). Products of two parts are exact in fp32, so a product of A and W is w0 a0 + (w0 a1 + w1 a0) + (w0 a2 + w1 a1 +
-// w2 a0) up to 2^-24 of it (the size of one rounding, of either sign), and a W whose values are bf16 numbers, as a widened checkpoint's are, has
+// (unscaled, a third part fell out of bf16's range below 2^-108, and operands of 2^-126 kept 9 bits). Products of two parts are exact in fp32, so a product of A and W is
+// w0 a0 + (w0 a1 + w1 a0) + (w0 a2 + w1 a1 + w2 a0) up to 2^-24 of it (w1 a2, w2 a1 and w2 a2 are left out), and a W whose values are bf16 numbers, as a widened checkpoint's are, has
 // w1 = w2 = 0: three products, exact. Sums: over each chunk of 64 k the head products w0 a0 go into one accumulator in tensor memory and the others into a second one;
-// the two are added, and then to a sum in registers, rounded to nearest; each segment of k (1,024 of them or more, by K alone) has a sum of its own, and
-// the segments' sums are added in order. So an element's result depends on its row and column alone, not on M, the tile, or how the work is dealt out,
-// and fewer roundings stand behind it than behind K fused multiply-adds one after the other.
+// the two are added, and then to a sum in registers, rounded to nearest; K / 1,024 segments of k, one at least and four at most, of whole chunks (the last is shorter), have
+// a sum each, and these are added in order. So an element's result depends on its row and column alone, not on M, the tile, or how the work is dealt out.
+// Error of an element: 16 + K / 64 times 2^-24 of the magnitudes' sum at most (a chunk's sixteen-term sums inside the tensor core lose up to 2^-23 of what is there, K / 64 + 4
+// roundings follow), where K fused multiply-adds one after the other allow K times 2^-24.
 //
 // Two kernels. `split_rows_kernel` writes A's parts, [3][M][K] in bf16. `gemm_f32_kernel` has W on the 128-row side of the tcgen05 tile
 // (split on the way from global to shared memory) and the rows of A as the tile's width, any multiple of 16, so that a trace's few hundred rows waste none.
-// Relative error (2-norms) against 64 bits, normal inputs, here and of K fused multiply-adds in the order of k: K = 2,048 1.1e-7 and 8.1e-7, 8,192 1.3e-7 and 1.6e-6,
-// all positive 1.0e-7 and 7.0e-7.
+// Measured (2-norms against 64 bits, normal inputs, and of K fused multiply-adds in the order of k): K = 128 7.5e-8 and 2.0e-7, 1,024 1.0e-7 and 5.7e-7, 2,048 1.1e-7 and 8.1e-7,
+// 8,192 1.3e-7 and 1.6e-6; all positive 128 9.0e-8 and 1.8e-7, 2,048 9.6e-8 and 7.0e-7.
 // What bounds it: a chunk's way through a block, 1.0 us and 0.006 for each row of the tile: the issuing thread's waits, W's trip to the splitters and the adders' reads
 // of tensor memory, eight columns at a time for want of registers; its products take 0.4 us. 333 rows, a graph of products with other weights each, against 8 x 8 register
 // tiles of fused multiply-adds (42 TFLOP/s at best): 3,072 x 2,048 31 us (124), 2,048 x 2,048 29 (107), 16,384 x 2,048 169 (527), 2,048 x 8,192 88 (431); 40 rows 16,384 x
-// 2,048 57 (117); one row 16,384 x 2,048 51 (330), 3,072 x 2,048 24 (316).
+// 2,048 57 (117); one row 16,384 x 2,048 51 (330), 3,072 x 2,048 24 (316); 2,048 rows 16,384 x 2,048 776 (2,609), 2,048 x 8,192 413 (1,532). A W of 24-bit numbers takes six
+// products and a full split: 333 rows 41, 39, 223 and 125 us in the order above, one row 63 and 31, 2,048 rows 1,044 and 556.
 #include "umma.cuh"
 
 namespace {

@@ -891,7 +891,8 @@ def _f32_clusters(segments: int) -> int:
 @functools.lru_cache(maxsize=None)
 def _gemm_f32_plan(m: int, n: int, k: int) -> tuple[int, bool]:
     """(rows of x per block, whether the segments of k go to the blocks of a cluster) of the 32-bit product: the least rounds of blocks times what a block
-    takes, 1 + 0.006 * rows microseconds per 64 k and 4 at its ends. Measured on a B200 with 1 to 1,000 rows and 2,048 to 16,384 columns, the formula is within 15 % of it:
+    takes, 1 + 0.006 * rows microseconds per 64 k and 4 at its ends. Measured on a B200 with 1 to 1,000 rows and 2,048 to 16,384 columns, and a W widened from bf16, the formula is within 15 % of it (a W of 24-bit numbers
+    takes 1.2 to 1.4 times as long in the same tiles):
     333 rows x 16,384 x 2,048 in three tiles of 112 rows 169 us (in four of 96: 209), 333 x 2,048 x 8,192 183 us in one block a tile, 91 in clusters of four."""
     best, best_cost = (16, False), None
     segments = _lib().oxr_gemm_f32_segments(k)
@@ -1012,7 +1013,8 @@ def _gemm_split_buffers(device: torch.device) -> tuple[torch.Tensor, torch.Tenso
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """``x @ weight.T`` for ``weight [out, in]``, no bias (oxr_runtime/language.py:223-231), fp32 accumulation.
 
-    float32 x float32 runs the tensor-core kernel on parts of eight bits, whose error is that of fewer 32-bit roundings than K (no TF32). bfloat16 x bfloat16 runs the skinny kernel up to
+    float32 x float32 runs the tensor-core kernel on parts of eight bits (no TF32): an element is off by (16 + k / 64) 2^-24 of its magnitudes' sum at most; products of short
+    rows (``oxr_gemm_f32_is_short``) are summed in 64 bits and rounded once. bfloat16 x bfloat16 runs the skinny kernel up to
     ``SKINNY_MAX_ROWS`` rows and the TMA + tcgen05 kernel beyond (cuBLAS only when a row is not a whole number of
     16-byte words). A weight kept in float32 under bfloat16 activations is multiplied in fp32 and the result
     rounded once; it takes up to ``F32_PARTS_BYTES`` of scratch for the parts of x. ``out`` (contiguous ``[rows, out]`` of the output dtype) receives the product instead of a new tensor.
