@@ -81,3 +81,25 @@ def test_another_thread_does_not_change_the_activation(ops, grouped):
         return out
 
     assert torch.equal(product(True), product(False))
+
+
+@pytest.mark.parametrize("spread", [True, False], ids=["evenly", "all the same"])
+def test_a_layer_of_experts_at_its_real_size(ops, spread):
+    """1,421 tokens of ordinary size, 4 of 16 experts: some 355 rows each, or all tokens on the same four. Forty tokens against 64 bits."""
+    tokens, hidden, ff, experts, top = 1421, 4096, 1536, 16, 4
+    h = randn(tokens, hidden, seed=21).bfloat16()
+    up, down = (randn(experts * 2 * ff, hidden, seed=22) * 0.02).bfloat16(), (randn(experts * hidden, ff, seed=23) * 0.02).bfloat16()
+    ids = randn(tokens, experts, seed=24).topk(top).indices.int() if spread else torch.tensor([[3, 7, 8, 15]], dtype=torch.int32, device=DEV).repeat(tokens, 1)
+    weights = torch.softmax(randn(tokens, top, seed=25), -1)
+    status = ops.new_status(DEV)
+    _, order, place, tile_group = ops.expert_sort(ids, experts, pad=ops.GROUP_TILE_ROWS)
+    a = ops.grouped_gated_linear(ops.gather_rows(h, order, top), up, tile_group, 2 * ff)
+    got = ops.combine_rows(ops.grouped_linear(a, down, tile_group, hidden), place, weights)
+    ops.check_status(status)
+    for t in range(0, tokens, 36):
+        want = torch.zeros(hidden, dtype=torch.float64, device=DEV)
+        for e, share in zip(ids[t].tolist(), weights[t].double()):
+            g, u = (up[e * 2 * ff:(e + 1) * 2 * ff].double() @ h[t].double()).split(ff)
+            want += share * (down[e * hidden:(e + 1) * hidden].double() @ (torch.nn.functional.silu(g) * u))
+        # three roundings to 16 bits (activation, each expert's row, their sum), 2^-9 of a value each and of either sign
+        assert (got[t].double() - want).norm() <= 3 * 2 ** -9 * want.norm()
