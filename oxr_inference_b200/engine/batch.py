@@ -11,6 +11,7 @@ beyond the real requests are padding that writes and reads the scratch page (oxr
 
 from __future__ import annotations
 
+import weakref
 from dataclasses import dataclass
 
 import numpy as np
@@ -81,6 +82,18 @@ class BatchBuilder:
         self._same_requests: dict[int, tuple] = {}
         """Per fixed device block: the serials of the requests its rows were last filled for. While the same requests
         decode on, only what moves with a token is written again."""
+        self._fixed_blocks: dict[int, weakref.ref] = {}
+        """The fixed device blocks that the entries above are of, by their ``id()``."""
+
+    def _recognise(self, block: torch.Tensor) -> None:
+        """What is kept for a fixed block that is gone does not belong to another that has its ``id()`` now: the graphs of a dropped
+        ``DecodeGraphs`` leave such blocks behind."""
+        key = id(block)
+        held = self._fixed_blocks.get(key)
+        if held is None or held() is not block:
+            for kept in (self._fixed_pinned, self._fixed_views, self._rows, self._same_requests):
+                kept.pop(key, None)
+            self._fixed_blocks[key] = weakref.ref(block)
 
     # ---- host memory
     def _staging(self, words: int, fixed_block: torch.Tensor | None) -> torch.Tensor:
@@ -128,6 +141,8 @@ class BatchBuilder:
         if not fixed:
             layout = self.eager_layout(entries)
         n_real = len(entries)
+        if fixed:
+            self._recognise(device_block)
         if fixed and (n_real > layout.requests or any(len(e.tokens) != 1 or e.want != [0] for e in entries)):
             raise ValueError("a fixed layout takes single-token entries that want their logits, up to its size")
         pinned = self._staging(layout.total, device_block if fixed else None)
