@@ -910,6 +910,7 @@ def _gemm_f32_plan(m: int, n: int, k: int) -> tuple[int, bool]:
     return best
 
 
+F32_MAX_COLUMNS = 65535 * 128      # a grid has as many rows; with the tiles of rows and columns along its first axis the kernel took 4 % longer
 F32_PARTS_BYTES = 128 << 20
 
 
@@ -1010,6 +1011,13 @@ def _gemm_split_buffers(device: torch.device) -> tuple[torch.Tensor, torch.Tenso
     return got
 
 
+def _given_or_cast(out: torch.Tensor, given: torch.Tensor | None, dtype: torch.dtype) -> torch.Tensor:
+    if given is not None and dtype != torch.float32:
+        given.copy_(out)
+        return given
+    return cast(out, dtype)
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """``x @ weight.T`` for ``weight [out, in]``, no bias (oxr_runtime/language.py:223-231), fp32 accumulation.
 
@@ -1042,6 +1050,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
         out = given if given is not None and out_dtype == torch.float32 else torch.empty((m, n), dtype=torch.float32, device=x.device)
         if m == 0 or n == 0:
             return cast(out, out_dtype) if given is None else given
+        if n > F32_MAX_COLUMNS:
+            for at in range(0, n, F32_MAX_COLUMNS):
+                out[:, at:at + F32_MAX_COLUMNS].copy_(linear(x32, weight[at:at + F32_MAX_COLUMNS]))
+            return _given_or_cast(out, given, out_dtype)
         short = bool(lib.oxr_gemm_f32_is_short(n, k))
         rows = m if short else _gemm_f32_rows(m, k)
         parts = None if short else torch.empty((3, rows, -(-k // 8) * 8), dtype=torch.bfloat16, device=x.device)
@@ -1052,10 +1064,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
             _done(lib.oxr_gemm_f32_nt(out[at:].data_ptr(), x32[at:].data_ptr(), weight.data_ptr(), _ptr(parts), some, n, k, tile, int(shared),
                                       new_status(x.device).data_ptr(), _stream()), "gemm_f32")
             launch_count += 0 if short else 1  # two kernels
-        if given is not None and out_dtype != torch.float32:
-            given.copy_(out)
-            return given
-        return cast(out, out_dtype)
+        return _given_or_cast(out, given, out_dtype)
     if x.dtype != torch.bfloat16:
         raise KernelError(f"linear: activations {x.dtype} with weight {weight.dtype} is not a supported pair")
     if STREAM_GEMM and m <= STREAM_MAX_ROWS and k % 8 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0:

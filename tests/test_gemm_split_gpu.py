@@ -144,3 +144,13 @@ def test_what_is_not_finite_in_any_segment(ops, K, shared):
     there = want.isfinite()
     # K multiply-adds one after the other where the scale does not reach, each rounding at most 2^-24 of the magnitudes' sum
     assert ((out.double() - exact).abs()[there] <= (K + 16) * 2 ** -24 * size[there]).all()
+
+
+def test_more_columns_than_a_grid_has_rows(ops):
+    """8.4 million columns in tiles of 128: cut by columns."""
+    N, K = 65536 * 128 + 40, 24
+    x, w = randn(3, K, seed=51), randn(N, K, seed=52)
+    got = ops.linear(x, w)
+    some = torch.tensor([0, 127, 128, 65535 * 128 - 1, 65535 * 128, N - 41, N - 1], device=DEV)
+    want, size = x.double() @ w[some].double().T, x.double().abs() @ w[some].double().abs().T
+    assert ((got[:, some].double() - want).abs() <= (16 + K / 64) * 2 ** -24 * size).all()
